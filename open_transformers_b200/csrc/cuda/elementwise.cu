@@ -23,10 +23,59 @@ namespace {
 
 
 // ------------------------------------------------------------------ RMSNorm
-// one warp per row; lane_tree with VW = 8
+// One warp per row; lane_tree with VW = 8. The row stays in registers (as loaded) between the sum of squares and the
+// scaling, so all of its loads are in flight at once and x is read once. MAXC = max number of 8-wide column chunks per
+// lane (D <= 256 * MAXC); wider rows take the kernel below, which reads x twice.
+template <typename T, int MAXC>
+__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
+                                                         float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
+  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const T* xr = x + row * D;
+  Raw8<T> raw[MAXC];
+#pragma unroll
+  for (int j = 0; j < MAXC; ++j) {
+    const int c = lane * 8 + j * 256;
+    if (c < D) raw[j].load(xr + c);
+  }
+  float acc = 0.0f;
+#pragma unroll
+  for (int j = 0; j < MAXC; ++j) {
+    if (lane * 8 + j * 256 < D) {
+      float f[8];
+      raw[j].unpack(f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc = __fmaf_rn(f[e], f[e], acc);
+    }
+  }
+  const float ss = warp_butterfly(acc);
+  const float rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
+  if (lane == 0) rstd_out[row] = rstd;
+  T* yr = y + row * D;
+#pragma unroll
+  for (int j = 0; j < MAXC; ++j) {
+    const int c = lane * 8 + j * 256;
+    if (c < D) {
+      float f[8], o[8];
+      raw[j].unpack(f);
+      if (w) {
+        float g[8];
+        Vec8<T>::load(w + c, g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(__fmul_rn(f[e], rstd), g[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(f[e], rstd);
+      }
+      Vec8<T>::store(yr + c, o);
+    }
+  }
+}
+// The same row of any width.
 template <typename T>
-__global__ void rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
-                                   float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
+__global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
+                                        float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -179,143 +228,254 @@ inline void pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
 }
 
 // --------------------------------------------------- gain-free QK-norm + RoPE
-// One warp per (token, head) over the first `heads` heads of a [rows, ld_in] buffer with head
-// width D (<= 128, multiple of 4): lane l holds elements 4l..4l+3 (two rotation pairs).
-// out[row, head*D + i]; rstd[row*heads + head]. lane_tree with VW = 4.
-template <typename T>
-__global__ void qknorm_rope_fwd_kernel(const T* __restrict__ in, long ld_in, T* __restrict__ out, long ld_out,
+// Over the first `heads` heads of a [rows, ld_in] buffer with head width D (<= 128, multiple of 4): lane l of a warp holds
+// elements 4l..4l+3 of a head (two rotation pairs). out[row, head*D + i]; rstd[row*heads + head]. lane_tree with VW = 4.
+// A warp takes ROPE_HEADS heads of one token: the token's cos / sin are read once for all of them and their loads (8 bytes
+// per lane in bf16) are in flight together; one head per warp with 2-byte loads and two 64-bit divisions per warp was bound
+// by its instructions. VEC: bases and pitches allow the four-element accesses.
+constexpr int ROPE_HEADS = 4;
+template <typename T, bool VEC> struct Vec4;
+template <> struct Vec4<__nv_bfloat16, true> {
+  uint2 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void unpack(float (&f)[4]) const {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xFFFF0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xFFFF0000u);
+  }
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&f)[4]) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+  }
+};
+template <> struct Vec4<float, true> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void unpack(float (&f)[4]) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+  static __device__ __forceinline__ void store(float* p, const float (&f)[4]) { *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]); }
+};
+template <typename T> struct Vec4<T, false> {
+  T v[4];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = p[e];
+  }
+  __device__ __forceinline__ void unpack(float (&f)[4]) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = to_f<T>(v[e]);
+  }
+  static __device__ __forceinline__ void store(T* p, const float (&f)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[e] = from_f<T>(f[e]);
+  }
+};
+// warp -> (token, first head); false past the end
+__device__ __forceinline__ bool rope_place(long rows, int heads, long& row, int& head0) {
+  const int groups = (heads + ROPE_HEADS - 1) / ROPE_HEADS;
+  const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (wid >= rows * groups) return false;
+  row = (rows * groups) >> 31 ? wid / groups : (long)((unsigned)wid / (unsigned)groups);
+  head0 = (int)(wid - row * groups) * ROPE_HEADS;
+  return true;
+}
+__device__ __forceinline__ int rope_pos(long row, int seq_len) { return row >> 31 ? (int)(row % seq_len) : (int)((unsigned)row % (unsigned)seq_len); }
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restrict__ in, long ld_in, T* __restrict__ out, long ld_out,
                                        float* __restrict__ rstd_out, const float* __restrict__ cosb,
                                        const float* __restrict__ sinb, long rows, int heads, int D, int seq_len,
                                        int do_norm, float inv_d, float eps) {
-  const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long row;
+  int head0;
+  if (!rope_place(rows, heads, row, head0)) return;
   const int lane = threadIdx.x & 31;
-  if (wid >= rows * heads) return;
-  const long row = wid / heads;
-  const int head = (int)(wid - row * heads);
-  const int pos = (int)(row % seq_len);
   const bool active = lane * 4 < D;
-  float f[4] = {0.f, 0.f, 0.f, 0.f};
+  const int n = min(ROPE_HEADS, heads - head0);
+  Vec4<T, VEC> raw[ROPE_HEADS];
+  const T* p = in + row * ld_in + (long)head0 * D + lane * 4;
+#pragma unroll
+  for (int i = 0; i < ROPE_HEADS; ++i)
+    if (active && i < n) raw[i].load(p + i * D);
+  float c[2] = {0.f, 0.f}, s[2] = {0.f, 0.f};
   if (active) {
-    const T* p = in + row * ld_in + (long)head * D + lane * 4;
+    const long at = (long)rope_pos(row, seq_len) * (D >> 1) + lane * 2;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = to_f<T>(p[e]);
+    for (int pr = 0; pr < 2; ++pr) { c[pr] = cosb[at + pr]; s[pr] = sinb[at + pr]; }
   }
-  float rstd = 1.0f;
-  if (do_norm) {
-    float acc = 0.0f;
+  T* o = out + row * ld_out + (long)head0 * D + lane * 4;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc = __fmaf_rn(f[e], f[e], acc);
-    const float ss = warp_butterfly(acc);
-    rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
-    if (lane == 0) rstd_out[wid] = rstd;
+  for (int i = 0; i < ROPE_HEADS; ++i) {
+    if (i >= n) break;  // (the same for the whole warp)
+    float f[4] = {0.f, 0.f, 0.f, 0.f};
+    if (active) raw[i].unpack(f);
+    if (do_norm) {
+      float acc = 0.0f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = __fmul_rn(f[e], rstd);
-  }
-  if (active) {
-    const int half = D >> 1;
-    T* o = out + row * ld_out + (long)head * D + lane * 4;
+      for (int e = 0; e < 4; ++e) acc = __fmaf_rn(f[e], f[e], acc);
+      const float ss = warp_butterfly(acc);
+      const float rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
+      if (lane == 0) rstd_out[row * heads + head0 + i] = rstd;
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr) {
-      const float c = cosb[(long)pos * half + lane * 2 + pr];
-      const float s = sinb[(long)pos * half + lane * 2 + pr];
-      const float xe = f[2 * pr], xo = f[2 * pr + 1];
-      o[2 * pr] = from_f<T>(__fmaf_rn(xe, c, -__fmul_rn(xo, s)));
-      o[2 * pr + 1] = from_f<T>(__fmaf_rn(xe, s, __fmul_rn(xo, c)));
+      for (int e = 0; e < 4; ++e) f[e] = __fmul_rn(f[e], rstd);
+    }
+    if (active) {
+      float r[4];
+#pragma unroll
+      for (int pr = 0; pr < 2; ++pr) {
+        const float xe = f[2 * pr], xo = f[2 * pr + 1];
+        r[2 * pr] = __fmaf_rn(xe, c[pr], -__fmul_rn(xo, s[pr]));
+        r[2 * pr + 1] = __fmaf_rn(xe, s[pr], __fmul_rn(xo, c[pr]));
+      }
+      Vec4<T, VEC>::store(o + i * D, r);
     }
   }
 }
 
-template <typename T>
-__global__ void qknorm_rope_bwd_kernel(const T* __restrict__ dout, long ld_dout, const T* __restrict__ in, long ld_in,
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restrict__ dout, long ld_dout, const T* __restrict__ in, long ld_in,
                                        const float* __restrict__ rstd_in, T* __restrict__ din, long ld_din,
                                        const float* __restrict__ cosb, const float* __restrict__ sinb, long rows,
                                        int heads, int D, int seq_len, int do_norm, float inv_d) {
-  const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long row;
+  int head0;
+  if (!rope_place(rows, heads, row, head0)) return;
   const int lane = threadIdx.x & 31;
-  if (wid >= rows * heads) return;
-  const long row = wid / heads;
-  const int head = (int)(wid - row * heads);
-  const int pos = (int)(row % seq_len);
   const bool active = lane * 4 < D;
-  float g[4] = {0.f, 0.f, 0.f, 0.f};
-  if (active) {
-    const int half = D >> 1;
-    const T* p = dout + row * ld_dout + (long)head * D + lane * 4;
+  const int n = min(ROPE_HEADS, heads - head0);
+  Vec4<T, VEC> rd[ROPE_HEADS], rx[ROPE_HEADS];
+  float rstd[ROPE_HEADS];
+  const T* pd = dout + row * ld_dout + (long)head0 * D + lane * 4;
+  const T* px = in + row * ld_in + (long)head0 * D + lane * 4;
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr) {
-      const float c = cosb[(long)pos * half + lane * 2 + pr];
-      const float s = sinb[(long)pos * half + lane * 2 + pr];
-      const float de = to_f<T>(p[2 * pr]), dd = to_f<T>(p[2 * pr + 1]);
-      g[2 * pr] = __fmaf_rn(de, c, __fmul_rn(dd, s));
-      g[2 * pr + 1] = __fmaf_rn(dd, c, -__fmul_rn(de, s));
+  for (int i = 0; i < ROPE_HEADS; ++i) {
+    if (active && i < n) {
+      rd[i].load(pd + i * D);
+      if (do_norm) rx[i].load(px + i * D);
     }
+    rstd[i] = do_norm && i < n ? rstd_in[row * heads + head0 + i] : 0.0f;
   }
-  if (do_norm) {
-    const float rstd = rstd_in[wid];
-    float xh[4] = {0.f, 0.f, 0.f, 0.f};
+  float c[2] = {0.f, 0.f}, s[2] = {0.f, 0.f};
+  if (active) {
+    const long at = (long)rope_pos(row, seq_len) * (D >> 1) + lane * 2;
+#pragma unroll
+    for (int pr = 0; pr < 2; ++pr) { c[pr] = cosb[at + pr]; s[pr] = sinb[at + pr]; }
+  }
+  T* o = din + row * ld_din + (long)head0 * D + lane * 4;
+#pragma unroll
+  for (int i = 0; i < ROPE_HEADS; ++i) {
+    if (i >= n) break;
+    float g[4] = {0.f, 0.f, 0.f, 0.f};
     if (active) {
-      const T* p = in + row * ld_in + (long)head * D + lane * 4;
+      float d[4];
+      rd[i].unpack(d);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) xh[e] = __fmul_rn(to_f<T>(p[e]), rstd);
+      for (int pr = 0; pr < 2; ++pr) {
+        const float de = d[2 * pr], dd = d[2 * pr + 1];
+        g[2 * pr] = __fmaf_rn(de, c[pr], __fmul_rn(dd, s[pr]));
+        g[2 * pr + 1] = __fmaf_rn(dd, c[pr], -__fmul_rn(de, s[pr]));
+      }
     }
-    float acc = 0.0f;
+    if (do_norm) {
+      float xh[4] = {0.f, 0.f, 0.f, 0.f};
+      if (active) {
+        rx[i].unpack(xh);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc = __fmaf_rn(g[e], xh[e], acc);
-    const float cs = __fmul_rn(warp_butterfly(acc), inv_d);
+        for (int e = 0; e < 4; ++e) xh[e] = __fmul_rn(xh[e], rstd[i]);
+      }
+      float acc = 0.0f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) g[e] = __fmul_rn(rstd, __fmaf_rn(-xh[e], cs, g[e]));
-  }
-  if (active) {
-    T* o = din + row * ld_din + (long)head * D + lane * 4;
+      for (int e = 0; e < 4; ++e) acc = __fmaf_rn(g[e], xh[e], acc);
+      const float cs = __fmul_rn(warp_butterfly(acc), inv_d);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = from_f<T>(g[e]);
+      for (int e = 0; e < 4; ++e) g[e] = __fmul_rn(rstd[i], __fmaf_rn(-xh[e], cs, g[e]));
+    }
+    if (active) Vec4<T, VEC>::store(o + i * D, g);
   }
 }
 
 // ------------------------------------------------------------------- SwiGLU
 // gate_up [rows, 2F] (gate = cols [0,F), up = cols [F,2F)) -> h [rows, F] = silu(gate) * up
+constexpr int SWIGLU_MAX_THREADS = 384;
+// One CTA per row, two 8-element groups per thread and sweep with all their loads in flight: no index division (a 64-bit
+// one per group cost as much as the activation), and enough bytes in flight per SM to hold the memory's rate.
 template <typename T>
-__global__ void swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ h, long rows, int F) {
-  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (idx >= rows * F) return;
-  const long row = idx / F;
-  const int col = (int)(idx - row * F);
-  float g[8], u[8], o[8];
-  Vec8<T>::load(gu + row * 2 * F + col, g);
-  Vec8<T>::load(gu + row * 2 * F + F + col, u);
+__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ h, int F) {
+  const T* gr = gu + (long)blockIdx.x * 2 * F;
+  T* hr = h + (long)blockIdx.x * F;
+  for (int c0 = threadIdx.x * 8; c0 < F; c0 += blockDim.x * 16) {
+    Raw8<T> rg[2], ru[2];
 #pragma unroll
-  for (int e = 0; e < 8; e += 2) {
-    const tc05::f2 g2 = tc05::pack2(g[e], g[e + 1]);
-    tc05::unpack2(tc05::mul2(tc05::mul2(g2, tc05::sigmoid_fast2(g2)), tc05::pack2(u[e], u[e + 1])), o[e], o[e + 1]);
+    for (int u = 0; u < 2; ++u) {
+      const int c = c0 + u * blockDim.x * 8;
+      if (c < F) {
+        rg[u].load(gr + c);
+        ru[u].load(gr + F + c);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int c = c0 + u * blockDim.x * 8;
+      if (c < F) {
+        float g[8], v[8], o[8];
+        rg[u].unpack(g);
+        ru[u].unpack(v);
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          const tc05::f2 g2 = tc05::pack2(g[e], g[e + 1]);
+          tc05::unpack2(tc05::mul2(tc05::mul2(g2, tc05::sigmoid_fast2(g2)), tc05::pack2(v[e], v[e + 1])), o[e], o[e + 1]);
+        }
+        Vec8<T>::store(hr + c, o);
+      }
+    }
   }
-  Vec8<T>::store(h + idx, o);
 }
 // d_gate_up [rows, 2F] from dh [rows, F]
 template <typename T>
-__global__ void swiglu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, long rows,
-                                  int F) {
-  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (idx >= rows * F) return;
-  const long row = idx / F;
-  const int col = (int)(idx - row * F);
-  float g[8], u[8], d[8], og[8], ou[8];
-  Vec8<T>::load(gu + row * 2 * F + col, g);
-  Vec8<T>::load(gu + row * 2 * F + F + col, u);
-  Vec8<T>::load(dh + idx, d);
+__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, int F) {
+  const T* gr = gu + (long)blockIdx.x * 2 * F;
+  const T* dr = dh + (long)blockIdx.x * F;
+  T* or_ = dgu + (long)blockIdx.x * 2 * F;
+  for (int c0 = threadIdx.x * 8; c0 < F; c0 += blockDim.x * 16) {
+    Raw8<T> rg[2], ru[2], rd[2];
 #pragma unroll
-  for (int e = 0; e < 8; e += 2) {
-    using namespace tc05;
-    const f2 g2 = pack2(g[e], g[e + 1]), u2 = pack2(u[e], u[e + 1]), d2 = pack2(d[e], d[e + 1]);
-    const f2 sg = sigmoid_fast2(g2);
-    const f2 silu = mul2(g2, sg);
-    // d silu / dg = sg * (1 + g (1 - sg))
-    const f2 one = pack2(1.0f, 1.0f);
-    const f2 dsilu = mul2(sg, fma2(g2, add2(one, mul2(sg, pack2(-1.0f, -1.0f))), one));
-    unpack2(mul2(mul2(d2, u2), dsilu), og[e], og[e + 1]);
-    unpack2(mul2(d2, silu), ou[e], ou[e + 1]);
+    for (int u = 0; u < 2; ++u) {
+      const int c = c0 + u * blockDim.x * 8;
+      if (c < F) {
+        rg[u].load(gr + c);
+        ru[u].load(gr + F + c);
+        rd[u].load(dr + c);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int c = c0 + u * blockDim.x * 8;
+      if (c < F) {
+        float g[8], v[8], d[8], og[8], ou[8];
+        rg[u].unpack(g);
+        ru[u].unpack(v);
+        rd[u].unpack(d);
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          using namespace tc05;
+          const f2 g2 = pack2(g[e], g[e + 1]), u2 = pack2(v[e], v[e + 1]), d2 = pack2(d[e], d[e + 1]);
+          const f2 sg = sigmoid_fast2(g2);
+          const f2 silu = mul2(g2, sg);
+          // d silu / dg = sg * (1 + g (1 - sg))
+          const f2 one = pack2(1.0f, 1.0f);
+          const f2 dsilu = mul2(sg, fma2(g2, add2(one, mul2(sg, pack2(-1.0f, -1.0f))), one));
+          unpack2(mul2(mul2(d2, u2), dsilu), og[e], og[e + 1]);
+          unpack2(mul2(d2, silu), ou[e], ou[e + 1]);
+        }
+        Vec8<T>::store(or_ + c, og);
+        Vec8<T>::store(or_ + F + c, ou);
+      }
+    }
   }
-  Vec8<T>::store(dgu + row * 2 * F + col, og);
-  Vec8<T>::store(dgu + row * 2 * F + F + col, ou);
+}
+// threads per row: the row's groups split evenly over the sweeps of two groups per thread
+inline int swiglu_threads(int F) {
+  const int groups = F / 8, sweeps = (groups + 2 * SWIGLU_MAX_THREADS - 1) / (2 * SWIGLU_MAX_THREADS);
+  const int t = (groups + 2 * sweeps - 1) / (2 * sweeps);
+  return (t + 31) / 32 * 32;
 }
 
 // --------------------------------------------------------- fused CE + z-loss
@@ -454,6 +614,8 @@ __global__ void add_kernel(const T* __restrict__ a, const T* __restrict__ b, T* 
 }
 
 inline unsigned blocks_for(long n, int per) { return (unsigned)((n + per - 1) / per); }
+// whether four elements of any row that start at a multiple of four are one aligned access
+inline bool four_aligned(const void* p, long ld, int bf16) { return ld % 4 == 0 && reinterpret_cast<uintptr_t>(p) % (bf16 ? 8 : 16) == 0; }
 
 }  // namespace
 
@@ -466,8 +628,11 @@ inline unsigned blocks_for(long n, int per) { return (unsigned)((n + per - 1) / 
 extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long rows, int D, float inv_d,
                                float eps, int dtype, void* stream) {
   if (D % 8) return -2;
-  DISPATCH_T(dtype, rmsnorm_fwd_kernel<T><<<blocks_for(rows, 8), 256, 0, S(stream)>>>(
-                        (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps);)
+#define RF(KERN) DISPATCH_T(dtype, KERN<<<blocks_for(rows, 8), 256, 0, S(stream)>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps);)
+#define RFC(MAXC) RF((rmsnorm_fwd_kernel<T, MAXC>))
+  if (D <= 256) { RFC(1) } else if (D <= 1024) { RFC(4) } else if (D <= 2048) { RFC(8) } else if (D <= 4096) { RFC(16) } else { RF(rmsnorm_fwd_wide_kernel<T>) }
+#undef RFC
+#undef RF
   return (int)cudaGetLastError();
 }
 extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
@@ -497,30 +662,34 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
                                    const float* sinb, long rows, int heads, int D, int seq_len, int do_norm,
                                    float inv_d, float eps, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
-  DISPATCH_T(dtype, qknorm_rope_fwd_kernel<T><<<blocks_for(rows * heads, 8), 256, 0, S(stream)>>>(
-                        (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d,
-                        eps);)
+  const unsigned grid = blocks_for(rows * ((heads + ROPE_HEADS - 1) / ROPE_HEADS), 8);
+  const bool vec = four_aligned(in, ld_in, dtype) && four_aligned(out, ld_out, dtype);
+#define QF(V) DISPATCH_T(dtype, qknorm_rope_fwd_kernel<T, V><<<grid, 256, 0, S(stream)>>>( \
+                        (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d, eps);)
+  if (vec) { QF(true) } else { QF(false) }
+#undef QF
   return (int)cudaGetLastError();
 }
 extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* in, long ld_in, const float* rstd,
                                    void* din, long ld_din, const float* cosb, const float* sinb, long rows, int heads,
                                    int D, int seq_len, int do_norm, float inv_d, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
-  DISPATCH_T(dtype, qknorm_rope_bwd_kernel<T><<<blocks_for(rows * heads, 8), 256, 0, S(stream)>>>(
-                        (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D,
-                        seq_len, do_norm, inv_d);)
+  const unsigned grid = blocks_for(rows * ((heads + ROPE_HEADS - 1) / ROPE_HEADS), 8);
+  const bool vec = four_aligned(dout, ld_dout, dtype) && four_aligned(in, ld_in, dtype) && four_aligned(din, ld_din, dtype);
+#define QB(V) DISPATCH_T(dtype, qknorm_rope_bwd_kernel<T, V><<<grid, 256, 0, S(stream)>>>( \
+                        (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d);)
+  if (vec) { QB(true) } else { QB(false) }
+#undef QB
   return (int)cudaGetLastError();
 }
 extern "C" int otb_swiglu_fwd(const void* gu, void* h, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
-  DISPATCH_T(dtype, swiglu_fwd_kernel<T><<<blocks_for(rows * F / 8, 256), 256, 0, S(stream)>>>((const T*)gu, (T*)h,
-                                                                                                 rows, F);)
+  DISPATCH_T(dtype, swiglu_fwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (T*)h, F);)
   return (int)cudaGetLastError();
 }
 extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
-  DISPATCH_T(dtype, swiglu_bwd_kernel<T><<<blocks_for(rows * F / 8, 256), 256, 0, S(stream)>>>(
-                        (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
+  DISPATCH_T(dtype, swiglu_bwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (const T*)dh, (T*)dgu, F);)
   return (int)cudaGetLastError();
 }
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
