@@ -1311,31 +1311,62 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-// delta[b,h,t] = sum_d dO[t,h,d] * O[t,h,d]; one warp per (row, head), lane_tree with VW = 4. The scratch has three
-// [B, H, T] planes: delta, -lse and -delta (the negated copies feed the transposed dK/dV kernel's packed arithmetic).
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, long lddo, const __nv_bfloat16* __restrict__ O,
+// delta[b,h,t] = sum_d dO[t,h,d] * O[t,h,d], lane_tree with VW = 4. The scratch has three [B, H, T] planes: delta, -lse and
+// -delta (the negated copies feed the transposed dK/dV kernel's packed arithmetic). A warp takes DELTA_ROWS consecutive
+// rows of one head: all of their loads (8 bytes per lane) are in flight together and the rows' results leave as whole
+// 32-byte sectors. Memory-bound then (134 MB at 4 x 4096 rows, 16 heads x 128); one row per warp with 2-byte loads, two
+// 64-bit divisions and 4-byte stores took 56 us there. VEC: both operands allow the 8-byte loads.
+constexpr int DELTA_ROWS = 8;
+template <bool VEC>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, long lddo, const __nv_bfloat16* __restrict__ O,
                                   long ldo, const float* __restrict__ lse, float* __restrict__ delta, int B, int T, int H, int D) {
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const long rows = (long)B * T;
-  if (wid >= rows * H) return;
-  const long row = wid / H;
-  const int h = (int)(wid - row * H);
-  float acc = 0.0f;
-  if (lane * 4 < D) {
-    const __nv_bfloat16* a = dO + row * lddo + (long)h * D + lane * 4;
-    const __nv_bfloat16* o = O + row * ldo + (long)h * D + lane * 4;
+  const long rows = (long)B * T, groups = (rows + DELTA_ROWS - 1) / DELTA_ROWS;
+  if (wid >= groups * H) return;
+  const long grp = (groups * H) >> 31 ? wid / H : (long)((unsigned)wid / (unsigned)H);  // heads vary fastest: neighbouring warps read one row
+  const int h = (int)(wid - grp * H);
+  const long row0 = grp * DELTA_ROWS;
+  const int n = (int)min((long)DELTA_ROWS, rows - row0);
+  const bool active = lane * 4 < D;
+  const __nv_bfloat16* pa = dO + row0 * lddo + (long)h * D + lane * 4;
+  const __nv_bfloat16* po = O + row0 * ldo + (long)h * D + lane * 4;
+  uint2 a[DELTA_ROWS], o[DELTA_ROWS];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc = __fmaf_rn(__bfloat162float(a[e]), __bfloat162float(o[e]), acc);
+  for (int r = 0; r < DELTA_ROWS; ++r) {
+    a[r] = o[r] = make_uint2(0u, 0u);
+    if (active && r < n) {
+      if (VEC) {
+        a[r] = *reinterpret_cast<const uint2*>(pa + r * lddo);
+        o[r] = *reinterpret_cast<const uint2*>(po + r * ldo);
+      } else {
+        const uint16_t* x = reinterpret_cast<const uint16_t*>(pa + r * lddo);
+        const uint16_t* y = reinterpret_cast<const uint16_t*>(po + r * ldo);
+        a[r] = make_uint2(x[0] | (uint32_t)x[1] << 16, x[2] | (uint32_t)x[3] << 16);
+        o[r] = make_uint2(y[0] | (uint32_t)y[1] << 16, y[2] | (uint32_t)y[3] << 16);
+      }
+    }
   }
+  float mine = 0.0f;
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-  if (lane == 0) {
-    const long bb = row / T, t = row - bb * T;
+  for (int r = 0; r < DELTA_ROWS; ++r) {
+    float acc = 0.0f;
+    if (active) {
+      acc = __fmaf_rn(__uint_as_float(a[r].x << 16), __uint_as_float(o[r].x << 16), acc);
+      acc = __fmaf_rn(__uint_as_float(a[r].x & 0xFFFF0000u), __uint_as_float(o[r].x & 0xFFFF0000u), acc);
+      acc = __fmaf_rn(__uint_as_float(a[r].y << 16), __uint_as_float(o[r].y << 16), acc);
+      acc = __fmaf_rn(__uint_as_float(a[r].y & 0xFFFF0000u), __uint_as_float(o[r].y & 0xFFFF0000u), acc);
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+    if (lane == r) mine = acc;
+  }
+  if (lane < n) {
+    const long row = row0 + lane, bb = row >> 31 ? row / T : (long)((unsigned)row / (unsigned)T), t = row - bb * T;
     const long idx = (bb * H + h) * T + t, plane = (long)B * H * T;
-    delta[idx] = acc;
+    delta[idx] = mine;
     delta[plane + idx] = -lse[idx];
-    delta[2 * plane + idx] = -acc;
+    delta[2 * plane + idx] = -mine;
   }
 }
 
@@ -1495,9 +1526,10 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   r = encode_3d(&tdo, dO, (uint64_t)lddo, (uint64_t)T, (uint64_t)B, (uint64_t)lddo);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
-  const long warps = (long)B * T * H;
-  attn_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O,
-                                                               ldo, lse, delta, B, T, H, D);
+  const long warps = ((long)B * T + DELTA_ROWS - 1) / DELTA_ROWS * H;
+  const bool vec = ((reinterpret_cast<uintptr_t>(O) | reinterpret_cast<uintptr_t>(dO)) & 7) == 0;  // pitches are multiples of 8 elements
+  auto delta_kernel = vec ? attn_delta_kernel<true> : attn_delta_kernel<false>;
+  delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse, delta, B, T, H, D);
   __nv_bfloat16* dQp = (__nv_bfloat16*)dqk;
   __nv_bfloat16* dKp = dQp + (long)H * D;
   __nv_bfloat16* dVp = (__nv_bfloat16*)dqkv + (long)(H + Hkv) * D;

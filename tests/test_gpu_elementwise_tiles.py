@@ -1,0 +1,82 @@
+"""Memory-bound kernels on a GPU at the edges of their tilings: bit for bit against the CPU twin."""
+import pytest
+import torch
+
+from open_transformers_b200.ops import functional as K
+
+pytestmark = pytest.mark.gpu
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+def _same(dev, host, what):
+    assert torch.equal(dev.cpu(), host), what
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("rows,D", [(1, 8), (9, 248), (7, 1032), (3, 4096), (5, 4104)])  # register widths, and one past the last
+def test_rmsnorm_forward_widths(dtype, rows, D):
+    g = torch.Generator().manual_seed(D)
+    x, w = torch.randn(rows, D, generator=g).to(dtype), torch.randn(D, generator=g).to(dtype)
+    for weight in (w, None):
+        dev = K.rmsnorm_fwd(x.cuda(), None if weight is None else weight.cuda(), 1e-5)
+        for a, b in zip(dev, K.rmsnorm_fwd(x, weight, 1e-5)):
+            _same(a, b, "rmsnorm")
+
+
+# heads that do not fill a warp's group, narrow heads, and ``pad``: a row pitch (or an offset) that forbids the wide loads
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("rows,heads,D,seq,pad", [(1, 1, 4, 1, 0), (37, 5, 128, 10, 0), (50, 3, 64, 50, 0), (33, 6, 20, 11, 1), (16, 4, 128, 16, 2)])
+def test_qknorm_rope_groups(dtype, norm, rows, heads, D, seq, pad):
+    g = torch.Generator().manual_seed(rows + D)
+    cos, sin = K.rope_tables(seq, D, 10000.0, "cpu")
+    wide = torch.randn(rows, heads * D + 8 + pad, generator=g).to(dtype)
+    dwide = torch.randn(rows, heads * D + pad, generator=g).to(dtype)
+
+    def run(dev):
+        x, dy = wide.to(dev)[:, pad:], dwide.to(dev)[:, pad:]
+        out, rstd = K.qknorm_rope_fwd(x, cos.to(dev), sin.to(dev), heads, D, seq, norm, 1e-5)
+        din = torch.zeros(rows, heads * D + pad, dtype=dtype, device=dev)[:, pad:]
+        K.qknorm_rope_bwd(dy, x, rstd, din, cos.to(dev), sin.to(dev), heads, D, seq, norm)
+        return (out, rstd, din) if norm else (out, din)
+
+    for a, b in zip(run("cuda"), run("cpu")):
+        _same(a, b, "rope")
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("rows,F", [(1, 8), (3, 264), (2, 3072), (2, 3080), (2, 6152)])  # one group, one sweep, two sweeps of 384 threads
+def test_swiglu_widths(dtype, rows, F):
+    g = torch.Generator().manual_seed(F)
+    gu, dh = torch.randn(rows, 2 * F, generator=g).to(dtype), torch.randn(rows, F, generator=g).to(dtype)
+    _same(K.swiglu_fwd(gu.cuda()), K.swiglu_fwd(gu), "forward")
+    _same(K.swiglu_bwd(gu.cuda(), dh.cuda()), K.swiglu_bwd(gu, dh), "backward")
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("V", [8, 4096, 4104, 16392, 70008, 128256])  # one group, whole sweeps, a ragged unroll, every occupancy
+def test_loss_row_widths(dtype, V):
+    g = torch.Generator().manual_seed(V)
+    x = (3 * torch.randn(3, V, generator=g)).to(dtype)
+    labels = torch.tensor([0, V - 1, -100])
+    for grad in (False, True):
+        a, b = x.clone().cuda(), x.clone()
+        dev, host = K.ce_zloss_(a, labels.cuda(), 1e-4, 0.25, grad), K.ce_zloss_(b, labels, 1e-4, 0.25, grad)
+        for p, q in zip((*dev, a), (*host, b)):
+            _same(p, q, "loss")
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D", [(1, 64, 3, 1, 64), (3, 37, 4, 2, 64), (2, 131, 2, 1, 128)])  # rows that end inside a group of 8
+def test_attention_row_groups(B, T, H, Hkv, D):
+    g = torch.Generator().manual_seed(T)
+    qk, qkv, dO = (torch.randn(B * T, n * D, generator=g).to(BF16) for n in (H + Hkv, H + 2 * Hkv, H))
+
+    def run(dev):
+        a, b, d = qk.to(dev), qkv.to(dev), dO.to(dev)
+        O, lse = K.attn_fwd(a, b, B, T, H, Hkv, D, 0)
+        dqk, dqkv = torch.zeros_like(a), torch.zeros_like(b)
+        K.attn_bwd(a, b, O, d, lse, dqk, dqkv, B, T, H, Hkv, D, 0)
+        return O, lse, dqk, dqkv
+
+    for p, q in zip(run("cuda"), run("cpu")):
+        _same(p, q, "attention")
