@@ -1578,3 +1578,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   }
   return (int)cudaGetLastError();
 }
+
+OTB_PACKED(otb_attn_fwd)
+OTB_PACKED(otb_attn_bwd)
+OTB_PACKED(otb_attn_fwd_i8pv)

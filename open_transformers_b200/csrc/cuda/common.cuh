@@ -3,6 +3,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
+
+#include <type_traits>
+#include <utility>
 
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -42,3 +46,33 @@ inline int otb_sm_count() {
     cudaError_t _e = (expr);                  \
     if (_e != cudaSuccess) return (int)_e;    \
   } while (0)
+
+// OTB_PACKED(entry) adds `entry_p`, which takes the arguments of the C entry point as one array of 8-byte words (integers
+// and pointers as 64-bit integers, floats as doubles). Python builds that array with one struct.pack, several times cheaper
+// than an object per argument; the hot entry points are called this way.
+template <typename T>
+inline T otb_packed_arg(const char* word) {
+  if constexpr (std::is_pointer<T>::value) {
+    uint64_t v;
+    memcpy(&v, word, 8);
+    return reinterpret_cast<T>(static_cast<uintptr_t>(v));
+  } else if constexpr (std::is_floating_point<T>::value) {
+    double v;
+    memcpy(&v, word, 8);
+    return static_cast<T>(v);
+  } else {
+    int64_t v;
+    memcpy(&v, word, 8);
+    return static_cast<T>(v);
+  }
+}
+template <typename... A, size_t... I>
+inline int otb_packed_call(int (*f)(A...), const char* words, std::index_sequence<I...>) {
+  return f(otb_packed_arg<A>(words + 8 * I)...);
+}
+template <typename... A>
+inline int otb_packed(int (*f)(A...), const char* words) {
+  return otb_packed_call(f, words, std::index_sequence_for<A...>());
+}
+#define OTB_PACKED(entry) \
+  extern "C" int entry##_p(const char* words) { return otb_packed(entry, words); }

@@ -765,3 +765,14 @@ extern "C" int otb_add(const void* a, const void* b, void* out, long n, int dtyp
   DISPATCH_T(dtype, add_kernel<T><<<blocks_for(n / 8, 256), 256, 0, S(stream)>>>((const T*)a, (const T*)b, (T*)out, n);)
   return (int)cudaGetLastError();
 }
+
+OTB_PACKED(otb_rmsnorm_fwd)
+OTB_PACKED(otb_rmsnorm_bwd)
+OTB_PACKED(otb_qknorm_rope_fwd)
+OTB_PACKED(otb_qknorm_rope_bwd)
+OTB_PACKED(otb_swiglu_fwd)
+OTB_PACKED(otb_swiglu_bwd)
+OTB_PACKED(otb_ce_zloss)
+OTB_PACKED(otb_det_sum)
+OTB_PACKED(otb_embedding_fwd)
+OTB_PACKED(otb_embedding_bwd)

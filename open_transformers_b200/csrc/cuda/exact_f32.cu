@@ -700,3 +700,7 @@ extern "C" int otb_attn_f32_bwd(const float* qk, long ldqk, const float* qkv, lo
     return attn_f32_bwd<64>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv, B, T, H, Hkv, D, window, c_log2, scale, vec, s);
   return attn_f32_bwd<128>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv, B, T, H, Hkv, D, window, c_log2, scale, vec, s);
 }
+
+OTB_PACKED(otb_gemm_f32)
+OTB_PACKED(otb_attn_f32_fwd)
+OTB_PACKED(otb_attn_f32_bwd)

@@ -1047,3 +1047,6 @@ extern "C" int otb_tp_finish(const float* acc, const void* flags, unsigned seq, 
       reinterpret_cast<__nv_bfloat16*>(y), rows, N, BN, rank, ld_acc, ldr, ldy, status);
   return (int)cudaGetLastError();
 }
+
+OTB_PACKED(otb_gemm_bf16)
+OTB_PACKED(otb_gemm_i8)

@@ -227,3 +227,10 @@ extern "C" int otb_i8_widen(const void* q, void* out, long n, int out_dtype, voi
   else i8_widen_kernel<float><<<blocks_for(n, 8 * 256), 256, 0, S(stream)>>>((const int8_t*)q, (float*)out, n);
   return (int)cudaGetLastError();
 }
+
+OTB_PACKED(otb_absmax)
+OTB_PACKED(otb_quant_act)
+OTB_PACKED(otb_quant_weight)
+OTB_PACKED(otb_lsq_bwd)
+OTB_PACKED(otb_row_stat)
+OTB_PACKED(otb_i8_widen)

