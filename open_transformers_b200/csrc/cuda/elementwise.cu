@@ -227,6 +227,92 @@ inline void pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
   }
 }
 
+// ------------------------------------------------------------ per-head RMSNorm with gain
+// The RMSNorm of every head of a [tokens, ld] buffer (head h in columns h*D .. h*D + D - 1, D <= 128, multiple of 8), read
+// and written in place of its columns: the same sums as the row kernels above on [tokens * heads, D] (lane_tree with VW = 8
+// uses 16 of its 32 lanes at this width; the other sixteen add +0.0 once), without copies that make the heads contiguous and
+// copies that join them again. Sixteen lanes per row, so a warp works on two.
+__device__ __forceinline__ float half_butterfly(float v) {
+  v = __fadd_rn(v, 0.0f);  // the partner at distance 16 holds no element
+#pragma unroll
+  for (int off = 8; off >= 1; off >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, off));
+  return v;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) head_rmsnorm_fwd_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, T* __restrict__ y, long ldy,
+                                                              float* __restrict__ rstd_out, long rows, int heads, int D, float inv_d, float eps) {
+  const long row = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
+  const int c = (threadIdx.x & 15) * 8;
+  const bool on = row < rows && c < D;
+  const long tok = row / heads;
+  const long at = (row - tok * heads) * D + c;
+  Raw8<T> raw;
+  float acc = 0.0f;
+  if (on) {
+    raw.load(x + tok * ldx + at);
+    float f[8];
+    raw.unpack(f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc = __fmaf_rn(f[e], f[e], acc);
+  }
+  const float ss = half_butterfly(acc);
+  const float rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
+  if (on) {
+    if (c == 0) rstd_out[row] = rstd;
+    float f[8], g[8], o[8];
+    raw.unpack(f);
+    Vec8<T>::load(w + c, g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(__fmul_rn(f[e], rstd), g[e]);
+    Vec8<T>::store(y + tok * ldy + at, o);
+  }
+}
+// dx and the dgamma partials of NORM_SLAB-row slabs (rows = (token, head) pairs); two slabs per CTA.
+template <typename T>
+__global__ void __launch_bounds__(256) head_rmsnorm_bwd_kernel(const T* __restrict__ dy, long lddy, const T* __restrict__ x, long ldx, const T* __restrict__ w,
+                                                              const float* __restrict__ rstd_in, T* __restrict__ dx, long lddx,
+                                                              float* __restrict__ dgamma_partial, long rows, int heads, int D, float inv_d) {
+  __shared__ float prod[16][128];
+  const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
+  const long row = (long)blockIdx.x * 16 + r;
+  const bool on = row < rows && c < D;
+  const long tok = row / heads;
+  const long at = (row - tok * heads) * D + c;
+  float xh[8], gy[8], acc = 0.0f, rstd = 0.0f;
+  if (on) {
+    rstd = rstd_in[row];
+    float xf[8], df[8], g[8];
+    Vec8<T>::load(x + tok * ldx + at, xf);
+    Vec8<T>::load(dy + tok * lddy + at, df);
+    Vec8<T>::load(w + c, g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      xh[e] = __fmul_rn(xf[e], rstd);
+      gy[e] = __fmul_rn(df[e], g[e]);
+      acc = __fmaf_rn(gy[e], xh[e], acc);
+      if (dgamma_partial) prod[r][c + e] = __fmul_rn(df[e], xh[e]);
+    }
+  }
+  const float cs = __fmul_rn(half_butterfly(acc), inv_d);
+  if (on) {
+    float o[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(rstd, __fmaf_rn(-xh[e], cs, gy[e]));
+    Vec8<T>::store(dx + tok * lddx + at, o);
+  }
+  if (dgamma_partial) {
+    __syncthreads();
+    const int slab = threadIdx.x >> 7, col = threadIdx.x & 127;
+    const long first = (long)blockIdx.x * 16 + slab * NORM_SLAB;
+    if (first < rows && col < D) {
+      const int n = (int)min((long)NORM_SLAB, rows - first);
+      float t = 0.0f;
+      for (int i = 0; i < n; ++i) t = __fadd_rn(t, prod[slab * NORM_SLAB + i][col]);
+      dgamma_partial[(first / NORM_SLAB) * D + col] = t;
+    }
+  }
+}
+
 // --------------------------------------------------- gain-free QK-norm + RoPE
 // Over the first `heads` heads of a [rows, ld_in] buffer with head width D (<= 128, multiple of 4): lane l of a warp holds
 // elements 4l..4l+3 of a head (two rotation pairs). out[row, head*D + i]; rstd[row*heads + head]. lane_tree with VW = 4.
@@ -683,6 +769,22 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
   if (dgamma_partial) pair_tree_cols_launch(dgamma_partial, slabs, D, S(stream));
   return (int)cudaGetLastError();
 }
+// x, y, dy, dx: 16-byte aligned, pitches (in elements) that keep every row so; D <= 128, multiple of 8. rows = tokens * heads.
+extern "C" int otb_head_rmsnorm_fwd(const void* x, long ldx, const void* w, void* y, long ldy, float* rstd, long rows, int heads, int D,
+                                    float inv_d, float eps, int dtype, void* stream) {
+  if (D % 8 || D > 128 || ldx % 8 || ldy % 8) return -2;
+  DISPATCH_T(dtype, head_rmsnorm_fwd_kernel<T><<<blocks_for(rows, 16), 256, 0, S(stream)>>>((const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
+                                                                                          D, inv_d, eps);)
+  return (int)cudaGetLastError();
+}
+extern "C" int otb_head_rmsnorm_bwd(const void* dy, long lddy, const void* x, long ldx, const void* w, const float* rstd, void* dx, long lddx,
+                                    float* dgamma_partial, long rows, int heads, int D, float inv_d, int dtype, void* stream) {
+  if (D % 8 || D > 128 || lddy % 8 || ldx % 8 || lddx % 8) return -2;
+  DISPATCH_T(dtype, head_rmsnorm_bwd_kernel<T><<<blocks_for(rows, 16), 256, 0, S(stream)>>>((const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
+                                                                                          (T*)dx, lddx, dgamma_partial, rows, heads, D, inv_d);)
+  if (dgamma_partial) pair_tree_cols_launch(dgamma_partial, (rows + NORM_SLAB - 1) / NORM_SLAB, D, S(stream));
+  return (int)cudaGetLastError();
+}
 extern "C" long otb_rmsnorm_slabs(long rows) { return (rows + NORM_SLAB - 1) / NORM_SLAB; }
 
 extern "C" int otb_pair_tree_cols(float* v, long n, int D, void* stream) {
@@ -768,6 +870,8 @@ extern "C" int otb_add(const void* a, const void* b, void* out, long n, int dtyp
 
 OTB_PACKED(otb_rmsnorm_fwd)
 OTB_PACKED(otb_rmsnorm_bwd)
+OTB_PACKED(otb_head_rmsnorm_fwd)
+OTB_PACKED(otb_head_rmsnorm_bwd)
 OTB_PACKED(otb_qknorm_rope_fwd)
 OTB_PACKED(otb_qknorm_rope_bwd)
 OTB_PACKED(otb_swiglu_fwd)

@@ -23,6 +23,13 @@ class ParamMixin:
         return getattr(self, "_slot_" + name, None)
 
 
+def _untouched(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` would run ``cls.forward`` and nothing else: no subclass, no hook, no replaced method. Only
+    then may a fused function take the module's place."""
+    return type(module) is cls and "forward" not in module.__dict__ and not nn.modules.module._has_any_global_hook() and not (
+        module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+
+
 class Linear(nn.Module, ParamMixin):
     def __init__(self, in_features: int, out_features: int):
         super().__init__()
@@ -90,13 +97,22 @@ class QuantLinear(Linear):
             return K.row_stat(w, "absmax", 1.0 / self.qmax_w, 1e-12)
         return (K.absmax(w) * (1.0 / self.qmax_w)).clamp_min(1e-12).expand(w.shape[0]).contiguous()
 
+    def _operand(self, dtype):
+        """The weight that is quantised, in the activation dtype."""
+        w = self._cw()
+        if w is None:
+            w = self.weight if dtype == self.weight.dtype else self.weight.to(dtype)
+        return w.detach()
+
+    def quant_operands(self, dtype):
+        """(w, weight slot, step, step slot, qmax, learned step?, cache) for ``A.quant_qkv``."""
+        w, lsq = self._operand(dtype), self.method == "lsq"
+        return w, self._slot(), self._step(w), self._slot("weight_scale") if lsq else None, self.qmax_w, lsq, self._qcache
+
     def forward(self, x, residual=None, tp_mode=None):
         if not self.qat_active:
             return super().forward(x, residual)
-        w = self._cw()
-        if w is None:
-            w = self.weight if x.dtype == self.weight.dtype else self.weight.to(x.dtype)
-        w = w.detach()
+        w = self._operand(x.dtype)
         lsq = self.method == "lsq"
         st = A.tp()
         mode = tp_mode or self.tp_mode
@@ -161,13 +177,18 @@ class RMSNorm(nn.Module, ParamMixin):
         else:
             self.register_parameter("weight", None)
 
+    def operands(self, dtype):
+        """(fp32 parameter, gain in the activation dtype, gradient slot)."""
+        w = self._cw()
+        if w is None:
+            w = self.weight if dtype == self.weight.dtype else self.weight.to(dtype)
+        return self.weight, w, self._slot()
+
     def forward(self, x, tp_heads: int = 0):
         if self.weight is None:
             return A.rms_norm(x, None, eps=self.eps)
-        w = self._cw()
-        if w is None and x.dtype != self.weight.dtype:
-            w = self.weight.to(x.dtype)
-        return A.rms_norm(x, self.weight, w, self._slot(), self.eps, tp_heads)
+        master, w, slot = self.operands(x.dtype)
+        return A.rms_norm(x, master, w, slot, self.eps, tp_heads)
 
 
 @ROPE.register("rope_default")
@@ -275,7 +296,15 @@ class _GQABase(nn.Module, ParamMixin):
 
     def _qkv(self, x):
         if isinstance(self.wq, QuantLinear) and self.wq.qat_active:
-            return torch.cat([self.wq(x), self.wk(x), self.wv(x)], -1)
+            layers = (self.wq, self.wk, self.wv)
+            # one fused call when the three are plain active layers that quantise their input alike; rows of the joint output
+            # and of its gradient then start at multiples of 16 bytes (out_features % 8)
+            if all(_untouched(m, QuantLinear) and m.qat_active and not m.ste_bwd_hadamard and m.qmax_a == self.wq.qmax_a and
+                   m.out_features % 8 == 0 for m in layers):
+                parts = [m.quant_operands(x.dtype) for m in layers]
+                masters = [p for m in layers for p in (m.weight, m.weight_scale if m.method == "lsq" else None)]
+                return A.quant_qkv(x, self.wq.qmax_a, parts, masters)
+            return torch.cat([m(x) for m in layers], -1)
         fused = getattr(self, "_fused_qkv", None)
         if fused is not None:  # (master view, compute view, slot) spanning wq|wk|wv in the flat buffers
             return A.linear(x, fused[0], fused[1], fused[2])
@@ -316,7 +345,11 @@ class _GQABase(nn.Module, ParamMixin):
         B, T, _ = x.shape
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
         qkv = self._qkv(x)
-        if self.qk_norm_gain:
+        if self.qk_norm_gain and _untouched(self.q_norm, RMSNorm) and _untouched(self.k_norm, RMSNorm) and \
+                self.q_norm.eps == self.k_norm.eps and K.head_norm_supported(qkv.reshape(B * T, -1), D):
+            o = A.gain_attention(qkv, cos, sin, self.q_norm.operands(qkv.dtype), self.k_norm.operands(qkv.dtype), H, Hkv, D, self.window,
+                                 self.q_norm.eps, self._int8_pv(qkv))
+        elif self.qk_norm_gain:
             q, k, v = qkv.split([H * D, Hkv * D, Hkv * D], -1)
             q = self.q_norm(q.reshape(B, T, H, D)).reshape(B, T, H * D)
             k = self.k_norm(k.reshape(B, T, Hkv, D)).reshape(B, T, Hkv * D)

@@ -122,6 +122,34 @@ def rmsnorm_bwd(dy, x, w, rstd, need_dgamma: bool):
     return dx, (part[0] if need_dgamma else None)
 
 
+_head_rmsnorm_fwd = packed_entry("otb_head_rmsnorm_fwd", "9q2d2q")
+_head_rmsnorm_bwd = packed_entry("otb_head_rmsnorm_bwd", "12qd2q")
+
+
+def head_norm_supported(x: torch.Tensor, D: int) -> bool:
+    """Whether the per-head RMSNorm kernels take the heads of this [tokens, columns] CUDA buffer in place."""
+    return x.is_cuda and D % 8 == 0 and D <= 128 and _ld(x) % 8 == 0 and x.data_ptr() % 16 == 0
+
+
+def head_rmsnorm_fwd(x, w, y, heads: int, D: int, eps: float):
+    """RMSNorm with gain ``w`` [D] of every head of ``x`` [tokens, heads * D] (any row pitch) into ``y``; returns rstd
+    [tokens * heads]. Same bits as ``rmsnorm_fwd`` on the heads as contiguous rows."""
+    rows = x.shape[0] * heads
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+    check(_head_rmsnorm_fwd(ptr(x), _ld(x), ptr(w), ptr(y), _ld(y), ptr(rstd), rows, heads, D, 1.0 / D, eps, is_bf16(x), raw_stream()),
+          "head_rmsnorm_fwd")
+    return rstd
+
+
+def head_rmsnorm_bwd(dy, x, w, rstd, dx, heads: int, D: int, need_dgamma: bool):
+    """Gradient of ``head_rmsnorm_fwd``: writes ``dx`` (any row pitch) and returns dgamma [D] or None."""
+    rows = x.shape[0] * heads
+    part = torch.empty(((rows + NORM_SLAB - 1) // NORM_SLAB, D), dtype=torch.float32, device=x.device) if need_dgamma else None
+    check(_head_rmsnorm_bwd(ptr(dy), _ld(dy), ptr(x), _ld(x), ptr(w), ptr(rstd), ptr(dx), _ld(dx), ptr(part), rows, heads, D, 1.0 / D,
+                            is_bf16(x), raw_stream()), "head_rmsnorm_bwd")
+    return part[0] if need_dgamma else None
+
+
 # ------------------------------------------------------------------ QK-norm + RoPE, attention
 _qknorm_rope_fwd = packed_entry("otb_qknorm_rope_fwd", "12q2d2q")
 _qknorm_rope_bwd = packed_entry("otb_qknorm_rope_bwd", "14qd2q")
@@ -388,14 +416,17 @@ def quant_weight(w: torch.Tensor, s: torch.Tensor, qmax: int, hat_dtype: torch.d
 
 
 def gemm_i8(aq: torch.Tensor, bq: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor, out_dtype: torch.dtype,
-            residual: torch.Tensor | None = None) -> torch.Tensor:
+            residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``C = float(A_q B_q^T) * (sa * sb[n]) (+ residual)``: int8 [M,K] x int8 [N,K], exact int32 accumulation
-    (tcgen05 kind::i8 on the GPU), one rounding at the dequantisation."""
+    (tcgen05 kind::i8 on the GPU), one rounding at the dequantisation. ``out``: where to put it (a column range of a wider
+    buffer, say)."""
     M, Kd = aq.shape
     N, Kb = bq.shape
     assert Kd == Kb and aq.dtype == torch.int8 and bq.dtype == torch.int8
     assert sa.dtype == torch.float32 and sb.dtype == torch.float32 and sb.numel() == N
-    out = torch.empty((M, N), dtype=out_dtype, device=aq.device)
+    if out is None:
+        out = torch.empty((M, N), dtype=out_dtype, device=aq.device)
+    assert out.dtype == out_dtype and tuple(out.shape) == (M, N)
     bf = is_bf16(out)
     epi = EPI_RESIDUAL if residual is not None else (EPI_STORE if bf else EPI_STORE_F32)
     if residual is not None:
