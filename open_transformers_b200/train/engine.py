@@ -1295,20 +1295,18 @@ class TrainEngine:
         lay = self.layout
         if self.sharded and td != "tree":
             raise ValueError("sharded multi-GPU hashing needs train.state_hash.tensor_digest=tree")
-        handle = {"td": td, "include_grads": include_grads, "opt_step": self.opt_step, "keys": None, "plan": None, "digests": None}
+        handle = {"td": td, "include_grads": include_grads, "opt_step": self.opt_step, "plan": None, "digests": None}
         if td != "tree":
             return handle
         fields = self._hash_fields(include_grads)
-        keys, views = [], []
-        for si in range(self.seg_lo, self.seg_hi) if self.sharded else range(self.n_segs):
-            seg = lay.segments[si]
-            for tag, flat in fields:
-                keys.append((seg.param, seg.shard, tag))
-                views.append(self._segment_view(flat, si, packed=tag != "weight"))
-        handle["keys"] = keys
-        if self.is_cuda and views:
-            plans = self.__dict__.setdefault("_hash_plans", {})
-            plan = plans.get(include_grads)
+        plans = self.__dict__.setdefault("_hash_plans", {})
+        plan = plans.get(include_grads)
+        views = []
+        if plan is None:  # (a plan holds the same views, in the same order)
+            for si in range(self.seg_lo, self.seg_hi) if self.sharded else range(self.n_segs):
+                for tag, flat in fields:
+                    views.append(self._segment_view(flat, si, packed=tag != "weight"))
+        if self.is_cuda and (plan is not None or views):
             if plan is None:
                 plan = plans[include_grads] = SH.TreeDigestPlan(views)
                 lo, _hi = torch.cuda.Stream.priority_range()
@@ -1330,27 +1328,20 @@ class TrainEngine:
         when ownership is sharded, and fold everything into the v3 byte stream on the host."""
         td, include_grads = handle["td"], handle["include_grads"]
         lay = self.layout
-        seg_digests = {}
         if td == "tree":
+            streams = self._hash_streams(include_grads)  # (the first time: laid out while the device still hashes)
             if handle["plan"] is not None:
                 handle["done"].synchronize()
-                digs = handle["plan"].digests()
+                raw = handle["plan"].digest_bytes()
             else:
-                digs = handle["digests"]
-            seg_digests = dict(zip(handle["keys"], digs))
+                raw = b"".join(handle["digests"])
             if self.sharded:
                 # every process knows which (parameter, shard, field) digests every other one owns, so only the 32-byte
                 # values travel: one all-gather of a fixed-size byte tensor
-                cache = self.__dict__.setdefault("_hash_keys_by_rank", {})
-                keys_by_rank = cache.get(include_grads)
-                if keys_by_rank is None:
-                    fields = [tag for tag, _ in self._hash_fields(include_grads)]
-                    keys_by_rank = cache[include_grads] = [
-                        [(lay.segments[si].param, lay.segments[si].shard, tag) for si in range(slo, shi) for tag in fields]
-                        for slo, shi in lay.owner_ranges(self.world)]
-                width = 32 * max(max(len(k) for k in keys_by_rank), 1)
+                n_fields = len(self._hash_fields(include_grads))
+                counts = [(shi - slo) * n_fields for slo, shi in lay.owner_ranges(self.world)]
+                width = 32 * max(max(counts), 1)
                 mine = torch.zeros(width, dtype=torch.uint8)
-                raw = b"".join(digs)
                 mine[: len(raw)] = torch.frombuffer(bytearray(raw), dtype=torch.uint8)
                 if self._host_gloo:  # the digests are host bytes already: no reason to touch the device or its streams
                     parts = [torch.empty_like(mine) for _ in range(self.world)]
@@ -1360,42 +1351,93 @@ class TrainEngine:
                     parts = [torch.empty_like(mine) for _ in range(self.world)]
                     dist.all_gather(parts, mine, group=self.group)
                 allraw = torch.stack(parts).cpu().numpy().tobytes()
-                seg_digests = {}
-                for r, keys in enumerate(keys_by_rank):
-                    base = r * width
-                    for j, k in enumerate(keys):
-                        seg_digests[k] = allraw[base + 32 * j: base + 32 * j + 32]
-        order = sorted(range(len(self.names)), key=lambda i: self.names[i])
-        step_bytes = b"optim_step\0" + int(handle["opt_step"]).to_bytes(8, "little", signed=True)
-        empty = SH.tree_digest_bytes(b"") if td == "tree" else None
-        locals_ = []
-        for s in range(self.dp_shard):
-            h = SH._new()
-            for pi in order:
-                shape = lay.shapes[pi] if lay.shapes[pi] else (1,)
-                lo, hi = SH.shard_rows(shape[0], self.dp_shard, s)
-                sshape = (hi - lo,) + tuple(shape[1:])
-                h.update(self.names[pi].encode() + b"\0")
-                head = b"\0torch.float32\0" + str(sshape).encode() + b"\0"
-
-                def feed(tag, key, flat):
-                    if td == "tree":
-                        h.update(tag + head + b"tree\0" + (seg_digests[(pi, s, key)] if hi > lo else empty))
-                    else:
-                        h.update(tag + head)
-                        row = lay.numels[pi] // max(shape[0], 1)
-                        st = lay.offsets[pi] + lo * row
-                        SH.feed_raw(h, flat[st:st + (hi - lo) * row])
-
-                feed(b"weight", "weight", self.master)
-                h.update(step_bytes)
-                feed(b"optim_exp_avg", "exp_avg", self.m1)
-                feed(b"optim_exp_avg_sq", "exp_avg_sq", self.m2)
-                if include_grads:
-                    feed(b"grad", "grad", self.grad_red)
-            locals_.append(h.digest())
+                raw = b"".join(allraw[r * width: r * width + 32 * c] for r, c in enumerate(counts))
+            locals_ = self._fold_digests(streams, np.frombuffer(raw, dtype=np.uint8).reshape(-1, 32), handle["opt_step"])
+        else:
+            locals_ = [self._shard_stream(s, include_grads, handle["opt_step"]) for s in range(self.dp_shard)]
         shard_state = SH.combine_shard_state(locals_, self.V)
         return SH.finalize_state_hash(shard_state, self.param_groups, prev, batch_digest)
+
+    def _shard_records(self, s: int, include_grads: bool):
+        """The v3 stream of virtual shard ``s`` as (kind, value) items: "bytes" a constant, "step" the optimizer step's eight
+        bytes, "data" one tensor's content as (parameter, field index, rows lo, rows hi)."""
+        lay = self.layout
+        tags = (b"weight", b"optim_exp_avg", b"optim_exp_avg_sq", b"grad")
+        for pi in sorted(range(len(self.names)), key=lambda i: self.names[i]):
+            shape = lay.shapes[pi] if lay.shapes[pi] else (1,)
+            lo, hi = SH.shard_rows(shape[0], self.dp_shard, s)
+            head = b"\0torch.float32\0" + str((hi - lo,) + tuple(shape[1:])).encode() + b"\0"
+            yield "bytes", self.names[pi].encode() + b"\0"
+            for f in range(4 if include_grads else 3):
+                yield "bytes", tags[f] + head
+                yield "data", (pi, f, lo, hi)
+                if f == 0:
+                    yield "bytes", b"optim_step\0"
+                    yield "step", None
+
+    def _shard_stream(self, s: int, include_grads: bool, opt_step: int) -> bytes:
+        """Digest of shard ``s`` over the raw tensor bytes."""
+        lay, h = self.layout, SH._new()
+        flats = [flat for _, flat in self._hash_fields(include_grads)]
+        for kind, v in self._shard_records(s, include_grads):
+            if kind == "data":
+                pi, f, lo, hi = v
+                row = lay.numels[pi] // max(lay.shapes[pi][0] if lay.shapes[pi] else 1, 1)
+                st = lay.offsets[pi] + lo * row
+                SH.feed_raw(h, flats[f][st:st + (hi - lo) * row])
+            else:
+                h.update(v if kind == "bytes" else int(opt_step).to_bytes(8, "little", signed=True))
+        return h.digest()
+
+    def _hash_streams(self, include_grads: bool) -> list:
+        """Every shard's stream with a place for each digest and for the step: (bytes, byte positions of the digests, which
+        digest goes there, byte positions of the step), laid out once per engine. Only the digests and the step change from
+        one hash to the next, so a hash is two scatters and one blake2b call per shard; the device has nothing to do
+        meanwhile when the hash is not overlapped. (126 M parameters in 8 shards, 608 digests: building the views and the
+        stream item by item took 1.4 ms of a 3.9 ms hash.)"""
+        cache = self.__dict__.setdefault("_hash_templates", {})
+        shards = cache.get(include_grads)
+        if shards is not None:
+            return shards
+        n_fields = 4 if include_grads else 3
+        at_seg = {(sg.param, sg.shard): i for i, sg in enumerate(self.layout.segments)}
+        empty, byte = SH.tree_digest_bytes(b""), np.arange(32)
+        shards = []
+        for s in range(self.dp_shard):
+            text, places, source, steps = bytearray(), [], [], []
+            for kind, v in self._shard_records(s, include_grads):
+                if kind == "bytes":
+                    text += v
+                elif kind == "step":
+                    steps.append(len(text))
+                    text += bytes(8)
+                else:
+                    pi, f, lo, hi = v
+                    text += b"tree\0"
+                    if hi > lo:
+                        places.append(len(text))
+                        source.append(at_seg[(pi, s)] * n_fields + f)
+                    text += empty
+            places = (np.asarray(places, dtype=np.int64)[:, None] + byte).reshape(-1)
+            steps = (np.asarray(steps, dtype=np.int64)[:, None] + byte[:8]).reshape(-1)
+            shards.append((np.frombuffer(bytes(text), dtype=np.uint8), places, np.asarray(source, dtype=np.int64), steps))
+        cache[include_grads] = shards
+        return shards
+
+    @staticmethod
+    def _fold_digests(streams: list, digests: np.ndarray, opt_step: int) -> list[bytes]:
+        """Digest of every shard's stream, each tensor represented by its tree digest: ``digests`` [segments x fields, 32] in
+        segment order."""
+        step = np.frombuffer(int(opt_step).to_bytes(8, "little", signed=True), dtype=np.uint8)
+        out = []
+        for text, places, source, steps in streams:
+            buf = text.copy()
+            buf[places] = digests[source].reshape(-1)
+            buf[steps] = np.tile(step, len(steps) // 8)
+            h = SH._new()
+            h.update(buf)
+            out.append(h.digest())
+        return out
 
     def sharded_state_hash(self, prev, batch_digest: bytes | None, include_grads: bool = True, tensor_digest: str | None = None) -> str:
         """v3 hash of the current state. With peer-sharded ownership each process digests the segments it

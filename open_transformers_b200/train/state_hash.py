@@ -180,8 +180,12 @@ class TreeDigestPlan:
                                           ctypes.c_void_p(st.cuda_stream)), "tree_digest_plan")
             self.host.copy_(self.out, non_blocking=True)
 
+    def digest_bytes(self) -> bytes:
+        """All n digests, 32 bytes each."""
+        return self.host.numpy().tobytes()
+
     def digests(self) -> list[bytes]:
-        raw = self.host.numpy().tobytes()
+        raw = self.digest_bytes()
         return [raw[i * 32:(i + 1) * 32] for i in range(self.n)]
 
 
