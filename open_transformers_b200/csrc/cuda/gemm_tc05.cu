@@ -10,6 +10,11 @@
 //     (cp.async.bulk.tensor store; cp.reduce.async.bulk.tensor .add for the fp32 accumulate
 //     epilogue, one add per element, so still a fixed order).
 //
+// Large products run on CTA PAIRS (PAIR = true): the two SMs of a cluster share one 256 x 256 tile
+// (tcgen05 cta_group::2). Each CTA stages its 128 rows of A and half of B's rows, the first CTA's barrier counts both CTAs'
+// loads, its elected thread issues the products, which read both shared memories and accumulate 128 rows in each CTA's
+// tensor memory, and a multicast commit releases the stage, or the finished tile, in both. The epilogue is the same.
+//
 // Reduction order (the hashed contract): every output element is the tensor-core fp32
 // accumulation of its K products taken in ascending k, 16 at a time, with NO split-K and no
 // atomics, so the result does not depend on the grid, the tile schedule or the GPU count.
@@ -154,10 +159,10 @@ __device__ __forceinline__ void release_peer_flag(uint32_t* flag, uint32_t seq) 
   asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(seq) : "memory");
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool PAIR = false>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK_BYTES;
-  static constexpr int B_BYTES = BN * BK_BYTES;
+  static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK_BYTES;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int EPI_OFFSET = STAGES * STAGE_BYTES;       // 4 warps x 2 buffers x [32 rows][128 B]
   static constexpr int EPI_BYTES = 4 * 2 * 4096;
@@ -165,7 +170,7 @@ struct SmemLayout {
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;  // + barriers + alignment slack
 };
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8, int TP, typename TPA>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8, int TP, typename TPA, bool PAIR = false>
 __global__ void __launch_bounds__(TP >= 2 ? NUM_THREADS + 128 : NUM_THREADS, 1)
 gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, void* __restrict__ Cv,
@@ -175,7 +180,12 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   static_assert(!I8 || (!A_MN && !B_MN), "the int8 path takes K-major operands only");
   static_assert(TP == 0 || !I8, "the tensor-parallel variants are bf16");
   static_assert(TP != 2 || EPI == EPI_F32, "the chained GEMM hands fp32 accumulator tiles on");
-  int nctas = gridDim.x;
+  static_assert(TP == 0 || !PAIR, "the tensor-parallel variants work on single CTAs");
+  constexpr int CTAS = PAIR ? 2 : 1;                  // CTAs that work on one tile
+  constexpr int TM = BM * CTAS;                       // rows of a tile; each CTA of a pair holds 128 of them
+  constexpr int BROWS = BN / CTAS;                    // rows of B this CTA stages
+  const int half = PAIR ? (int)(blockIdx.x & 1) : 0;  // rank in the pair (clusters are two consecutive blocks)
+  int nctas = gridDim.x / CTAS;
   if constexpr (TP == 1) {
     nctas = tp.gemm_ctas;
     if ((int)blockIdx.x >= nctas) {
@@ -207,8 +217,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   }
   constexpr int BK = I8 ? BK_BYTES : BK_BYTES / 2;  // elements of K per k-block
-  const int cta = ((int)blockIdx.x + g_cta_rotation) % nctas;  // which persistent worker this CTA is
-  using L = SmemLayout<BN, STAGES>;
+  const int cta = ((int)blockIdx.x / CTAS + g_cta_rotation) % nctas;  // which persistent worker this CTA (or pair) is
+  using L = SmemLayout<BN, STAGES, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
@@ -225,7 +235,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int lane = threadIdx.x & 31;
   constexpr uint32_t TMEM_COLS = 2 * BN >= 512 ? 512 : (2 * BN <= 32 ? 32 : 2 * BN);
 
-  const int tiles_m = (M + BM - 1) / BM;
+  const int tiles_m = (M + TM - 1) / TM;
   const int tiles_n = (N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int k_blocks = (K + BK - 1) / BK;
@@ -237,18 +247,24 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 4);  // one arrive per epilogue warp
+      mbar_init(&tempty_bar[b], 4 * CTAS);  // one arrive per epilogue warp
       mbar_init(&tloaded_bar[b], 4);  // one arrive per accumulator-loading warp
     }
     *abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_slot, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything arrives on them
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -305,26 +321,36 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag)) { ok = false; break; }
           uint8_t* sa = smem + s * L::STAGE_BYTES;
           uint8_t* sb = sa + L::A_BYTES;
-          mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+          // a pair's loads (each CTA its own rows of A and its half of B) are all counted on the first CTA's barrier
+          if (half == 0) mbar_expect_tx(&full_bar[s], CTAS * L::STAGE_BYTES);
+          auto load = [&](uint8_t* dst, const CUtensorMap* tmap, int x, int y) {
+            if constexpr (PAIR) tma_load_2d_pair(dst, tmap, pair_leader(&full_bar[s]), x, y);
+            else tma_load_2d(dst, tmap, &full_bar[s], x, y);
+          };
+          const int arow = tm * TM + half * BM, brow = tn * BN + half * BROWS;
           if (!A_MN) {
-            tma_load_2d(sa, &tmA, &full_bar[s], kb * BK, tm * BM);
+            load(sa, &tmA, kb * BK, arow);
           } else {
 #pragma unroll
-            for (int c = 0; c < BM / 64; ++c) tma_load_2d(sa + c * 8192, &tmA, &full_bar[s], tm * BM + c * 64, kb * BK);
+            for (int c = 0; c < BM / 64; ++c) load(sa + c * 8192, &tmA, arow + c * 64, kb * BK);
           }
           if (!B_MN) {
-            tma_load_2d(sb, &tmB, &full_bar[s], kb * BK, tn * BN);
+            load(sb, &tmB, kb * BK, brow);
           } else {
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c) tma_load_2d(sb + c * 8192, &tmB, &full_bar[s], tn * BN + c * 64, kb * BK);
+            for (int c = 0; c < BROWS / 64; ++c) load(sb + c * 8192, &tmB, brow + c * 64, kb * BK);
           }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc = I8 ? make_idesc(BM, BN, 0, 0, 2, 1) : make_idesc(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    if (half == 0 && elect_one()) {  // the first CTA's thread issues the products of both
+      constexpr uint32_t idesc = I8 ? make_idesc(TM, BN, 0, 0, 2, 1) : make_idesc(TM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      auto commit = [](uint64_t* bar) {
+        if constexpr (PAIR) mma_commit_pair(bar);
+        else mma_commit(bar);
+      };
       uint32_t it = 0, lt = 0;
       bool ok = true;
       for (int t = cta; t < num_tiles && ok; t += nctas, ++lt) {
@@ -333,7 +359,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (chain_in) {  // the loading warps waited for the buffer to be free and filled it with the incoming partial sum
           if (!mbar_wait(&tloaded_bar[buf], bph, abort_flag)) { ok = false; break; }
         } else {
-          if (!mbar_wait(&tempty_bar[buf], bph ^ 1, abort_flag)) { ok = false; break; }
+          if (!(PAIR ? mbar_wait_cluster(&tempty_bar[buf], bph ^ 1, abort_flag) : mbar_wait(&tempty_bar[buf], bph ^ 1, abort_flag))) { ok = false; break; }
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
@@ -348,12 +374,14 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int kk = 0; kk < BK_BYTES / UMMA_K_BYTES; ++kk) {
             const uint64_t ad = A_MN ? make_smem_desc(sa + kk * 2048, 8192, 1024) : make_smem_desc(sa + kk * 32, 16, 1024);
             const uint64_t bd = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024) : make_smem_desc(sb + kk * 32, 16, 1024);
-            if (I8) mma_i8_ss(d_tmem, ad, bd, idesc, (kb | kk) != 0);
+            if constexpr (PAIR && I8) mma_i8_ss_pair(d_tmem, ad, bd, idesc, (kb | kk) != 0);
+            else if constexpr (PAIR) mma_f16_ss_pair(d_tmem, ad, bd, idesc, (kb | kk) != 0);
+            else if constexpr (I8) mma_i8_ss(d_tmem, ad, bd, idesc, (kb | kk) != 0);
             else mma_f16_ss(d_tmem, ad, bd, idesc, ((kb | kk) != 0) || chain_in);
           }
-          mma_commit(&empty_bar[s]);  // smem stage reusable once these MMAs have read it
+          commit(&empty_bar[s]);  // smem stage reusable once these MMAs have read it
         }
-        if (ok) mma_commit(&tfull_bar[buf]);  // accumulator complete
+        if (ok) commit(&tfull_bar[buf]);  // accumulator complete
       }
     }
   } else if (TP == 3 && warp >= 6) {
@@ -470,7 +498,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t bph = (lt >> 1) & 1;
       if (!mbar_wait(&tfull_bar[buf], bph, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      const long row = (long)tm * BM + q * 32 + lane;
+      const int row0 = tm * TM + half * BM + q * 32;  // first row of this warp
+      const long row = row0 + lane;
       const int col0 = tn * BN;
       // Software pipeline over 32-column chunks with two register buffers: the TMEM load of the next chunk is
       // in flight while the current one is converted and written to this warp's staging slice
@@ -485,7 +514,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncwarp();
         if (lane == 0) {
           const uint32_t src = smem_u32(stage0 + (slice & 1) * 4096);
-          const int y = tm * BM + q * 32;
+          const int y = row0;
           if (EPI == EPI_F32_ACC) {
             asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                              reinterpret_cast<uint64_t>(tmc)),
@@ -582,7 +611,10 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_leader(&tempty_bar[buf]);
+        else mbar_arrive(&tempty_bar[buf]);
+      }
       if constexpr (TP == 2) {
         // this warp's 32 rows of the tile have been written into the next rank's memory: tell it
         if (lane == 0) {
@@ -598,11 +630,14 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   tc_fence_before();
-  __syncthreads();
+  // a pair ends together: until here the other CTA's loads, arrivals and products may still reach this one
+  if constexpr (PAIR) cluster_sync_all();
+  else __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && status) atomicExch(status, 1u);  // a bounded wait ran out
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
@@ -627,6 +662,62 @@ CUresult encode_2d(CUtensorMap* out, const void* ptr, uint64_t dim0, uint64_t di
   return fn(out, dt, 2, const_cast<void*>(ptr), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+// One tile per CTA pair (cluster of two): 256 rows x 256 columns, max_ctas / 2 persistent pairs.
+constexpr int PAIR_STAGES = 6;
+template <int EPI, bool A_MN, bool B_MN, bool I8 = false>
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N, int K, long ldc, long ldr,
+                uint32_t* status, int max_ctas, cudaStream_t stream, const float* scale_a = nullptr, const float* scale_b = nullptr) {
+  using L = SmemLayout<256, PAIR_STAGES, true>;
+  auto kern = gemm_tc05_kernel<256, PAIR_STAGES, A_MN, B_MN, EPI, I8, 0, TpNone, true>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    if (e != cudaSuccess) return (int)e;
+    attr_done = true;
+  }
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  const int pairs = (int)(tiles < max_ctas / 2 ? tiles : max_ctas / 2);
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 2;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = L::TOTAL;
+  cfg.stream = stream;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  const int group_m = 8;
+  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m, scale_a, scale_b,
+                                 status, TpNone{});
+}
+
+// Share of the chip's tensor-core time that goes into wanted products when tm x tn tiles of an M x N result run on `workers`:
+// the last wave's idle workers and the padding of ragged edges are the loss.
+double tile_efficiency(int M, int N, int tm, int tn, int workers) {
+  const long t = (long)((M + tm - 1) / tm) * ((N + tn - 1) / tn);
+  const long slots = (t + workers - 1) / workers * workers;
+  return (double)M * N / ((double)tm * tn * (double)slots);
+}
+// What a 128-column tile achieves of a 256-column one: it reads shared memory more often per product, and an MN-major
+// operand, whose panels come as 64-wide boxes, costs it more (the same products with both tiles: 1.18 times the time with two
+// K-major operands, 1.19 - 1.30 with an MN-major one).
+constexpr double NARROW = 0.84, NARROW_MN = 0.78;
+// Whether pairs take a product whose best single-CTA tiling has efficiency `single`. A pair reads each row of A and B from
+// shared memory half as often per product as two single CTAs and so runs PAIR_GAIN times as fast (back to back, single and
+// paired: 16384 x 3072 x 2048 149 and 140 us, 16384 x 11264 x 2048 543 and 508, 16384 x 128256 x 2048 6243 and 5680; data
+// gradient 16384 x 5632 x 2048 267 and 251, weight gradient 2048 x 5632 x 16384 302 and 280), but its tiles are twice as
+// large: it loses where they leave SMs idle, less than one wave of pairs above all, or pad more rows (1024 x 3072 x 2048: 30
+// and 32; 1111 x 4096 x 768: 24 and 32). With an MN-major operand the gain fades as the product grows and turns into a loss
+// (378 GFLOP 0.93 - 0.99 of the single time, 756 GFLOP 1.00, 8.6 TFLOP 1.06): pairs take those up to PAIR_MN_FLOPS.
+constexpr double PAIR_GAIN = 1.07, PAIR_MN_FLOPS = 5e11;
+bool pair_wins(int M, int N, int K, bool mn_major, int max_ctas, double single) {
+  const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  return N > 128 && tiles >= max_ctas / 2 && max_ctas >= 2 && (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) &&
+         PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
 }
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8 = false>
@@ -708,6 +799,15 @@ __global__ void tp_finish_kernel(const float* __restrict__ acc, const uint32_t* 
   }
 }
 
+template <int EPI>
+int launch_pair_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N,
+                      int K, long ldc, long ldr, uint32_t* status, int max_ctas, cudaStream_t s) {
+  if (!a_mn && !b_mn) return launch_pair<EPI, false, false>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+  if (!a_mn && b_mn) return launch_pair<EPI, false, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+  if (a_mn && b_mn) return launch_pair<EPI, true, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+  return launch_pair<EPI, true, false>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+}
+
 template <int BN, int STAGES, int EPI>
 int launch_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N,
                  int K, long ldc, long ldr, uint32_t* status, int max_ctas, cudaStream_t s) {
@@ -735,18 +835,13 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   const bool bf16_out = (epi == EPI_BF16 || epi == EPI_BF16_RES);
   if ((bf16_out && (ldc & 7)) || (!bf16_out && (ldc & 3)) || (epi == EPI_BF16_RES && (ldr & 7))) return -2;
   if (max_ctas <= 0) max_ctas = otb_sm_count();
-  // Tile width: the 256-wide tile is the more efficient one per tile; the 128-wide one wins when
-  // it fills the last wave of CTAs noticeably better.
-  int BN = 128;
-  if (N >= 256) {
-    const long t256 = (long)((M + 127) / 128) * ((N + 255) / 256);
-    const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
-    const double e256 = (double)t256 / (double)(((t256 + max_ctas - 1) / max_ctas) * max_ctas) *
-                        ((double)N / (double)(((N + 255) / 256) * 256));
-    const double e128 = 0.88 * (double)t128 / (double)(((t128 + max_ctas - 1) / max_ctas) * max_ctas) *
-                        ((double)N / (double)(((N + 127) / 128) * 128));
-    BN = e256 >= e128 ? 256 : 128;
-  }
+  // Tile shape: the 256-wide tile is the more efficient one per tile; the 128-wide one wins when it fills the last wave of
+  // CTAs noticeably better, the pair's 256 x 256 one when the product is large (pair_wins).
+  const bool mn_major = a_mn || b_mn;
+  const double e128 = (mn_major ? NARROW_MN : NARROW) * tile_efficiency(M, N, BM, 128, max_ctas);
+  const double e256 = N >= 256 ? tile_efficiency(M, N, BM, 256, max_ctas) : 0.0;
+  const int BN = e256 >= e128 ? 256 : 128;
+  const bool pair = pair_wins(M, N, K, mn_major, max_ctas, BN == 256 ? e256 : e128);
   CUtensorMap ta, tb;
   CUresult r;
   constexpr int BK = BK_BYTES / 2;
@@ -754,7 +849,7 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* C, const void* 
            : encode_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   r = b_mn ? encode_2d(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BK)
-           : encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, (uint32_t)BN);
+           : encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, (uint32_t)(pair ? 128 : BN));
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   CUtensorMap tc;
   r = bf16_out ? encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32, 2)
@@ -762,6 +857,15 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   if (reinterpret_cast<uintptr_t>(C) & 15) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (pair) {
+    switch (epi) {
+      case EPI_BF16: return launch_pair_major<EPI_BF16>(a_mn, b_mn, ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+      case EPI_F32: return launch_pair_major<EPI_F32>(a_mn, b_mn, ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+      case EPI_F32_ACC: return launch_pair_major<EPI_F32_ACC>(a_mn, b_mn, ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+      case EPI_BF16_RES: return launch_pair_major<EPI_BF16_RES>(a_mn, b_mn, ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s);
+      default: return -3;
+    }
+  }
 #define OTB_DISPATCH(BN_, ST_)                                                                                      \
   switch (epi) {                                                                                                    \
     case EPI_BF16: return launch_major<BN_, ST_, EPI_BF16>(a_mn, b_mn, ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s); \
@@ -796,15 +900,21 @@ extern "C" int otb_gemm_i8(const void* A, const void* B, void* C, const void* R,
   if (!scale_a || !scale_b) return -2;
   if (max_ctas <= 0) max_ctas = otb_sm_count();
   const int BN = N > 128 ? 256 : 128;
+  const bool pair = pair_wins(M, N, K, false, max_ctas, tile_efficiency(M, N, BM, BN, max_ctas));
   CUtensorMap ta, tb, tc;
   CUresult r = encode_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK_BYTES, BM, 1);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
-  r = encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK_BYTES, (uint32_t)BN, 1);
+  r = encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK_BYTES, (uint32_t)(pair ? 128 : BN), 1);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   r = bf16_out ? encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32, 2)
                : encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 32, 32, 4);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (pair) {
+    if (epi == EPI_BF16) return launch_pair<EPI_BF16, false, false, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s, scale_a, scale_b);
+    if (epi == EPI_F32) return launch_pair<EPI_F32, false, false, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s, scale_a, scale_b);
+    return launch_pair<EPI_BF16_RES, false, false, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s, scale_a, scale_b);
+  }
 #define OTB_I8(BN_, ST_, EPI_) \
   return launch<BN_, ST_, false, false, EPI_, true>(ta, tb, tc, C, R, M, N, K, ldc, ldr, status, max_ctas, s, scale_a, scale_b);
   if (BN == 256) {
