@@ -14,23 +14,26 @@ namespace {
 inline bool aligned16(const void* p, long ld) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(ld * 4)) & 15) == 0; }
 
 // ------------------------------------------------------------------------------ GEMM
-// TM x TN tile of C per CTA, RM x RN chains per thread, k-slabs of 16 double-buffered in shared memory as [k][row] (the
-// next slab travels through registers while this one is multiplied). The chains are independent, so the tile shape only
+// TM x TN tile of C per CTA, RM x RN chains per thread, k-slabs double-buffered in shared memory as [k][row] (the next
+// slabs travel through registers while this one is multiplied). The chains are independent, so the tile shape only
 // decides how many CTAs there are and how many shared-memory words a multiply-add costs:
 //   128 x 128 (8 x 8 per thread: 4 float4 per 64 multiply-adds), 64 x 64 and 32 x 32 (4 x 4: 2 per 16).
 // The rule takes the largest tile that still gives every SM a CTA (two for the 128-wide one, whose last wave costs most).
 // Bound by the serial chains of the few tiles a small product has, then by shared-memory words per multiply-add. A 2-layer,
 // 256-wide micro-batch of 4 x 512 tokens spent 5.1 ms in these products with one 64 x 64 tile shape, scalar shared-memory
-// reads and no overlap of load and multiply, 6.8 ms in attention; the whole pass went from 11.47 to 2.69 ms.
-constexpr int GK = 16;
-
+// reads and no overlap of load and multiply, 6.8 ms in attention; the whole pass went from 11.47 to 2.69 ms, and with the deeper fetch of the small tiles (and
+// cheaper launches) to 2.31.
 template <int TM, int TN, int RM, int RN>
 struct F32Tile {
   static constexpr int NT = (TM / RM) * (TN / RN);
+  // The small tiles have too few multiply-adds per slab to cover a load from L2 or DRAM (a 2048 x 256 x 768 product took 58 us
+  // with slabs of 16 fetched one ahead): they take slabs of 32 and fetch two ahead.
+  static constexpr int GK = TM >= 128 ? 16 : 32;
+  static constexpr int AHEAD = TM >= 128 ? 1 : 2;
 };
 
 // One operand's share of a k-slab, held in registers between the global load and the shared-memory store.
-template <int TR, int NT, bool MN>
+template <int TR, int NT, bool MN, int GK>
 struct Slab {
   static constexpr int PER = TR * GK / 4 / NT;  // float4 per thread
   static_assert(TR * GK / 4 % NT == 0, "the slab splits evenly over the CTA");
@@ -75,7 +78,8 @@ template <int TM, int TN, int RM, int RN, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(F32Tile<TM, TN, RM, RN>::NT)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
                 const float* __restrict__ R, int M, int N, int K, long lda, long ldb, long ldc, long ldr, int vec) {
-  constexpr int NT = F32Tile<TM, TN, RM, RN>::NT, GX = TN / RN;
+  using Tile = F32Tile<TM, TN, RM, RN>;
+  constexpr int NT = Tile::NT, GX = TN / RN, GK = Tile::GK, AHEAD = Tile::AHEAD;
   __shared__ __align__(16) float sa[2][GK][TM + 4], sb[2][GK][TN + 4];
   const int tx = threadIdx.x % GX, ty = threadIdx.x / GX;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
@@ -89,13 +93,17 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
     for (int j = 0; j < RN; ++j)
       // the accumulating epilogue continues the chain from the value already in C
       acc[i][j] = (EPI == 2 && mrow(i) < M && ncol(j) < N) ? C[(long)mrow(i) * ldc + ncol(j)] : 0.0f;
-  Slab<TM, NT, A_MN> la;
-  Slab<TN, NT, B_MN> lb;
+  Slab<TM, NT, A_MN, GK> la[AHEAD];
+  Slab<TN, NT, B_MN, GK> lb[AHEAD];
   const bool va = vec & 1, vb = vec & 2, vc = vec & 4;
-  la.load(A, lda, m0, M, 0, K, va);
-  lb.load(B, ldb, n0, N, 0, K, vb);
-  la.store(sa[0]);
-  lb.store(sb[0]);
+  la[0].load(A, lda, m0, M, 0, K, va);
+  lb[0].load(B, ldb, n0, N, 0, K, vb);
+  la[0].store(sa[0]);
+  lb[0].store(sb[0]);
+  if (AHEAD == 2) {
+    la[AHEAD - 1].load(A, lda, m0, M, GK, K, va);
+    lb[AHEAD - 1].load(B, ldb, n0, N, GK, K, vb);
+  }
   __syncthreads();
   auto step = [&](int buf, int k) {
     float a[RM], b[RN];
@@ -114,24 +122,27 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 #pragma unroll
       for (int j = 0; j < RN; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
   };
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += GK, buf ^= 1) {
-    const bool more = k0 + GK < K;
-    if (more) {
-      la.load(A, lda, m0, M, k0 + GK, K, va);
-      lb.load(B, ldb, n0, N, k0 + GK, K, vb);
-    }
-    if (k0 + GK <= K) {
+  for (int k00 = 0; k00 < K; k00 += 2 * GK) {
 #pragma unroll
-      for (int k = 0; k < GK; ++k) step(buf, k);
-    } else {  // the chain ends at K: no links of padding
-      for (int k = 0; k < K - k0; ++k) step(buf, k);
+    for (int u = 0; u < 2; ++u) {  // slab k0 / GK has parity u: so do its buffer and, two ahead, its registers
+      const int k0 = k00 + u * GK;
+      if (k0 >= K) break;
+      if (k0 + AHEAD * GK < K) {
+        la[AHEAD == 2 ? u : 0].load(A, lda, m0, M, k0 + AHEAD * GK, K, va);
+        lb[AHEAD == 2 ? u : 0].load(B, ldb, n0, N, k0 + AHEAD * GK, K, vb);
+      }
+      if (k0 + GK <= K) {
+#pragma unroll
+        for (int k = 0; k < GK; ++k) step(u, k);
+      } else {  // the chain ends at K: no links of padding
+        for (int k = 0; k < K - k0; ++k) step(u, k);
+      }
+      if (k0 + GK < K) {
+        la[AHEAD == 2 ? u ^ 1 : 0].store(sa[u ^ 1]);  // that buffer was last read before the barrier that ended the previous slab
+        lb[AHEAD == 2 ? u ^ 1 : 0].store(sb[u ^ 1]);
+      }
+      __syncthreads();
     }
-    if (more) {
-      la.store(sa[buf ^ 1]);  // that buffer was last read before the barrier that ended the previous slab
-      lb.store(sb[buf ^ 1]);
-    }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
