@@ -57,15 +57,28 @@ __global__ void absmax_final_kernel(const float* __restrict__ partial, int n, fl
   if (threadIdx.x == 0) out[0] = m;
 }
 
+// as many 256-thread CTAs as are resident at once, fewer where there is less to do
+inline unsigned quant_blocks(long n) { return (unsigned)min((long)blocks_for(n, 8 * 256), (long)otb_sm_count() * 8); }
+
 __device__ __forceinline__ float clamp_q(float q, float qmax) { return fminf(fmaxf(q, -qmax), qmax); }
 
+// The maximum is that of `parts` partial maxima: a resident CTA folds them itself (a few KB from L2, once) and then walks
+// its share of x, which spares a one-CTA launch between the two passes.
 template <typename T>
-__global__ void quant_act_kernel(const T* __restrict__ x, long n, const float* __restrict__ amax, float inv_qmax,
+__global__ void __launch_bounds__(256) quant_act_kernel(const T* __restrict__ x, long n, const float* __restrict__ amax, int parts, float inv_qmax,
                                  float qmax, int8_t* __restrict__ q, float* __restrict__ step_out) {
-  const float step = fmaxf(__fmul_rn(amax[0], inv_qmax), FLT_MIN);
+  __shared__ float sh[32];
+  float m = 0.0f;
+  for (int i = threadIdx.x; i < parts; i += blockDim.x) m = fmaxf(m, amax[i]);
+  m = block_max(m, sh);
+  const float step = fmaxf(__fmul_rn(m, inv_qmax), FLT_MIN);
   if (blockIdx.x == 0 && threadIdx.x == 0) step_out[0] = step;
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (i + 8 <= n) {
+  const long stride = (long)gridDim.x * blockDim.x * 8;
+  for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += stride) {
+    if (i + 8 > n) {
+      for (long j = i; j < n; ++j) q[j] = (int8_t)(int)clamp_q(rintf(__fdiv_rn(to_f<T>(x[j]), step)), qmax);
+      break;
+    }
     float f[8];
     Vec8<T>::load(x + i, f);
     uint32_t w[2] = {0, 0};
@@ -75,8 +88,6 @@ __global__ void quant_act_kernel(const T* __restrict__ x, long n, const float* _
       w[e >> 2] |= (uint32_t)(v & 0xFF) << (8 * (e & 3));
     }
     *reinterpret_cast<uint2*>(q + i) = make_uint2(w[0], w[1]);
-  } else {
-    for (long j = i; j < n; ++j) q[j] = (int8_t)(int)clamp_q(rintf(__fdiv_rn(to_f<T>(x[j]), step)), qmax);
   }
 }
 
@@ -103,11 +114,15 @@ __global__ void quant_weight_kernel(const T* __restrict__ w, const float* __rest
   }
 }
 
+// `mode` of the backward: the step size is learned; dW / ds hold nothing yet (the first micro-batch of a step): taken as zero
+// instead of being cleared by a pass of its own and read back.
+enum LsqMode : int { LSQ_LEARN = 1, LSQ_FRESH_W = 2, LSQ_FRESH_S = 4 };
 // one warp per row; G fp32 [N,K] (this micro-batch's dL/dw_hat before the activation step is applied)
 template <typename T>
 __global__ void lsq_bwd_kernel(const float* __restrict__ G, const T* __restrict__ w, const float* __restrict__ s,
                                const float* __restrict__ ga, long N, int K, float qmax, float gs,
-                               float* __restrict__ dW, float* __restrict__ ds, int learn_step) {
+                               float* __restrict__ dW, float* __restrict__ ds, int mode) {
+  const bool fresh = mode & LSQ_FRESH_W;
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= N) return;
@@ -119,7 +134,12 @@ __global__ void lsq_bwd_kernel(const float* __restrict__ G, const T* __restrict_
     Vec8<T>::load(w + row * K + c, f);
     float g[8], d[8];
     Vec8<float>::load(G + row * K + c, g);
-    Vec8<float>::load(dW + row * K + c, d);
+    if (fresh) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) d[e] = 0.0f;
+    } else {
+      Vec8<float>::load(dW + row * K + c, d);
+    }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const float t = __fdiv_rn(f[e], sr);
@@ -131,9 +151,9 @@ __global__ void lsq_bwd_kernel(const float* __restrict__ G, const T* __restrict_
     }
     Vec8<float>::store(dW + row * K + c, d);
   }
-  if (learn_step) {
+  if (mode & LSQ_LEARN) {
     const float tot = warp_butterfly(acc);
-    if (lane == 0) ds[row] = __fadd_rn(ds[row], __fmul_rn(tot, gs));
+    if (lane == 0) ds[row] = __fadd_rn(mode & LSQ_FRESH_S ? 0.0f : ds[row], __fmul_rn(tot, gs));
   }
 }
 
@@ -190,8 +210,17 @@ extern "C" int otb_absmax(const void* x, long n, int dtype, float* scratch, floa
 extern "C" int otb_quant_act(const void* x, long n, int dtype, const float* amax, int qmax, void* q, float* step,
                              void* stream) {
   if (n <= 0) return 0;
-  DISPATCH_T(dtype, quant_act_kernel<T><<<blocks_for(n, 8 * 256), 256, 0, S(stream)>>>(
-                        (const T*)x, n, amax, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);)
+  DISPATCH_T(dtype, quant_act_kernel<T><<<quant_blocks(n), 256, 0, S(stream)>>>(
+                        (const T*)x, n, amax, 1, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);)
+  return (int)cudaGetLastError();
+}
+// Both passes: absmax of x, then its quantisation. scratch: otb_absmax_scratch_floats() device floats.
+extern "C" int otb_absmax_quant_act(const void* x, long n, int dtype, float* scratch, int qmax, void* q, float* step, void* stream) {
+  if (n <= 0) return 0;
+  DISPATCH_T(dtype, {
+    absmax_partial_kernel<T><<<AMAX_BLOCKS, 256, 0, S(stream)>>>((const T*)x, n, scratch);
+    quant_act_kernel<T><<<quant_blocks(n), 256, 0, S(stream)>>>((const T*)x, n, scratch, AMAX_BLOCKS, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);
+  })
   return (int)cudaGetLastError();
 }
 // w [N,K] (dtype), s [N] fp32 -> q int8 [N,K] and, when w_hat is not null, w_hat = q*s in out_dtype. K % 8 == 0.
@@ -208,10 +237,10 @@ extern "C" int otb_quant_weight(const void* w, const float* s, long N, int K, in
   return (int)cudaGetLastError();
 }
 extern "C" int otb_lsq_bwd(const float* G, const void* w, const float* s, const float* ga, long N, int K, int dtype,
-                           int qmax, float gs, float* dW, float* ds, int learn_step, void* stream) {
+                           int qmax, float gs, float* dW, float* ds, int mode, void* stream) {
   if (K % 8) return -2;
   DISPATCH_T(dtype, lsq_bwd_kernel<T><<<blocks_for(N, 8), 256, 0, S(stream)>>>(G, (const T*)w, s, ga, N, K, (float)qmax,
-                                                                               gs, dW, ds, learn_step);)
+                                                                               gs, dW, ds, mode);)
   return (int)cudaGetLastError();
 }
 extern "C" int otb_row_stat(const void* w, long N, int K, int dtype, int mode, float c, float floor_v, float* s,
@@ -230,6 +259,7 @@ extern "C" int otb_i8_widen(const void* q, void* out, long n, int out_dtype, voi
 
 OTB_PACKED(otb_absmax)
 OTB_PACKED(otb_quant_act)
+OTB_PACKED(otb_absmax_quant_act)
 OTB_PACKED(otb_quant_weight)
 OTB_PACKED(otb_lsq_bwd)
 OTB_PACKED(otb_row_stat)

@@ -712,17 +712,15 @@ def _quant_weight_grads(G, w, step, sa, qmax_w, learn_step, slot_w, slot_s, w_dt
     N, Kd = w.shape
     gs = 1.0 / math.sqrt(float(Kd) * float(qmax_w))
     use_slot = slot_w is not None and slot_w.buf is not None
-    if use_slot:
-        slot_w.zero_if_first()
-    dW = slot_w.buf if use_slot else torch.zeros((N, Kd), dtype=torch.float32, device=w.device)
-    ds, s_slot = None, False
+    fresh_w = slot_w.take() if use_slot else True
+    dW = slot_w.buf if use_slot else torch.empty((N, Kd), dtype=torch.float32, device=w.device)
+    ds, s_slot, fresh_s = None, False, False
     if learn_step:
         s_slot = slot_s is not None and slot_s.buf is not None
-        if s_slot:
-            slot_s.zero_if_first()
-        ds = slot_s.buf if s_slot else torch.zeros(N, dtype=torch.float32, device=w.device)
+        fresh_s = slot_s.take() if s_slot else True
+        ds = slot_s.buf if s_slot else torch.empty(N, dtype=torch.float32, device=w.device)
     # a fixed (absmax) step never clips, so its mask bound is one grid point wider than the grid
-    K.lsq_bwd_(G, w, step, sa, qmax_w if learn_step else qmax_w + 1, gs, dW, ds)
+    K.lsq_bwd_(G, w, step, sa, qmax_w if learn_step else qmax_w + 1, gs, dW, ds, fresh_w, fresh_s)
     return (None if use_slot else dW.to(w_dtype)), (ds.to(s_dtype) if learn_step and not s_slot else None)
 
 

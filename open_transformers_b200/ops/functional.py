@@ -366,11 +366,16 @@ weight_epoch: int | None = None  # set (and bumped at every weight change) by th
 
 _absmax = packed_entry("otb_absmax", "6q")
 _quant_act = packed_entry("otb_quant_act", "8q")
+_absmax_quant_act = packed_entry("otb_absmax_quant_act", "8q")
 _quant_weight = packed_entry("otb_quant_weight", "10q")
 _gemm_i8 = packed_entry("otb_gemm_i8", "17q")
 _lsq_bwd = packed_entry("otb_lsq_bwd", "8qd4q")
 _row_stat = packed_entry("otb_row_stat", "5q2d2q")
 _i8_widen = packed_entry("otb_i8_widen", "5q")
+
+
+def _absmax_scratch() -> int:
+    return cuda_lib().otb_absmax_scratch_floats()
 
 
 def absmax(x: torch.Tensor) -> torch.Tensor:
@@ -379,8 +384,7 @@ def absmax(x: torch.Tensor) -> torch.Tensor:
     assert x.is_contiguous()
     out = torch.empty(1, dtype=torch.float32, device=x.device)
     if x.is_cuda:
-        lib = cuda_lib()
-        scratch = torch.empty(lib.otb_absmax_scratch_floats(), dtype=torch.float32, device=x.device)
+        scratch = torch.empty(_absmax_scratch(), dtype=torch.float32, device=x.device)
         check(_absmax(ptr(x), x.numel(), is_bf16(x), ptr(scratch), ptr(out), raw_stream()), "absmax")
     else:
         check(cpu_lib().otb_cpu_absmax(P(x), L(x.numel()), I(is_bf16(x)), P(out)), "absmax")
@@ -390,9 +394,13 @@ def absmax(x: torch.Tensor) -> torch.Tensor:
 def quant_act(x: torch.Tensor, qmax: int):
     """Per-tensor symmetric quantisation: step = max|x| / qmax, q = clamp(rint(x / step)). Returns (q int8, step[1])."""
     assert x.is_contiguous()
-    am = absmax(x)
     q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
     step = torch.empty(1, dtype=torch.float32, device=x.device)
+    if x.is_cuda and x.numel() > 0:
+        scratch = torch.empty(_absmax_scratch(), dtype=torch.float32, device=x.device)
+        check(_absmax_quant_act(ptr(x), x.numel(), is_bf16(x), ptr(scratch), qmax, ptr(q), ptr(step), raw_stream()), "quant_act")
+        return q, step
+    am = absmax(x)
     if x.is_cuda:
         check(_quant_act(ptr(x), x.numel(), is_bf16(x), ptr(am), qmax, ptr(q), ptr(step), raw_stream()), "quant_act")
     else:
@@ -447,15 +455,20 @@ def gemm_i8(aq: torch.Tensor, bq: torch.Tensor, sa: torch.Tensor, sb: torch.Tens
 
 
 def lsq_bwd_(G: torch.Tensor, w: torch.Tensor, s: torch.Tensor, ga: torch.Tensor | None, qmax: int, gs: float,
-             dW: torch.Tensor, ds: torch.Tensor | None) -> None:
+             dW: torch.Tensor, ds: torch.Tensor | None, fresh_w: bool = False, fresh_s: bool = False) -> None:
     """Straight-through backward of the learned step size, accumulating into ``dW`` [N,K] and ``ds`` [N] (fp32):
+    ``fresh_w`` / ``fresh_s``: the buffer's contents are stale and count as zero.
     ``dW += inside ? G*ga : 0``, ``ds += gs * sum_k G*ga * (inside ? rint(t)-t : sign(t) qmax)`` with t = w/s."""
     N, Kd = w.shape
     assert G.dtype == torch.float32 and G.is_contiguous() and dW.dtype == torch.float32 and dW.is_contiguous()
     learn = ds is not None
     if w.is_cuda:
-        check(_lsq_bwd(ptr(G), ptr(w), ptr(s), ptr(ga), N, Kd, is_bf16(w), qmax, gs, ptr(dW), ptr(ds), learn, raw_stream()), "lsq_bwd")
+        check(_lsq_bwd(ptr(G), ptr(w), ptr(s), ptr(ga), N, Kd, is_bf16(w), qmax, gs, ptr(dW), ptr(ds), learn | fresh_w << 1 | fresh_s << 2, raw_stream()), "lsq_bwd")
     else:
+        if fresh_w:
+            dW.zero_()
+        if fresh_s and learn:
+            ds.zero_()
         check(cpu_lib().otb_cpu_lsq_bwd(P(G), P(w), P(s), P(ga), L(N), I(Kd), I(is_bf16(w)), I(qmax), F(gs), P(dW), P(ds), I(learn)), "lsq_bwd")
 
 
