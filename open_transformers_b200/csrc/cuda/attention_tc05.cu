@@ -74,6 +74,15 @@ struct BarsX : Bars {
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
+// The bf16 kernels are persistent, one CTA per SM: every role walks the same list of work items, barrier phases and ring
+// positions running on, so the loads and first products of an item are under way while the previous one's results are read
+// out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about 8 us, were
+// exposed: a quarter of an item's time with a 512-key window. 4 x 4096 tokens, 16 heads x 128, forward and backward: 1790 ->
+// 1612 us full causal, 744 -> 691 us windowed.) Item r * gridDim + c of the list goes to CTA c in even rounds
+// r and to the mirrored CTA in odd ones; the list is sorted by falling work, so the sums come out even.
+__device__ __forceinline__ int work_item(int round) {
+  return round * (int)gridDim.x + (round & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+}
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
@@ -410,7 +419,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
 constexpr int F2_THREADS = 64 + 256;
 
 struct Bars2 {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done[2];
+  uint64_t q_full, q_empty, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done[2];
   uint32_t tmem_slot;
   uint32_t abort_flag;
 };
@@ -418,7 +427,7 @@ struct Bars2 {
 template <int D>
 __global__ void __launch_bounds__(F2_THREADS, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV,
-                 __nv_bfloat16* __restrict__ O, long ldo, float* __restrict__ lse_out, int T, int H, int Hkv, int window,
+                 __nv_bfloat16* __restrict__ O, long ldo, float* __restrict__ lse_out, int B, int T, int H, int Hkv, int window,
                  float c_log2, uint32_t* __restrict__ status) {
   constexpr int TILE = BQ * D * 2;
   constexpr int ST = 2;
@@ -431,22 +440,35 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = (T + BQ - 1) / BQ;
-  const int pr = (int)gridDim.x - 1 - (int)((blockIdx.x + g_attn_rotation) % gridDim.x);  // heavy pairs first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int g = h / (H / Hkv);
-  const int tile0 = 2 * pr;
-  const bool hasB = tile0 + 1 < nq;
-  // key-block range [jlo_X, jhi_X] of tile X; the CTA walks [jlo_A, jhi_B] (jlo_A <= jlo_B, jhi_A < jhi_B)
-  auto jlo_of = [&](int t) { const int q0 = t * BQ; return (window > 0 && q0 - window + 1 > 0) ? (q0 - window + 1) / BKV : 0; };
-  const int jloA = jlo_of(tile0), jhiA = tile0;
-  const int jloB = hasB ? jlo_of(tile0 + 1) : 0, jhiB = tile0 + 1;
-  const int jlo = jloA, jhi = hasB ? jhiB : jhiA;
-  const int n = jhi - jlo + 1;
-  auto act = [&](int X, int j) { return X == 0 ? (j <= jhiA) : (hasB && j >= jloB && j <= jhiB); };
+  const int nq = (T + BQ - 1) / BQ, npairs = (nq + 1) / 2, heads = B * H;
+  const int items = npairs * heads;
+  // Item -> pair of tiles (heavy pairs first), head, sequence, and the key blocks: [jlo_X, jhi_X] of tile X; the CTA walks
+  // [jlo_A, jhi_B] (jlo_A <= jlo_B, jhi_A < jhi_B)
+  struct Item {
+    int tile0, h, b, g, jlo, n, jhiA, jloB, jhiB;
+    bool hasB;
+    __device__ __forceinline__ bool act(int X, int j) const { return X == 0 ? j <= jhiA : (hasB && j >= jloB && j <= jhiB); }
+  };
+  auto item_of = [&](int w) {
+    Item it;
+    const int hb = w % heads;
+    it.tile0 = 2 * (npairs - 1 - (w / heads + g_attn_rotation) % npairs);
+    it.h = hb % H;
+    it.b = hb / H;
+    it.g = it.h / (H / Hkv);
+    it.hasB = it.tile0 + 1 < nq;
+    auto jlo_of = [&](int t) { const int q0 = t * BQ; return (window > 0 && q0 - window + 1 > 0) ? (q0 - window + 1) / BKV : 0; };
+    it.jlo = jlo_of(it.tile0);
+    it.jhiA = it.tile0;
+    it.jloB = it.hasB ? jlo_of(it.tile0 + 1) : 0;
+    it.jhiB = it.tile0 + 1;
+    it.n = (it.hasB ? it.jhiB : it.jhiA) - it.jlo + 1;
+    return it;
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
+    mbar_init(&bars->q_empty, 1);
     for (int s = 0; s < ST; ++s) {
       mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1); mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], 1);
     }
@@ -462,100 +484,104 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->q_full, hasB ? 2 * TILE : TILE);
-      load_tile<D>(sQ, &tmQK, &bars->q_full, h * D, tile0 * BQ, b);
-      if (hasB) load_tile<D>(sQ + TILE, &tmQK, &bars->q_full, h * D, (tile0 + 1) * BQ, b);
-      for (int i = 0; i < n; ++i) {
-        const int st = i % ST;
-        const uint32_t ph = (i / ST) & 1;
-        const int k0 = (jlo + i) * BKV;
-        if (!mbar_wait(&bars->k_empty[st], ph ^ 1, abort_flag)) break;
-        mbar_expect_tx(&bars->k_full[st], TILE);
-        load_tile<D>(sK + st * TILE, &tmQK, &bars->k_full[st], (H + g) * D, k0, b);
-        if (!mbar_wait(&bars->v_empty[st], ph ^ 1, abort_flag)) break;
-        mbar_expect_tx(&bars->v_full[st], TILE);
-        load_tile<D>(sV + st * TILE, &tmV, &bars->v_full[st], (H + Hkv + g) * D, k0, b);
+      uint32_t ring = 0;  // key blocks loaded so far
+      bool ok = true;
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const Item it = item_of(w);
+        if (!mbar_wait(&bars->q_empty, (round & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(&bars->q_full, it.hasB ? 2 * TILE : TILE);
+        load_tile<D>(sQ, &tmQK, &bars->q_full, it.h * D, it.tile0 * BQ, it.b);
+        if (it.hasB) load_tile<D>(sQ + TILE, &tmQK, &bars->q_full, it.h * D, (it.tile0 + 1) * BQ, it.b);
+        for (int i = 0; i < it.n; ++i, ++ring) {
+          const int st = ring % ST;
+          const uint32_t ph = (ring / ST) & 1;
+          const int k0 = (it.jlo + i) * BKV;
+          if (!(ok = mbar_wait(&bars->k_empty[st], ph ^ 1, abort_flag))) break;
+          mbar_expect_tx(&bars->k_full[st], TILE);
+          load_tile<D>(sK + st * TILE, &tmQK, &bars->k_full[st], (H + it.g) * D, k0, it.b);
+          if (!(ok = mbar_wait(&bars->v_empty[st], ph ^ 1, abort_flag))) break;
+          mbar_expect_tx(&bars->v_full[st], TILE);
+          load_tile<D>(sV + st * TILE, &tmV, &bars->v_full[st], (H + Hkv + it.g) * D, k0, it.b);
+        }
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idS = make_idesc(128, BKV, 0, 0);
       constexpr uint32_t idPV = make_idesc(128, D, 0, 1);
-      bool ok = mbar_wait(&bars->q_full, 0, abort_flag);
-      int done[2] = {0, 0};  // P V products issued per tile
-      // S of block i for every tile that takes part in it; frees the K stage afterwards
-      auto issue_S = [&](int i) {
-        const int st = i % ST;
-        if (!mbar_wait(&bars->k_full[st], (i / ST) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t aK = smem_u32(sK + st * TILE);
-        for (int X = 0; X < 2; ++X) {
-          if (!act(X, jlo + i)) continue;
-          const uint32_t aQ = smem_u32(sQ + X * TILE);
+      bool ok = true;
+      uint32_t ring = 0, parity[2] = {0, 0};  // key blocks before this item; P tiles consumed per tile
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const Item it = item_of(w);
+        const int n = it.n;
+        if (!(ok = mbar_wait(&bars->q_full, round & 1, abort_flag))) break;
+        bool first[2] = {true, true};
+        auto k_ready = [&](int i) { return mbar_wait(&bars->k_full[(ring + i) % ST], ((ring + i) / ST) & 1, abort_flag); };
+        // S of tile X (block i); K stage not released
+        auto issue_S1 = [&](int X, int i) {
+          const uint32_t aK = smem_u32(sK + ((ring + i) % ST) * TILE), aQ = smem_u32(sQ + X * TILE);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 128, desc_k(aQ, kk), desc_k(aK, kk), idS, kk != 0);
           mma_commit(&bars->s_full[X]);
-        }
-        mma_commit(&bars->k_empty[st]);
-        return true;
-      };
-      // S of tile X only (block i), K stage not released
-      auto issue_S1 = [&](int X, int i) {
-        const uint32_t aK = smem_u32(sK + (i % ST) * TILE), aQ = smem_u32(sQ + X * TILE);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 128, desc_k(aQ, kk), desc_k(aK, kk), idS, kk != 0);
-        mma_commit(&bars->s_full[X]);
-      };
-      if (ok) ok = issue_S(0);
-      for (int i = 0; i < n && ok; ++i) {
-        const int st = i % ST, j = jlo + i;
-        const bool more = i + 1 < n;
-        bool k_next = false;  // K of block i + 1 is in shared memory
-        for (int X = 0; X < 2 && ok; ++X) {
-          if (act(X, j)) {
-            if (!mbar_wait(&bars->p_ready[X], done[X] & 1, abort_flag)) { ok = false; break; }
-            if (!mbar_wait(&bars->v_full[st], (i / ST) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t aV = smem_u32(sV + st * TILE);
-#pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk)
-              mma_f16_ts(tmem + 256 + X * 128, tmem + X * 128 + kk * 8, desc_mn(aV, kk), idPV, (done[X] | kk) != 0);
-            ++done[X];
-            if (j == (X == 0 ? jhiA : jhiB)) mma_commit(&bars->o_done[X]);
-          }
-          // this tile's next S goes right behind its P V (it overwrites the P just consumed)
-          if (more && act(X, j + 1)) {
-            if (!k_next) {
-              if (!mbar_wait(&bars->k_full[(i + 1) % ST], ((i + 1) / ST) & 1, abort_flag)) { ok = false; break; }
+        };
+        if (!(ok = k_ready(0))) break;
+        tc_fence_after();
+        for (int X = 0; X < 2; ++X)
+          if (it.act(X, it.jlo)) issue_S1(X, 0);
+        mma_commit(&bars->k_empty[ring % ST]);
+        for (int i = 0; i < n && ok; ++i) {
+          const int st = (ring + i) % ST, j = it.jlo + i;
+          const bool more = i + 1 < n;
+          bool k_next = false;  // K of block i + 1 is in shared memory
+          for (int X = 0; X < 2 && ok; ++X) {
+            if (it.act(X, j)) {
+              if (!(ok = mbar_wait(&bars->p_ready[X], parity[X] & 1, abort_flag))) break;
+              ++parity[X];
+              if (!(ok = mbar_wait(&bars->v_full[st], ((ring + i) / ST) & 1, abort_flag))) break;
               tc_fence_after();
-              k_next = true;
+              const uint32_t aV = smem_u32(sV + st * TILE);
+#pragma unroll
+              for (int kk = 0; kk < BKV / 16; ++kk)
+                mma_f16_ts(tmem + 256 + X * 128, tmem + X * 128 + kk * 8, desc_mn(aV, kk), idPV, !first[X] || kk != 0);
+              first[X] = false;
+              if (j == (X == 0 ? it.jhiA : it.jhiB)) mma_commit(&bars->o_done[X]);
             }
-            issue_S1(X, i + 1);
+            // this tile's next S goes right behind its P V (it overwrites the P just consumed)
+            if (more && it.act(X, j + 1)) {
+              if (!k_next) {
+                if (!(ok = k_ready(i + 1))) break;
+                tc_fence_after();
+                k_next = true;
+              }
+              issue_S1(X, i + 1);
+            }
           }
+          if (!ok) break;
+          mma_commit(&bars->v_empty[st]);
+          if (more) mma_commit(&bars->k_empty[(ring + i + 1) % ST]);
+          if (i + 2 == n || n == 1) mma_commit(&bars->q_empty);  // the item's last scores are on their way
         }
-        if (!ok) break;
-        mma_commit(&bars->v_empty[st]);
-        if (more) mma_commit(&bars->k_empty[(i + 1) % ST]);
+        ring += n;
       }
     }
   } else {
     const int X = (warp - 2) >> 2;           // tile of this warp
     const int quad = warp & 3;               // TMEM lane quadrant this warp may touch
     const int r = quad * 32 + lane;          // row inside the tile == TMEM lane
-    const int q0 = (tile0 + X) * BQ;
-    const int qi = q0 + r;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     const uint32_t tS = tmem + X * 128 + lane_off, tO = tmem + 256 + X * 128 + lane_off;
-    const int jhiX = X == 0 ? jhiA : jhiB;
-    float m_run = -INFINITY, l_run[NSPLIT] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int cnt = 0;
+    uint32_t scores = 0, outputs = 0;  // score tiles and results of this tile so far (barrier phases)
     bool ok = true;
-    if (X == 0 || hasB) {
-      for (int i = 0; i < n && ok; ++i) {
-        const int j = jlo + i;
-        if (!act(X, j)) continue;
+    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      const Item it = item_of(w);
+      if (X == 1 && !it.hasB) continue;
+      const int q0 = (it.tile0 + X) * BQ, qi = q0 + r, h = it.h, b = it.b;
+      const int jloX = X == 0 ? it.jlo : it.jloB, jhiX = X == 0 ? it.jhiA : it.jhiB;
+      float m_run = -INFINITY, l_run[NSPLIT] = {0.0f, 0.0f, 0.0f, 0.0f};
+      for (int j = jloX; j <= jhiX && ok; ++j) {
         const bool need_mask = (j == jhiX) || (window > 0 && j * BKV < q0 + BQ - window);
-        if (!mbar_wait(&bars->s_full[X], cnt & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(&bars->s_full[X], scores & 1, abort_flag)) { ok = false; break; }
+        ++scores;
         tc_fence_after();
         // pass 1: row maximum. Fully visible blocks take the unrolled path with the next 32 columns already in flight
         // while the current ones are reduced; blocks on the diagonal or the window edge take a compact loop.
@@ -587,7 +613,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
         const float m_safe = (m_new == -INFINITY) ? 0.0f : m_new;
         const float alpha = det_exp2_attn(__fadd_rn(m_run, -m_safe));
         // O row *= alpha (the previous P V is complete: its S product was issued behind it)
-        if (cnt > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+        if (j > jloX && __any_sync(0xffffffffu, alpha != 1.0f)) {
           const f2 a2 = pack2(alpha, alpha);
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
@@ -647,12 +673,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
         }
         tmem_st_wait();
         m_run = m_new;
-        ++cnt;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_ready[X]);
       }
-      ok = ok && mbar_wait(&bars->o_done[X], 0, abort_flag);
+      ok = ok && mbar_wait(&bars->o_done[X], outputs & 1, abort_flag);
+      ++outputs;
       tc_fence_after();
       if (ok) {
         const float l_tot = __fadd_rn(__fadd_rn(__fadd_rn(l_run[0], l_run[1]), l_run[2]), l_run[3]);
@@ -925,7 +951,7 @@ __device__ __forceinline__ uint64_t desc_mn_r(uint32_t base, int kk) {
 }
 
 struct BarsQ2 {
-  uint64_t qdo_full, kv_full[3], kv_empty[3], sdp_full[2], ds_ready[2], dq_done[2];
+  uint64_t qdo_full, qdo_empty, kv_full[3], kv_empty[3], sdp_full[2], ds_ready[2], dq_done[2];
   uint32_t tmem_slot;
   uint32_t abort_flag;
 };
@@ -934,7 +960,7 @@ template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmDO,
                    const __grid_constant__ CUtensorMap tmK64, const __grid_constant__ CUtensorMap tmV64,
-                   const float* __restrict__ lse, const float* __restrict__ delta, __nv_bfloat16* __restrict__ dQ, long lddq, int T,
+                   const float* __restrict__ lse, const float* __restrict__ delta, __nv_bfloat16* __restrict__ dQ, long lddq, int B, int T,
                    int H, int Hkv, int window, float scale, float c_log2, uint32_t* __restrict__ status) {
   constexpr int TILE = BQ * D * 2;    // a [128][D] query-side tile
   constexpr int KT = HK * D * 2;      // a [64][D] key-side tile
@@ -949,22 +975,35 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = (T + BQ - 1) / BQ;
-  const int pr = (int)gridDim.x - 1 - (int)((blockIdx.x + g_attn_rotation) % gridDim.x);
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int g = h / (H / Hkv);
-  const int tile0 = 2 * pr;
-  const bool hasB = tile0 + 1 < nq;
-  // 64-key steps [ulo_X, uhi_X] of tile X: every step that holds a key some row of the tile can see
-  auto ulo_of = [&](int t) { const int q0 = t * BQ; return (window > 0 && q0 - window + 1 > 0) ? (q0 - window + 1) / HK : 0; };
-  const int uloA = ulo_of(tile0), uhiA = 2 * tile0 + 1;
-  const int uloB = hasB ? ulo_of(tile0 + 1) : 0, uhiB = 2 * tile0 + 3;
-  const int ulo = uloA, uhi = hasB ? uhiB : uhiA;
-  const int n = uhi - ulo + 1;
-  auto act = [&](int X, int u) { return X == 0 ? (u <= uhiA) : (hasB && u >= uloB && u <= uhiB); };
+  const int nq = (T + BQ - 1) / BQ, npairs = (nq + 1) / 2, heads = B * H;
+  const int items = npairs * heads;
+  // Item -> pair of tiles (heavy pairs first), head, sequence, and the 64-key steps [ulo_X, uhi_X] of tile X: every step that
+  // holds a key some row of the tile can see
+  struct Item {
+    int tile0, h, b, g, ulo, n, uhiA, uloB, uhiB;
+    bool hasB;
+    __device__ __forceinline__ bool act(int X, int u) const { return X == 0 ? u <= uhiA : (hasB && u >= uloB && u <= uhiB); }
+  };
+  auto item_of = [&](int w) {
+    Item it;
+    const int hb = w % heads;
+    it.tile0 = 2 * (npairs - 1 - (w / heads + g_attn_rotation) % npairs);
+    it.h = hb % H;
+    it.b = hb / H;
+    it.g = it.h / (H / Hkv);
+    it.hasB = it.tile0 + 1 < nq;
+    auto ulo_of = [&](int t) { const int q0 = t * BQ; return (window > 0 && q0 - window + 1 > 0) ? (q0 - window + 1) / HK : 0; };
+    it.ulo = ulo_of(it.tile0);
+    it.uhiA = 2 * it.tile0 + 1;
+    it.uloB = it.hasB ? ulo_of(it.tile0 + 1) : 0;
+    it.uhiB = 2 * it.tile0 + 3;
+    it.n = (it.hasB ? it.uhiB : it.uhiA) - it.ulo + 1;
+    return it;
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->qdo_full, 1);
+    mbar_init(&bars->qdo_empty, 1);
     for (int s = 0; s < ST; ++s) { mbar_init(&bars->kv_full[s], 1); mbar_init(&bars->kv_empty[s], 1); }
     for (int x = 0; x < 2; ++x) { mbar_init(&bars->sdp_full[x], 1); mbar_init(&bars->ds_ready[x], 8); mbar_init(&bars->dq_done[x], 1); }
     bars->abort_flag = 0;
@@ -978,67 +1017,81 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->qdo_full, (hasB ? 4 : 2) * TILE);
-      for (int X = 0; X < (hasB ? 2 : 1); ++X) {
-        load_tile<D>(sQ + X * TILE, &tmQK, &bars->qdo_full, h * D, (tile0 + X) * BQ, b);
-        load_tile<D>(sDO + X * TILE, &tmDO, &bars->qdo_full, h * D, (tile0 + X) * BQ, b);
-      }
-      for (int i = 0; i < n; ++i) {
-        const int st = i % ST;
-        const int k0 = (ulo + i) * HK;
-        if (!mbar_wait(&bars->kv_empty[st], ((i / ST) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(&bars->kv_full[st], 2 * KT);
-        load_tile_r<D, HK>(sK + st * KT, &tmK64, &bars->kv_full[st], (H + g) * D, k0, b);
-        load_tile_r<D, HK>(sV + st * KT, &tmV64, &bars->kv_full[st], (H + Hkv + g) * D, k0, b);
+      uint32_t ring = 0;
+      bool ok = true;
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const Item it = item_of(w);
+        if (!mbar_wait(&bars->qdo_empty, (round & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(&bars->qdo_full, (it.hasB ? 4 : 2) * TILE);
+        for (int X = 0; X < (it.hasB ? 2 : 1); ++X) {
+          load_tile<D>(sQ + X * TILE, &tmQK, &bars->qdo_full, it.h * D, (it.tile0 + X) * BQ, it.b);
+          load_tile<D>(sDO + X * TILE, &tmDO, &bars->qdo_full, it.h * D, (it.tile0 + X) * BQ, it.b);
+        }
+        for (int i = 0; i < it.n; ++i, ++ring) {
+          const int st = ring % ST;
+          const int k0 = (it.ulo + i) * HK;
+          if (!(ok = mbar_wait(&bars->kv_empty[st], ((ring / ST) & 1) ^ 1, abort_flag))) break;
+          mbar_expect_tx(&bars->kv_full[st], 2 * KT);
+          load_tile_r<D, HK>(sK + st * KT, &tmK64, &bars->kv_full[st], (H + it.g) * D, k0, it.b);
+          load_tile_r<D, HK>(sV + st * KT, &tmV64, &bars->kv_full[st], (H + Hkv + it.g) * D, k0, it.b);
+        }
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idS = make_idesc(128, HK, 0, 0);  // S = Q K^T, dP = dO V^T: 128 x 64
       constexpr uint32_t idQ = make_idesc(128, D, 0, 1);   // dQ = dS K: A in tensor memory, B MN-major
-      bool ok = mbar_wait(&bars->qdo_full, 0, abort_flag);
-      int done[2] = {0, 0};
-      auto issue_sdp = [&](int X, int i) {
-        const uint32_t aK = smem_u32(sK + (i % ST) * KT), aV = smem_u32(sV + (i % ST) * KT);
-        const uint32_t aQ = smem_u32(sQ + X * TILE), aDO = smem_u32(sDO + X * TILE);
+      bool ok = true;
+      uint32_t ring = 0, parity[2] = {0, 0};  // key steps before this item; dS tiles consumed per tile
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const Item it = item_of(w);
+        const int n = it.n;
+        if (!(ok = mbar_wait(&bars->qdo_full, round & 1, abort_flag))) break;
+        bool first[2] = {true, true};
+        auto kv_ready = [&](int i) { return mbar_wait(&bars->kv_full[(ring + i) % ST], ((ring + i) / ST) & 1, abort_flag); };
+        auto issue_sdp = [&](int X, int i) {
+          const uint32_t aK = smem_u32(sK + ((ring + i) % ST) * KT), aV = smem_u32(sV + ((ring + i) % ST) * KT);
+          const uint32_t aQ = smem_u32(sQ + X * TILE), aDO = smem_u32(sDO + X * TILE);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 256, desc_k(aQ, kk), desc_k_r<HK>(aK, kk), idS, kk != 0);
+          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 256, desc_k(aQ, kk), desc_k_r<HK>(aK, kk), idS, kk != 0);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 256 + 64, desc_k(aDO, kk), desc_k_r<HK>(aV, kk), idS, kk != 0);
-        mma_commit(&bars->sdp_full[X]);
-      };
-      if (ok) ok = mbar_wait(&bars->kv_full[0], 0, abort_flag);
-      if (ok) {
+          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 256 + 64, desc_k(aDO, kk), desc_k_r<HK>(aV, kk), idS, kk != 0);
+          mma_commit(&bars->sdp_full[X]);
+        };
+        if (!(ok = kv_ready(0))) break;
         tc_fence_after();
         for (int X = 0; X < 2; ++X)
-          if (act(X, ulo)) issue_sdp(X, 0);
-      }
-      for (int i = 0; i < n && ok; ++i) {
-        const int st = i % ST, u = ulo + i;
-        const bool more = i + 1 < n;
-        bool kv_next = false;
-        for (int X = 0; X < 2 && ok; ++X) {
-          if (act(X, u)) {
-            if (!mbar_wait(&bars->ds_ready[X], done[X] & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t aK = smem_u32(sK + st * KT);
-#pragma unroll
-            for (int kk = 0; kk < HK / 16; ++kk)
-              mma_f16_ts(tmem + X * 256 + 128, tmem + X * 256 + (kk >> 1) * 32 + (kk & 1) * 8, desc_mn_r<HK>(aK, kk), idQ, (done[X] | kk) != 0);
-            ++done[X];
-            if (u == (X == 0 ? uhiA : uhiB)) mma_commit(&bars->dq_done[X]);
-          }
-          if (more && act(X, u + 1)) {
-            if (!kv_next) {
-              if (!mbar_wait(&bars->kv_full[(i + 1) % ST], ((i + 1) / ST) & 1, abort_flag)) { ok = false; break; }
+          if (it.act(X, it.ulo)) issue_sdp(X, 0);
+        for (int i = 0; i < n && ok; ++i) {
+          const int st = (ring + i) % ST, u = it.ulo + i;
+          const bool more = i + 1 < n;
+          bool kv_next = false;
+          for (int X = 0; X < 2 && ok; ++X) {
+            if (it.act(X, u)) {
+              if (!(ok = mbar_wait(&bars->ds_ready[X], parity[X] & 1, abort_flag))) break;
+              ++parity[X];
               tc_fence_after();
-              kv_next = true;
+              const uint32_t aK = smem_u32(sK + st * KT);
+#pragma unroll
+              for (int kk = 0; kk < HK / 16; ++kk)
+                mma_f16_ts(tmem + X * 256 + 128, tmem + X * 256 + (kk >> 1) * 32 + (kk & 1) * 8, desc_mn_r<HK>(aK, kk), idQ, !first[X] || kk != 0);
+              first[X] = false;
+              if (u == (X == 0 ? it.uhiA : it.uhiB)) mma_commit(&bars->dq_done[X]);
             }
-            issue_sdp(X, i + 1);
+            if (more && it.act(X, u + 1)) {
+              if (!kv_next) {
+                if (!(ok = kv_ready(i + 1))) break;
+                tc_fence_after();
+                kv_next = true;
+              }
+              issue_sdp(X, i + 1);
+            }
           }
+          if (!ok) break;
+          mma_commit(&bars->kv_empty[st]);
+          if (i + 2 == n || n == 1) mma_commit(&bars->qdo_empty);  // the item's last scores are on their way
         }
-        if (!ok) break;
-        mma_commit(&bars->kv_empty[st]);
+        ring += n;
       }
     }
   } else {
@@ -1047,23 +1100,24 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
     const int quad = warp & 3;
     const int hf = ((warp - 2) & 7) >> 2;    // which half of the step's keys
     const int r = quad * 32 + lane;
-    const int q0 = (tile0 + X) * BQ;
-    const int qi = q0 + r;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     const uint32_t tS = tmem + X * 256 + lane_off + hf * 32, tDP = tS + 64, tDQ = tmem + X * 256 + 128 + lane_off;
-    const bool row_ok = qi < T;
+    uint32_t scores = 0, outputs = 0;  // score tiles and results of this tile so far (barrier phases)
     bool ok = true;
-    if (X == 0 || hasB) {
+    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      const Item it = item_of(w);
+      if (X == 1 && !it.hasB) continue;
+      const int q0 = (it.tile0 + X) * BQ, qi = q0 + r, h = it.h, b = it.b;
+      const bool row_ok = qi < T;
       const float lse_r = row_ok ? lse[((long)b * H + h) * T + qi] : 0.0f;
       const float dl_r = row_ok ? delta[((long)b * H + h) * T + qi] : 0.0f;
-      int cnt = 0;
-      for (int i = 0; i < n && ok; ++i) {
-        const int u = ulo + i;
-        if (!act(X, u)) continue;
+      const int uloX = X == 0 ? it.ulo : it.uloB, uhiX = X == 0 ? it.uhiA : it.uhiB;
+      for (int u = uloX; u <= uhiX && ok; ++u) {
         const int k0 = u * HK;
         // some (row, key) pair of this step is hidden, or the tile has rows past the end of the sequence
         const bool need_mask = (k0 + HK - 1 > q0) || (window > 0 && k0 <= q0 + BQ - 1 - window) || (q0 + BQ > T);
-        if (!mbar_wait(&bars->sdp_full[X], cnt & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(&bars->sdp_full[X], scores & 1, abort_flag)) { ok = false; break; }
+        ++scores;
         tc_fence_after();
         // dS (bf16 pairs, 8 columns per 16 keys) goes over the thread's own score columns, which it has read by then
 #pragma unroll
@@ -1077,12 +1131,12 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
           tmem_st_32x32b_x8(tS + c * 8, pk);
         }
         tmem_st_wait();
-        ++cnt;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->ds_ready[X]);
       }
-      ok = ok && mbar_wait(&bars->dq_done[X], 0, abort_flag);
+      ok = ok && mbar_wait(&bars->dq_done[X], outputs & 1, abort_flag);
+      ++outputs;
       tc_fence_after();
       if (ok) {
         constexpr int DHALF = D / 2;
@@ -1124,7 +1178,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
 constexpr int KV2_ST = 4;
 
 struct BarsKV2 {
-  uint64_t kv_full, qdo_full[KV2_ST], qdo_empty[KV2_ST], sdp_full[2], pds_ready[2], acc_done;
+  uint64_t kv_full, kv_empty, qdo_full[KV2_ST], qdo_empty[KV2_ST], sdp_full[2], pds_ready[2], acc_done;
   uint32_t tmem_slot;
   uint32_t abort_flag;
 };
@@ -1162,7 +1216,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV,
                     const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmDO64,
                     const float* __restrict__ nlse, const float* __restrict__ ndelta, __nv_bfloat16* __restrict__ dK, long lddk,
-                    __nv_bfloat16* __restrict__ dV, long lddv, int T, int H, int Hkv, int window, float scale, float c_log2,
+                    __nv_bfloat16* __restrict__ dV, long lddv, int B, int T, int H, int Hkv, int window, float scale, float c_log2,
                     uint32_t* __restrict__ status) {
   constexpr int TILE = BKV * D * 2;  // [128 keys][D]
   constexpr int QT = HK * D * 2;     // [64 queries][D]
@@ -1178,18 +1232,26 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb = (int)((blockIdx.x + g_attn_rotation) % gridDim.x), g = blockIdx.y, b = blockIdx.z;
-  const int G = H / Hkv;
-  const int k0 = kb * BKV;
-  const int nu = T / HK;  // query steps in the sequence
-  const int ulo = k0 / HK;
-  int uhi = nu - 1;
-  if (window > 0) uhi = min(uhi, (k0 + BKV - 1 + window - 1) / HK);
-  const int nqi = uhi - ulo + 1;  // query steps per head
-  const int n = G * nqi;
+  const int G = H / Hkv, nkb = (T + BKV - 1) / BKV, heads = B * Hkv;
+  const int items = nkb * heads;
+  // Item -> key block (the first ones are seen by the most queries), KV head, sequence, and the query steps per head
+  struct Item { int k0, g, b, ulo, nqi, n; };
+  auto item_of = [&](int w) {
+    Item it;
+    it.k0 = (w / heads + g_attn_rotation) % nkb * BKV;
+    it.g = w % heads % Hkv;
+    it.b = w % heads / Hkv;
+    it.ulo = it.k0 / HK;
+    int uhi = T / HK - 1;
+    if (window > 0) uhi = min(uhi, (it.k0 + BKV - 1 + window - 1) / HK);
+    it.nqi = uhi - it.ulo + 1;
+    it.n = G * it.nqi;
+    return it;
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
+    mbar_init(&bars->kv_empty, 1);
     for (int s = 0; s < ST; ++s) { mbar_init(&bars->qdo_full[s], 1); mbar_init(&bars->qdo_empty[s], 1); }
     for (int z = 0; z < 2; ++z) { mbar_init(&bars->sdp_full[z], 1); mbar_init(&bars->pds_ready[z], SOFTMAX_WARPS); }
     mbar_init(&bars->acc_done, 1);
@@ -1205,19 +1267,25 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->kv_full, 2 * TILE);
-      load_tile<D>(sK, &tmQK, &bars->kv_full, (H + g) * D, k0, b);
-      load_tile<D>(sV, &tmV, &bars->kv_full, (H + Hkv + g) * D, k0, b);
-      for (int i = 0; i < n; ++i) {
-        const int st = i % ST;
-        const int h = g * G + i / nqi;
-        const int q0 = (ulo + i % nqi) * HK;
-        if (!mbar_wait(&bars->qdo_empty[st], ((i / ST) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(&bars->qdo_full[st], 2 * QT + 2 * HK * 4);
-        load_tile_r<D, HK>(sQ + st * QT, &tmQ64, &bars->qdo_full[st], h * D, q0, b);
-        load_tile_r<D, HK>(sDO + st * QT, &tmDO64, &bars->qdo_full[st], h * D, q0, b);
-        bulk_load(sStat + st * 2 * HK, nlse + ((long)b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
-        bulk_load(sStat + st * 2 * HK + HK, ndelta + ((long)b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
+      uint32_t step = 0;  // query steps loaded so far
+      bool ok = true;
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const Item it = item_of(w);
+        if (!mbar_wait(&bars->kv_empty, (round & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(&bars->kv_full, 2 * TILE);
+        load_tile<D>(sK, &tmQK, &bars->kv_full, (H + it.g) * D, it.k0, it.b);
+        load_tile<D>(sV, &tmV, &bars->kv_full, (H + Hkv + it.g) * D, it.k0, it.b);
+        for (int i = 0; i < it.n; ++i, ++step) {
+          const int st = step % ST;
+          const int h = it.g * G + i / it.nqi;
+          const int q0 = (it.ulo + i % it.nqi) * HK;
+          if (!(ok = mbar_wait(&bars->qdo_empty[st], ((step / ST) & 1) ^ 1, abort_flag))) break;
+          mbar_expect_tx(&bars->qdo_full[st], 2 * QT + 2 * HK * 4);
+          load_tile_r<D, HK>(sQ + st * QT, &tmQ64, &bars->qdo_full[st], h * D, q0, it.b);
+          load_tile_r<D, HK>(sDO + st * QT, &tmDO64, &bars->qdo_full[st], h * D, q0, it.b);
+          bulk_load(sStat + st * 2 * HK, nlse + ((long)it.b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
+          bulk_load(sStat + st * 2 * HK + HK, ndelta + ((long)it.b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
+        }
       }
     }
   } else if (warp == 1) {
@@ -1225,35 +1293,44 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
       constexpr uint32_t idS = make_idesc(128, HK, 0, 0);  // S^T = K Q^T, dP^T = V dO^T: 128 keys x 64 queries
       constexpr uint32_t idG = make_idesc(128, D, 0, 1);   // dV = P^T dO, dK = dS^T Q: A in tensor memory, B MN-major
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
-      bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
-      auto issue_sdp = [&](int i) {
-        const int st = i % ST, z = i & 1;
-        if (!mbar_wait(&bars->qdo_full[st], (i / ST) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
+      bool ok = true;
+      uint32_t step = 0;  // query steps before this item: their number decides stage, buffer and phases
+      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+        const int n = item_of(w).n;
+        if (!(ok = mbar_wait(&bars->kv_full, round & 1, abort_flag))) break;
+        auto issue_sdp = [&](int i) {
+          const uint32_t c = step + i;
+          const int st = c % ST, z = c & 1;
+          if (!mbar_wait(&bars->qdo_full[st], (c / ST) & 1, abort_flag)) return false;
+          tc_fence_after();
+          const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128, desc_k(aK, kk), desc_k_r<HK>(aQ, kk), idS, kk != 0);
+          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128, desc_k(aK, kk), desc_k_r<HK>(aQ, kk), idS, kk != 0);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128 + 64, desc_k(aV, kk), desc_k_r<HK>(aDO, kk), idS, kk != 0);
-        mma_commit(&bars->sdp_full[z]);
-        return true;
-      };
-      if (ok) ok = issue_sdp(0);
-      if (ok && n > 1) ok = issue_sdp(1);
-      for (int i = 0; i < n && ok; ++i) {
-        const int st = i % ST, z = i & 1;
-        if (!mbar_wait(&bars->pds_ready[z], (i >> 1) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
+          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128 + 64, desc_k(aV, kk), desc_k_r<HK>(aDO, kk), idS, kk != 0);
+          mma_commit(&bars->sdp_full[z]);
+          if (i + 1 == n) mma_commit(&bars->kv_empty);  // the item's last scores are on their way
+          return true;
+        };
+        ok = issue_sdp(0);
+        if (ok && n > 1) ok = issue_sdp(1);
+        for (int i = 0; i < n && ok; ++i) {
+          const uint32_t c = step + i;
+          const int st = c % ST, z = c & 1;
+          if (!(ok = mbar_wait(&bars->pds_ready[z], (c >> 1) & 1, abort_flag))) break;
+          tc_fence_after();
+          const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
 #pragma unroll
-        for (int kk = 0; kk < HK / 16; ++kk)
-          mma_f16_ts(tDV, tBuf + z * 128 + kk * 16, desc_mn_r<HK>(aDO, kk), idG, (i | kk) != 0);
+          for (int kk = 0; kk < HK / 16; ++kk)
+            mma_f16_ts(tDV, tBuf + z * 128 + kk * 16, desc_mn_r<HK>(aDO, kk), idG, (i | kk) != 0);
 #pragma unroll
-        for (int kk = 0; kk < HK / 16; ++kk)
-          mma_f16_ts(tDK, tBuf + z * 128 + 64 + kk * 16, desc_mn_r<HK>(aQ, kk), idG, (i | kk) != 0);
-        mma_commit(&bars->qdo_empty[st]);
-        if (i + 1 == n) mma_commit(&bars->acc_done);
-        if (i + 2 < n) { if (!issue_sdp(i + 2)) { ok = false; break; } }  // into the buffer just consumed
+          for (int kk = 0; kk < HK / 16; ++kk)
+            mma_f16_ts(tDK, tBuf + z * 128 + 64 + kk * 16, desc_mn_r<HK>(aQ, kk), idG, (i | kk) != 0);
+          mma_commit(&bars->qdo_empty[st]);
+          if (i + 1 == n) mma_commit(&bars->acc_done);
+          if (i + 2 < n) ok = issue_sdp(i + 2);  // into the buffer just consumed
+        }
+        step += n;
       }
     }
   } else {
@@ -1261,61 +1338,66 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
     const int quad = warp & 3;
     const int cq = (warp - 2) >> 2;          // which 16 of the step's 64 queries
     const int r = quad * 32 + lane;          // key row == TMEM lane
-    const int kj = k0 + r;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    uint32_t step = 0;
     bool ok = true;
-    for (int i = 0; i < n && ok; ++i) {
-      const int st = i % ST, z = i & 1;
-      const int q0 = (ulo + i % nqi) * HK;
-      const int qbase = q0 + cq * 16;
-      // some (key, query) pair of the step is hidden
-      const bool need_mask = (k0 + BKV - 1 > q0) || (window > 0 && k0 <= q0 + HK - 1 - window);
-      if (!mbar_wait(&bars->qdo_full[st], (i / ST) & 1, abort_flag)) { ok = false; break; }  // the statistics are in shared memory
-      if (!mbar_wait(&bars->sdp_full[z], (i >> 1) & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t tSt = tBuf + z * 128 + cq * 16 + lane_off, tDPt = tSt + 64;
-      const float* nl = sStat + st * 2 * HK + cq * 16;
-      const float* nd = nl + HK;
-      uint32_t vs[16], vd[16], pk[8], dsr[8];
-      // (512-key window, 4 x 4096 tokens, 16 heads x 128: 222 -> 209 us against position tests in every pair of such a step)
-      const Seen sn = need_mask ? seen(k0 + quad * 32, k0 + quad * 32 + 31, qbase, qbase + 15, window) : VISIBLE;
-      if (sn == HIDDEN) {
+    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      const Item it = item_of(w);
+      const int k0 = it.k0, g = it.g, b = it.b, kj = k0 + r;
+      for (int i = 0; i < it.n && ok; ++i, ++step) {
+        const int st = step % ST, z = step & 1;
+        const int q0 = (it.ulo + i % it.nqi) * HK;
+        const int qbase = q0 + cq * 16;
+        // some (key, query) pair of the step is hidden
+        const bool need_mask = (k0 + BKV - 1 > q0) || (window > 0 && k0 <= q0 + HK - 1 - window);
+        if (!mbar_wait(&bars->qdo_full[st], (step / ST) & 1, abort_flag)) { ok = false; break; }  // the statistics are in shared memory
+        if (!mbar_wait(&bars->sdp_full[z], (step >> 1) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t tSt = tBuf + z * 128 + cq * 16 + lane_off, tDPt = tSt + 64;
+        const float* nl = sStat + st * 2 * HK + cq * 16;
+        const float* nd = nl + HK;
+        uint32_t vs[16], vd[16], pk[8], dsr[8];
+        // (512-key window, 4 x 4096 tokens, 16 heads x 128: 222 -> 209 us against position tests in every pair of such a step)
+        const Seen sn = need_mask ? seen(k0 + quad * 32, k0 + quad * 32 + 31, qbase, qbase + 15, window) : VISIBLE;
+        if (sn == HIDDEN) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) pk[e] = dsr[e] = 0u;
-      } else {
-        tmem_ld_32x32b_x16(tSt, vs);
-        tmem_ld_32x32b_x16(tDPt, vd);
-        tmem_ld_wait();
-        if (sn == MIXED) bwd_probs_t<true>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
-        else bwd_probs_t<false>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
-      }
-      tmem_st_32x32b_x8(tSt, pk);
-      tmem_st_32x32b_x8(tDPt, dsr);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->pds_ready[z]);
-    }
-    if (ok && mbar_wait(&bars->acc_done, 0, abort_flag)) {
-      tc_fence_after();
-      const bool in_range = kj < T;
-      __nv_bfloat16* dkrow = dK + ((long)b * T + kj) * lddk + (long)g * D + cq * DH;
-      __nv_bfloat16* dvrow = dV + ((long)b * T + kj) * lddv + (long)g * D + cq * DH;
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-#pragma unroll
-        for (int c = 0; c < DH / 16; ++c) {
-          uint32_t v[16];
-          tmem_ld_32x32b_x16((which ? tDK : tDV) + lane_off + cq * DH + c * 16, v);
+          for (int e = 0; e < 8; ++e) pk[e] = dsr[e] = 0u;
+        } else {
+          tmem_ld_32x32b_x16(tSt, vs);
+          tmem_ld_32x32b_x16(tDPt, vd);
           tmem_ld_wait();
-          if (in_range) {
-            uint4* dst = reinterpret_cast<uint4*>((which ? dkrow : dvrow) + c * 16);
+          if (sn == MIXED) bwd_probs_t<true>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
+          else bwd_probs_t<false>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
+        }
+        tmem_st_32x32b_x8(tSt, pk);
+        tmem_st_32x32b_x8(tDPt, dsr);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->pds_ready[z]);
+      }
+      ok = ok && mbar_wait(&bars->acc_done, round & 1, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        const bool in_range = kj < T;
+        __nv_bfloat16* dkrow = dK + ((long)b * T + kj) * lddk + (long)g * D + cq * DH;
+        __nv_bfloat16* dvrow = dV + ((long)b * T + kj) * lddv + (long)g * D + cq * DH;
 #pragma unroll
-            for (int w = 0; w < 2; ++w)
-              dst[w] = make_uint4(pack_bf16(__uint_as_float(v[8 * w]), __uint_as_float(v[8 * w + 1])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 2]), __uint_as_float(v[8 * w + 3])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 4]), __uint_as_float(v[8 * w + 5])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 6]), __uint_as_float(v[8 * w + 7])));
+        for (int which = 0; which < 2; ++which) {
+#pragma unroll
+          for (int c = 0; c < DH / 16; ++c) {
+            uint32_t v[16];
+            tmem_ld_32x32b_x16((which ? tDK : tDV) + lane_off + cq * DH + c * 16, v);
+            tmem_ld_wait();
+            if (in_range) {
+              uint4* dst = reinterpret_cast<uint4*>((which ? dkrow : dvrow) + c * 16);
+#pragma unroll
+              for (int w = 0; w < 2; ++w)
+                dst[w] = make_uint4(pack_bf16(__uint_as_float(v[8 * w]), __uint_as_float(v[8 * w + 1])),
+                                    pack_bf16(__uint_as_float(v[8 * w + 2]), __uint_as_float(v[8 * w + 3])),
+                                    pack_bf16(__uint_as_float(v[8 * w + 4]), __uint_as_float(v[8 * w + 5])),
+                                    pack_bf16(__uint_as_float(v[8 * w + 6]), __uint_as_float(v[8 * w + 7])));
+            }
           }
         }
       }
@@ -1470,6 +1552,9 @@ int set_smem(K kern, int bytes) {
 
 // qk: [B*T, ldqk] bf16 holding H query heads then Hkv key heads (width D each); qkv: [B*T, ldqkv] bf16 whose
 // value heads start at column (H + Hkv) * D; O: [B*T, ldo]; lse: [B, H, T] fp32. D in {64, 128}.
+// one CTA per SM, fewer when there are fewer items
+static inline unsigned persistent_grid(long items) { return (unsigned)(items < otb_sm_count() ? items : otb_sm_count()); }
+
 extern "C" int otb_set_attn_rotation(int rotation) {
   if (rotation < 0) return -2;
   return (int)cudaMemcpyToSymbol(g_attn_rotation, &rotation, sizeof(rotation));
@@ -1484,17 +1569,17 @@ extern "C" int otb_attn_fwd(const void* qk, long ldqk, const void* qkv, long ldq
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
   const int nq = (T + BQ - 1) / BQ;
-  dim3 grid((nq + 1) / 2, H, B);
+  const unsigned grid = persistent_grid((long)((nq + 1) / 2) * H * B);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (D == 128) {
     static int once = set_smem(attn_fwd2_kernel<128>, attn_fwd2_smem_bytes<128>());
     if (once) return once;
-    attn_fwd2_kernel<128><<<grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, T, H, Hkv, window,
+    attn_fwd2_kernel<128><<<grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                               c_log2, status);
   } else {
     static int once = set_smem(attn_fwd2_kernel<64>, attn_fwd2_smem_bytes<64>());
     if (once) return once;
-    attn_fwd2_kernel<64><<<grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, T, H, Hkv, window,
+    attn_fwd2_kernel<64><<<grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                             c_log2, status);
   }
   return (int)cudaGetLastError();
@@ -1555,7 +1640,9 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   r = encode_3d(&tv64, qkv, (uint64_t)ldqkv, (uint64_t)T, (uint64_t)B, (uint64_t)ldqkv, HK);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   const int nq = (T + BQ - 1) / BQ;
-  dim3 gkv((T + BKV - 1) / BKV, Hkv, B), gq((nq + 1) / 2, H, B);
+  const int nkb = (T + BKV - 1) / BKV;
+  const unsigned gq = persistent_grid((long)((nq + 1) / 2) * H * B), gkv2 = persistent_grid((long)nkb * Hkv * B);
+  const dim3 gkv(nkb, Hkv, B);
   const bool kv2 = T % HK == 0;  // the transposed dK/dV kernel walks whole 64-query steps
   const long plane = (long)B * H * T;
   CUtensorMap tq64, tdo64;
@@ -1571,12 +1658,12 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
                       set_smem(attn_bwd_q2_kernel<128>, attn_bwd_q2_smem_bytes<128>());
     if (once) return once;
     if (kv2)
-      attn_bwd_kv2_kernel<128><<<gkv, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s>>>(
-          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, T, H, Hkv, window, scale, c_log2, status);
+      attn_bwd_kv2_kernel<128><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s>>>(
+          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
     else
       attn_bwd_kv_kernel<128><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    attn_bwd_q2_kernel<128><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, T, H,
+    attn_bwd_q2_kernel<128><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                                                                   Hkv, window, scale, c_log2, status);
   } else {
     static int once = set_smem(attn_bwd_kv_kernel<64>, attn_bwd_smem_bytes<64>()) |
@@ -1584,12 +1671,12 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
                       set_smem(attn_bwd_q2_kernel<64>, attn_bwd_q2_smem_bytes<64>());
     if (once) return once;
     if (kv2)
-      attn_bwd_kv2_kernel<64><<<gkv, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s>>>(
-          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, T, H, Hkv, window, scale, c_log2, status);
+      attn_bwd_kv2_kernel<64><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s>>>(
+          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
     else
       attn_bwd_kv_kernel<64><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                  lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    attn_bwd_q2_kernel<64><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, T, H, Hkv,
+    attn_bwd_q2_kernel<64><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H, Hkv,
                                                                                 window, scale, c_log2, status);
   }
   return (int)cudaGetLastError();
