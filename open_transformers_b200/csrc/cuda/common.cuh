@@ -28,6 +28,20 @@ inline PFN_encodeTiled get_encode_tiled() {
   return fn;
 }
 
+// Encoding a tensor map is a driver call and needs a current context, which the runtime gives a thread only with its first
+// runtime call that needs one: a thread whose first device work is a product into memory that it already holds (autograd's
+// own thread, say) has none yet and gets CUDA_ERROR_INVALID_CONTEXT. It then takes its device's primary context and repeats.
+template <typename F>
+inline CUresult otb_encode(F encode) {
+  CUresult r = encode();
+  int dev = 0;
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) {
+    r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaFree(nullptr) == cudaSuccess) r = encode();
+  }
+  return r;
+}
+
 inline int otb_sm_count() {
   static int sm[64] = {0};
   int dev = 0;
