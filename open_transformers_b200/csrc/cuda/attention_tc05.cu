@@ -78,10 +78,10 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // positions running on, so the loads and first products of an item are under way while the previous one's results are read
 // out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about 8 us, were
 // exposed: a quarter of an item's time with a 512-key window. 4 x 4096 tokens, 16 heads x 128, forward and backward: 1790 ->
-// 1612 us full causal, 744 -> 691 us windowed.) Item r * gridDim + c of the list goes to CTA c in even rounds
+// 1612 us full causal, 744 -> 691 us windowed.) Item r * gridDim + c of the list goes to CTA c in even turns
 // r and to the mirrored CTA in odd ones; the list is sorted by falling work, so the sums come out even.
-__device__ __forceinline__ int work_item(int round) {
-  return round * (int)gridDim.x + (round & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+__device__ __forceinline__ int work_item(int turn) {
+  return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
@@ -486,9 +486,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
     if (elect_one()) {
       uint32_t ring = 0;  // key blocks loaded so far
       bool ok = true;
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const Item it = item_of(w);
-        if (!mbar_wait(&bars->q_empty, (round & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait(&bars->q_empty, (turn & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(&bars->q_full, it.hasB ? 2 * TILE : TILE);
         load_tile<D>(sQ, &tmQK, &bars->q_full, it.h * D, it.tile0 * BQ, it.b);
         if (it.hasB) load_tile<D>(sQ + TILE, &tmQK, &bars->q_full, it.h * D, (it.tile0 + 1) * BQ, it.b);
@@ -511,10 +511,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
       constexpr uint32_t idPV = make_idesc(128, D, 0, 1);
       bool ok = true;
       uint32_t ring = 0, parity[2] = {0, 0};  // key blocks before this item; P tiles consumed per tile
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const Item it = item_of(w);
         const int n = it.n;
-        if (!(ok = mbar_wait(&bars->q_full, round & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->q_full, turn & 1, abort_flag))) break;
         bool first[2] = {true, true};
         auto k_ready = [&](int i) { return mbar_wait(&bars->k_full[(ring + i) % ST], ((ring + i) / ST) & 1, abort_flag); };
         // S of tile X (block i); K stage not released
@@ -572,7 +572,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
     const uint32_t tS = tmem + X * 128 + lane_off, tO = tmem + 256 + X * 128 + lane_off;
     uint32_t scores = 0, outputs = 0;  // score tiles and results of this tile so far (barrier phases)
     bool ok = true;
-    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+    for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
       const Item it = item_of(w);
       if (X == 1 && !it.hasB) continue;
       const int q0 = (it.tile0 + X) * BQ, qi = q0 + r, h = it.h, b = it.b;
@@ -1019,9 +1019,9 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
     if (elect_one()) {
       uint32_t ring = 0;
       bool ok = true;
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const Item it = item_of(w);
-        if (!mbar_wait(&bars->qdo_empty, (round & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait(&bars->qdo_empty, (turn & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(&bars->qdo_full, (it.hasB ? 4 : 2) * TILE);
         for (int X = 0; X < (it.hasB ? 2 : 1); ++X) {
           load_tile<D>(sQ + X * TILE, &tmQK, &bars->qdo_full, it.h * D, (it.tile0 + X) * BQ, it.b);
@@ -1043,10 +1043,10 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
       constexpr uint32_t idQ = make_idesc(128, D, 0, 1);   // dQ = dS K: A in tensor memory, B MN-major
       bool ok = true;
       uint32_t ring = 0, parity[2] = {0, 0};  // key steps before this item; dS tiles consumed per tile
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const Item it = item_of(w);
         const int n = it.n;
-        if (!(ok = mbar_wait(&bars->qdo_full, round & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->qdo_full, turn & 1, abort_flag))) break;
         bool first[2] = {true, true};
         auto kv_ready = [&](int i) { return mbar_wait(&bars->kv_full[(ring + i) % ST], ((ring + i) / ST) & 1, abort_flag); };
         auto issue_sdp = [&](int X, int i) {
@@ -1104,7 +1104,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
     const uint32_t tS = tmem + X * 256 + lane_off + hf * 32, tDP = tS + 64, tDQ = tmem + X * 256 + 128 + lane_off;
     uint32_t scores = 0, outputs = 0;  // score tiles and results of this tile so far (barrier phases)
     bool ok = true;
-    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+    for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
       const Item it = item_of(w);
       if (X == 1 && !it.hasB) continue;
       const int q0 = (it.tile0 + X) * BQ, qi = q0 + r, h = it.h, b = it.b;
@@ -1269,9 +1269,9 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
     if (elect_one()) {
       uint32_t step = 0;  // query steps loaded so far
       bool ok = true;
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const Item it = item_of(w);
-        if (!mbar_wait(&bars->kv_empty, (round & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait(&bars->kv_empty, (turn & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(&bars->kv_full, 2 * TILE);
         load_tile<D>(sK, &tmQK, &bars->kv_full, (H + it.g) * D, it.k0, it.b);
         load_tile<D>(sV, &tmV, &bars->kv_full, (H + Hkv + it.g) * D, it.k0, it.b);
@@ -1295,9 +1295,9 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
       bool ok = true;
       uint32_t step = 0;  // query steps before this item: their number decides stage, buffer and phases
-      for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
         const int n = item_of(w).n;
-        if (!(ok = mbar_wait(&bars->kv_full, round & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->kv_full, turn & 1, abort_flag))) break;
         auto issue_sdp = [&](int i) {
           const uint32_t c = step + i;
           const int st = c % ST, z = c & 1;
@@ -1341,7 +1341,7 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     uint32_t step = 0;
     bool ok = true;
-    for (int round = 0, w; ok && (w = work_item(round)) < items; ++round) {
+    for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
       const Item it = item_of(w);
       const int k0 = it.k0, g = it.g, b = it.b, kj = k0 + r;
       for (int i = 0; i < it.n && ok; ++i, ++step) {
@@ -1376,7 +1376,7 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->pds_ready[z]);
       }
-      ok = ok && mbar_wait(&bars->acc_done, round & 1, abort_flag);
+      ok = ok && mbar_wait(&bars->acc_done, turn & 1, abort_flag);
       if (ok) {
         tc_fence_after();
         const bool in_range = kj < T;
