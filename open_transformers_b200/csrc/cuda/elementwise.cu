@@ -574,18 +574,62 @@ inline int swiglu_threads(int F) {
 // and the row is overwritten with d loss / d logits = e_i * k - onehot * scale, k = ((1 + 2 z lse) / s) * scale
 // (scale = 1 / (tokens * accum), host reciprocal; the label's element is fma(e, k, -scale)).
 // Rows with label < 0 are ignored: zero loss, zero gradient.
-// The row is read three times (maximum, sum, gradient) and only the first read should come from DRAM: the launch asks for
-// so much shared memory that the rows being worked on (CTAs per SM x SMs) stay inside two thirds of L2, and CE_UNROLL groups per
-// thread are in flight to make up for the fewer threads. (16384 rows of 128 256 bf16 logits took 2.41 ms with four CTAs per
-// SM and 152 MB of rows in work; head and loss together went from 23.89 to 23.49 ms.)
-constexpr int CE_THREADS = 512, CE_UNROLL = 4;
-template <typename T>
+// Bound by instructions, not by the three reads (the maximum of bf16 logits is taken two at a time as bf16, the exponent's clamp
+// is left out where it does nothing). UNROLL groups per thread are in flight: 4 for long rows (16384 rows of 128 256 bf16
+// logits with their gradient: 2435 -> 2147 us), 1 for rows of at most 8 sweeps (8192 rows of 8192: 130 -> 123 us), which the
+// wider loop's registers slow (140 us).
+constexpr int CE_THREADS = 512, CE_SWEEP = CE_THREADS * 8;
+template <typename T, int CE_UNROLL>
+__device__ __forceinline__ void ce_fetch(Raw8<T> (&raw)[CE_UNROLL], const T* __restrict__ xr, int c0, int V) {
+#pragma unroll
+  for (int u = 0; u < CE_UNROLL; ++u)
+    if (c0 + u * CE_SWEEP < V) raw[u].load(xr + c0 + u * CE_SWEEP);
+}
+// the thread's even and odd chains of sum e_i
+template <typename T, int CE_UNROLL, bool CLAMP>
+__device__ __forceinline__ tc05::f2 ce_sum(const T* __restrict__ xr, int V, tc05::f2 l2, tc05::f2 nm2) {
+  using namespace tc05;
+  Raw8<T> raw[CE_UNROLL];
+  f2 acc2 = pack2(0.0f, 0.0f);
+  for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * CE_SWEEP) {
+    ce_fetch(raw, xr, c0, V);
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u) {
+      if (c0 + u * CE_SWEEP >= V) break;
+      float f[8];
+      raw[u].unpack(f);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) acc2 = add2(acc2, exp2_acc2<CLAMP>(fma2(pack2(f[e], f[e + 1]), l2, nm2)));
+    }
+  }
+  return acc2;
+}
+// the thread's groups of the row become e_i * k; the owner of the label's group rewrites that one element
+template <typename T, int CE_UNROLL, bool CLAMP>
+__device__ __forceinline__ void ce_grad(T* __restrict__ xr, int V, tc05::f2 l2, tc05::f2 nm2, tc05::f2 k2, long label, float at_label) {
+  using namespace tc05;
+  Raw8<T> raw[CE_UNROLL];
+  for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * CE_SWEEP) {
+    ce_fetch(raw, xr, c0, V);
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u) {
+      const int c = c0 + u * CE_SWEEP;
+      if (c >= V) break;
+      float f[8], o[8];
+      raw[u].unpack(f);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) unpack2(mul2(exp2_acc2<CLAMP>(fma2(pack2(f[e], f[e + 1]), l2, nm2)), k2), o[e], o[e + 1]);
+      Vec8<T>::store(xr + c, o);
+      if (label >= c && label < c + 8) xr[label] = from_f<T>(at_label);
+    }
+  }
+}
+template <typename T, int CE_UNROLL>
 __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ logits, const long* __restrict__ labels,
                                                               float* __restrict__ ce_out, float* __restrict__ lse_out,
                                                               long rows, int V, float two_z, float scale, int write_grad) {
   using namespace tc05;
   __shared__ float sh[32];
-  constexpr int SWEEP = CE_THREADS * 8;
   const long row = blockIdx.x;
   T* xr = logits + row * V;
   const long label = labels[row];
@@ -593,27 +637,21 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
     if (threadIdx.x == 0) { ce_out[row] = 0.0f; lse_out[row] = 0.0f; }
     if (write_grad) {
       float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int c = threadIdx.x * 8; c < V; c += SWEEP) Vec8<T>::store(xr + c, z);
+      for (int c = threadIdx.x * 8; c < V; c += CE_SWEEP) Vec8<T>::store(xr + c, z);
     }
     return;
   }
   const float x_label = to_f<T>(xr[label]);
-  Raw8<T> raw[CE_UNROLL];
-  auto fetch = [&](int c0) {
+  float mx = -INFINITY, mn = INFINITY;
+  {
+    Raw8<T> raw[CE_UNROLL];
+    for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * CE_SWEEP) {
+      ce_fetch(raw, xr, c0, V);
 #pragma unroll
-    for (int u = 0; u < CE_UNROLL; ++u)
-      if (c0 + u * SWEEP < V) raw[u].load(xr + c0 + u * SWEEP);
-  };
-  float mx = -INFINITY;
-  for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * SWEEP) {
-    fetch(c0);
-#pragma unroll
-    for (int u = 0; u < CE_UNROLL; ++u) {
-      if (c0 + u * SWEEP >= V) break;
-      float f[8];
-      raw[u].unpack(f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, f[e]);
+      for (int u = 0; u < CE_UNROLL; ++u) {
+        if (c0 + u * CE_SWEEP >= V) break;
+        raw[u].extremes(mx, mn);
+      }
     }
   }
   mx = block_max(mx, sh);
@@ -621,18 +659,10 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
   const f2 l2 = pack2(LOG2E, LOG2E);
   const float nm = -__fmul_rn(mx, LOG2E);
   const f2 nm2 = pack2(nm, nm);
-  f2 acc2 = pack2(0.0f, 0.0f);
-  for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * SWEEP) {
-    fetch(c0);
-#pragma unroll
-    for (int u = 0; u < CE_UNROLL; ++u) {
-      if (c0 + u * SWEEP >= V) break;
-      float f[8];
-      raw[u].unpack(f);
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) acc2 = add2(acc2, exp2_acc2(fma2(pack2(f[e], f[e + 1]), l2, nm2)));
-    }
-  }
+  // The exponent's clamp at -126 does nothing in a row whose smallest logit is above it (the exponent grows with the logit;
+  // a NaN or an infinity fails the test): such rows, all of them in practice, leave it out, one instruction in eight.
+  const bool inside = __syncthreads_and(__fmaf_rn(mn, LOG2E, nm) >= -126.0f);
+  const f2 acc2 = inside ? ce_sum<T, CE_UNROLL, false>(xr, V, l2, nm2) : ce_sum<T, CE_UNROLL, true>(xr, V, l2, nm2);
   float a0, a1;
   unpack2(acc2, a0, a1);
   const float s = block_tree_sum(__fadd_rn(a0, a1), sh);
@@ -645,26 +675,9 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
   __syncthreads();  // every thread has its copy of the label logit before anyone overwrites the row
   const float k = __fmul_rn(__fdiv_rn(__fmaf_rn(two_z, lse, 1.0f), s), scale);
   const f2 k2 = pack2(k, k);
-  for (int c0 = threadIdx.x * 8; c0 < V; c0 += CE_UNROLL * SWEEP) {
-    fetch(c0);
-#pragma unroll
-    for (int u = 0; u < CE_UNROLL; ++u) {
-      const int c = c0 + u * SWEEP;
-      if (c >= V) break;
-      float f[8], o[8];
-      raw[u].unpack(f);
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) unpack2(mul2(exp2_acc2(fma2(pack2(f[e], f[e + 1]), l2, nm2)), k2), o[e], o[e + 1]);
-      Vec8<T>::store(xr + c, o);
-      if (label >= c && label < c + 8)  // the owner of the label's group rewrites that one element
-        xr[label] = from_f<T>(__fmaf_rn(det_exp2_acc(__fmaf_rn(x_label, LOG2E, nm)), k, -scale));
-    }
-  }
-}
-// dynamic shared memory that leaves as many CTAs on an SM as their rows fit two thirds of L2 (one at least; four fill the SM anyway)
-inline int ce_smem(int V, int elem) {
-  const long rows = (80L << 20) / ((long)V * elem * otb_sm_count());
-  return rows >= 4 ? 0 : rows >= 3 ? 72 * 1024 : rows == 2 ? 100 * 1024 : 120 * 1024;
+  const float at_label = __fmaf_rn(det_exp2_acc(__fmaf_rn(x_label, LOG2E, nm)), k, -scale);
+  if (inside) ce_grad<T, CE_UNROLL, false>(xr, V, l2, nm2, k2, label, at_label);
+  else ce_grad<T, CE_UNROLL, true>(xr, V, l2, nm2, k2, label, at_label);
 }
 
 // sum (or sum of squares) of n floats: element i -> thread i % 1024, ascending fold, block_tree_sum.
@@ -829,12 +842,10 @@ extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long ro
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
-  const int smem = ce_smem(V, dtype ? 2 : 4);
-  DISPATCH_T(dtype, {
-    static int attr = cudaFuncSetAttribute(ce_zloss_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
-    if (attr) return attr;
-    ce_zloss_kernel<T><<<(unsigned)rows, CE_THREADS, smem, S(stream)>>>((T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);
-  })
+#define CE(U) \
+  DISPATCH_T(dtype, ce_zloss_kernel<T, U><<<(unsigned)rows, CE_THREADS, 0, S(stream)>>>((T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+  if (V <= 8 * CE_SWEEP) { CE(1) } else { CE(4) }
+#undef CE
   return (int)cudaGetLastError();
 }
 extern "C" int otb_det_sum(const float* x, long n, int mode, float post_scale, float* out, void* stream) {

@@ -44,6 +44,18 @@ template <> struct Vec8<float> {
 template <typename T> struct Raw8;
 template <> struct Raw8<__nv_bfloat16> {
   uint4 v;
+  // the larger of mx and the elements (numbers win over NaN), the smaller of mn and the elements (NaN wins)
+  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    __nv_bfloat162 b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
+    const __nv_bfloat162 hi = __hmax2(__hmax2(b[0], b[1]), __hmax2(b[2], b[3]));
+    const __nv_bfloat162 lo = __hmin2_nan(__hmin2_nan(b[0], b[1]), __hmin2_nan(b[2], b[3]));
+    mx = fmaxf(mx, fmaxf(__low2float(hi), __high2float(hi)));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(__low2float(lo)));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(__high2float(lo)));
+  }
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ void unpack(float (&f)[8]) const {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -56,6 +68,14 @@ template <> struct Raw8<__nv_bfloat16> {
 };
 template <> struct Raw8<float> {
   float4 a, b;
+  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      mx = fmaxf(mx, f[e]);
+      asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(f[e]));
+    }
+  }
   __device__ __forceinline__ void load(const float* p) {
     a = *reinterpret_cast<const float4*>(p);
     b = *reinterpret_cast<const float4*>(p + 4);

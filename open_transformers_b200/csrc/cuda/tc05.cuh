@@ -335,11 +335,16 @@ __device__ __forceinline__ f2 exp2_attn2(f2 y) {
   return pack2(__uint_as_float(e0), __uint_as_float(e1));
 }
 
-// det_exp2_acc (csrc/common/det_math.h) on two values at once: same operations, same bits
+// det_exp2_acc (csrc/common/det_math.h) on two values at once: same operations, same bits. CLAMP = false: the caller knows
+// that both are numbers of at least -126.
+template <bool CLAMP = true>
 __device__ __forceinline__ f2 exp2_acc2(f2 y) {
-  float y0, y1;
-  unpack2(y, y0, y1);
-  const f2 yc = pack2(fmaxf(y0, -126.0f), fmaxf(y1, -126.0f));
+  f2 yc = y;
+  if constexpr (CLAMP) {
+    float y0, y1;
+    unpack2(y, y0, y1);
+    yc = pack2(fmaxf(y0, -126.0f), fmaxf(y1, -126.0f));
+  }
   const f2 t = add2(yc, pack2(12582912.0f, 12582912.0f));
   const f2 kf = add2(t, pack2(-12582912.0f, -12582912.0f));
   const f2 r = fma2(kf, pack2(-1.0f, -1.0f), yc);

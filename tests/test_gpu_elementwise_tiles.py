@@ -80,3 +80,20 @@ def test_attention_row_groups(B, T, H, Hkv, D):
 
     for p, q in zip(run("cuda"), run("cpu")):
         _same(p, q, "attention")
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_loss_rows_with_far_values(dtype):
+    """Rows whose exponents reach the clamp, at its edge, or hold infinities, beside an ordinary one."""
+    V = 5000
+    x = torch.randn(5, V, generator=torch.Generator().manual_seed(9))
+    x[1] *= 100
+    x[2, 17] = -87.0 + float(x[2].max())
+    x[3, 4321] = -float("inf")
+    x[4, 1:] = -float("inf")
+    x = x.to(dtype)
+    labels = torch.tensor([1, 2, 17, 4, 0])
+    a, b = x.clone().cuda(), x.clone()
+    dev, host = K.ce_zloss_(a, labels.cuda(), 1e-4, 0.25), K.ce_zloss_(b, labels, 1e-4, 0.25)
+    for p, q in zip((*dev, a), (*host, b)):
+        _same(p, q, "loss")
