@@ -342,6 +342,13 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
       }
+      if constexpr (PAIR) {
+        // The commits that release the last stages arrive in both CTAs, and nothing else waits for them (the epilogue's
+        // barrier is another one, and arrivals of separate commits come in no stated order): each CTA takes them in before
+        // it ends, as if it were about to fill every stage once more. They are done long before the last epilogue is.
+        for (int d = 0; d < STAGES; ++d, ++it)
+          if (!mbar_wait(&empty_bar[it % STAGES], ((it / STAGES) & 1) ^ 1, abort_flag)) break;
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
@@ -630,7 +637,9 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   tc_fence_before();
-  // a pair ends together: until here the other CTA's loads, arrivals and products may still reach this one
+  // A pair ends together: until here the other CTA's loads, arrivals and products may still reach this one. After it none
+  // does: the products have read every load, both producers have seen every stage released, both epilogues every finished
+  // tile, and the epilogues' arrivals on the first CTA come before this barrier.
   if constexpr (PAIR) cluster_sync_all();
   else __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && status) atomicExch(status, 1u);  // a bounded wait ran out

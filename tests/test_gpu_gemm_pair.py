@@ -38,3 +38,21 @@ def test_int8_pairs(M, N, K_):
         assert torch.equal(K.gemm_i8(*dev, dtype).cpu(), K.gemm_i8(a, b, sa, sb, dtype))
     assert torch.equal(K.gemm_i8(*dev, torch.bfloat16, res.cuda()).cpu(), K.gemm_i8(a, b, sa, sb, torch.bfloat16, res))
     assert K.kernel_status("cuda") == 0
+
+
+# The shortest pipelines, one tile per pair and launches back to back: a pair has to leave nothing under way behind it (the
+# arrivals that release its last stages would land in the shared memory of the pair that follows). K of one step, of a ragged
+# last step, of one step less than the ring, of the whole ring and of one more.
+@pytest.mark.parametrize("K_", [64, 72, 320, 384, 448])
+def test_pairs_that_follow_one_another(K_):
+    g = torch.Generator().manual_seed(K_)
+    M, N = 2 * 256, 37 * 256  # 74 tiles: one per pair of 148 SMs
+    a, b = (torch.randn(r, K_, generator=g).bfloat16() for r in (M, N))
+    want = K.gemm(a, b, epi=K.EPI_STORE_F32)
+    ac, bc = a.cuda(), b.cuda()
+    outs = [torch.empty(M, N, device="cuda") for _ in range(8)]
+    for _ in range(25):
+        for out in outs:
+            K.gemm(ac, bc, epi=K.EPI_STORE_F32, out=out)
+    assert all(torch.equal(out.cpu(), want) for out in outs)
+    assert K.kernel_status("cuda") == 0
