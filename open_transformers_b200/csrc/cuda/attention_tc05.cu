@@ -41,9 +41,12 @@ using namespace tc05;
 
 namespace {
 
-// Launch-order permutation for the race tests: block x works as block (x + g_attn_rotation) mod gridDim.x. A block owns
+// Launch-order permutation for the race tests: block x works as block (x + g_attn_rotation) mod gridDim.x, and the persistent
+// kernels permute the tiles in their list of items the same way. A block owns
 // its query tile (or key block) and sums in a fixed order, so any rotation must give the same bytes (0 in production).
 __device__ int g_attn_rotation = 0;
+// index i of n under the permutation (unsigned: any rotation that the setter takes may be added)
+__device__ __forceinline__ int rotated(int i, int n) { return (int)(((unsigned)i + (unsigned)g_attn_rotation) % (unsigned)n); }
 
 constexpr int BQ = 128;   // query rows per tile
 constexpr int BKV = 128;  // keys per block
@@ -452,7 +455,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
   auto item_of = [&](int w) {
     Item it;
     const int hb = w % heads;
-    it.tile0 = 2 * (npairs - 1 - (w / heads + g_attn_rotation) % npairs);
+    it.tile0 = 2 * (npairs - 1 - rotated(w / heads, npairs));
     it.h = hb % H;
     it.b = hb / H;
     it.g = it.h / (H / Hkv);
@@ -987,7 +990,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   auto item_of = [&](int w) {
     Item it;
     const int hb = w % heads;
-    it.tile0 = 2 * (npairs - 1 - (w / heads + g_attn_rotation) % npairs);
+    it.tile0 = 2 * (npairs - 1 - rotated(w / heads, npairs));
     it.h = hb % H;
     it.b = hb / H;
     it.g = it.h / (H / Hkv);
@@ -1238,7 +1241,7 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   struct Item { int k0, g, b, ulo, nqi, n; };
   auto item_of = [&](int w) {
     Item it;
-    it.k0 = (w / heads + g_attn_rotation) % nkb * BKV;
+    it.k0 = rotated(w / heads, nkb) * BKV;
     it.g = w % heads % Hkv;
     it.b = w % heads / Hkv;
     it.ulo = it.k0 / HK;

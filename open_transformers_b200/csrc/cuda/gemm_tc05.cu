@@ -217,7 +217,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   }
   constexpr int BK = I8 ? BK_BYTES : BK_BYTES / 2;  // elements of K per k-block
-  const int cta = ((int)blockIdx.x / CTAS + g_cta_rotation) % nctas;  // which persistent worker this CTA (or pair) is
+  // which persistent worker this CTA (or pair) is (unsigned: any rotation that the setter takes may be added)
+  const int cta = (int)((blockIdx.x / CTAS + (unsigned)g_cta_rotation) % (unsigned)nctas);
   using L = SmemLayout<BN, STAGES, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

@@ -24,7 +24,7 @@ def test_many_items(B, T, H, Hkv, D, window):
 
     want = run("cpu")
     try:
-        for rotation in (0, 1):
+        for rotation in (0, 1, 2**31 - 1):  # (the last: the sum of item and rotation needs all 32 bits)
             assert cuda_lib().otb_set_attn_rotation(rotation) == 0
             for got, ref in zip(run("cuda"), want):
                 assert torch.equal(got, ref)

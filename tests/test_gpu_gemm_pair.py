@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from open_transformers_b200.ops import functional as K
+from open_transformers_b200.ops.native import cuda_lib
 
 pytestmark = pytest.mark.gpu
 
@@ -55,4 +56,18 @@ def test_pairs_that_follow_one_another(K_):
         for out in outs:
             K.gemm(ac, bc, epi=K.EPI_STORE_F32, out=out)
     assert all(torch.equal(out.cpu(), want) for out in outs)
+    assert K.kernel_status("cuda") == 0
+
+
+@pytest.mark.parametrize("M,N", [(512, 9472), (300, 704)])  # pairs, single CTAs
+def test_any_order_of_the_tiles(M, N):
+    g = torch.Generator().manual_seed(N)
+    a, b = (torch.randn(r, 64, generator=g).bfloat16() for r in (M, N))
+    want, ac, bc = K.gemm(a, b), a.cuda(), b.cuda()
+    try:
+        for rotation in (1, 2**31 - 1):  # (the last: the sum of block and rotation needs all 32 bits)
+            assert cuda_lib().otb_set_cta_rotation(rotation) == 0
+            assert torch.equal(K.gemm(ac, bc).cpu(), want)
+    finally:
+        assert cuda_lib().otb_set_cta_rotation(0) == 0
     assert K.kernel_status("cuda") == 0
