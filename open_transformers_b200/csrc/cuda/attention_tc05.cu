@@ -1550,11 +1550,6 @@ template <int D> constexpr int attn_bwd_q2_smem_bytes() { return 4 * (BQ * D * 2
 template <int D> constexpr int attn_bwd_kv2_smem_bytes() { return 2 * (BKV * D * 2) + 2 * KV2_ST * (HK * D * 2) + KV2_ST * 2 * HK * 4 + 1024 + 256; }
 template <int D> constexpr int attn_fwd2_smem_bytes() { return (2 + 2 * 2) * (BQ * D * 2) + 1024 + 256; }
 
-template <typename K>
-int set_smem(K kern, int bytes) {
-  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 }  // namespace
 
 // qk: [B*T, ldqk] bf16 holding H query heads then Hkv key heads (width D each); qkv: [B*T, ldqkv] bf16 whose
@@ -1579,13 +1574,13 @@ extern "C" int otb_attn_fwd(const void* qk, long ldqk, const void* qkv, long ldq
   const unsigned grid = persistent_grid((long)((nq + 1) / 2) * H * B);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (D == 128) {
-    static int once = set_smem(attn_fwd2_kernel<128>, attn_fwd2_smem_bytes<128>());
-    if (once) return once;
+    const int rc = otb_allow_smem<attn_fwd2_kernel<128>>(attn_fwd2_smem_bytes<128>());
+    if (rc) return rc;
     attn_fwd2_kernel<128><<<grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                               c_log2, status);
   } else {
-    static int once = set_smem(attn_fwd2_kernel<64>, attn_fwd2_smem_bytes<64>());
-    if (once) return once;
+    const int rc = otb_allow_smem<attn_fwd2_kernel<64>>(attn_fwd2_smem_bytes<64>());
+    if (rc) return rc;
     attn_fwd2_kernel<64><<<grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                             c_log2, status);
   }
@@ -1609,8 +1604,8 @@ extern "C" int otb_attn_fwd_i8pv(const void* qk, long ldqk, const void* qkv, lon
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
   dim3 grid((T + BQ - 1) / BQ, H, B);
-  static int once = set_smem(attn_fwd_kernel<128, true>, attn_smem_bytes<128>());
-  if (once) return once;
+  const int rc = otb_allow_smem<attn_fwd_kernel<128, true>>(attn_smem_bytes<128>());
+  if (rc) return rc;
   attn_fwd_kernel<128, true><<<grid, ATT_THREADS, attn_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, T, H, Hkv, window,
                                                                                scale, c_log2, vstep, status);
   return (int)cudaGetLastError();
@@ -1660,10 +1655,10 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     if (r != CUDA_SUCCESS) return 1000 + (int)r;
   }
   if (D == 128) {
-    static int once = set_smem(attn_bwd_kv_kernel<128>, attn_bwd_smem_bytes<128>()) |
-                      set_smem(attn_bwd_kv2_kernel<128>, attn_bwd_kv2_smem_bytes<128>()) |
-                      set_smem(attn_bwd_q2_kernel<128>, attn_bwd_q2_smem_bytes<128>());
-    if (once) return once;
+    const int rc = otb_allow_smem<attn_bwd_kv_kernel<128>>(attn_bwd_smem_bytes<128>()) |
+                   otb_allow_smem<attn_bwd_kv2_kernel<128>>(attn_bwd_kv2_smem_bytes<128>()) |
+                   otb_allow_smem<attn_bwd_q2_kernel<128>>(attn_bwd_q2_smem_bytes<128>());
+    if (rc) return rc;
     if (kv2)
       attn_bwd_kv2_kernel<128><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s>>>(
           tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
@@ -1673,10 +1668,10 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     attn_bwd_q2_kernel<128><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                                                                   Hkv, window, scale, c_log2, status);
   } else {
-    static int once = set_smem(attn_bwd_kv_kernel<64>, attn_bwd_smem_bytes<64>()) |
-                      set_smem(attn_bwd_kv2_kernel<64>, attn_bwd_kv2_smem_bytes<64>()) |
-                      set_smem(attn_bwd_q2_kernel<64>, attn_bwd_q2_smem_bytes<64>());
-    if (once) return once;
+    const int rc = otb_allow_smem<attn_bwd_kv_kernel<64>>(attn_bwd_smem_bytes<64>()) |
+                   otb_allow_smem<attn_bwd_kv2_kernel<64>>(attn_bwd_kv2_smem_bytes<64>()) |
+                   otb_allow_smem<attn_bwd_q2_kernel<64>>(attn_bwd_q2_smem_bytes<64>());
+    if (rc) return rc;
     if (kv2)
       attn_bwd_kv2_kernel<64><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s>>>(
           tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);

@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <atomic>
 #include <type_traits>
 #include <utility>
 
@@ -53,6 +54,20 @@ inline int otb_sm_count() {
     sm[dev] = n;
   }
   return sm[dev];
+}
+
+// Lets KERN take `bytes` of dynamic shared memory. The attribute belongs to the current device, so it is remembered for each
+// device by itself; two threads that come first together both set it. An error is not remembered.
+template <auto KERN>
+inline int otb_allow_smem(int bytes) {
+  static std::atomic<bool> allowed[64];
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+  const bool kept = dev >= 0 && dev < 64;
+  if (kept && allowed[dev].load(std::memory_order_acquire)) return 0;
+  if (const cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return (int)e;
+  if (kept) allowed[dev].store(true, std::memory_order_release);
+  return 0;
 }
 
 #define OTB_CUDA_CHECK_RET(expr)              \

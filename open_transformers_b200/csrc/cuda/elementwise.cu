@@ -772,8 +772,7 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
   const long slabs = (rows + NORM_SLAB - 1) / NORM_SLAB;
 #define RB(MAXC)                                                                                                          \
   DISPATCH_T(dtype, {                                                                                                     \
-    static int attr = cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, MAXC>, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_SLAB * 256 * MAXC * 4); \
-    if (attr) return attr;                                                                                                \
+    if (const int rc = otb_allow_smem<rmsnorm_bwd_kernel<T, MAXC>>(NORM_SLAB * 256 * MAXC * 4)) return rc;                   \
     rmsnorm_bwd_kernel<T, MAXC><<<(unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream)>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
                                                                                      dgamma_partial, rows, D, inv_d);     \
   })

@@ -652,22 +652,12 @@ extern "C" int otb_gemm_f32(const float* A, const float* B, float* C, const floa
 }
 
 namespace {
-template <typename K>
-int allow_smem(K kern, int bytes, bool& done) {
-  if (!done) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return (int)e;
-    done = true;
-  }
-  return 0;
-}
 template <int DM>
 int attn_f32_fwd(const float* qk, long ldqk, const float* qkv, long ldqkv, float* O, long ldo, float* lse, int B, int T, int H, int Hkv, int D,
                  int window, float c_log2, int vec, cudaStream_t s) {
   constexpr int KV = DM * FLD > FKB * (DM + 4) ? DM * FLD : FKB * (DM + 4);
   constexpr int bytes = 4 * (DM * ALD + KV + FKB * ALD + 5 * AT);
-  static bool done = false;
-  if (const int rc = allow_smem(attn_f32_fwd_kernel<DM>, bytes, done)) return rc;
+  if (const int rc = otb_allow_smem<attn_f32_fwd_kernel<DM>>(bytes)) return rc;
   attn_f32_fwd_kernel<DM><<<(unsigned)((T + AT - 1) / AT * (long)H * B), 256, bytes, s>>>(qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2, vec);
   return (int)cudaGetLastError();
 }
@@ -676,9 +666,8 @@ int attn_f32_bwd(const float* qk, long ldqk, const float* qkv, long ldqkv, const
                  float* dqk, long lddqk, float* dqkv, long lddqkv, int B, int T, int H, int Hkv, int D, int window, float c_log2, float scale,
                  int vec, cudaStream_t s) {
   constexpr int kv_bytes = 4 * (4 * DM * ALD + 2 * AT * ALD), q_bytes = 4 * (4 * DM * ALD + AT * ALD);
-  static bool done_kv = false, done_q = false;
-  if (const int rc = allow_smem(attn_f32_bwd_kv_kernel<DM>, kv_bytes, done_kv)) return rc;
-  if (const int rc = allow_smem(attn_f32_bwd_q_kernel<DM>, q_bytes, done_q)) return rc;
+  if (const int rc = otb_allow_smem<attn_f32_bwd_kv_kernel<DM>>(kv_bytes)) return rc;
+  if (const int rc = otb_allow_smem<attn_f32_bwd_q_kernel<DM>>(q_bytes)) return rc;
   const long nt = (T + AT - 1) / AT;
   attn_f32_bwd_kv_kernel<DM><<<(unsigned)(nt * Hkv * B), 256, kv_bytes, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv, B, T, H,
                                                                      Hkv, D, window, c_log2, scale, vec);

@@ -682,13 +682,8 @@ template <int EPI, bool A_MN, bool B_MN, bool I8 = false>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N, int K, long ldc, long ldr,
                 uint32_t* status, int max_ctas, cudaStream_t stream, const float* scale_a = nullptr, const float* scale_b = nullptr) {
   using L = SmemLayout<256, PAIR_STAGES, true>;
-  auto kern = gemm_tc05_kernel<256, PAIR_STAGES, A_MN, B_MN, EPI, I8, 0, TpNone, true>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  constexpr auto kern = gemm_tc05_kernel<256, PAIR_STAGES, A_MN, B_MN, EPI, I8, 0, TpNone, true>;
+  if (const int rc = otb_allow_smem<kern>(L::TOTAL)) return rc;
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
   const int pairs = (int)(tiles < max_ctas / 2 ? tiles : max_ctas / 2);
   cudaLaunchAttribute cluster;
@@ -736,13 +731,8 @@ template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8 = false>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N, int K, long ldc, long ldr,
            uint32_t* status, int max_ctas, cudaStream_t stream, const float* scale_a = nullptr, const float* scale_b = nullptr) {
   using L = SmemLayout<BN, STAGES>;
-  auto kern = gemm_tc05_kernel<BN, STAGES, A_MN, B_MN, EPI, I8, 0, TpNone>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  constexpr auto kern = gemm_tc05_kernel<BN, STAGES, A_MN, B_MN, EPI, I8, 0, TpNone>;
+  if (const int rc = otb_allow_smem<kern>(L::TOTAL)) return rc;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   int grid = tiles < max_ctas ? tiles : max_ctas;
   if (grid < 1) grid = 1;
@@ -756,13 +746,8 @@ template <int BN, int STAGES, bool B_MN, int EPI, int TP>
 int launch_tp(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* C, const void* R, int M, int N, int K, long ldc,
               long ldr, uint32_t* status, int grid, const TpArgs& tp, cudaStream_t stream, int group_m = 8) {
   using L = SmemLayout<BN, STAGES>;
-  auto kern = gemm_tc05_kernel<BN, STAGES, false, B_MN, EPI, false, TP, TpArgs>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  constexpr auto kern = gemm_tc05_kernel<BN, STAGES, false, B_MN, EPI, false, TP, TpArgs>;
+  if (const int rc = otb_allow_smem<kern>(L::TOTAL)) return rc;
   kern<<<grid, TP >= 2 ? NUM_THREADS + 128 : NUM_THREADS, L::TOTAL, stream>>>(
       ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m, nullptr, nullptr, status, tp);
   return (int)cudaGetLastError();
