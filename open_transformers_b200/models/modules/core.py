@@ -24,10 +24,11 @@ class ParamMixin:
 
 
 def _untouched(module: nn.Module, cls: type) -> bool:
-    """Whether calling ``module`` would run ``cls.forward`` and nothing else: no subclass, no hook, no replaced method. Only
-    then may a fused function take the module's place."""
-    return type(module) is cls and "forward" not in module.__dict__ and not nn.modules.module._has_any_global_hook() and not (
-        module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+    """Whether calling ``module`` would run ``cls``'s own forward as it is written here and nothing else: no subclass, no hook,
+    no ``forward`` put in its place on the module or on the class. Only then may a fused function take the module's place."""
+    return type(module) is cls and "forward" not in module.__dict__ and cls.forward is _OWN_FORWARD[cls] and \
+        not nn.modules.module._has_any_global_hook() and not (
+            module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
 
 
 class Linear(nn.Module, ParamMixin):
@@ -189,6 +190,9 @@ class RMSNorm(nn.Module, ParamMixin):
             return A.rms_norm(x, None, eps=self.eps)
         master, w, slot = self.operands(x.dtype)
         return A.rms_norm(x, master, w, slot, self.eps, tp_heads)
+
+
+_OWN_FORWARD = {cls: cls.forward for cls in (QuantLinear, RMSNorm)}
 
 
 @ROPE.register("rope_default")

@@ -55,6 +55,21 @@ def test_a_hooked_layer_is_called():
     assert seen == ["wk", "k_norm"]
 
 
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])  # (the gains are fused on a GPU only)
+@pytest.mark.parametrize("cls", [core.QuantLinear, core.RMSNorm])
+def test_a_forward_replaced_on_the_class_is_called(monkeypatch, device, cls):
+    mod = core.GQAQKNorm(64, 2, 1, 64, qat=QATConfig(enabled=True, method="absmax"))
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.fill_(0.01)
+    mod = mod.to(device)
+    cos, sin = K.rope_tables(4, 64, 10000.0, device)
+    seen, own = [], cls.forward
+    monkeypatch.setattr(cls, "forward", lambda self, *a, **kw: (seen.append(self), own(self, *a, **kw))[1])
+    mod(torch.ones(1, 4, 64, device=device), cos, sin)
+    assert seen == ([mod.wq, mod.wk, mod.wv, mod.wo] if cls is core.QuantLinear else [mod.q_norm, mod.k_norm])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("tokens,heads,D,pad", [(1, 1, 8, 0), (5, 3, 64, 8), (33, 5, 128, 16), (130, 2, 120, 0)])
