@@ -350,7 +350,8 @@ class _GQABase(nn.Module, ParamMixin):
         H, Hkv, D = self.n_heads, self.n_kv_heads, self.head_dim
         qkv = self._qkv(x)
         if self.qk_norm_gain and _untouched(self.q_norm, RMSNorm) and _untouched(self.k_norm, RMSNorm) and \
-                self.q_norm.eps == self.k_norm.eps and K.head_norm_supported(qkv.reshape(B * T, -1), D):
+                self.q_norm.weight is not None and self.k_norm.weight is not None and self.q_norm.eps == self.k_norm.eps and \
+                K.head_norm_supported(qkv.reshape(B * T, -1), D):
             o = A.gain_attention(qkv, cos, sin, self.q_norm.operands(qkv.dtype), self.k_norm.operands(qkv.dtype), H, Hkv, D, self.window,
                                  self.q_norm.eps, self._int8_pv(qkv))
         elif self.qk_norm_gain:

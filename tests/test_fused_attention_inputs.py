@@ -70,6 +70,25 @@ def test_a_forward_replaced_on_the_class_is_called(monkeypatch, device, cls):
     assert seen == ([mod.wq, mod.wk, mod.wv, mod.wo] if cls is core.QuantLinear else [mod.q_norm, mod.k_norm])
 
 
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("name", ["q_norm", "k_norm"])
+def test_head_norm_without_a_gain(monkeypatch, device, name):
+    """A module whose query or key norm was replaced by one without a weight: no gain to fuse."""
+    g = torch.Generator().manual_seed(3)
+    mod = core.GQAQKNorm(64, 2, 1, 64)
+    setattr(mod, name, core.RMSNorm(64, gain=False))
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * 0.05)
+    mod = mod.to(device)
+    cos, sin = K.rope_tables(9, 64, 10000.0, device)
+    x, dy = (torch.randn(2, 9, 64, generator=g).to(device) for _ in range(2))
+    want = _run(mod, x, dy, cos, sin, False)
+    monkeypatch.setattr(K, "head_norm_supported", lambda x, D: True)  # (so that the CPU run asks the same question)
+    for a, b in zip(_run(mod, x, dy, cos, sin, True), want):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("tokens,heads,D,pad", [(1, 1, 8, 0), (5, 3, 64, 8), (33, 5, 128, 16), (130, 2, 120, 0)])
