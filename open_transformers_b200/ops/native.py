@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import re
 import struct
 import threading
 from pathlib import Path
@@ -129,8 +130,10 @@ def raw_stream() -> int:
 
 
 def packed_entry(name: str, words: str):
-    """Callable for a CUDA entry point: ``words`` has one letter per argument (q integer or pointer, d float)."""
+    """Callable for a CUDA entry point: ``words`` has one letter per argument (q integer or pointer, d float). Numbers of other
+    types are taken as ``I`` / ``L`` / ``F`` take them (a window of 512.0, a one-element tensor)."""
     pack = struct.Struct("=" + words).pack
+    kinds = [kind for count, kind in re.findall(r"(\d*)([qd])", words) for _ in range(int(count or 1))]
     fn = None
 
     def call(*args) -> int:
@@ -139,7 +142,11 @@ def packed_entry(name: str, words: str):
             f = getattr(cuda_lib(), name + "_p")
             f.argtypes = [ctypes.c_char_p]
             fn = f
-        return fn(pack(*args))
+        try:
+            packed = pack(*args)
+        except (struct.error, TypeError):
+            packed = pack(*[int(a) if kind == "q" else float(a) for a, kind in zip(args, kinds, strict=True)])
+        return fn(packed)
 
     return call
 
