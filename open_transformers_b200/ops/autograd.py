@@ -767,8 +767,8 @@ class QuantQkvFn(Function):
     def backward(ctx, dy):
         xq, sa, *rest = ctx.saved_tensors
         dy2 = _flat2d(dy)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
+        if not dy2.is_contiguous() or dy2.data_ptr() % 16:  # the products read its columns in place, in 16-byte pieces
+            dy2 = dy2.clone(memory_format=torch.contiguous_format)
         xw = K.i8_widen(xq, dy2.dtype)
         dx, grads, at = None, [], dy2.shape[1]
         for i in reversed(range(len(ctx.parts))):

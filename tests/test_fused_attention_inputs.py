@@ -89,6 +89,22 @@ def test_head_norm_without_a_gain(monkeypatch, device, name):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_gradient_of_the_joint_projections_at_any_address(device):
+    """A contiguous gradient that starts at an odd element (the layers by themselves get aligned copies of their columns)."""
+    g = torch.Generator().manual_seed(5)
+    mod = core.GQAQKNorm(64, 2, 1, 64, qat=QATConfig(enabled=True, method="absmax"))
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * 0.05)
+    mod = mod.to(device)
+    x = torch.randn(2, 9, 64, generator=g).to(device, torch.bfloat16).requires_grad_()
+    dy = torch.randn(2 * 9 * 256 + 1, generator=g).to(device, torch.bfloat16)[1:].view(2, 9, 256)
+    weights = [m.weight for m in (mod.wq, mod.wk, mod.wv)]
+    for a, b in zip(torch.autograd.grad(mod._qkv(x), [x, *weights], dy), torch.autograd.grad(mod._qkv(x), [x, *weights], dy.clone())):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("tokens,heads,D,pad", [(1, 1, 8, 0), (5, 3, 64, 8), (33, 5, 128, 16), (130, 2, 120, 0)])
