@@ -31,7 +31,7 @@ namespace {
 
 inline unsigned blocks_for(long n, int per) { return (unsigned)((n + per - 1) / per); }
 
-constexpr int AMAX_BLOCKS = 592;  // 4 per SM; partial maxima, then one block folds them
+constexpr int AMAX_BLOCKS = 592;  // 4 per SM; one partial maximum each, folded by whoever needs the whole
 
 template <typename T>
 __global__ void absmax_partial_kernel(const T* __restrict__ x, long n, float* __restrict__ partial) {
@@ -57,19 +57,19 @@ __global__ void absmax_final_kernel(const float* __restrict__ partial, int n, fl
   if (threadIdx.x == 0) out[0] = m;
 }
 
-// as many 256-thread CTAs as are resident at once, fewer where there is less to do
-inline unsigned quant_blocks(long n) { return (unsigned)min((long)blocks_for(n, 8 * 256), (long)otb_sm_count() * 8); }
+// as many 256-thread CTAs as are resident at once, fewer where there is less to do (one writes the step)
+inline unsigned quant_blocks(long n) { return (unsigned)max(1L, min((long)blocks_for(n, 8 * 256), (long)otb_sm_count() * 8)); }
 
 __device__ __forceinline__ float clamp_q(float q, float qmax) { return fminf(fmaxf(q, -qmax), qmax); }
 
-// The maximum is that of `parts` partial maxima: a resident CTA folds them itself (a few KB from L2, once) and then walks
+// The maximum is that of the AMAX_BLOCKS partial maxima: a resident CTA folds them itself (a few KB from L2, once) and then walks
 // its share of x, which spares a one-CTA launch between the two passes.
 template <typename T>
-__global__ void __launch_bounds__(256) quant_act_kernel(const T* __restrict__ x, long n, const float* __restrict__ amax, int parts, float inv_qmax,
+__global__ void __launch_bounds__(256) quant_act_kernel(const T* __restrict__ x, long n, const float* __restrict__ amax, float inv_qmax,
                                  float qmax, int8_t* __restrict__ q, float* __restrict__ step_out) {
   __shared__ float sh[32];
   float m = 0.0f;
-  for (int i = threadIdx.x; i < parts; i += blockDim.x) m = fmaxf(m, amax[i]);
+  for (int i = threadIdx.x; i < AMAX_BLOCKS; i += blockDim.x) m = fmaxf(m, amax[i]);
   m = block_max(m, sh);
   const float step = fmaxf(__fmul_rn(m, inv_qmax), FLT_MIN);
   if (blockIdx.x == 0 && threadIdx.x == 0) step_out[0] = step;
@@ -207,19 +207,12 @@ extern "C" int otb_absmax(const void* x, long n, int dtype, float* scratch, floa
   absmax_final_kernel<<<1, 256, 0, S(stream)>>>(scratch, AMAX_BLOCKS, amax);
   return (int)cudaGetLastError();
 }
-extern "C" int otb_quant_act(const void* x, long n, int dtype, const float* amax, int qmax, void* q, float* step,
-                             void* stream) {
-  if (n <= 0) return 0;
-  DISPATCH_T(dtype, quant_act_kernel<T><<<quant_blocks(n), 256, 0, S(stream)>>>(
-                        (const T*)x, n, amax, 1, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);)
-  return (int)cudaGetLastError();
-}
-// Both passes: absmax of x, then its quantisation. scratch: otb_absmax_scratch_floats() device floats.
+// Both passes: absmax of x, then its quantisation (of nothing, n = 0: the step alone). x and q 16- and 8-byte aligned; scratch:
+// otb_absmax_scratch_floats() device floats.
 extern "C" int otb_absmax_quant_act(const void* x, long n, int dtype, float* scratch, int qmax, void* q, float* step, void* stream) {
-  if (n <= 0) return 0;
   DISPATCH_T(dtype, {
     absmax_partial_kernel<T><<<AMAX_BLOCKS, 256, 0, S(stream)>>>((const T*)x, n, scratch);
-    quant_act_kernel<T><<<quant_blocks(n), 256, 0, S(stream)>>>((const T*)x, n, scratch, AMAX_BLOCKS, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);
+    quant_act_kernel<T><<<quant_blocks(n), 256, 0, S(stream)>>>((const T*)x, n, scratch, 1.0f / (float)qmax, (float)qmax, (int8_t*)q, step);
   })
   return (int)cudaGetLastError();
 }
@@ -258,7 +251,6 @@ extern "C" int otb_i8_widen(const void* q, void* out, long n, int out_dtype, voi
 }
 
 OTB_PACKED(otb_absmax)
-OTB_PACKED(otb_quant_act)
 OTB_PACKED(otb_absmax_quant_act)
 OTB_PACKED(otb_quant_weight)
 OTB_PACKED(otb_lsq_bwd)

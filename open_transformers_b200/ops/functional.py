@@ -365,7 +365,6 @@ weight_epoch: int | None = None  # set (and bumped at every weight change) by th
 
 
 _absmax = packed_entry("otb_absmax", "6q")
-_quant_act = packed_entry("otb_quant_act", "8q")
 _absmax_quant_act = packed_entry("otb_absmax_quant_act", "8q")
 _quant_weight = packed_entry("otb_quant_weight", "10q")
 _gemm_i8 = packed_entry("otb_gemm_i8", "17q")
@@ -396,14 +395,11 @@ def quant_act(x: torch.Tensor, qmax: int):
     assert x.is_contiguous()
     q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
     step = torch.empty(1, dtype=torch.float32, device=x.device)
-    if x.is_cuda and x.numel() > 0:
+    if x.is_cuda:
         scratch = torch.empty(_absmax_scratch(), dtype=torch.float32, device=x.device)
         check(_absmax_quant_act(ptr(x), x.numel(), is_bf16(x), ptr(scratch), qmax, ptr(q), ptr(step), raw_stream()), "quant_act")
-        return q, step
-    am = absmax(x)
-    if x.is_cuda:
-        check(_quant_act(ptr(x), x.numel(), is_bf16(x), ptr(am), qmax, ptr(q), ptr(step), raw_stream()), "quant_act")
     else:
+        am = absmax(x)
         check(cpu_lib().otb_cpu_quant_act(P(x), L(x.numel()), I(is_bf16(x)), P(am), I(qmax), P(q), P(step)), "quant_act")
     return q, step
 

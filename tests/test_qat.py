@@ -353,3 +353,13 @@ def test_every_recipe_switch_together_trains_and_replays_in_bf16(tmp_path):
     assert audit_replay(ck, data_root=tmp, until_step=3)["match"] is True
     r = audit_replay(from_init=True, descriptor_checkpoint=ck, data_root=tmp, until_step=3, offload_grads=True, offload_optimizer=True)
     assert r["match"] is True and r["state_hash"] == res["hashes"][-1][1]
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_quantiser_of_an_empty_tensor(device, dtype):
+    """No element: the maximum is 0 and the step its floor, the smallest normal number."""
+    old = torch.full((1,), 7.0, device=device)
+    del old  # (what an unwritten step would hold)
+    q, step = K.quant_act(torch.empty(0, 16, dtype=dtype, device=device), 127)
+    assert q.shape == (0, 16) and q.dtype == torch.int8 and float(step) == torch.finfo(torch.float32).tiny
