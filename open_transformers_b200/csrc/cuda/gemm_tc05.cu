@@ -720,11 +720,33 @@ constexpr double NARROW = 0.84, NARROW_MN = 0.78;
 // large: it loses where they leave SMs idle, less than one wave of pairs above all, or pad more rows (1024 x 3072 x 2048: 30
 // and 32; 1111 x 4096 x 768: 24 and 32). With an MN-major operand the gain fades as the product grows and turns into a loss
 // (378 GFLOP 0.93 - 0.99 of the single time, 756 GFLOP 1.00, 8.6 TFLOP 1.06): pairs take those up to PAIR_MN_FLOPS.
+// With few K steps the stores are the time, and a pair's next tile waits until the slower of its two CTAs has read its
+// accumulator: 16384 x 5632, single and paired, us: K 64 36 and 51, 256 51 and 58, 384 66 and 68, 512 89 and 85, 640 107 and
+// 97; as int8, twice the rate for the same stores: K 512 75 and 86, 1024 80 and 92, 1280 95 and 99, 1536 111 and 111, and
+// 9081 x 5312 x 2256 133 and 103. 4096 x 4096, 16384 x 2048, 2048 x 11264 and 512 x 128256 cross at the same K.
 constexpr double PAIR_GAIN = 1.07, PAIR_MN_FLOPS = 5e11;
-bool pair_wins(int M, int N, int K, bool mn_major, int max_ctas, double single) {
+constexpr int PAIR_ABOVE_K = 512, PAIR_ABOVE_K_I8 = 1536;
+bool pair_wins(int M, int N, int K, bool mn_major, bool i8, int max_ctas, double single) {
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
-  return N > 128 && tiles >= max_ctas / 2 && max_ctas >= 2 && (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) &&
-         PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
+  return N > 128 && K > (i8 ? PAIR_ABOVE_K_I8 : PAIR_ABOVE_K) && tiles >= max_ctas / 2 && max_ctas >= 2 &&
+         (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) && PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
+}
+// Tile of a product: columns of a single CTA's tile, or PAIR_TILE.
+constexpr int PAIR_TILE = 512;
+int choose_tile(int M, int N, int K, bool mn_major, bool i8, int max_ctas) {
+  int BN;
+  double single;
+  if (i8) {
+    BN = N > 128 ? 256 : 128;
+    single = tile_efficiency(M, N, BM, BN, max_ctas);
+  } else {
+    // the 256-wide tile is the more efficient one per tile; the 128-wide one wins when it fills the last wave noticeably better
+    const double e128 = (mn_major ? NARROW_MN : NARROW) * tile_efficiency(M, N, BM, 128, max_ctas);
+    const double e256 = N >= 256 ? tile_efficiency(M, N, BM, 256, max_ctas) : 0.0;
+    BN = e256 >= e128 ? 256 : 128;
+    single = BN == 256 ? e256 : e128;
+  }
+  return pair_wins(M, N, K, mn_major, i8, max_ctas, single) ? PAIR_TILE : BN;
 }
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8 = false>
@@ -816,6 +838,11 @@ int launch_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& t
 
 }  // namespace
 
+// The tile that the entry points below choose: 128 or 256 columns on one CTA, 512 for a CTA pair (max_ctas 0: every SM).
+extern "C" int otb_gemm_tile(int M, int N, int K, int mn_major, int i8, int max_ctas) {
+  return choose_tile(M, N, K, mn_major != 0, i8 != 0, max_ctas > 0 ? max_ctas : otb_sm_count());
+}
+
 // C[M,N] = op(A) op(B)^T with bf16 operands and fp32 tensor-core accumulation.
 //   a_mn = 0: A is [M,K] row-major with leading dimension lda;  a_mn = 1: A is [K,M] row-major.
 //   b_mn = 0: B is [N,K] row-major with leading dimension ldb;  b_mn = 1: B is [K,N] row-major.
@@ -832,13 +859,8 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   const bool bf16_out = (epi == EPI_BF16 || epi == EPI_BF16_RES);
   if ((bf16_out && (ldc & 7)) || (!bf16_out && (ldc & 3)) || (epi == EPI_BF16_RES && (ldr & 7))) return -2;
   if (max_ctas <= 0) max_ctas = otb_sm_count();
-  // Tile shape: the 256-wide tile is the more efficient one per tile; the 128-wide one wins when it fills the last wave of
-  // CTAs noticeably better, the pair's 256 x 256 one when the product is large (pair_wins).
-  const bool mn_major = a_mn || b_mn;
-  const double e128 = (mn_major ? NARROW_MN : NARROW) * tile_efficiency(M, N, BM, 128, max_ctas);
-  const double e256 = N >= 256 ? tile_efficiency(M, N, BM, 256, max_ctas) : 0.0;
-  const int BN = e256 >= e128 ? 256 : 128;
-  const bool pair = pair_wins(M, N, K, mn_major, max_ctas, BN == 256 ? e256 : e128);
+  const int BN = choose_tile(M, N, K, a_mn || b_mn, false, max_ctas);
+  const bool pair = BN == PAIR_TILE;
   CUtensorMap ta, tb;
   CUresult r;
   constexpr int BK = BK_BYTES / 2;
@@ -896,8 +918,8 @@ extern "C" int otb_gemm_i8(const void* A, const void* B, void* C, const void* R,
   if ((bf16_out && (ldc & 7)) || (!bf16_out && (ldc & 3)) || (epi == EPI_BF16_RES && (ldr & 7))) return -2;
   if (!scale_a || !scale_b) return -2;
   if (max_ctas <= 0) max_ctas = otb_sm_count();
-  const int BN = N > 128 ? 256 : 128;
-  const bool pair = pair_wins(M, N, K, false, max_ctas, tile_efficiency(M, N, BM, BN, max_ctas));
+  const int BN = choose_tile(M, N, K, false, true, max_ctas);
+  const bool pair = BN == PAIR_TILE;
   CUtensorMap ta, tb, tc;
   CUresult r = encode_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK_BYTES, BM, 1);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;

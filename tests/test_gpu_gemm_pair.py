@@ -6,14 +6,18 @@ from open_transformers_b200.ops import functional as K
 from open_transformers_b200.ops.native import cuda_lib
 
 pytestmark = pytest.mark.gpu
+PAIR = 512  # otb_gemm_tile's answer for CTA pairs
 
 
 # 256-row tiles whose second CTA holds few, no or all rows; ragged column tiles; one K step, a ragged one, more than the ring
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
-@pytest.mark.parametrize("M,N,K_", [(2304, 4864, 8), (2104, 5008, 72), (2184, 5120, 64), (2056, 9480, 48), (2304, 4872, 456)])
+# (the K up to 512 run the same results on single CTAs)
+@pytest.mark.parametrize("M,N,K_", [(2304, 4864, 8), (2104, 5008, 72), (2184, 5120, 64), (2056, 9480, 48), (2304, 4872, 456),
+                                    (2304, 4864, 520), (2104, 5008, 576), (2056, 9480, 584), (2304, 4872, 1000)])
 def test_bf16_pairs(a_mn, b_mn, M, N, K_):
     g = torch.Generator().manual_seed(K_)
     a, b = torch.randn(M, K_, generator=g).bfloat16(), torch.randn(N, K_, generator=g).bfloat16()
+    assert (cuda_lib().otb_gemm_tile(M, N, K_, a_mn or b_mn, 0, 0) == PAIR) == (K_ > 512)
     want = K.gemm(a, b, epi=K.EPI_STORE_F32)
     ac, bc = (t.t().contiguous().cuda() if mn else t.cuda() for t, mn in ((a, a_mn), (b, b_mn)))
     kw = dict(a_mn=a_mn, b_mn=b_mn)
@@ -28,8 +32,9 @@ def test_bf16_pairs(a_mn, b_mn, M, N, K_):
     assert bool((big == 7.0).all()) and K.kernel_status("cuda") == 0
 
 
-@pytest.mark.parametrize("M,N,K_", [(2100, 5008, 144), (2304, 4864, 16), (2049, 9480, 1040)])
+@pytest.mark.parametrize("M,N,K_", [(2100, 5008, 144), (2304, 4864, 16), (2049, 9480, 1040), (2100, 5008, 1552), (2304, 4872, 1680), (2049, 9480, 1664)])
 def test_int8_pairs(M, N, K_):
+    assert (cuda_lib().otb_gemm_tile(M, N, K_, 0, 1, 0) == PAIR) == (K_ > 1536)
     g = torch.Generator().manual_seed(N)
     a, b = (torch.randint(-127, 128, (r, K_), dtype=torch.int8, generator=g) for r in (M, N))
     sa, sb = torch.rand(1, generator=g) * 0.01, torch.rand(N, generator=g) * 0.01
@@ -42,12 +47,13 @@ def test_int8_pairs(M, N, K_):
 
 
 # The shortest pipelines, one tile per pair and launches back to back: a pair has to leave nothing under way behind it (the
-# arrivals that release its last stages would land in the shared memory of the pair that follows). K of one step, of a ragged
-# last step, of one step less than the ring, of the whole ring and of one more.
-@pytest.mark.parametrize("K_", [64, 72, 320, 384, 448])
+# arrivals that release its last stages would land in the shared memory of the pair that follows). K steps of 64 around one and
+# a half and two turns of the ring of six, with and without a ragged last one.
+@pytest.mark.parametrize("K_", [520, 576, 640, 704, 768, 776])
 def test_pairs_that_follow_one_another(K_):
     g = torch.Generator().manual_seed(K_)
     M, N = 2 * 256, 37 * 256  # 74 tiles: one per pair of 148 SMs
+    assert cuda_lib().otb_gemm_tile(M, N, K_, 0, 0, 0) == PAIR
     a, b = (torch.randn(r, K_, generator=g).bfloat16() for r in (M, N))
     want = K.gemm(a, b, epi=K.EPI_STORE_F32)
     ac, bc = a.cuda(), b.cuda()
@@ -59,10 +65,11 @@ def test_pairs_that_follow_one_another(K_):
     assert K.kernel_status("cuda") == 0
 
 
-@pytest.mark.parametrize("M,N", [(512, 9472), (300, 704)])  # pairs, single CTAs
-def test_any_order_of_the_tiles(M, N):
+@pytest.mark.parametrize("M,N,pair", [(512, 9472, True), (300, 704, False)])
+def test_any_order_of_the_tiles(M, N, pair):
+    assert (cuda_lib().otb_gemm_tile(M, N, 520, 0, 0, 0) == PAIR) == pair
     g = torch.Generator().manual_seed(N)
-    a, b = (torch.randn(r, 64, generator=g).bfloat16() for r in (M, N))
+    a, b = (torch.randn(r, 520, generator=g).bfloat16() for r in (M, N))
     want, ac, bc = K.gemm(a, b), a.cuda(), b.cuda()
     try:
         for rotation in (1, 2**31 - 1):  # (the last: the sum of block and rotation needs all 32 bits)
