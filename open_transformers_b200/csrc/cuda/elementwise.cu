@@ -481,9 +481,71 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restric
 
 // ------------------------------------------------------------------- SwiGLU
 // gate_up [rows, 2F] (gate = cols [0,F), up = cols [F,2F)) -> h [rows, F] = silu(gate) * up
+// silu(g) * u of eight elements, and its gradient (dg, du) from d
+template <typename T>
+__device__ __forceinline__ void swiglu8(const Raw8<T>& rg, const Raw8<T>& ru, T* h) {
+  float g[8], u[8], o[8];
+  rg.unpack(g);
+  ru.unpack(u);
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) {
+    const tc05::f2 g2 = tc05::pack2(g[e], g[e + 1]);
+    tc05::unpack2(tc05::mul2(tc05::mul2(g2, tc05::sigmoid_fast2(g2)), tc05::pack2(u[e], u[e + 1])), o[e], o[e + 1]);
+  }
+  Vec8<T>::store(h, o);
+}
+template <typename T>
+__device__ __forceinline__ void swiglu8_bwd(const Raw8<T>& rg, const Raw8<T>& ru, const Raw8<T>& rd, T* dg, T* du) {
+  using namespace tc05;
+  float g[8], u[8], d[8], og[8], ou[8];
+  rg.unpack(g);
+  ru.unpack(u);
+  rd.unpack(d);
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) {
+    const f2 g2 = pack2(g[e], g[e + 1]), u2 = pack2(u[e], u[e + 1]), d2 = pack2(d[e], d[e + 1]);
+    const f2 sg = sigmoid_fast2(g2);
+    const f2 silu = mul2(g2, sg);
+    // d silu / dg = sg * (1 + g (1 - sg))
+    const f2 one = pack2(1.0f, 1.0f);
+    const f2 dsilu = mul2(sg, fma2(g2, add2(one, mul2(sg, pack2(-1.0f, -1.0f))), one));
+    unpack2(mul2(mul2(d2, u2), dsilu), og[e], og[e + 1]);
+    unpack2(mul2(d2, silu), ou[e], ou[e + 1]);
+  }
+  Vec8<T>::store(dg, og);
+  Vec8<T>::store(du, ou);
+}
+// One thread per group of eight, wherever its row is.
+template <typename T>
+__global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* __restrict__ gu, T* __restrict__ h, long rows, int F) {
+  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (idx >= rows * F) return;
+  const long row = idx / F;
+  const T* gr = gu + row * 2 * F + (idx - row * F);
+  Raw8<T> g, u;
+  g.load(gr);
+  u.load(gr + F);
+  swiglu8(g, u, h + idx);
+}
+template <typename T>
+__global__ void __launch_bounds__(256) swiglu_bwd_flat_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, long rows, int F) {
+  const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (idx >= rows * F) return;
+  const long row = idx / F, at = row * 2 * F + (idx - row * F);
+  Raw8<T> g, u, d;
+  g.load(gu + at);
+  u.load(gu + at + F);
+  d.load(dh + idx);
+  swiglu8_bwd(g, u, d, dgu + at, dgu + at + F);
+}
+// One CTA per row, two groups per thread and sweep with all their loads in flight: no index division (a 64-bit one per group
+// costs as much as the activation), and enough bytes in flight per SM to hold the memory's rate. It needs rows that fill its
+// warps and enough of them; narrow rows leave lanes idle and end up as many CTAs with next to nothing to do, and a few wide rows
+// leave SMs idle. bf16, flat and per row, us, forward: 20000 x 5632 120 and 101, 10000 x 2048 24.1 and 20.5, 4800 x 1024 6.7
+// and 6.3; 20000 x 704 16.0 and 19.2, 20000 x 352 8.8 and 12.4, 1048576 x 64 73 and 544; 64 x 5632 2.4 and 2.8, 600 x 16384
+// 11.4 and 12.5, 1200 x 1024 3.0 and 3.3. (Backward alike, its gain smaller: 20000 x 5632 164 and 160.)
 constexpr int SWIGLU_MAX_THREADS = 384;
-// One CTA per row, two 8-element groups per thread and sweep with all their loads in flight: no index division (a 64-bit
-// one per group cost as much as the activation), and enough bytes in flight per SM to hold the memory's rate.
+inline bool swiglu_per_row(long rows, int F) { return F >= 1024 && rows >= 2048 && rows <= 0x7fffffffL; }
 template <typename T>
 __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ h, int F) {
   const T* gr = gu + (long)blockIdx.x * 2 * F;
@@ -501,17 +563,7 @@ __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T*
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int c = c0 + u * blockDim.x * 8;
-      if (c < F) {
-        float g[8], v[8], o[8];
-        rg[u].unpack(g);
-        ru[u].unpack(v);
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const tc05::f2 g2 = tc05::pack2(g[e], g[e + 1]);
-          tc05::unpack2(tc05::mul2(tc05::mul2(g2, tc05::sigmoid_fast2(g2)), tc05::pack2(v[e], v[e + 1])), o[e], o[e + 1]);
-        }
-        Vec8<T>::store(hr + c, o);
-      }
+      if (c < F) swiglu8(rg[u], ru[u], hr + c);
     }
   }
 }
@@ -535,26 +587,7 @@ __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_bwd_kernel(const T*
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int c = c0 + u * blockDim.x * 8;
-      if (c < F) {
-        float g[8], v[8], d[8], og[8], ou[8];
-        rg[u].unpack(g);
-        ru[u].unpack(v);
-        rd[u].unpack(d);
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          using namespace tc05;
-          const f2 g2 = pack2(g[e], g[e + 1]), u2 = pack2(v[e], v[e + 1]), d2 = pack2(d[e], d[e + 1]);
-          const f2 sg = sigmoid_fast2(g2);
-          const f2 silu = mul2(g2, sg);
-          // d silu / dg = sg * (1 + g (1 - sg))
-          const f2 one = pack2(1.0f, 1.0f);
-          const f2 dsilu = mul2(sg, fma2(g2, add2(one, mul2(sg, pack2(-1.0f, -1.0f))), one));
-          unpack2(mul2(mul2(d2, u2), dsilu), og[e], og[e + 1]);
-          unpack2(mul2(d2, silu), ou[e], ou[e + 1]);
-        }
-        Vec8<T>::store(or_ + c, og);
-        Vec8<T>::store(or_ + F + c, ou);
-      }
+      if (c < F) swiglu8_bwd(rg[u], ru[u], rd[u], or_ + c, or_ + F + c);
     }
   }
 }
@@ -830,12 +863,20 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
 }
 extern "C" int otb_swiglu_fwd(const void* gu, void* h, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
-  DISPATCH_T(dtype, swiglu_fwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (T*)h, F);)
+  if (swiglu_per_row(rows, F)) {
+    DISPATCH_T(dtype, swiglu_fwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (T*)h, F);)
+  } else {
+    DISPATCH_T(dtype, swiglu_fwd_flat_kernel<T><<<blocks_for(rows * F / 8, 256), 256, 0, S(stream)>>>((const T*)gu, (T*)h, rows, F);)
+  }
   return (int)cudaGetLastError();
 }
 extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
-  DISPATCH_T(dtype, swiglu_bwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (const T*)dh, (T*)dgu, F);)
+  if (swiglu_per_row(rows, F)) {
+    DISPATCH_T(dtype, swiglu_bwd_kernel<T><<<(unsigned)rows, swiglu_threads(F), 0, S(stream)>>>((const T*)gu, (const T*)dh, (T*)dgu, F);)
+  } else {
+    DISPATCH_T(dtype, swiglu_bwd_flat_kernel<T><<<blocks_for(rows * F / 8, 256), 256, 0, S(stream)>>>((const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
+  }
   return (int)cudaGetLastError();
 }
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,

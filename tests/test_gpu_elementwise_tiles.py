@@ -53,6 +53,16 @@ def test_swiglu_widths(dtype, rows, F):
     _same(K.swiglu_bwd(gu.cuda(), dh.cuda()), K.swiglu_bwd(gu, dh), "backward")
 
 
+# both forms of the kernel at the line between them: 1024 columns, 2048 rows (and the widths above on a CTA per row)
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("rows,F", [(2048, 1016), (2047, 1024), (2048, 1024), (2049, 3072), (2050, 3080), (2048, 6152), (70000, 8)])
+def test_swiglu_forms(dtype, rows, F):
+    g = torch.Generator().manual_seed(F)
+    gu, dh = torch.randn(rows, 2 * F, generator=g).to(dtype), torch.randn(rows, F, generator=g).to(dtype)
+    _same(K.swiglu_fwd(gu.cuda()), K.swiglu_fwd(gu), "forward")
+    _same(K.swiglu_bwd(gu.cuda(), dh.cuda()), K.swiglu_bwd(gu, dh), "backward")
+
+
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("V", [8, 4096, 4104, 16392, 70008, 128256])  # one group, whole sweeps, a ragged unroll, every occupancy
 def test_loss_row_widths(dtype, V):
