@@ -607,10 +607,14 @@ inline int swiglu_threads(int F) {
 // and the row is overwritten with d loss / d logits = e_i * k - onehot * scale, k = ((1 + 2 z lse) / s) * scale
 // (scale = 1 / (tokens * accum), host reciprocal; the label's element is fma(e, k, -scale)).
 // Rows with label < 0 are ignored: zero loss, zero gradient.
-// Bound by instructions, not by the three reads (the maximum of bf16 logits is taken two at a time as bf16, the exponent's clamp
-// is left out where it does nothing). UNROLL groups per thread are in flight: 4 for long rows (16384 rows of 128 256 bf16
-// logits with their gradient: 2435 -> 2147 us), 1 for rows of at most 8 sweeps (8192 rows of 8192: 130 -> 123 us), which the
-// wider loop's registers slow (140 us).
+// Bound by instructions, not by the three reads (the maximum of bf16 logits is taken two at a time as bf16). Two things help
+// long rows and cost short ones registers, and with them CTAs per SM (ce_form chooses):
+//   TEST: the first pass finds the smallest logit too, and where it is near enough the exponent's clamp is left out;
+//   UNROLL groups per thread are in flight.
+// us for 16384 rows with their gradient; neither / TEST / TEST and four groups: bf16 V 1024 89 / 95 / 130, 8192 211 / 216 / 248,
+// 16384 296 / 296 / 346, 32768 525 / 516 / 568, 65536 986 / 967 / 1073, 98304 1714 / 1672 / 1552; 4000 rows of 128256 622 / 624 /
+// 542. fp32, 4000 rows: 1024 22 / 26 / 36, 8192 60 / 67 / 83, 16384 99 / 104 / 135, 32768 256 / 198 / 225, 65536 611 / 584 / 448;
+// with a few rows per SM neither helps (64 rows of 128256: 30 / 34 / 37, 149: 52 / - / 60, 600: 222 / 231 / 209).
 constexpr int CE_THREADS = 512, CE_SWEEP = CE_THREADS * 8;
 template <typename T, int CE_UNROLL>
 __device__ __forceinline__ void ce_fetch(Raw8<T> (&raw)[CE_UNROLL], const T* __restrict__ xr, int c0, int V) {
@@ -657,7 +661,7 @@ __device__ __forceinline__ void ce_grad(T* __restrict__ xr, int V, tc05::f2 l2, 
     }
   }
 }
-template <typename T, int CE_UNROLL>
+template <typename T, int CE_UNROLL, bool TEST>
 __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ logits, const long* __restrict__ labels,
                                                               float* __restrict__ ce_out, float* __restrict__ lse_out,
                                                               long rows, int V, float two_z, float scale, int write_grad) {
@@ -683,7 +687,8 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
 #pragma unroll
       for (int u = 0; u < CE_UNROLL; ++u) {
         if (c0 + u * CE_SWEEP >= V) break;
-        raw[u].extremes(mx, mn);
+        raw[u].largest(mx);
+        if (TEST) raw[u].smallest(mn);
       }
     }
   }
@@ -694,7 +699,8 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
   const f2 nm2 = pack2(nm, nm);
   // The exponent's clamp at -126 does nothing in a row whose smallest logit is above it (the exponent grows with the logit;
   // a NaN or an infinity fails the test): such rows, all of them in practice, leave it out, one instruction in eight.
-  const bool inside = __syncthreads_and(__fmaf_rn(mn, LOG2E, nm) >= -126.0f);
+  bool inside = false;
+  if constexpr (TEST) inside = __syncthreads_and(__fmaf_rn(mn, LOG2E, nm) >= -126.0f);
   const f2 acc2 = inside ? ce_sum<T, CE_UNROLL, false>(xr, V, l2, nm2) : ce_sum<T, CE_UNROLL, true>(xr, V, l2, nm2);
   float a0, a1;
   unpack2(acc2, a0, a1);
@@ -711,6 +717,12 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ lo
   const float at_label = __fmaf_rn(det_exp2_acc(__fmaf_rn(x_label, LOG2E, nm)), k, -scale);
   if (inside) ce_grad<T, CE_UNROLL, false>(xr, V, l2, nm2, k2, label, at_label);
   else ce_grad<T, CE_UNROLL, true>(xr, V, l2, nm2, k2, label, at_label);
+}
+
+// Form of the loss kernel: 0 neither, 1 TEST, 4 TEST and four groups in flight. The lines lie where the figures above cross.
+inline int ce_form(long rows, int V, bool bf16) {
+  if (bf16) return V <= 2 * CE_SWEEP ? 0 : V <= 20 * CE_SWEEP ? 1 : 4;
+  return V <= 6 * CE_SWEEP || rows <= 4 * otb_sm_count() ? 0 : V <= 8 * CE_SWEEP ? 1 : 4;
 }
 
 // sum (or sum of squares) of n floats: element i -> thread i % 1024, ascending fold, block_tree_sum.
@@ -882,9 +894,10 @@ extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long ro
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
-#define CE(U) \
-  DISPATCH_T(dtype, ce_zloss_kernel<T, U><<<(unsigned)rows, CE_THREADS, 0, S(stream)>>>((T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
-  if (V <= 8 * CE_SWEEP) { CE(1) } else { CE(4) }
+#define CE(U, TEST) \
+  DISPATCH_T(dtype, ce_zloss_kernel<T, U, TEST><<<(unsigned)rows, CE_THREADS, 0, S(stream)>>>((T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+  const int form = ce_form(rows, V, dtype);
+  if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
   return (int)cudaGetLastError();
 }

@@ -44,15 +44,22 @@ template <> struct Vec8<float> {
 template <typename T> struct Raw8;
 template <> struct Raw8<__nv_bfloat16> {
   uint4 v;
-  // the larger of mx and the elements (numbers win over NaN), the smaller of mn and the elements (NaN wins)
-  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+  // the larger of mx and the elements (numbers win over NaN)
+  __device__ __forceinline__ void largest(float& mx) const {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     __nv_bfloat162 b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) b[i] = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
     const __nv_bfloat162 hi = __hmax2(__hmax2(b[0], b[1]), __hmax2(b[2], b[3]));
-    const __nv_bfloat162 lo = __hmin2_nan(__hmin2_nan(b[0], b[1]), __hmin2_nan(b[2], b[3]));
     mx = fmaxf(mx, fmaxf(__low2float(hi), __high2float(hi)));
+  }
+  // the smaller of mn and the elements (NaN wins)
+  __device__ __forceinline__ void smallest(float& mn) const {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    __nv_bfloat162 b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
+    const __nv_bfloat162 lo = __hmin2_nan(__hmin2_nan(b[0], b[1]), __hmin2_nan(b[2], b[3]));
     asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(__low2float(lo)));
     asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(__high2float(lo)));
   }
@@ -68,13 +75,15 @@ template <> struct Raw8<__nv_bfloat16> {
 };
 template <> struct Raw8<float> {
   float4 a, b;
-  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+  __device__ __forceinline__ void largest(float& mx) const {
     const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      mx = fmaxf(mx, f[e]);
-      asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(f[e]));
-    }
+    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, f[e]);
+  }
+  __device__ __forceinline__ void smallest(float& mn) const {
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(f[e]));
   }
   __device__ __forceinline__ void load(const float* p) {
     a = *reinterpret_cast<const float4*>(p);

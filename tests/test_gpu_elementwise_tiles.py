@@ -64,7 +64,7 @@ def test_swiglu_forms(dtype, rows, F):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("V", [8, 4096, 4104, 16392, 70008, 128256])  # one group, whole sweeps, a ragged unroll, every occupancy
+@pytest.mark.parametrize("V", [8, 4096, 4104, 16392, 70008, 128256])  # one group, whole sweeps, ragged ones, both unrolls
 def test_loss_row_widths(dtype, V):
     g = torch.Generator().manual_seed(V)
     x = (3 * torch.randn(3, V, generator=g)).to(dtype)
@@ -107,3 +107,25 @@ def test_loss_rows_with_far_values(dtype):
     dev, host = K.ce_zloss_(a, labels.cuda(), 1e-4, 0.25), K.ce_zloss_(b, labels, 1e-4, 0.25)
     for p, q in zip((*dev, a), (*host, b)):
         _same(p, q, "loss")
+
+
+# every form of the loss kernel on both sides of each line (bf16: 8192 and 81920 columns, fp32: 24576 and 32768, and four rows per SM)
+@pytest.mark.parametrize("dtype,V", [(BF16, 8192), (BF16, 8200), (BF16, 81920), (BF16, 81928), (F32, 24576), (F32, 24584), (F32, 32768), (F32, 32776)])
+@pytest.mark.parametrize("rows", [8, 593])
+def test_loss_forms_with_far_values(dtype, V, rows):
+    """Ordinary rows beside rows whose exponents reach the clamp, at its edge, or hold infinities of either sign or a NaN."""
+    x = torch.randn(rows, V, generator=torch.Generator().manual_seed(V))
+    x[1] *= 100
+    x[2, 17] = -87.0 + float(x[2].max())
+    x[3, 4321] = -float("inf")
+    x[4, 1:] = -float("inf")
+    x[5, V - 1] = float("inf")
+    x[6, 100] = float("nan")
+    x[7, V - 3] = -87.5 + float(x[7].max())
+    x = x.to(dtype)
+    labels = torch.randint(0, V, (rows,), generator=torch.Generator().manual_seed(1))
+    labels[4] = 0
+    a, b = x.clone().cuda(), x.clone()
+    dev, host = K.ce_zloss_(a, labels.cuda(), 1e-4, 0.25), K.ce_zloss_(b, labels, 1e-4, 0.25)
+    for p, q, what in zip((*dev, a), (*host, b), ("ce", "lse", "gradient")):
+        torch.testing.assert_close(p.cpu(), q, rtol=0, atol=0, equal_nan=True, msg=what)
