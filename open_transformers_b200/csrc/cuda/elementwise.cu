@@ -316,11 +316,15 @@ __global__ void __launch_bounds__(256) head_rmsnorm_bwd_kernel(const T* __restri
 // --------------------------------------------------- gain-free QK-norm + RoPE
 // Over the first `heads` heads of a [rows, ld_in] buffer with head width D (<= 128, multiple of 4): lane l of a warp holds
 // elements 4l..4l+3 of a head (two rotation pairs). out[row, head*D + i]; rstd[row*heads + head]. lane_tree with VW = 4.
-// A warp takes ROPE_HEADS heads of one token: the token's cos / sin are read once for all of them and their loads (8 bytes
+// A warp takes NH heads of one token: the token's cos / sin are read once for all of them and their loads (8 bytes
 // per lane in bf16) are in flight together; one head per warp with 2-byte loads and two 64-bit divisions per warp was bound
 // by its instructions (76 us forward, 86 us backward at 16384 tokens x 20 heads x 128; with the row sums of the attention
 // backward regrouped the same way, that layer's pass went from 864 to 761 us with a 512-key window). VEC: bases and pitches allow the four-element accesses.
+// Four heads per warp need enough heads to fill the chip: us, one and four per warp, 100 tokens x 5 heads x 128 2.5 and 2.9,
+// 300 x 16 3.0 and 3.0, 1000 x 5 3.2 and 3.1, 2000 x 5 4.5 and 3.9; a single head per token leaves three quarters of the registers
+// unused (32768 x 1 x 64 backward: 9.5 and 11.5).
 constexpr int ROPE_HEADS = 4;
+inline bool rope_one_head(long rows, int heads) { return heads == 1 || rows * heads < 4800; }
 template <typename T, bool VEC> struct Vec4;
 template <> struct Vec4<__nv_bfloat16, true> {
   uint2 v;
@@ -356,31 +360,32 @@ template <typename T> struct Vec4<T, false> {
   }
 };
 // warp -> (token, first head); false past the end
+template <int NH>
 __device__ __forceinline__ bool rope_place(long rows, int heads, long& row, int& head0) {
-  const int groups = (heads + ROPE_HEADS - 1) / ROPE_HEADS;
+  const int groups = (heads + NH - 1) / NH;
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wid >= rows * groups) return false;
   row = (rows * groups) >> 31 ? wid / groups : (long)((unsigned)wid / (unsigned)groups);
-  head0 = (int)(wid - row * groups) * ROPE_HEADS;
+  head0 = (int)(wid - row * groups) * NH;
   return true;
 }
 __device__ __forceinline__ int rope_pos(long row, int seq_len) { return row >> 31 ? (int)(row % seq_len) : (int)((unsigned)row % (unsigned)seq_len); }
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, int NH>
 __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restrict__ in, long ld_in, T* __restrict__ out, long ld_out,
                                        float* __restrict__ rstd_out, const float* __restrict__ cosb,
                                        const float* __restrict__ sinb, long rows, int heads, int D, int seq_len,
                                        int do_norm, float inv_d, float eps) {
   long row;
   int head0;
-  if (!rope_place(rows, heads, row, head0)) return;
+  if (!rope_place<NH>(rows, heads, row, head0)) return;
   const int lane = threadIdx.x & 31;
   const bool active = lane * 4 < D;
-  const int n = min(ROPE_HEADS, heads - head0);
-  Vec4<T, VEC> raw[ROPE_HEADS];
+  const int n = min(NH, heads - head0);
+  Vec4<T, VEC> raw[NH];
   const T* p = in + row * ld_in + (long)head0 * D + lane * 4;
 #pragma unroll
-  for (int i = 0; i < ROPE_HEADS; ++i)
+  for (int i = 0; i < NH; ++i)
     if (active && i < n) raw[i].load(p + i * D);
   float c[2] = {0.f, 0.f}, s[2] = {0.f, 0.f};
   if (active) {
@@ -390,7 +395,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restric
   }
   T* o = out + row * ld_out + (long)head0 * D + lane * 4;
 #pragma unroll
-  for (int i = 0; i < ROPE_HEADS; ++i) {
+  for (int i = 0; i < NH; ++i) {
     if (i >= n) break;  // (the same for the whole warp)
     float f[4] = {0.f, 0.f, 0.f, 0.f};
     if (active) raw[i].unpack(f);
@@ -417,23 +422,23 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restric
   }
 }
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, int NH>
 __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restrict__ dout, long ld_dout, const T* __restrict__ in, long ld_in,
                                        const float* __restrict__ rstd_in, T* __restrict__ din, long ld_din,
                                        const float* __restrict__ cosb, const float* __restrict__ sinb, long rows,
                                        int heads, int D, int seq_len, int do_norm, float inv_d) {
   long row;
   int head0;
-  if (!rope_place(rows, heads, row, head0)) return;
+  if (!rope_place<NH>(rows, heads, row, head0)) return;
   const int lane = threadIdx.x & 31;
   const bool active = lane * 4 < D;
-  const int n = min(ROPE_HEADS, heads - head0);
-  Vec4<T, VEC> rd[ROPE_HEADS], rx[ROPE_HEADS];
-  float rstd[ROPE_HEADS];
+  const int n = min(NH, heads - head0);
+  Vec4<T, VEC> rd[NH], rx[NH];
+  float rstd[NH];
   const T* pd = dout + row * ld_dout + (long)head0 * D + lane * 4;
   const T* px = in + row * ld_in + (long)head0 * D + lane * 4;
 #pragma unroll
-  for (int i = 0; i < ROPE_HEADS; ++i) {
+  for (int i = 0; i < NH; ++i) {
     if (active && i < n) {
       rd[i].load(pd + i * D);
       if (do_norm) rx[i].load(px + i * D);
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restric
   }
   T* o = din + row * ld_din + (long)head0 * D + lane * 4;
 #pragma unroll
-  for (int i = 0; i < ROPE_HEADS; ++i) {
+  for (int i = 0; i < NH; ++i) {
     if (i >= n) break;
     float g[4] = {0.f, 0.f, 0.f, 0.f};
     if (active) {
@@ -853,11 +858,14 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
                                    const float* sinb, long rows, int heads, int D, int seq_len, int do_norm,
                                    float inv_d, float eps, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
-  const unsigned grid = blocks_for(rows * ((heads + ROPE_HEADS - 1) / ROPE_HEADS), 8);
   const bool vec = four_aligned(in, ld_in, dtype) && four_aligned(out, ld_out, dtype);
-#define QF(V) DISPATCH_T(dtype, qknorm_rope_fwd_kernel<T, V><<<grid, 256, 0, S(stream)>>>( \
+#define QF(V, NH) DISPATCH_T(dtype, qknorm_rope_fwd_kernel<T, V, NH><<<blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream)>>>( \
                         (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d, eps);)
-  if (vec) { QF(true) } else { QF(false) }
+  if (rope_one_head(rows, heads)) {
+    if (vec) { QF(true, 1) } else { QF(false, 1) }
+  } else {
+    if (vec) { QF(true, ROPE_HEADS) } else { QF(false, ROPE_HEADS) }
+  }
 #undef QF
   return (int)cudaGetLastError();
 }
@@ -865,11 +873,14 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
                                    void* din, long ld_din, const float* cosb, const float* sinb, long rows, int heads,
                                    int D, int seq_len, int do_norm, float inv_d, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
-  const unsigned grid = blocks_for(rows * ((heads + ROPE_HEADS - 1) / ROPE_HEADS), 8);
   const bool vec = four_aligned(dout, ld_dout, dtype) && four_aligned(in, ld_in, dtype) && four_aligned(din, ld_din, dtype);
-#define QB(V) DISPATCH_T(dtype, qknorm_rope_bwd_kernel<T, V><<<grid, 256, 0, S(stream)>>>( \
+#define QB(V, NH) DISPATCH_T(dtype, qknorm_rope_bwd_kernel<T, V, NH><<<blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream)>>>( \
                         (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d);)
-  if (vec) { QB(true) } else { QB(false) }
+  if (rope_one_head(rows, heads)) {
+    if (vec) { QB(true, 1) } else { QB(false, 1) }
+  } else {
+    if (vec) { QB(true, ROPE_HEADS) } else { QB(false, ROPE_HEADS) }
+  }
 #undef QB
   return (int)cudaGetLastError();
 }

@@ -26,7 +26,9 @@ def test_rmsnorm_forward_widths(dtype, rows, D):
 # heads that do not fill a warp's group, narrow heads, and ``pad``: a row pitch (or an offset) that forbids the wide loads
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("norm", [True, False])
-@pytest.mark.parametrize("rows,heads,D,seq,pad", [(1, 1, 4, 1, 0), (37, 5, 128, 10, 0), (50, 3, 64, 50, 0), (33, 6, 20, 11, 1), (16, 4, 128, 16, 2)])
+@pytest.mark.parametrize("rows,heads,D,seq,pad", [(1, 1, 4, 1, 0), (37, 5, 128, 10, 0), (50, 3, 64, 50, 0), (33, 6, 20, 11, 1), (16, 4, 128, 16, 2),
+                                                  # four heads per warp (4800 heads and more), not all of them there; one head per token
+                                                  (961, 5, 128, 31, 0), (1600, 3, 64, 50, 0), (800, 6, 20, 11, 1), (1201, 4, 128, 1201, 2), (5000, 1, 64, 100, 0)])
 def test_qknorm_rope_groups(dtype, norm, rows, heads, D, seq, pad):
     g = torch.Generator().manual_seed(rows + D)
     cos, sin = K.rope_tables(seq, D, 10000.0, "cpu")
