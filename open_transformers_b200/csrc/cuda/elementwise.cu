@@ -25,7 +25,7 @@ namespace {
 // ------------------------------------------------------------------ RMSNorm
 // One warp per row; lane_tree with VW = 8. The row stays in registers (as loaded) between the sum of squares and the
 // scaling, so all of its loads are in flight at once and x is read once. MAXC = max number of 8-wide column chunks per
-// lane (D <= 256 * MAXC); wider rows take the kernel below, which reads x twice.
+// lane (D <= 256 * MAXC).
 template <typename T, int MAXC>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                                          float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
     }
   }
 }
-// The same row of any width.
+// The same row of any width: x is read twice, the second time from the nearer caches.
 template <typename T>
 __global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                         float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
@@ -105,6 +105,16 @@ __global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __rest
     }
     Vec8<T>::store(yr + c, o);
   }
+}
+
+// Where the row stays in registers. The second reading of a bf16 row is cheap (L1) and a warp that holds a long row has less to
+// overlap, so bf16 rows of 1024 columns and more gain only where that reading misses, in long rows of a tensor far above the
+// L2; fp32 rows, twice the bytes, gain at every width. us, two readings and registers: bf16 64 x 2048 3.6 and 4.5, 1200 x 1024
+// 2.95 and 3.3, 8192 x 2048 9.2 and 10.4, 16384 x 2048 23.0 and 24.7, 4096 x 4096 10.3 and 13.9, 16384 x 4096 57.6 and 50.1; 1200 x
+// 768 3.15 and 3.05; fp32 64 x 2048 5.2 and 4.7, 16384 x 2048 64 and 53.
+inline bool rmsnorm_in_registers(long rows, int D, bool bf16) {
+  if (D > 4096) return false;
+  return !bf16 || D <= 768 || (D > 2048 && rows >= 12288);
 }
 
 // One CTA of SLAB warps per slab of SLAB rows, one warp per row: the row stays in registers (as loaded, 16-byte
@@ -809,9 +819,17 @@ inline bool four_aligned(const void* p, long ld, int bf16) { return ld % 4 == 0 
 extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long rows, int D, float inv_d,
                                float eps, int dtype, void* stream) {
   if (D % 8) return -2;
-#define RF(KERN) DISPATCH_T(dtype, KERN<<<blocks_for(rows, 8), 256, 0, S(stream)>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps);)
+#define RF(KERN) KERN<<<blocks_for(rows, 8), 256, 0, S(stream)>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
 #define RFC(MAXC) RF((rmsnorm_fwd_kernel<T, MAXC>))
-  if (D <= 256) { RFC(1) } else if (D <= 1024) { RFC(4) } else if (D <= 2048) { RFC(8) } else if (D <= 4096) { RFC(16) } else { RF(rmsnorm_fwd_wide_kernel<T>) }
+  if (!rmsnorm_in_registers(rows, D, dtype)) {
+    DISPATCH_T(dtype, RF(rmsnorm_fwd_wide_kernel<T>);)
+  } else if (dtype) {
+    using T = __nv_bfloat16;
+    if (D <= 256) RFC(1); else if (D <= 768) RFC(3); else RFC(16);
+  } else {
+    using T = float;
+    if (D <= 256) RFC(1); else if (D <= 1024) RFC(4); else if (D <= 2048) RFC(8); else RFC(16);
+  }
 #undef RFC
 #undef RF
   return (int)cudaGetLastError();
