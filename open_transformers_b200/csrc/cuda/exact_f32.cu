@@ -189,7 +189,7 @@ int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, in
 }
 
 // ------------------------------------------------------------------------- attention
-// All three kernels work on 64-row tiles whose operands sit TRANSPOSED in shared memory ([d][64 + 4]): a product over d
+// The three main kernels work on 64-row tiles whose operands sit TRANSPOSED in shared memory ([d][64 + 4]): a product over d
 // reads one float4 of rows and one of columns per step for 4 x 4 (or 4 x 8) chains, and the accumulations over queries /
 // keys read the same arrays as float4 along the row index, four links of each chain at a time. Before (one warp per row,
 // every operand straight from global memory, one key per lane) each multiply-add cost a strided load:
@@ -412,6 +412,162 @@ __global__ void attn_f32_delta_kernel(const float* __restrict__ dO, long lddo, c
     const long bb = row / T, t = row - bb * T;
     delta[(bb * H + h) * T + t] = acc;
   }
+}
+
+// ---- sequences far shorter than a tile: one warp per query, or per key in dK / dV, and one pair per lane; no block of keys
+// ever moves the running maximum (T <= FKB). Same chains, same bits. The tiles above spend as long on one query as on 64 (4
+// heads, us, this form and tiles: forward 1 token x 64 5.5 and 15.8, 16 tokens 9.7 and 17.4, 33 tokens 15.8 and 18.5, x 128 19.9
+// and 28.7; 48 tokens 27.6 and 18.5; backward 1 token x 64 13.7 and 27.2, 16 tokens 20.2 and 29.2, 32 tokens 31.2 and 30.1).
+__device__ __forceinline__ float chain(const float* __restrict__ a, const float* __restrict__ b, int D) {
+  float s = 0.0f;
+  for (int d = 0; d < D; ++d) s = __fmaf_rn(a[d], b[d], s);
+  return s;
+}
+__global__ void __launch_bounds__(128)
+attn_f32_fwd_short_kernel(const float* __restrict__ qk, long ldqk, const float* __restrict__ qkv, long ldqkv, float* __restrict__ O, long ldo,
+                          float* __restrict__ lse, int B, int T, int H, int Hkv, int D, int window, float c_log2) {
+  __shared__ float sp[4][FKB];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long wid = (long)blockIdx.x * 4 + w;
+  if (wid >= (long)B * H * T) return;
+  const int qi = (int)(wid % T), h = (int)((wid / T) % H), g = h / (H / Hkv);
+  const long row0 = wid / ((long)T * H) * T, qrow = row0 + qi;  // first row of the sequence; this query's
+  float s[4], mx = -INFINITY;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int kj = lane + 32 * u;
+    s[u] = kj < T && !masked(qi, kj, window) ? chain(qk + qrow * ldqk + (long)h * D, qk + (row0 + kj) * ldqk + (long)(H + g) * D, D) : -INFINITY;
+    mx = fmaxf(mx, s[u]);
+  }
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const float m_run = __fmul_rn(mx, c_log2);
+  const float m_safe = (m_run == -INFINITY) ? 0.0f : m_run;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) sp[w][lane + 32 * u] = (s[u] == -INFINITY) ? 0.0f : det_exp2_attn(__fmaf_rn(s[u], c_log2, -m_safe));
+  __syncwarp();
+  float l_part = 0.0f;
+  if (lane < 4) {  // the four quarter-row sums: even and odd keys are ascending chains, then added
+    float le = 0.0f, lo = 0.0f;
+    for (int e = lane * 32; e < lane * 32 + 32; e += 2) { le = __fadd_rn(le, sp[w][e]); lo = __fadd_rn(lo, sp[w][e + 1]); }
+    l_part = __fadd_rn(le, lo);
+  }
+  float pv[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int e = 0; e < T; ++e) {
+    const float p = sp[w][e];
+    if (p == 0.0f) continue;
+    const float* vr = qkv + (row0 + e) * ldqkv + (long)(H + Hkv + g) * D;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int d = lane + 32 * u;
+      if (d < D) pv[u] = __fmaf_rn(p, vr[d], pv[u]);
+    }
+  }
+  const float l0 = __shfl_sync(0xffffffffu, l_part, 0), l1 = __shfl_sync(0xffffffffu, l_part, 1);
+  const float l2 = __shfl_sync(0xffffffffu, l_part, 2), l3 = __shfl_sync(0xffffffffu, l_part, 3);
+  const float l_tot = __fadd_rn(__fadd_rn(__fadd_rn(l0, l1), l2), l3);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int d = lane + 32 * u;
+    if (d < D) O[qrow * ldo + (long)h * D + d] = __fdiv_rn(__fadd_rn(0.0f, pv[u]), l_tot);  // (0: the output before this block)
+  }
+  if (lane == 0) lse[(wid / T) * T + qi] = __fmaf_rn(det_logf(l_tot), 1.44269504088896341f, m_run);
+}
+// p and ds of one (query, key) pair
+__device__ __forceinline__ void pair_p_ds(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ dor,
+                                          const float* __restrict__ v, float l2, float dl, int D, float c_log2, float scale, float& p, float& ds) {
+  p = det_exp2_attn(__fmaf_rn(chain(q, k, D), c_log2, -l2));
+  ds = __fmul_rn(__fmul_rn(p, __fadd_rn(chain(dor, v, D), -dl)), scale);
+}
+__global__ void __launch_bounds__(128)
+attn_f32_bwd_kv_short_kernel(const float* __restrict__ qk, long ldqk, const float* __restrict__ qkv, long ldqkv, const float* __restrict__ dO, long lddo,
+                             const float* __restrict__ lse, const float* __restrict__ delta, float* __restrict__ dqk, long lddqk,
+                             float* __restrict__ dqkv, long lddqkv, int B, int T, int H, int Hkv, int D, int window, float c_log2, float scale) {
+  __shared__ float sp[4][32], sds[4][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long wid = (long)blockIdx.x * 4 + w;
+  if (wid >= (long)B * Hkv * T) return;
+  const int kj = (int)(wid % T), g = (int)((wid / T) % Hkv), G = H / Hkv;
+  const long b = wid / ((long)T * Hkv), krow = b * T + kj;
+  const float* k = qk + krow * ldqk + (long)(H + g) * D;
+  const float* v = qkv + krow * ldqkv + (long)(H + Hkv + g) * D;
+  float dk[4] = {0.f, 0.f, 0.f, 0.f}, dv[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int h = g * G; h < (g + 1) * G; ++h) {
+    for (int qb = kj / 32 * 32; qb < T; qb += 32) {
+      const int qi = qb + lane;
+      const long qrow = b * T + qi, st = (b * H + h) * T + qi;
+      float p = 0.0f, ds = 0.0f;
+      if (qi < T && !masked(qi, kj, window))
+        pair_p_ds(qk + qrow * ldqk + (long)h * D, k, dO + qrow * lddo + (long)h * D, v, lse[st], delta[st], D, c_log2, scale, p, ds);
+      sp[w][lane] = p;
+      sds[w][lane] = ds;
+      __syncwarp();
+      for (int e = 0; e < 32 && qb + e < T; ++e) {
+        if (masked(qb + e, kj, window)) continue;
+        const long row = b * T + qb + e;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int d = lane + 32 * u;
+          if (d < D) {
+            dv[u] = __fmaf_rn(sp[w][e], dO[row * lddo + (long)h * D + d], dv[u]);
+            dk[u] = __fmaf_rn(sds[w][e], qk[row * ldqk + (long)h * D + d], dk[u]);
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int d = lane + 32 * u;
+    if (d < D) {
+      dqk[krow * lddqk + (long)(H + g) * D + d] = dk[u];
+      dqkv[krow * lddqkv + (long)(H + Hkv + g) * D + d] = dv[u];
+    }
+  }
+}
+__global__ void __launch_bounds__(128)
+attn_f32_bwd_q_short_kernel(const float* __restrict__ qk, long ldqk, const float* __restrict__ qkv, long ldqkv, const float* __restrict__ dO, long lddo,
+                            const float* __restrict__ lse, const float* __restrict__ delta, float* __restrict__ dqk, long lddqk, int B, int T, int H,
+                            int Hkv, int D, int window, float c_log2, float scale) {
+  __shared__ float sds[4][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long wid = (long)blockIdx.x * 4 + w;
+  if (wid >= (long)B * H * T) return;
+  const int qi = (int)(wid % T), h = (int)((wid / T) % H), g = h / (H / Hkv);
+  const long row0 = wid / ((long)T * H) * T, qrow = row0 + qi;
+  float dq[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int kb = 0; kb <= qi; kb += 32) {
+    const int kj = kb + lane;
+    float p = 0.0f, ds = 0.0f;
+    if (kj < T && !masked(qi, kj, window))
+      pair_p_ds(qk + qrow * ldqk + (long)h * D, qk + (row0 + kj) * ldqk + (long)(H + g) * D, dO + qrow * lddo + (long)h * D,
+                qkv + (row0 + kj) * ldqkv + (long)(H + Hkv + g) * D, lse[(wid / T) * T + qi], delta[(wid / T) * T + qi], D, c_log2, scale, p, ds);
+    sds[w][lane] = ds;
+    __syncwarp();
+    for (int e = 0; e < 32 && kb + e <= qi; ++e) {
+      if (masked(qi, kb + e, window)) continue;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int d = lane + 32 * u;
+        if (d < D) dq[u] = __fmaf_rn(sds[w][e], qk[(row0 + kb + e) * ldqk + (long)(H + g) * D + d], dq[u]);
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int d = lane + 32 * u;
+    if (d < D) dqk[qrow * lddqk + (long)h * D + d] = dq[u];
+  }
+}
+// Whether a call takes these: where the tiles leave SMs idle up to 40 tokens (backward 31); with more tiles than SMs, whose rate
+// then counts, up to 16 (8): 256 heads of 16 tokens x 64 forward 23.7 and 25.6, of 31 57 and 27; backward 4 tokens 15 and 41, 16
+// tokens 72 and 43; 2048 heads of 8 tokens 36 and 155, backward 106 and 251, of 16 331 and 267.
+inline bool short_rows(int T, long heads, bool backward) {
+  static_assert(FKB >= 40, "one block of keys");
+  if (heads <= otb_sm_count()) return T <= (backward ? 31 : 40);
+  return T <= (backward ? 8 : 16);
 }
 
 // s and dp of a 4 x 4 patch (rows from tiles R1 / R2, columns from C1 / C2), each one chain ascending in d
@@ -682,6 +838,10 @@ extern "C" int otb_attn_f32_fwd(const float* qk, long ldqk, const float* qkv, lo
   if (D > 128 || H % Hkv) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
+  if (short_rows(T, (long)B * H, false)) {
+    attn_f32_fwd_short_kernel<<<(unsigned)(((long)B * H * T + 3) / 4), 128, 0, s>>>(qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2);
+    return (int)cudaGetLastError();
+  }
   const int vec = D % 4 == 0 && aligned16(qk, ldqk) && aligned16(qkv, ldqkv);
   if (D <= 64) return attn_f32_fwd<64>(qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2, vec, s);
   return attn_f32_fwd<128>(qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2, vec, s);
@@ -695,6 +855,13 @@ extern "C" int otb_attn_f32_bwd(const float* qk, long ldqk, const float* qkv, lo
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
   const long w1 = (long)B * T * H;
   attn_f32_delta_kernel<<<(unsigned)((w1 + 7) / 8), 256, 0, s>>>(dO, lddo, O, ldo, delta, B, T, H, D);
+  if (short_rows(T, (long)B * H, true)) {
+    attn_f32_bwd_kv_short_kernel<<<(unsigned)(((long)B * Hkv * T + 3) / 4), 128, 0, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv,
+                                                                                        B, T, H, Hkv, D, window, c_log2, scale);
+    attn_f32_bwd_q_short_kernel<<<(unsigned)((w1 + 3) / 4), 128, 0, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, B, T, H, Hkv, D, window,
+                                                                        c_log2, scale);
+    return (int)cudaGetLastError();
+  }
   const int vec = D % 4 == 0 && aligned16(qk, ldqk) && aligned16(qkv, ldqkv) && aligned16(dO, lddo);
   if (D <= 64)
     return attn_f32_bwd<64>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv, B, T, H, Hkv, D, window, c_log2, scale, vec, s);

@@ -33,7 +33,11 @@ def test_gemm_tiles(a_mn, b_mn, M, N, K_, pad):
 
 
 @pytest.mark.parametrize("B,T,H,Hkv,D,window", [(1, 1, 1, 1, 4, 0), (2, 63, 2, 1, 64, 0), (1, 65, 4, 2, 48, 0), (1, 200, 2, 2, 128, 0),
-                                                (1, 129, 2, 1, 72, 32), (2, 300, 2, 1, 64, 96), (1, 330, 1, 1, 6, 128)])
+                                                (1, 129, 2, 1, 72, 32), (2, 300, 2, 1, 64, 96), (1, 330, 1, 1, 6, 128),
+                                                # one warp per row up to 31 (backward) and 40 (forward) tokens, tiles above; with more heads
+                                                # than SMs up to 8 and 16
+                                                (3, 5, 4, 2, 64, 0), (2, 31, 2, 1, 128, 8), (2, 32, 4, 1, 40, 0), (1, 40, 2, 2, 6, 32), (2, 41, 3, 1, 64, 16),
+                                                (120, 8, 4, 2, 16, 0), (120, 9, 4, 2, 16, 3), (120, 16, 2, 1, 64, 0), (120, 17, 2, 2, 8, 0)])
 def test_attention_tiles(B, T, H, Hkv, D, window):
     g = torch.Generator().manual_seed(T + D)
     qk = torch.randn(B * T, (H + Hkv) * D, generator=g)
