@@ -74,8 +74,9 @@ struct Slab {
   }
 };
 
-template <int TM, int TN, int RM, int RN, bool A_MN, bool B_MN, int EPI>
-__global__ void __launch_bounds__(F32Tile<TM, TN, RM, RN>::NT)
+// RES: CTAs that an SM holds at least, at the cost of spilled registers (0: as the compiler likes).
+template <int TM, int TN, int RM, int RN, int RES, bool A_MN, bool B_MN, int EPI>
+__global__ void __launch_bounds__(F32Tile<TM, TN, RM, RN>::NT, RES)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
                 const float* __restrict__ R, int M, int N, int K, long lda, long ldb, long ldc, long ldr, int vec) {
   using Tile = F32Tile<TM, TN, RM, RN>;
@@ -168,12 +169,12 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   }
 }
 
-template <int TM, int TN, int RM, int RN>
+template <int TM, int TN, int RM, int RN, int RES = 0>
 int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, int M, int N, int K, long lda, long ldb, long ldc, long ldr,
                     int a_mn, int b_mn, int epi, int vec, cudaStream_t s) {
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
 #define GF(AM, BM, E) \
-  gemm_f32_kernel<TM, TN, RM, RN, AM, BM, E><<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec)
+  gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E><<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec)
 #define GE(AM, BM)                                      \
   switch (epi) {                                         \
     case 0: case 1: GF(AM, BM, 0); break;                \
@@ -803,7 +804,14 @@ extern "C" int otb_gemm_f32(const float* A, const float* B, float* C, const floa
   const long sms = otb_sm_count();
   auto tiles = [&](int t) { return (long)((M + t - 1) / t) * ((N + t - 1) / t); };
   if (tiles(128) >= 2 * sms) return launch_gemm_f32<128, 128, 8, 8>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
-  if (tiles(64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
+  if (tiles(64) >= sms) {
+    // Two 64-wide tiles are resident on an SM, or three with some registers spilled; r tiles take r times as long as one, so
+    // the smaller r x waves wins (K-major, 1429 x 1214 x 2307, 437 tiles: 502 us with two, 365 with three; 1337 x 1734 x 696, 588
+    // tiles: 127 and 154). An MN-major B takes fewer registers and fits three as it is, but for the accumulating epilogue.
+    auto cost = [&](long r) { return r * ((tiles(64) + r * sms - 1) / (r * sms)); };
+    if ((!b_mn || epi == 2) && cost(3) < cost(2)) return launch_gemm_f32<64, 64, 4, 4, 3>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
+    return launch_gemm_f32<64, 64, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
+  }
   return launch_gemm_f32<32, 32, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
 }
 

@@ -14,7 +14,8 @@ def _same(dev, host, what):
 # one shape per tile size (32, 64 and 128 wide: the rule counts tiles against the SMs), ragged in every direction; ``pad``
 # makes the row pitch no multiple of four elements, which takes the scalar loads
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
-@pytest.mark.parametrize("M,N,K_,pad", [(33, 31, 5, 0), (65, 130, 67, 3), (770, 900, 33, 0), (2309, 2311, 17, 0), (2309, 2311, 18, 1)])
+@pytest.mark.parametrize("M,N,K_,pad", [(33, 31, 5, 0), (65, 130, 67, 3), (770, 900, 33, 0), (2309, 2311, 17, 0), (2309, 2311, 18, 1),
+                                        (1180, 1155, 37, 0), (1180, 1155, 70, 1)])  # (64-wide tiles, three to an SM)
 def test_gemm_tiles(a_mn, b_mn, M, N, K_, pad):
     g = torch.Generator().manual_seed(M + K_)
 
