@@ -1092,7 +1092,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
           }
           if (!ok) break;
           mma_commit(&bars->kv_empty[st]);
-          if (i + 2 == n || n == 1) mma_commit(&bars->qdo_empty);  // the item's last scores are on their way
+          if (i + 2 == n) mma_commit(&bars->qdo_empty);  // the item's last scores are on their way (an item has two steps at least)
         }
         ring += n;
       }

@@ -9,8 +9,10 @@ from open_transformers_b200.ops.native import cuda_lib
 pytestmark = pytest.mark.gpu
 
 
-# one pair of tiles per head; a lone last tile (its partner's warps sit the item out); a window that skips key blocks
-@pytest.mark.parametrize("B,T,H,Hkv,D,window", [(90, 192, 4, 2, 64, 0), (40, 320, 4, 4, 64, 96), (33, 384, 6, 2, 128, 128)])
+# one pair of tiles per head; a lone last tile (its partner's warps sit the item out); a window that skips key blocks; several
+# items of a single key block, whole and ragged, on every CTA
+@pytest.mark.parametrize("B,T,H,Hkv,D,window", [(90, 192, 4, 2, 64, 0), (40, 320, 4, 4, 64, 96), (33, 384, 6, 2, 128, 128), (200, 64, 4, 4, 64, 0),
+                                                (120, 100, 4, 2, 128, 0)])
 def test_many_items(B, T, H, Hkv, D, window):
     g = torch.Generator().manual_seed(T)
     qk, qkv, dO = (torch.randn(B * T, n * D, generator=g).to(torch.bfloat16) for n in (H + Hkv, H + 2 * Hkv, H))
