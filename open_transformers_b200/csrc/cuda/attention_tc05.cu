@@ -77,12 +77,15 @@ struct BarsX : Bars {
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
-// The bf16 kernels are persistent, one CTA per SM: every role walks the same list of work items, barrier phases and ring
+// The bf16 forward, dQ and transposed dK/dV kernels are persistent, one CTA per SM (the dK/dV kernel for lengths that are no
+// multiple of 64 and the int8 P V forward are not): every role walks the same list of work items, barrier phases and ring
 // positions running on, so the loads and first products of an item are under way while the previous one's results are read
 // out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about 8 us, were
 // exposed: a quarter of an item's time with a 512-key window. 4 x 4096 tokens, 16 heads x 128, forward and backward: 1790 ->
-// 1612 us full causal, 744 -> 691 us windowed.) Item r * gridDim + c of the list goes to CTA c in even turns
-// r and to the mirrored CTA in odd ones; the list is sorted by falling work, so the sums come out even.
+// 1612 us full causal, 744 -> 691 us windowed. Where every item has a CTA of its own the walk costs a little: forward 1 x 2048
+// 56 -> 59 us, 1 x 333 x 12 heads x 64 14.6 -> 15.1.) Item r * gridDim + c of the list goes to CTA c in even turns
+// r and to the mirrored CTA in odd ones; the list is sorted by falling work (but for a lone last tile, which comes first), so
+// the sums come out nearly even.
 __device__ __forceinline__ int work_item(int turn) {
   return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
