@@ -32,8 +32,16 @@ struct F32Tile {
   static constexpr int AHEAD = TM >= 128 ? 1 : 2;
 };
 
-// One operand's share of a k-slab, held in registers between the global load and the shared-memory store.
-template <int TR, int NT, bool MN, int GK>
+// v = *p where `in`, else v stays: a predicated load. A branch around it would make the loaded value meet the zeros of the
+// other side in a move, which waits for the load there and then instead of two slabs later.
+__device__ __forceinline__ void load_if(float4& v, const float* p, bool in) {
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+      : "l"(p), "r"((int)in));
+}
+// One operand's share of a k-slab, held in registers between the global load and the shared-memory store. WHOLE: every float4
+// is aligned and lies inside the operand or outside it as a whole.
+template <int TR, int NT, bool MN, int GK, bool WHOLE>
 struct Slab {
   static constexpr int PER = TR * GK / 4 / NT;  // float4 per thread
   static_assert(TR * GK / 4 % NT == 0, "the slab splits evenly over the CTA");
@@ -44,8 +52,13 @@ struct Slab {
       const int i = threadIdx.x + p * NT;
       // MN-major: four rows of one k; K-major: four k of one row (lanes along the rows: conflict-free stores)
       const int r = r0 + (MN ? (i % (TR / 4)) * 4 : i % TR), k = k0 + (MN ? i / (TR / 4) : (i / TR) * 4);
-      float f[4] = {0.f, 0.f, 0.f, 0.f};
       const bool in = r < R && k < K;
+      if constexpr (WHOLE) {
+        v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        load_if(v[p], X + (MN ? (long)k * ld + r : (long)r * ld + k), in);
+        continue;
+      }
+      float f[4] = {0.f, 0.f, 0.f, 0.f};
       if (in) {
         const float* q = X + (MN ? (long)k * ld + r : (long)r * ld + k);
         if (vec && (MN ? r + 4 <= R : k + 4 <= K)) {
@@ -75,7 +88,7 @@ struct Slab {
 };
 
 // RES: CTAs that an SM holds at least, at the cost of spilled registers (0: as the compiler likes).
-template <int TM, int TN, int RM, int RN, int RES, bool A_MN, bool B_MN, int EPI>
+template <int TM, int TN, int RM, int RN, int RES, bool A_MN, bool B_MN, int EPI, bool WHOLE>
 __global__ void __launch_bounds__(F32Tile<TM, TN, RM, RN>::NT, RES)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
                 const float* __restrict__ R, int M, int N, int K, long lda, long ldb, long ldc, long ldr, int vec) {
@@ -94,8 +107,8 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
     for (int j = 0; j < RN; ++j)
       // the accumulating epilogue continues the chain from the value already in C
       acc[i][j] = (EPI == 2 && mrow(i) < M && ncol(j) < N) ? C[(long)mrow(i) * ldc + ncol(j)] : 0.0f;
-  Slab<TM, NT, A_MN, GK> la[AHEAD];
-  Slab<TN, NT, B_MN, GK> lb[AHEAD];
+  Slab<TM, NT, A_MN, GK, WHOLE> la[AHEAD];
+  Slab<TN, NT, B_MN, GK, WHOLE> lb[AHEAD];
   const bool va = vec & 1, vb = vec & 2, vc = vec & 4;
   la[0].load(A, lda, m0, M, 0, K, va);
   lb[0].load(B, ldb, n0, N, 0, K, vb);
@@ -173,8 +186,12 @@ template <int TM, int TN, int RM, int RN, int RES = 0>
 int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, int M, int N, int K, long lda, long ldb, long ldc, long ldr,
                     int a_mn, int b_mn, int epi, int vec, cudaStream_t s) {
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-#define GF(AM, BM, E) \
-  gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E><<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec)
+  const bool whole = (vec & 3) == 3 && (a_mn ? M : K) % 4 == 0 && (b_mn ? N : K) % 4 == 0;
+#define GF(AM, BM, E)                                                                                                            \
+  do {                                                                                                                           \
+    auto kern = whole ? gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, true> : gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, false>; \
+    kern<<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec);                              \
+  } while (0)
 #define GE(AM, BM)                                      \
   switch (epi) {                                         \
     case 0: case 1: GF(AM, BM, 0); break;                \
