@@ -62,6 +62,20 @@ inline unsigned quant_blocks(long n) { return (unsigned)max(1L, min((long)blocks
 
 __device__ __forceinline__ float clamp_q(float q, float qmax) { return fminf(fmaxf(q, -qmax), qmax); }
 
+// Bits whose low byte is the two's complement of rint(x / step), for a finite x of at most 128 step. The division is an
+// IEEE one without the divider: with y = 1 / step correctly rounded, two steps q <- q + (x - q step) y from q = x y give the
+// correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990: the first makes q faithful, the second correct), provided
+// that nothing over- or underflows, which the bounds on the step see to (a tiny x whose remainder is subnormal has a quotient
+// near 0). Adding 1.5 * 2^23 rounds half to even and leaves the integer in the low bits. A NaN gives -qmax, as in the general
+// form.
+constexpr float DIVIDES_FROM = 0x1p-80f, DIVIDES_TO = 0x1p100f;
+__device__ __forceinline__ uint32_t quant_bits(float x, float step, float y, float qmax) {
+  float q = __fmul_rn(x, y);
+  q = __fmaf_rn(__fmaf_rn(-q, step, x), y, q);
+  q = __fmaf_rn(__fmaf_rn(-q, step, x), y, q);
+  return __float_as_uint(__fadd_rn(clamp_q(q, qmax), 12582912.0f));
+}
+
 // The maximum is that of the AMAX_BLOCKS partial maxima: a resident CTA folds them itself (a few KB from L2, once) and then walks
 // its share of x, which spares a one-CTA launch between the two passes.
 template <typename T>
@@ -73,6 +87,8 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const T* __restrict__ x,
   m = block_max(m, sh);
   const float step = fmaxf(__fmul_rn(m, inv_qmax), FLT_MIN);
   if (blockIdx.x == 0 && threadIdx.x == 0) step_out[0] = step;
+  const bool divides = step >= DIVIDES_FROM && step <= DIVIDES_TO;
+  const float y = __frcp_rn(step);
   const long stride = (long)gridDim.x * blockDim.x * 8;
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += stride) {
     if (i + 8 > n) {
@@ -82,10 +98,19 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const T* __restrict__ x,
     float f[8];
     Vec8<T>::load(x + i, f);
     uint32_t w[2] = {0, 0};
+    if (divides) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int v = (int)clamp_q(rintf(__fdiv_rn(f[e], step)), qmax);
-      w[e >> 2] |= (uint32_t)(v & 0xFF) << (8 * (e & 3));
+      for (int e = 0; e < 8; e += 4) {
+        const uint32_t b01 = __byte_perm(quant_bits(f[e], step, y, qmax), quant_bits(f[e + 1], step, y, qmax), 0x0040);
+        const uint32_t b23 = __byte_perm(quant_bits(f[e + 2], step, y, qmax), quant_bits(f[e + 3], step, y, qmax), 0x0040);
+        w[e >> 2] = __byte_perm(b01, b23, 0x5410);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int v = (int)clamp_q(rintf(__fdiv_rn(f[e], step)), qmax);
+        w[e >> 2] |= (uint32_t)(v & 0xFF) << (8 * (e & 3));
+      }
     }
     *reinterpret_cast<uint2*>(q + i) = make_uint2(w[0], w[1]);
   }
