@@ -16,6 +16,7 @@ from ..config.schema import ModelConfig
 from ..ops import autograd as A
 from .registry import ATTENTION, EMBEDDING, FFN, NORM, ROPE
 from . import modules as _modules  # noqa: F401  (fills the registries)
+from .modules.core import block_without_gradients
 
 
 @dataclass
@@ -38,6 +39,9 @@ class TransformerBlock(nn.Module):
         self.ffn = FFN.get(cfg.modules.ffn)(cfg.d_model, cfg.ffn_intermediate, qat=cfg.qat, layer_idx=layer_idx)
 
     def forward(self, x, cos, sin):
+        y = block_without_gradients(x, cos, sin, self.norm1, self.attn, self.norm2, self.ffn)
+        if y is not None:
+            return y
         x = self.attn(self.norm1(x), cos, sin, residual=x)
         return self.ffn(self.norm2(x), residual=x)
 

@@ -192,7 +192,7 @@ class RMSNorm(nn.Module, ParamMixin):
         return A.rms_norm(x, master, w, slot, self.eps, tp_heads)
 
 
-_OWN_FORWARD = {cls: cls.forward for cls in (QuantLinear, RMSNorm)}
+_OWN_FORWARD = {cls: cls.forward for cls in (Linear, QuantLinear, RMSNorm)}
 
 
 @ROPE.register("rope_default")
@@ -395,6 +395,65 @@ class SwiGLU(nn.Module):
 
     def forward(self, x, residual=None):
         return self.w_down(A.swiglu(self.w_gate_up(x)), residual)
+
+
+_OWN_FORWARD.update({cls: cls.forward for cls in (GQAQKNorm, GQAPlain, SwiGLU)})
+_OWN_QKV = _GQABase._qkv
+
+
+def _no_transform() -> bool:
+    """Whether an autograd function would only run its forward here: gradients are off and nothing looks on - no functorch
+    transform, forward-mode level, tracer, compiler, or torch function / dispatch mode."""
+    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None and \
+        torch.autograd.forward_ad._current_level < 0 and not torch._C._len_torch_dispatch_stack() and \
+        not torch._C._len_torch_function_stack() and not torch.compiler.is_compiling()
+
+
+def _ready(w, x, shape):
+    """``w`` if it is a contiguous tensor of that shape and of the type and device of ``x``, else None."""
+    ok = type(w) in (torch.Tensor, nn.Parameter) and w.dtype == x.dtype and w.device == x.device and w.shape == shape and w.is_contiguous()
+    return w if ok else None
+
+
+def _own_weight(m, x, shape):
+    """The weight that ``m`` multiplies ``x`` by, if it is ready where it lies."""
+    slot = m._slot()
+    if slot is not None and slot.gather is not None:  # its rows may still have to be pulled from their owners
+        return None
+    w = m._cw()
+    return _ready(m.weight if w is None else w, x, shape)
+
+
+def block_without_gradients(x, cos, sin, norm1, attn, norm2, ffn):
+    """The block's output from one native call, or None where the modules have to be called one by one: with gradients, off
+    the GPU, under tensor parallelism or the per-call timer, with quantised or gathered weights, head-norm gains, int8 P V,
+    hooks, or any module or method that is not this file's own. (The host bounds the scoring of short prompts: 333 tokens
+    through the six-layer 100M model.)"""
+    if torch.is_grad_enabled() or not x.is_cuda or type(x) is not torch.Tensor or not _no_transform() or A.tp() is not None or K.timing():
+        return None
+    if x.dim() != 3 or not x.is_contiguous() or x.dtype not in (torch.bfloat16, torch.float32) or x.numel() == 0:
+        return None
+    cls = type(attn)
+    if cls not in (GQAQKNorm, GQAPlain) or cls._qkv is not _OWN_QKV or "_qkv" in attn.__dict__ or type(ffn) is not SwiGLU:
+        return None
+    wo, gate_up, down = attn.wo, ffn.w_gate_up, ffn.w_down
+    if not (_untouched(attn, cls) and _untouched(ffn, SwiGLU) and _untouched(norm1, RMSNorm) and _untouched(norm2, RMSNorm) and
+            _untouched(wo, Linear) and _untouched(gate_up, Linear) and _untouched(down, Linear)):
+        return None
+    if attn.qk_norm_gain or norm1.weight is None or norm2.weight is None or (isinstance(attn.wq, QuantLinear) and attn.wq.qat_active):
+        return None
+    fused = getattr(attn, "_fused_qkv", None)
+    if fused is None or (fused[2] is not None and fused[2].gather is not None) or attn._int8_pv(x):
+        return None
+    T, d = x.shape[1], x.shape[2]
+    H, Hkv, D, inner = attn.n_heads, attn.n_kv_heads, attn.head_dim, ffn.intermediate
+    if cos.shape != (T, D // 2) or sin.shape != (T, D // 2) or not (cos.is_contiguous() and sin.is_contiguous() and cos.device == sin.device == x.device):
+        return None
+    w = (_own_weight(norm1, x, (d,)), _ready(fused[0] if fused[1] is None else fused[1], x, ((H + 2 * Hkv) * D, d)), _own_weight(wo, x, (d, H * D)),
+         _own_weight(norm2, x, (d,)), _own_weight(gate_up, x, (2 * inner, d)), _own_weight(down, x, (d, inner)))
+    if any(v is None for v in w):
+        return None
+    return K.block_fwd(x, *w, cos, sin, H, Hkv, D, attn.window, attn.qk_norm, norm1.eps, norm2.eps, attn.eps)
 
 
 class Embedding(nn.Module, ParamMixin):

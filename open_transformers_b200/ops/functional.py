@@ -39,6 +39,11 @@ def _status_ptr(t: torch.Tensor) -> int:
     return p
 
 
+def timing() -> bool:
+    """Whether the per-entry-point timer is running (native.start_timing)."""
+    return _native._timing is not None
+
+
 def kernel_status(device=None) -> int:
     """Non-zero if a bounded in-kernel wait ever gave up on this device (sync point)."""
     device = torch.device(device or "cuda")
@@ -266,6 +271,29 @@ def swiglu_bwd(gu: torch.Tensor, dh: torch.Tensor) -> torch.Tensor:
     else:
         check(cpu_lib().otb_cpu_swiglu_bwd(P(gu), P(dh), P(dgu), L(rows), I(F2 // 2), I(is_bf16(gu))), "swiglu_bwd")
     return dgu
+
+
+# ------------------------------------------------------------------ a block without gradients
+_block_fwd = packed_entry("otb_block_fwd", "20q4d3q")
+
+
+def block_fwd(x, norm1, wqkv, wo, norm2, wgu, wdown, cos, sin, H: int, Hkv: int, D: int, window: int, qk_norm: bool, eps1: float, eps2: float,
+              eps_qk: float) -> torch.Tensor:
+    """Decoder block on CUDA activations ``x`` [B, T, d] in one native call (csrc/cuda/block.cu): the launches of ``rmsnorm_fwd``,
+    ``gemm``, ``qknorm_rope_fwd``, ``attn_fwd`` and ``swiglu_fwd`` in the modules' order, so the same bits. Weights are contiguous
+    and of the activations' type."""
+    B, T, d = x.shape
+    inner = wdown.shape[1]
+    y = torch.empty_like(x)
+    bf = is_bf16(x)
+    need = cuda_lib().otb_block_fwd_scratch
+    need.restype = ctypes.c_long
+    scratch = torch.empty(need(L(B * T), I(d), I(H), I(Hkv), I(D), I(inner), I(bf)), dtype=torch.uint8, device=x.device)
+    check(_block_fwd(x.data_ptr(), y.data_ptr(), scratch.data_ptr(), norm1.data_ptr(), wqkv.data_ptr(), wo.data_ptr(), norm2.data_ptr(),
+                     wgu.data_ptr(), wdown.data_ptr(), cos.data_ptr(), sin.data_ptr(), B, T, d, H, Hkv, D, inner, window, qk_norm, eps1, eps2,
+                     eps_qk, 1.0 / math.sqrt(D), bf, _status_ptr(x), raw_stream()), "block_fwd")
+    _native.launch_count += 8  # nine launches, one of them counted by ``check``
+    return y
 
 
 # ---------------------------------------------------------------------------------- loss
