@@ -89,6 +89,12 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 __device__ __forceinline__ int work_item(int turn) {
   return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
+// dQ and dK/dV need nothing of each other, so the second of the two kernels is launched while the first one runs: its CTAs
+// start on the SMs that the first leaves free (64 CTAs of dK/dV, 96 of dQ on 148 SMs at 2 x 1000 tokens, 12 heads x 64), or as
+// the first one's CTAs end. The first allows it when all its CTAs are there, so whatever ran before it in the stream is
+// complete; the second ends after the first, so that what follows in the stream waits for both.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
@@ -754,6 +760,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
                    float c_log2, uint32_t* __restrict__ status) {
   constexpr int TILE = BQ * D * 2;
   constexpr int ST = 2;
+  let_next_kernel_start();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem;
@@ -1167,6 +1174,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && blockIdx.x == 0) wait_for_kernel_before();
   if (threadIdx.x == 0 && bars->abort_flag && status) atomicExch(status, 4u);
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
@@ -1227,6 +1235,7 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   constexpr int TILE = BKV * D * 2;  // [128 keys][D]
   constexpr int QT = HK * D * 2;     // [64 queries][D]
   constexpr int ST = KV2_ST;
+  let_next_kernel_start();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem;
@@ -1560,6 +1569,22 @@ template <int D> constexpr int attn_fwd2_smem_bytes() { return (2 + 2 * 2) * (BQ
 // one CTA per SM, fewer when there are fewer items
 static inline unsigned persistent_grid(long items) { return (unsigned)(items < otb_sm_count() ? items : otb_sm_count()); }
 
+// KERN's launch may begin while the kernel before it in the stream runs, once that one lets it
+template <typename... P, typename... A>
+static inline int launch_beside(void (*kern)(P...), unsigned grid, int smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute beside;
+  beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  beside.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(ATT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &beside;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 extern "C" int otb_set_attn_rotation(int rotation) {
   if (rotation < 0) return -2;
   return (int)cudaMemcpyToSymbol(g_attn_rotation, &rotation, sizeof(rotation));
@@ -1668,8 +1693,9 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<128><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    attn_bwd_q2_kernel<128><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
-                                                                                  Hkv, window, scale, c_log2, status);
+    if (const int rl = launch_beside(attn_bwd_q2_kernel<128>, gq, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+                                     Hkv, window, scale, c_log2, status))
+      return rl;
   } else {
     const int rc = otb_allow_smem<attn_bwd_kv_kernel<64>>(attn_bwd_smem_bytes<64>()) |
                    otb_allow_smem<attn_bwd_kv2_kernel<64>>(attn_bwd_kv2_smem_bytes<64>()) |
@@ -1681,8 +1707,9 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<64><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                  lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    attn_bwd_q2_kernel<64><<<gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s>>>(tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H, Hkv,
-                                                                                window, scale, c_log2, status);
+    if (const int rl = launch_beside(attn_bwd_q2_kernel<64>, gq, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+                                     Hkv, window, scale, c_log2, status))
+      return rl;
   }
   return (int)cudaGetLastError();
 }
