@@ -1,0 +1,41 @@
+"""Fast forms of kernels at the edges of what chooses them, bit for bit against the CPU twin."""
+import pytest
+import torch
+
+from open_transformers_b200.ops import functional as K
+
+pytestmark = pytest.mark.gpu
+
+
+# every 16-byte piece whole (predicated loads): one size per tile, rows ragged against the tile, K below, at and past a slab
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,K_", [(4, 36, 4), (36, 60, 32), (100, 260, 68), (772, 900, 36), (2308, 2312, 20)])
+def test_exact_gemm_of_whole_pieces(a_mn, b_mn, M, N, K_):
+    g = torch.Generator().manual_seed(M + K_)
+    a = torch.randn((K_, M) if a_mn else (M, K_), generator=g)
+    b = torch.randn((K_, N) if b_mn else (N, K_), generator=g)
+    acc = torch.randn(M, N, generator=g)
+    assert torch.equal(K.gemm(a.cuda(), b.cuda(), a_mn=a_mn, b_mn=b_mn).cpu(), K.gemm(a, b, a_mn=a_mn, b_mn=b_mn))
+    assert torch.equal(K.gemm(a.cuda(), b.cuda(), a_mn=a_mn, b_mn=b_mn, epi=K.EPI_ACC_F32, out=acc.cuda()).cpu(),
+                       K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, epi=K.EPI_ACC_F32, out=acc.clone()))
+
+
+# values on and one step beside every tie k + 1/2, NaN, both zeros; steps in and out of the range of the fast division
+# (2^-80 .. 2^100), a subnormal and an infinite one; lengths with and without a ragged end
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("qmax", [127, 7, 1])
+@pytest.mark.parametrize("top", [1.0, 3.1415927, 2.0**-70, 127 * 2.0**-80, 2.0**-90, 2.0**-130, 2.0**100, 2.0**120, float("inf")])
+def test_quantiser_near_ties(dtype, qmax, top):
+    step = torch.tensor(top, dtype=torch.float32) * torch.tensor(1.0 / qmax, dtype=torch.float32)
+    k = torch.arange(-qmax, qmax, dtype=torch.float32) + 0.5
+    ties = k * step if top < float("inf") else k
+    x = torch.cat([ties, torch.nextafter(ties, ties * 2), torch.nextafter(ties, ties * 0), torch.tensor([0.0, -0.0, 1e-40, float("nan")]),
+                   torch.linspace(-1, 1, 1001) * min(top, 3e38)]).clamp(-min(top, 3.3e38), min(top, 3.3e38)).to(dtype)
+    x = torch.cat([x, torch.tensor([top, -top]).to(dtype)])
+    for n in (x.numel(), x.numel() // 8 * 8):
+        part = x[-n:].contiguous()
+        q, s = K.quant_act(part.cuda(), qmax)
+        want_q, want_s = K.quant_act(part, qmax)
+        assert torch.equal(s.cpu(), want_s)
+        keep = ~part.isnan() & ~part.isinf()  # (what the quotient NaN becomes is the platform's conversion)
+        assert torch.equal(q.cpu()[keep], want_q[keep])
