@@ -89,12 +89,6 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 __device__ __forceinline__ int work_item(int turn) {
   return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
-// dQ and dK/dV need nothing of each other, so the second of the two kernels is launched while the first one runs: its CTAs
-// start on the SMs that the first leaves free (64 CTAs of dK/dV, 96 of dQ on 148 SMs at 2 x 1000 tokens, 12 heads x 64), or as
-// the first one's CTAs end. The first allows it when all its CTAs are there, so whatever ran before it in the stream is
-// complete; the second ends after the first, so that what follows in the stream waits for both.
-__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
@@ -492,6 +486,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  after_predecessor();
   const uint32_t tmem = bars->tmem_slot;
 
   if (warp == 0) {
@@ -760,7 +755,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
                    float c_log2, uint32_t* __restrict__ status) {
   constexpr int TILE = BQ * D * 2;
   constexpr int ST = 2;
-  let_next_kernel_start();
+  let_successor_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem;
@@ -1174,7 +1169,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && blockIdx.x == 0) wait_for_kernel_before();
+  if (threadIdx.x == 0 && blockIdx.x == 0) wait_for_predecessor();
   if (threadIdx.x == 0 && bars->abort_flag && status) atomicExch(status, 4u);
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
@@ -1235,7 +1230,7 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   constexpr int TILE = BKV * D * 2;  // [128 keys][D]
   constexpr int QT = HK * D * 2;     // [64 queries][D]
   constexpr int ST = KV2_ST;
-  let_next_kernel_start();
+  let_successor_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem;
@@ -1433,6 +1428,7 @@ constexpr int DELTA_ROWS = 8;
 template <bool VEC>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, long lddo, const __nv_bfloat16* __restrict__ O,
                                   long ldo, const float* __restrict__ lse, float* __restrict__ delta, int B, int T, int H, int D) {
+  after_predecessor();
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const long rows = (long)B * T, groups = (rows + DELTA_ROWS - 1) / DELTA_ROWS;
@@ -1569,22 +1565,6 @@ template <int D> constexpr int attn_fwd2_smem_bytes() { return (2 + 2 * 2) * (BQ
 // one CTA per SM, fewer when there are fewer items
 static inline unsigned persistent_grid(long items) { return (unsigned)(items < otb_sm_count() ? items : otb_sm_count()); }
 
-// KERN's launch may begin while the kernel before it in the stream runs, once that one lets it
-template <typename... P, typename... A>
-static inline int launch_beside(void (*kern)(P...), unsigned grid, int smem, cudaStream_t s, A... args) {
-  cudaLaunchAttribute beside;
-  beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  beside.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &beside;
-  cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 extern "C" int otb_set_attn_rotation(int rotation) {
   if (rotation < 0) return -2;
   return (int)cudaMemcpyToSymbol(g_attn_rotation, &rotation, sizeof(rotation));
@@ -1604,12 +1584,12 @@ extern "C" int otb_attn_fwd(const void* qk, long ldqk, const void* qkv, long ldq
   if (D == 128) {
     const int rc = otb_allow_smem<attn_fwd2_kernel<128>>(attn_fwd2_smem_bytes<128>());
     if (rc) return rc;
-    attn_fwd2_kernel<128><<<grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
+    otb_chain(attn_fwd2_kernel<128>, grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                               c_log2, status);
   } else {
     const int rc = otb_allow_smem<attn_fwd2_kernel<64>>(attn_fwd2_smem_bytes<64>());
     if (rc) return rc;
-    attn_fwd2_kernel<64><<<grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
+    otb_chain(attn_fwd2_kernel<64>, grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
                                                                             c_log2, status);
   }
   return (int)cudaGetLastError();
@@ -1660,7 +1640,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   const long warps = ((long)B * T + DELTA_ROWS - 1) / DELTA_ROWS * H;
   const bool vec = ((reinterpret_cast<uintptr_t>(O) | reinterpret_cast<uintptr_t>(dO)) & 7) == 0;  // pitches are multiples of 8 elements
   auto delta_kernel = vec ? attn_delta_kernel<true> : attn_delta_kernel<false>;
-  delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse, delta, B, T, H, D);
+  otb_chain(delta_kernel, (unsigned)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse, delta, B, T, H, D);
   __nv_bfloat16* dQp = (__nv_bfloat16*)dqk;
   __nv_bfloat16* dKp = dQp + (long)H * D;
   __nv_bfloat16* dVp = (__nv_bfloat16*)dqkv + (long)(H + Hkv) * D;
@@ -1673,6 +1653,8 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   const int nkb = (T + BKV - 1) / BKV;
   const unsigned gq = persistent_grid((long)((nq + 1) / 2) * H * B), gkv2 = persistent_grid((long)nkb * Hkv * B);
   const dim3 gkv(nkb, Hkv, B);
+  // dQ runs beside dK/dV: its CTAs start on the SMs that the latter leaves free (64 and 96 CTAs on 148 SMs at 2 x 1000 tokens, 12
+  // heads x 64), or as its CTAs end.
   const bool kv2 = T % HK == 0;  // the transposed dK/dV kernel walks whole 64-query steps
   const long plane = (long)B * H * T;
   CUtensorMap tq64, tdo64;
@@ -1693,7 +1675,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<128><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = launch_beside(attn_bwd_q2_kernel<128>, gq, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+    if (const int rl = otb_chain(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                      Hkv, window, scale, c_log2, status))
       return rl;
   } else {
@@ -1707,7 +1689,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<64><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                  lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = launch_beside(attn_bwd_q2_kernel<64>, gq, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+    if (const int rl = otb_chain(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                      Hkv, window, scale, c_log2, status))
       return rl;
   }

@@ -70,6 +70,32 @@ inline int otb_allow_smem(int bytes) {
   return 0;
 }
 
+// Kernels of one stream in a chain: otb_chain lets a kernel's launch begin while its predecessor still runs, and the kernel
+// calls after_predecessor() before it touches any memory. What then overlaps is the launch itself, the CTAs' start and their
+// set-up (barriers, tensor memory); without it a chain of kernels that take 4 to 15 us each pays them one after the other. A
+// kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that it needs.
+// Behind anything but such a kernel, and in front of it, the order of the stream is the ordinary one.
+__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory"); }
+// Two kernels that need nothing of each other: the first, launched in the ordinary way, calls let_successor_begin(), so that
+// all that ran before it is complete by then; the second, launched by otb_chain, touches memory at once and lets one thread call
+// wait_for_predecessor() at its end, so that what follows in the stream waits for both.
+__device__ __forceinline__ void let_successor_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline int otb_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 #define OTB_CUDA_CHECK_RET(expr)              \
   do {                                        \
     cudaError_t _e = (expr);                  \
