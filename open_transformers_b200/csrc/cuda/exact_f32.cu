@@ -187,11 +187,16 @@ template <int TM, int TN, int RM, int RN, int RES = 0>
 int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, int M, int N, int K, long lda, long ldb, long ldc, long ldr,
                     int a_mn, int b_mn, int epi, int vec, cudaStream_t s) {
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
+  // Predicated loads pay with two MN-major operands, the weight gradients (256 x 704 x 2048 71.5 -> 46.5 us, 1408 x 256 x 2048 85.4 ->
+  // 68.3, 4096 x 4096 x 512 411 -> 376), and with two K-major ones in 64-wide tiles (2048 x 1408 x 256 66.7 -> 61.2); not in
+  // 128-wide ones (4096 x 4096 x 512 465 -> 480) and not with one of each kind (2048 x 256 x 1408 75 -> 78).
   const bool whole = (vec & 3) == 3 && (a_mn ? M : K) % 4 == 0 && (b_mn ? N : K) % 4 == 0;
-#define GF(AM, BM, E)                                                                                                            \
-  do {                                                                                                                           \
-    auto kern = whole ? gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, true> : gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, false>; \
-    otb_chain(kern, grid, F32Tile<TM, TN, RM, RN>::NT, 0, s, A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec);                              \
+#define GF(AM, BM, E)                                                                                    \
+  do {                                                                                                   \
+    constexpr bool PAYS = AM == BM && (AM || TM == 64);                                                  \
+    auto kern = whole && PAYS ? gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, PAYS>                    \
+                              : gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, false>;                  \
+    otb_chain(kern, grid, F32Tile<TM, TN, RM, RN>::NT, 0, s, A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec); \
   } while (0)
 #define GE(AM, BM)                                      \
   switch (epi) {                                         \

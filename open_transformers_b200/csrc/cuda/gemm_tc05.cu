@@ -734,6 +734,11 @@ bool pair_wins(int M, int N, int K, bool mn_major, bool i8, int max_ctas, double
   return N > 128 && K > (i8 ? PAIR_ABOVE_K_I8 : PAIR_ABOVE_K) && tiles >= max_ctas / 2 && max_ctas >= 2 &&
          (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) && PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
 }
+// Where even 64-wide tiles fit the chip in one wave, more SMs share the loads and each has less to load, multiply and store
+// (wider and 64-wide tiles, us: 333 x 768 x 768 with residual 9.0 and 7.4, 1111 x 768 x 2048 13.3 and 11.7, 1111 x 768 x 4096 20.0
+// and 18.2, its data gradient 18.0 and 17.3, 768 x 1280 x 333 as a weight gradient 6.3 and 5.7; nowhere longer). In a second wave
+// they would read A twice as often as 128-wide ones.
+constexpr int SLIM = 64;
 // Tile of a product: columns of a single CTA's tile, or PAIR_TILE.
 constexpr int PAIR_TILE = 512;
 int choose_tile(int M, int N, int K, bool mn_major, bool i8, int max_ctas) {
@@ -748,6 +753,7 @@ int choose_tile(int M, int N, int K, bool mn_major, bool i8, int max_ctas) {
     const double e256 = N >= 256 ? tile_efficiency(M, N, BM, 256, max_ctas) : 0.0;
     BN = e256 >= e128 ? 256 : 128;
     single = BN == 256 ? e256 : e128;
+    if ((long)((M + BM - 1) / BM) * ((N + SLIM - 1) / SLIM) <= max_ctas) return SLIM;
   }
   return pair_wins(M, N, K, mn_major, i8, max_ctas, single) ? PAIR_TILE : BN;
 }
@@ -840,7 +846,7 @@ int launch_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& t
 
 }  // namespace
 
-// The tile that the entry points below choose: 128 or 256 columns on one CTA, 512 for a CTA pair (max_ctas 0: every SM).
+// The tile that the entry points below choose: 64, 128 or 256 columns on one CTA, 512 for a CTA pair (max_ctas 0: every SM).
 extern "C" int otb_gemm_tile(int M, int N, int K, int mn_major, int i8, int max_ctas) {
   return choose_tile(M, N, K, mn_major != 0, i8 != 0, max_ctas > 0 ? max_ctas : otb_sm_count());
 }
@@ -897,8 +903,10 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   }
   if (BN == 256) {
     OTB_DISPATCH(256, 4)
-  } else {
+  } else if (BN == 128) {
     OTB_DISPATCH(128, 6)
+  } else {
+    OTB_DISPATCH(SLIM, 8)
   }
 #undef OTB_DISPATCH
 }

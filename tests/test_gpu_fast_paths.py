@@ -39,3 +39,23 @@ def test_quantiser_near_ties(dtype, qmax, top):
         assert torch.equal(s.cpu(), want_s)
         keep = ~part.isnan() & ~part.isinf()  # (what the quotient NaN becomes is the platform's conversion)
         assert torch.equal(q.cpu()[keep], want_q[keep])
+
+
+# 64-wide tiles where all of them fit the chip at once: one tile, ragged columns and rows, a K of one step and of many, the
+# first size past a wave of them
+@pytest.mark.parametrize("M,N,K_", [(1, 8, 8), (130, 200, 64), (129, 72, 520), (37 * 128, 256, 72), (37 * 128 + 1, 256, 72)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_slim_gemm_tiles(M, N, K_, a_mn, b_mn):
+    g = torch.Generator().manual_seed(M + K_)
+    Mr = (M + 7) // 8 * 8 if a_mn else M  # (a row pitch is a multiple of 16 bytes)
+    a = torch.randn((K_, Mr) if a_mn else (M, K_), generator=g).bfloat16()
+    b = torch.randn((K_, N) if b_mn else (N, K_), generator=g).bfloat16()
+    for epi in (K.EPI_STORE, K.EPI_STORE_F32, K.EPI_ACC_F32, K.EPI_RESIDUAL):
+        kw = {"epi": epi}
+        rows = Mr if a_mn else M
+        out = torch.randn(rows, N, generator=g) if epi == K.EPI_ACC_F32 else None
+        res = torch.randn(rows, N, generator=g).bfloat16() if epi == K.EPI_RESIDUAL else None
+        want = K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=None if out is None else out.clone(), residual=res, **kw)
+        got = K.gemm(a.cuda(), b.cuda(), a_mn=a_mn, b_mn=b_mn, out=None if out is None else out.cuda(), residual=None if res is None else res.cuda(), **kw)
+        assert torch.equal(got.cpu(), want)
+    assert K.kernel_status("cuda") == 0
