@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -81,6 +82,7 @@ __device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontr
 // wait_for_predecessor() at its end, so that what follows in the stream waits for both.
 __device__ __forceinline__ void let_successor_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A launch that is refused is tried once in the ordinary way, which is right in either use, and whose error is the one to report.
 template <typename... P, typename... A>
 inline int otb_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchAttribute early;
@@ -93,7 +95,15 @@ inline int otb_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.stream = s;
   cfg.attrs = &early;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  std::tuple<P...> values(static_cast<P>(args)...);
+  return std::apply(
+      [&](P&... v) {
+        void* argv[] = {const_cast<void*>(static_cast<const void*>(&v))...};
+        if (cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), argv) == cudaSuccess) return 0;
+        (void)cudaGetLastError();
+        return (int)cudaLaunchKernel(reinterpret_cast<const void*>(kern), grid, block, argv, smem, s);
+      },
+      values);
 }
 
 #define OTB_CUDA_CHECK_RET(expr)              \
