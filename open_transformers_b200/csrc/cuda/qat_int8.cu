@@ -67,7 +67,8 @@ __device__ __forceinline__ float clamp_q(float q, float qmax) { return fminf(fma
 // correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990: the first makes q faithful, the second correct), provided
 // that nothing over- or underflows, which the bounds on the step see to (a tiny x whose remainder is subnormal has a quotient
 // near 0). Adding 1.5 * 2^23 rounds half to even and leaves the integer in the low bits. A NaN gives -qmax, as in the general
-// form.
+// form. (With a division, a rounding and a conversion per element the pass was bound by instructions: maximum and quantisation
+// of 16.8 M bf16 elements 24.6 -> 16.6 us, 46 M 73 -> 52, 92 M 140 -> 92; up to 1 M elements unchanged.)
 constexpr float DIVIDES_FROM = 0x1p-80f, DIVIDES_TO = 0x1p100f;
 __device__ __forceinline__ uint32_t quant_bits(float x, float step, float y, float qmax) {
   float q = __fmul_rn(x, y);
