@@ -92,13 +92,20 @@ __device__ __forceinline__ int work_item(int turn) {
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
+// A descriptor `bytes` further into its operand: one addition to the address field (16-byte units, shared memory ends below its
+// top). One thread issues every product beside busy element warps, and what it spends on a descriptor is time: forward and
+// backward at 4 x 4096 tokens, 16 heads x 128, with the whole descriptor built for each: 404 and 976 us, so 388 and 938; 512-key
+// window 183 and 380, so 179 and 364.
+__device__ __forceinline__ uint64_t desc_plus(uint64_t d, uint32_t bytes) {
+  return (d & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4));
+}
 // K-major operand, tile made of [128 rows][64 elems] sub-tiles 16 KB apart; k-step kk = 16 elems
 __device__ __forceinline__ uint64_t desc_k(uint32_t base, int kk) {
-  return make_smem_desc(base + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
+  return desc_plus(make_smem_desc(base, 16, 1024), (kk >> 2) * 16384 + (kk & 3) * 32);
 }
 // MN-major operand, tile made of [128 k-rows][64 mn elems] chunks 16 KB apart; k-step kk = 16 rows
 __device__ __forceinline__ uint64_t desc_mn(uint32_t base, int kk) {
-  return make_smem_desc(base + kk * 2048, 16384, 1024);
+  return desc_plus(make_smem_desc(base, 16384, 1024), kk * 2048);
 }
 
 template <int D>
@@ -951,11 +958,11 @@ __device__ __forceinline__ void load_tile_r(uint8_t* dst, const CUtensorMap* tm,
 // K-major / MN-major operand descriptors for tiles of ROWS rows ([ROWS][64 elems] sub-tiles ROWS * 128 bytes apart)
 template <int ROWS>
 __device__ __forceinline__ uint64_t desc_k_r(uint32_t base, int kk) {
-  return make_smem_desc(base + (kk >> 2) * (ROWS * 128) + (kk & 3) * 32, 16, 1024);
+  return desc_plus(make_smem_desc(base, 16, 1024), (kk >> 2) * (ROWS * 128) + (kk & 3) * 32);
 }
 template <int ROWS>
 __device__ __forceinline__ uint64_t desc_mn_r(uint32_t base, int kk) {
-  return make_smem_desc(base + kk * 2048, ROWS * 128, 1024);
+  return desc_plus(make_smem_desc(base, ROWS * 128, 1024), kk * 2048);
 }
 
 struct BarsQ2 {
@@ -1653,8 +1660,8 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   const int nkb = (T + BKV - 1) / BKV;
   const unsigned gq = persistent_grid((long)((nq + 1) / 2) * H * B), gkv2 = persistent_grid((long)nkb * Hkv * B);
   const dim3 gkv(nkb, Hkv, B);
-  // dQ runs beside dK/dV: its CTAs start on the SMs that the latter leaves free (64 and 96 CTAs on 148 SMs at 2 x 1000 tokens, 12
-  // heads x 64), or as its CTAs end.
+  // dQ runs beside dK/dV: its CTAs start on the SMs that the latter leaves free, or as its CTAs end (backward, us, one after the
+  // other and so: 2 x 1000 tokens, 12 heads x 64, window 512 83 and 56; 1 x 2048, 16 x 128 198 and 141; 4 x 4096 1018 and 976).
   const bool kv2 = T % HK == 0;  // the transposed dK/dV kernel walks whole 64-query steps
   const long plane = (long)B * H * T;
   CUtensorMap tq64, tdo64;
@@ -1675,7 +1682,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<128><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = otb_chain(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+    if (const int rl = otb_launch_early(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                      Hkv, window, scale, c_log2, status))
       return rl;
   } else {
@@ -1689,7 +1696,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
     else
       attn_bwd_kv_kernel<64><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
                                                                                  lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = otb_chain(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
+    if (const int rl = otb_launch_early(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
                                      Hkv, window, scale, c_log2, status))
       return rl;
   }

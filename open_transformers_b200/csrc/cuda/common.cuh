@@ -6,7 +6,6 @@
 #include <string.h>
 
 #include <atomic>
-#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -71,39 +70,52 @@ inline int otb_allow_smem(int bytes) {
   return 0;
 }
 
-// Kernels of one stream in a chain: otb_chain lets a kernel's launch begin while its predecessor still runs, and the kernel
-// calls after_predecessor() before it touches any memory. What then overlaps is the launch itself, the CTAs' start and their
-// set-up (barriers, tensor memory); without it a chain of kernels that take 4 to 15 us each pays them one after the other. A
-// kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that it needs.
+// Launches that may begin while the kernel before them in the stream still runs.
+// In a chain: otb_chain launches small grids that way, and the kernel calls after_predecessor() before it touches any memory.
+// What then overlaps is the launch itself, the CTAs' start and their set-up (barriers, tensor memory); a chain of kernels that
+// take 4 to 15 us each pays them one after the other otherwise (logits of 333 tokens through the six-layer 100M model: 594 ->
+// 559 us). A kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that
+// it needs. Large grids gain nothing. Not for kernels with a few small CTAs per SM that all take long: placed before the SMs
+// are free they pile up on some (an exact fp32 product of 512 two-warp CTAs took 1.4 to 1.6 times as long).
+// Side by side, where two kernels need nothing of each other: the first, launched in the ordinary way, calls
+// let_successor_begin(), so that all that ran before it is complete by then; the second, launched by otb_launch_early, touches
+// memory at once and lets one thread call wait_for_predecessor() at its end, so that what follows in the stream waits for both.
 // Behind anything but such a kernel, and in front of it, the order of the stream is the ordinary one.
-__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory"); }
-// Two kernels that need nothing of each other: the first, launched in the ordinary way, calls let_successor_begin(), so that
-// all that ran before it is complete by then; the second, launched by otb_chain, touches memory at once and lets one thread call
-// wait_for_predecessor() at its end, so that what follows in the stream waits for both.
 __device__ __forceinline__ void let_successor_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_predecessor() {
+  let_successor_begin();
+  wait_for_predecessor();
+}
 // A launch that is refused is tried once in the ordinary way, which is right in either use, and whose error is the one to report.
+template <typename... P>
+inline int otb_launch_args(bool early, const void* kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s, P... v) {
+  void* argv[] = {const_cast<void*>(static_cast<const void*>(&v))...};
+  if (early) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelExC(&cfg, kern, argv) == cudaSuccess) return 0;
+    (void)cudaGetLastError();
+  }
+  return (int)cudaLaunchKernel(kern, grid, block, argv, smem, s);
+}
+template <typename... P, typename... A>
+inline int otb_launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  return otb_launch_args<P...>(true, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
+}
+constexpr unsigned CHAIN_CTAS_PER_SM = 8;
 template <typename... P, typename... A>
 inline int otb_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchAttribute early;
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &early;
-  cfg.numAttrs = 1;
-  std::tuple<P...> values(static_cast<P>(args)...);
-  return std::apply(
-      [&](P&... v) {
-        void* argv[] = {const_cast<void*>(static_cast<const void*>(&v))...};
-        if (cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), argv) == cudaSuccess) return 0;
-        (void)cudaGetLastError();
-        return (int)cudaLaunchKernel(reinterpret_cast<const void*>(kern), grid, block, argv, smem, s);
-      },
-      values);
+  const bool small = (unsigned long)grid.x * grid.y * grid.z <= (unsigned long)CHAIN_CTAS_PER_SM * otb_sm_count();
+  return otb_launch_args<P...>(small, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
 }
 
 #define OTB_CUDA_CHECK_RET(expr)              \

@@ -92,7 +92,6 @@ template <int TM, int TN, int RM, int RN, int RES, bool A_MN, bool B_MN, int EPI
 __global__ void __launch_bounds__(F32Tile<TM, TN, RM, RN>::NT, RES)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
                 const float* __restrict__ R, int M, int N, int K, long lda, long ldb, long ldc, long ldr, int vec) {
-  after_predecessor();
   using Tile = F32Tile<TM, TN, RM, RN>;
   constexpr int NT = Tile::NT, GX = TN / RN, GK = Tile::GK, AHEAD = Tile::AHEAD;
   __shared__ __align__(16) float sa[2][GK][TM + 4], sb[2][GK][TN + 4];
@@ -196,7 +195,7 @@ int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, in
     constexpr bool PAYS = AM == BM && (AM || TM == 64);                                                  \
     auto kern = whole && PAYS ? gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, PAYS>                    \
                               : gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, false>;                  \
-    otb_chain(kern, grid, F32Tile<TM, TN, RM, RN>::NT, 0, s, A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec); \
+    kern<<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec);     \
   } while (0)
 #define GE(AM, BM)                                      \
   switch (epi) {                                         \
@@ -268,7 +267,6 @@ __global__ void __launch_bounds__(256)
 attn_f32_fwd_kernel(const float* __restrict__ qk, long ldqk, const float* __restrict__ qkv, long ldqkv,
                     float* __restrict__ O, long ldo, float* __restrict__ lse, int B, int T, int H, int Hkv, int D,
                     int window, float c_log2, int vec) {
-  after_predecessor();
   extern __shared__ float4 smem4[];
   float* sQ = reinterpret_cast<float*>(smem4);   // [DM][ALD]
   float* sKV = sQ + DM * ALD;                    // K: [DM][FLD], then V: [FKB][DM + 4]
@@ -421,7 +419,6 @@ attn_f32_fwd_kernel(const float* __restrict__ qk, long ldqk, const float* __rest
 
 __global__ void attn_f32_delta_kernel(const float* __restrict__ dO, long lddo, const float* __restrict__ O, long ldo,
                                       float* __restrict__ delta, int B, int T, int H, int D) {
-  after_predecessor();
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wid >= (long)B * T * H) return;
@@ -681,7 +678,6 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ qk, long ldqk, const float* __r
                        const float* __restrict__ dO, long lddo, const float* __restrict__ lse,
                        const float* __restrict__ delta, float* __restrict__ dqk, long lddqk, float* __restrict__ dqkv,
                        long lddqkv, int B, int T, int H, int Hkv, int D, int window, float c_log2, float scale, int vec) {
-  let_successor_begin();
   extern __shared__ float4 smem4[];
   float* sK = reinterpret_cast<float*>(smem4);
   float* sV = sK + DM * ALD;
@@ -817,7 +813,6 @@ attn_f32_bwd_q_kernel(const float* __restrict__ qk, long ldqk, const float* __re
       if (d < D) dqk[qrow * lddqk + (long)h * D + d] = dq[i][u];
     }
   }
-  if (threadIdx.x == 0 && blockIdx.x == 0) wait_for_predecessor();  // it runs beside dK/dV
 }
 
 }  // namespace
@@ -849,7 +844,7 @@ int attn_f32_fwd(const float* qk, long ldqk, const float* qkv, long ldqkv, float
   constexpr int KV = DM * FLD > FKB * (DM + 4) ? DM * FLD : FKB * (DM + 4);
   constexpr int bytes = 4 * (DM * ALD + KV + FKB * ALD + 5 * AT);
   if (const int rc = otb_allow_smem<attn_f32_fwd_kernel<DM>>(bytes)) return rc;
-  otb_chain(attn_f32_fwd_kernel<DM>, (unsigned)((T + AT - 1) / AT * (long)H * B), 256, bytes, s, qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2, vec);
+  attn_f32_fwd_kernel<DM><<<(unsigned)((T + AT - 1) / AT * (long)H * B), 256, bytes, s>>>(qk, ldqk, qkv, ldqkv, O, ldo, lse, B, T, H, Hkv, D, window, c_log2, vec);
   return (int)cudaGetLastError();
 }
 template <int DM>
@@ -862,7 +857,7 @@ int attn_f32_bwd(const float* qk, long ldqk, const float* qkv, long ldqkv, const
   const long nt = (T + AT - 1) / AT;
   attn_f32_bwd_kv_kernel<DM><<<(unsigned)(nt * Hkv * B), 256, kv_bytes, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv, B, T, H,
                                                                      Hkv, D, window, c_log2, scale, vec);
-  otb_chain(attn_f32_bwd_q_kernel<DM>, (unsigned)(nt * H * B), 256, q_bytes, s, qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, B, T, H, Hkv, D, window,
+  attn_f32_bwd_q_kernel<DM><<<(unsigned)(nt * H * B), 256, q_bytes, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, B, T, H, Hkv, D, window,
                                                                  c_log2, scale, vec);
   return (int)cudaGetLastError();
 }
@@ -889,7 +884,7 @@ extern "C" int otb_attn_f32_bwd(const float* qk, long ldqk, const float* qkv, lo
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
   const long w1 = (long)B * T * H;
-  otb_chain(attn_f32_delta_kernel, (unsigned)((w1 + 7) / 8), 256, 0, s, dO, lddo, O, ldo, delta, B, T, H, D);
+  attn_f32_delta_kernel<<<(unsigned)((w1 + 7) / 8), 256, 0, s>>>(dO, lddo, O, ldo, delta, B, T, H, D);
   if (short_rows(T, (long)B * H, true)) {
     attn_f32_bwd_kv_short_kernel<<<(unsigned)(((long)B * Hkv * T + 3) / 4), 128, 0, s>>>(qk, ldqk, qkv, ldqkv, dO, lddo, lse, delta, dqk, lddqk, dqkv, lddqkv,
                                                                                         B, T, H, Hkv, D, window, c_log2, scale);

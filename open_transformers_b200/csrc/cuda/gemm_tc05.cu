@@ -268,7 +268,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (TP == 0) after_predecessor();
+  if constexpr (TP == 0 && !PAIR) after_predecessor();
 
   // tile -> (m, n): groups of `group_m` row-tiles sweep all column tiles, so that the A rows of
   // a group and the B columns being swept stay L2-resident across the CTAs working on them.
@@ -687,19 +687,17 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   if (const int rc = otb_allow_smem<kern>(L::TOTAL)) return rc;
   const long tiles = (long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
   const int pairs = (int)(tiles < max_ctas / 2 ? tiles : max_ctas / 2);
-  cudaLaunchAttribute attrs[2];
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = 2;
-  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as in otb_chain
-  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 2;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = stream;
-  cfg.attrs = attrs;
-  cfg.numAttrs = 2;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
   const int group_m = 8;
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m, scale_a, scale_b,
                                  status, TpNone{});
