@@ -92,13 +92,6 @@ __device__ __forceinline__ int work_item(int turn) {
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
-// A descriptor `bytes` further into its operand: one addition to the address field (16-byte units, shared memory ends below its
-// top). One thread issues every product beside busy element warps, and what it spends on a descriptor is time: forward and
-// backward at 4 x 4096 tokens, 16 heads x 128, with the whole descriptor built for each: 404 and 976 us, so 388 and 938; 512-key
-// window 183 and 380, so 179 and 364.
-__device__ __forceinline__ uint64_t desc_plus(uint64_t d, uint32_t bytes) {
-  return (d & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4));
-}
 // K-major operand, tile made of [128 rows][64 elems] sub-tiles 16 KB apart; k-step kk = 16 elems
 __device__ __forceinline__ uint64_t desc_k(uint32_t base, int kk) {
   return desc_plus(make_smem_desc(base, 16, 1024), (kk >> 2) * 16384 + (kk & 3) * 32);

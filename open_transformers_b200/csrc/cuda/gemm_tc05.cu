@@ -379,10 +379,10 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
           const uint32_t sb = sa + L::A_BYTES;
+          const uint64_t a0 = make_smem_desc(sa, A_MN ? 8192 : 16, 1024), b0 = make_smem_desc(sb, B_MN ? 8192 : 16, 1024);
 #pragma unroll
           for (int kk = 0; kk < BK_BYTES / UMMA_K_BYTES; ++kk) {
-            const uint64_t ad = A_MN ? make_smem_desc(sa + kk * 2048, 8192, 1024) : make_smem_desc(sa + kk * 32, 16, 1024);
-            const uint64_t bd = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024) : make_smem_desc(sb + kk * 32, 16, 1024);
+            const uint64_t ad = desc_plus(a0, kk * (A_MN ? 2048 : 32)), bd = desc_plus(b0, kk * (B_MN ? 2048 : 32));
             if constexpr (PAIR && I8) mma_i8_ss_pair(d_tmem, ad, bd, idesc, (kb | kk) != 0);
             else if constexpr (PAIR) mma_f16_ss_pair(d_tmem, ad, bd, idesc, (kb | kk) != 0);
             else if constexpr (I8) mma_i8_ss(d_tmem, ad, bd, idesc, (kb | kk) != 0);
@@ -733,8 +733,8 @@ bool pair_wins(int M, int N, int K, bool mn_major, bool i8, int max_ctas, double
          (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) && PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
 }
 // Where even 64-wide tiles fit the chip in one wave, more SMs share the loads and each has less to load, multiply and store
-// (wider and 64-wide tiles, us: 333 x 768 x 768 with residual 9.0 and 7.4, 1111 x 768 x 2048 13.3 and 11.7, 1111 x 768 x 4096 20.0
-// and 18.2, its data gradient 18.0 and 17.3, 768 x 1280 x 333 as a weight gradient 6.3 and 5.7; nowhere longer). In a second wave
+// (wider and 64-wide tiles, us: 333 x 768 x 768 with residual 8.8 and 6.0, 1111 x 768 x 2048 13.0 and 9.7, the data gradient
+// 1111 x 768 x 4096 17.8 and 14.8, the weight gradient 768 x 2048 x 1111 9.1 and 7.8; nowhere longer). In a second wave
 // they would read A twice as often as 128-wide ones.
 constexpr int SLIM = 64;
 // Tile of a product: columns of a single CTA's tile, or PAIR_TILE.

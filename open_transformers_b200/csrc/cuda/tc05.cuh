@@ -297,6 +297,14 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= 2ull << 61;  // SWIZZLE_128B
   return d;
 }
+// The descriptor `bytes` further into its operand: one addition to the address field (16-byte units, shared memory ends below
+// its top). One thread issues every product, in the attention kernels beside busy element warps, and what it spends on a
+// descriptor is time where a product is short. With the whole descriptor built for each and so, us: attention forward and backward
+// at 4 x 4096 tokens, 16 heads x 128, 404 and 388, 976 and 938, with a 512-key window 183 and 179, 380 and 364; products in
+// 64-wide tiles 333 x 768 x 2048 10.3 and 9.3, 1111 x 768 x 4096 17.0 and 14.8; 256-wide and paired ones as before.
+__device__ __forceinline__ uint64_t desc_plus(uint64_t d, uint32_t bytes) {
+  return (d & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4));
+}
 // 32-bit instruction descriptor for kind::f16 (bf16 x bf16 -> fp32) or kind::i8.
 //   c_format: 1 = F32, 2 = S32; ab_format: 1 = BF16 (kind::f16), 1 = signed int8 (kind::i8)
 __host__ __device__ constexpr uint32_t make_idesc(uint32_t M, uint32_t N, uint32_t a_mn_major, uint32_t b_mn_major,
