@@ -1,6 +1,6 @@
 """A process that works on a second GPU: the kernels that need more shared memory than the default ask for it on every device.
-The library's host code runs here against a fake of the few runtime calls involved, so no GPU takes part; the fake refuses a
-launch, as the real call does, when the current device has not been asked."""
+The library's host code runs here against a fake of the few runtime calls involved, launches of both kinds among them, and sees no
+device, so no GPU takes part; the fake refuses a launch, as the real calls do, when the current device has not been asked."""
 import os
 import subprocess
 import sys
@@ -13,14 +13,16 @@ from open_transformers_b200 import build_native
 FAKE = r"""
 #include <stddef.h>
 typedef struct { unsigned x, y, z; } dim3_;
+typedef struct { dim3_ grid, block; size_t smem; void* stream; void* attrs; unsigned n_attrs; } config_;  /* cudaLaunchConfig_t */
 static int device, last;
 static struct { const void* f; int dev, bytes; } asked[256];
 static int n_asked;
-int fake_launches;
+static int fake_launches, fake_early;
 int fake_refuse_next;
 void fake_set_device(int d) { device = d; }
 int fake_asked(void) { return n_asked; }
 int fake_launched(void) { return fake_launches; }
+int fake_launched_early(void) { return fake_early; }
 void fake_refuse(void) { fake_refuse_next = 1; }
 int cudaGetDevice(int* d) { *d = device; return 0; }
 int cudaGetLastError(void) { int e = last; last = 0; return e; }
@@ -30,13 +32,19 @@ int cudaFuncSetAttribute(const void* f, int attr, int value) {
   asked[n_asked].f = f; asked[n_asked].dev = device; asked[n_asked++].bytes = value;
   return 0;
 }
-int cudaLaunchKernel(const void* f, dim3_ g, dim3_ b, void** args, size_t smem, void* stream) {
+static int launch(const void* f, dim3_ g, size_t smem) {
   int most = 48 << 10, i;
   for (i = 0; i < n_asked; ++i)
     if (asked[i].f == f && asked[i].dev == device && asked[i].bytes > most) most = asked[i].bytes;
-  if (smem > (size_t)most) return last = 1;
+  if (smem > (size_t)most || !g.x || !g.y || !g.z) return last = 1;
   ++fake_launches;
   return 0;
+}
+int cudaLaunchKernel(const void* f, dim3_ g, dim3_ b, void** args, size_t smem, void* stream) { return launch(f, g, smem); }
+int cudaLaunchKernelExC(const config_* c, const void* f, void** args) {
+  int rc = launch(f, c->grid, c->smem);
+  if (!rc) ++fake_early;
+  return rc;
 }
 """
 
@@ -61,7 +69,8 @@ for dev in (0, 1, 0, 1):
     for D in (64, 128):
         assert calls(D) == (0, 0, 0), (dev, D, calls(D))
     counts.append(fake.fake_asked())
-assert fake.fake_launched() >= 4 * 2 * 5
+assert fake.fake_launched() == 4 * 2 * (1 + 3 + 1)
+assert fake.fake_launched_early() == 4 * 2 * 1  # the norm's: a small grid in a chain
 assert counts[1] == 2 * counts[0] and counts[3] == counts[1], counts  # once per kernel and device
 print("ok")
 """
@@ -75,6 +84,6 @@ def test_shared_memory_is_asked_for_on_every_device(tmp_path):
     fake = tmp_path / "libfake.so"
     cc = "/usr/bin/gcc" if Path("/usr/bin/gcc").exists() else "gcc"
     subprocess.run([cc, "-shared", "-fPIC", "-o", str(fake), str(tmp_path / "fake.c")], check=True)
-    r = subprocess.run([sys.executable, "-c", CHILD, str(fake), str(lib)], env=dict(os.environ, LD_PRELOAD=str(fake)), capture_output=True, text=True,
+    r = subprocess.run([sys.executable, "-c", CHILD, str(fake), str(lib)], env=dict(os.environ, LD_PRELOAD=str(fake), CUDA_VISIBLE_DEVICES=""), capture_output=True, text=True,
                        timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
