@@ -1584,15 +1584,14 @@ extern "C" int otb_attn_fwd(const void* qk, long ldqk, const void* qkv, long ldq
   if (D == 128) {
     const int rc = otb_allow_smem<attn_fwd2_kernel<128>>(attn_fwd2_smem_bytes<128>());
     if (rc) return rc;
-    otb_chain(attn_fwd2_kernel<128>, grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
-                                                                              c_log2, status);
+    return otb_chain(attn_fwd2_kernel<128>, grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv,
+                     window, c_log2, status);
   } else {
     const int rc = otb_allow_smem<attn_fwd2_kernel<64>>(attn_fwd2_smem_bytes<64>());
     if (rc) return rc;
-    otb_chain(attn_fwd2_kernel<64>, grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv, window,
-                                                                            c_log2, status);
+    return otb_chain(attn_fwd2_kernel<64>, grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv,
+                     window, c_log2, status);
   }
-  return (int)cudaGetLastError();
 }
 
 // Forward with P V on the int8 tensor cores (head_dim 128 only). vq: int8 scratch [B*T, Hkv*D]; vstep: fp32 scratch
@@ -1640,7 +1639,9 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   const long warps = ((long)B * T + DELTA_ROWS - 1) / DELTA_ROWS * H;
   const bool vec = ((reinterpret_cast<uintptr_t>(O) | reinterpret_cast<uintptr_t>(dO)) & 7) == 0;  // pitches are multiples of 8 elements
   auto delta_kernel = vec ? attn_delta_kernel<true> : attn_delta_kernel<false>;
-  otb_chain(delta_kernel, (unsigned)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse, delta, B, T, H, D);
+  if (const int rc = otb_chain(delta_kernel, (unsigned)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse,
+                               delta, B, T, H, D))
+    return rc;
   __nv_bfloat16* dQp = (__nv_bfloat16*)dqk;
   __nv_bfloat16* dKp = dQp + (long)H * D;
   __nv_bfloat16* dVp = (__nv_bfloat16*)dqkv + (long)(H + Hkv) * D;
@@ -1669,31 +1670,26 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
                    otb_allow_smem<attn_bwd_kv2_kernel<128>>(attn_bwd_kv2_smem_bytes<128>()) |
                    otb_allow_smem<attn_bwd_q2_kernel<128>>(attn_bwd_q2_smem_bytes<128>());
     if (rc) return rc;
-    if (kv2)
-      attn_bwd_kv2_kernel<128><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s>>>(
-          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
-    else
-      attn_bwd_kv_kernel<128><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
-                                                                                   lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = otb_launch_early(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
-                                     Hkv, window, scale, c_log2, status))
-      return rl;
+    const int kv = kv2 ? otb_launch(attn_bwd_kv2_kernel<128>, gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s, tq, tv, tq64, tdo64, delta + plane,
+                                    delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status)
+                       : otb_launch(attn_bwd_kv_kernel<128>, gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s, tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
+                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
+    if (kv) return kv;
+    return otb_launch_early(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T,
+                            H, Hkv, window, scale, c_log2, status);
   } else {
     const int rc = otb_allow_smem<attn_bwd_kv_kernel<64>>(attn_bwd_smem_bytes<64>()) |
                    otb_allow_smem<attn_bwd_kv2_kernel<64>>(attn_bwd_kv2_smem_bytes<64>()) |
                    otb_allow_smem<attn_bwd_q2_kernel<64>>(attn_bwd_q2_smem_bytes<64>());
     if (rc) return rc;
-    if (kv2)
-      attn_bwd_kv2_kernel<64><<<gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s>>>(
-          tq, tv, tq64, tdo64, delta + plane, delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
-    else
-      attn_bwd_kv_kernel<64><<<gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s>>>(tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
-                                                                                 lddqkv, T, H, Hkv, window, scale, c_log2, status);
-    if (const int rl = otb_launch_early(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T, H,
-                                     Hkv, window, scale, c_log2, status))
-      return rl;
+    const int kv = kv2 ? otb_launch(attn_bwd_kv2_kernel<64>, gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s, tq, tv, tq64, tdo64, delta + plane,
+                                    delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status)
+                       : otb_launch(attn_bwd_kv_kernel<64>, gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s, tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
+                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
+    if (kv) return kv;
+    return otb_launch_early(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T,
+                            H, Hkv, window, scale, c_log2, status);
   }
-  return (int)cudaGetLastError();
 }
 
 OTB_PACKED(otb_attn_fwd)

@@ -88,6 +88,8 @@ __device__ __forceinline__ void after_predecessor() {
   wait_for_predecessor();
 }
 // A launch that is refused is tried once in the ordinary way, which is right in either use, and whose error is the one to report.
+// The code returned is the only report: nothing is left pending for the next reader of the runtime's last error, and an entry
+// point with several launches looks at each, because the retry clears what an earlier one left there.
 template <typename... P>
 inline int otb_launch_args(bool early, const void* kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s, P... v) {
   void* argv[] = {const_cast<void*>(static_cast<const void*>(&v))...};
@@ -105,7 +107,13 @@ inline int otb_launch_args(bool early, const void* kern, dim3 grid, dim3 block, 
     if (cudaLaunchKernelExC(&cfg, kern, argv) == cudaSuccess) return 0;
     (void)cudaGetLastError();
   }
-  return (int)cudaLaunchKernel(kern, grid, block, argv, smem, s);
+  const int rc = (int)cudaLaunchKernel(kern, grid, block, argv, smem, s);
+  if (rc) (void)cudaGetLastError();
+  return rc;
+}
+template <typename... P, typename... A>
+inline int otb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  return otb_launch_args<P...>(false, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
 }
 template <typename... P, typename... A>
 inline int otb_launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {

@@ -230,15 +230,16 @@ __global__ void __launch_bounds__(256) pair_tree_cols_stage_kernel(float* __rest
   if (col < D && r == 0) v[g0 * row_stride * D + col] = sm[0][c];
 }
 
-inline void pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
+inline int pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
   long stride = 1;
   while (n > 1) {
     const long groups = (n + 63) / 64;
     dim3 grid((D + 31) / 32, (unsigned)groups);
-    otb_chain(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D);
+    if (const int rc = otb_chain(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D)) return rc;
     n = groups;
     stride *= 64;
   }
+  return 0;
 }
 
 // ------------------------------------------------------------ per-head RMSNorm with gain
@@ -834,7 +835,7 @@ inline bool four_aligned(const void* p, long ld, int bf16) { return ld % 4 == 0 
 extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long rows, int D, float inv_d,
                                float eps, int dtype, void* stream) {
   if (D % 8) return -2;
-#define RF(KERN) otb_chain(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
+#define RF(KERN) return otb_chain(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
 #define RFC(MAXC) RF((rmsnorm_fwd_kernel<T, MAXC>))
   if (!rmsnorm_in_registers(rows, D, dtype)) {
     DISPATCH_T(dtype, RF(rmsnorm_fwd_wide_kernel<T>);)
@@ -847,44 +848,43 @@ extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rst
   }
 #undef RFC
 #undef RF
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
                                float* dgamma_partial, long rows, int D, float inv_d, int dtype, void* stream) {
   if (D % 8 || D > 256 * 16) return -2;
+  int launched = 0;
   const long slabs = (rows + NORM_SLAB - 1) / NORM_SLAB;
 #define RB(MAXC)                                                                                                          \
   DISPATCH_T(dtype, {                                                                                                     \
     if (const int rc = otb_allow_smem<rmsnorm_bwd_kernel<T, MAXC>>(NORM_SLAB * 256 * MAXC * 4)) return rc;                   \
-    otb_chain(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
+    launched = otb_chain(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
                                                                                      dgamma_partial, rows, D, inv_d);     \
   })
   if (D <= 256) { RB(1) } else if (D <= 1024) { RB(4) } else if (D <= 2048) { RB(8) } else { RB(16) }
 #undef RB
-  if (dgamma_partial) pair_tree_cols_launch(dgamma_partial, slabs, D, S(stream));
-  return (int)cudaGetLastError();
+  if (launched || !dgamma_partial) return launched;
+  return pair_tree_cols_launch(dgamma_partial, slabs, D, S(stream));
 }
 // x, y, dy, dx: 16-byte aligned, pitches (in elements) that keep every row so; D <= 128, multiple of 8. rows = tokens * heads.
 extern "C" int otb_head_rmsnorm_fwd(const void* x, long ldx, const void* w, void* y, long ldy, float* rstd, long rows, int heads, int D,
                                     float inv_d, float eps, int dtype, void* stream) {
   if (D % 8 || D > 128 || ldx % 8 || ldy % 8) return -2;
-  DISPATCH_T(dtype, otb_chain(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
+  DISPATCH_T(dtype, return otb_chain(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
                                                                                           D, inv_d, eps);)
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_head_rmsnorm_bwd(const void* dy, long lddy, const void* x, long ldx, const void* w, const float* rstd, void* dx, long lddx,
                                     float* dgamma_partial, long rows, int heads, int D, float inv_d, int dtype, void* stream) {
   if (D % 8 || D > 128 || lddy % 8 || ldx % 8 || lddx % 8) return -2;
-  DISPATCH_T(dtype, otb_chain(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
+  int launched = 0;
+  DISPATCH_T(dtype, launched = otb_chain(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
                                                                                           (T*)dx, lddx, dgamma_partial, rows, heads, D, inv_d);)
-  if (dgamma_partial) pair_tree_cols_launch(dgamma_partial, (rows + NORM_SLAB - 1) / NORM_SLAB, D, S(stream));
-  return (int)cudaGetLastError();
+  if (launched || !dgamma_partial) return launched;
+  return pair_tree_cols_launch(dgamma_partial, (rows + NORM_SLAB - 1) / NORM_SLAB, D, S(stream));
 }
 extern "C" long otb_rmsnorm_slabs(long rows) { return (rows + NORM_SLAB - 1) / NORM_SLAB; }
 
 extern "C" int otb_pair_tree_cols(float* v, long n, int D, void* stream) {
-  pair_tree_cols_launch(v, n, D, S(stream));
-  return (int)cudaGetLastError();
+  return pair_tree_cols_launch(v, n, D, S(stream));
 }
 
 extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long ld_out, float* rstd, const float* cosb,
@@ -892,7 +892,7 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
                                    float inv_d, float eps, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(in, ld_in, dtype) && four_aligned(out, ld_out, dtype);
-#define QF(V, NH) DISPATCH_T(dtype, otb_chain(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QF(V, NH) DISPATCH_T(dtype, return otb_chain(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d, eps);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QF(true, 1) } else { QF(false, 1) }
@@ -900,14 +900,13 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
     if (vec) { QF(true, ROPE_HEADS) } else { QF(false, ROPE_HEADS) }
   }
 #undef QF
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* in, long ld_in, const float* rstd,
                                    void* din, long ld_din, const float* cosb, const float* sinb, long rows, int heads,
                                    int D, int seq_len, int do_norm, float inv_d, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(dout, ld_dout, dtype) && four_aligned(in, ld_in, dtype) && four_aligned(din, ld_din, dtype);
-#define QB(V, NH) DISPATCH_T(dtype, otb_chain(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QB(V, NH) DISPATCH_T(dtype, return otb_chain(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QB(true, 1) } else { QB(false, 1) }
@@ -915,46 +914,40 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
     if (vec) { QB(true, ROPE_HEADS) } else { QB(false, ROPE_HEADS) }
   }
 #undef QB
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_swiglu_fwd(const void* gu, void* h, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, otb_chain(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
+    DISPATCH_T(dtype, return otb_chain(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
   } else {
-    DISPATCH_T(dtype, otb_chain(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
+    DISPATCH_T(dtype, return otb_chain(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
   }
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, otb_chain(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
+    DISPATCH_T(dtype, return otb_chain(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
   } else {
-    DISPATCH_T(dtype, otb_chain(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
+    DISPATCH_T(dtype, return otb_chain(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
   }
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
 #define CE(U, TEST) \
-  DISPATCH_T(dtype, otb_chain(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+  DISPATCH_T(dtype, return otb_chain(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
   const int form = ce_form(rows, V, dtype);
   if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_det_sum(const float* x, long n, int mode, float post_scale, float* out, void* stream) {
-  otb_chain(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
-  return (int)cudaGetLastError();
+  return otb_chain(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
 }
 extern "C" int otb_embedding_fwd(const long* ids, const void* table, void* out, long rows, int D, int dtype,
                                  void* stream) {
   if (D % 8) return -2;
-  DISPATCH_T(dtype, otb_chain(embedding_fwd_kernel<T>, (unsigned)rows, 128, 0, S(stream), ids, (const T*)table, (T*)out, rows,
+  DISPATCH_T(dtype, return otb_chain(embedding_fwd_kernel<T>, (unsigned)rows, 128, 0, S(stream), ids, (const T*)table, (T*)out, rows,
                                                                                     D);)
-  return (int)cudaGetLastError();
 }
 extern "C" int otb_embedding_bwd(const void* dy, const long* sorted_ids, const long* sorted_tok, long n, float* dW, int D,
                                  int accumulate, int dtype, void* stream) {

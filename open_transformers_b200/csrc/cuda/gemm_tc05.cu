@@ -699,8 +699,10 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   cfg.attrs = &cluster;
   cfg.numAttrs = 1;
   const int group_m = 8;
-  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m, scale_a, scale_b,
-                                 status, TpNone{});
+  const int rc = (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m, scale_a,
+                                         scale_b, status, TpNone{});
+  if (rc) (void)cudaGetLastError();  // the code is the only report
+  return rc;
 }
 
 // Share of the chip's tensor-core time that goes into wanted products when tm x tn tiles of an M x N result run on `workers`:
