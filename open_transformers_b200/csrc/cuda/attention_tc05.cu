@@ -36,6 +36,7 @@
 #include "tc05.cuh"
 #include "common.cuh"
 #include "det_math.h"
+#include "entries.cuh"
 
 using namespace tc05;
 

@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "det_math.h"
+#include "entries.cuh"
 #include "ew_common.cuh"
 #include "tc05.cuh"
 

@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "det_math.h"
+#include "entries.cuh"
 
 namespace {
 

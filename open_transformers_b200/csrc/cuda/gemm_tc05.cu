@@ -49,6 +49,7 @@
 // (reference docs/MODEL_OP_DTYPE_TRACE.md:82,100).
 #include "tc05.cuh"
 #include "common.cuh"
+#include "entries.cuh"
 
 using namespace tc05;
 
