@@ -1429,7 +1429,6 @@ constexpr int DELTA_ROWS = 8;
 template <bool VEC>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, long lddo, const __nv_bfloat16* __restrict__ O,
                                   long ldo, const float* __restrict__ lse, float* __restrict__ delta, int B, int T, int H, int D) {
-  after_predecessor();
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const long rows = (long)B * T, groups = (rows + DELTA_ROWS - 1) / DELTA_ROWS;
@@ -1582,16 +1581,19 @@ extern "C" int otb_attn_fwd(const void* qk, long ldqk, const void* qkv, long ldq
   const int nq = (T + BQ - 1) / BQ;
   const unsigned grid = persistent_grid((long)((nq + 1) / 2) * H * B);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  // Early where most of the chip is free anyway (us, ordinary and early: 12 CTAs 9.0 and 8.4, 24 13.9 and 13.4, 48 24.5 and 23.8, 64
+  // 33.8 and 33.2, each heads x pairs of query tiles); with 128 and 148 CTAs it loses (56.6 and 58.0, 406 and 420, windowed 176 and 179).
+  const bool early = 2 * (int)grid <= otb_sm_count();
   if (D == 128) {
     const int rc = otb_allow_smem<attn_fwd2_kernel<128>>(attn_fwd2_smem_bytes<128>());
     if (rc) return rc;
-    return otb_chain(attn_fwd2_kernel<128>, grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv,
-                     window, c_log2, status);
+    return otb_launch_if_early(early, attn_fwd2_kernel<128>, grid, F2_THREADS, attn_fwd2_smem_bytes<128>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T,
+                               H, Hkv, window, c_log2, status);
   } else {
     const int rc = otb_allow_smem<attn_fwd2_kernel<64>>(attn_fwd2_smem_bytes<64>());
     if (rc) return rc;
-    return otb_chain(attn_fwd2_kernel<64>, grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T, H, Hkv,
-                     window, c_log2, status);
+    return otb_launch_if_early(early, attn_fwd2_kernel<64>, grid, F2_THREADS, attn_fwd2_smem_bytes<64>(), s, tq, tv, (__nv_bfloat16*)O, ldo, lse, B, T,
+                               H, Hkv, window, c_log2, status);
   }
 }
 
@@ -1640,7 +1642,7 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   const long warps = ((long)B * T + DELTA_ROWS - 1) / DELTA_ROWS * H;
   const bool vec = ((reinterpret_cast<uintptr_t>(O) | reinterpret_cast<uintptr_t>(dO)) & 7) == 0;  // pitches are multiples of 8 elements
   auto delta_kernel = vec ? attn_delta_kernel<true> : attn_delta_kernel<false>;
-  if (const int rc = otb_chain(delta_kernel, (unsigned)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse,
+  if (const int rc = otb_launch(delta_kernel, (unsigned)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)dO, lddo, (const __nv_bfloat16*)O, ldo, lse,
                                delta, B, T, H, D))
     return rc;
   __nv_bfloat16* dQp = (__nv_bfloat16*)dqk;

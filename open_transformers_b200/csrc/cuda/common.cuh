@@ -70,17 +70,19 @@ inline int otb_allow_smem(int bytes) {
   return 0;
 }
 
-// Launches that may begin while the kernel before them in the stream still runs.
-// In a chain: otb_chain launches small grids that way, and the kernel calls after_predecessor() before it touches any memory.
-// What then overlaps is the launch itself, the CTAs' start and their set-up (barriers, tensor memory); a chain of kernels that
-// take 4 to 15 us each pays them one after the other otherwise (logits of 333 tokens through the six-layer 100M model: 594 ->
-// 559 us). A kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that
-// it needs. Large grids gain nothing. Not for kernels with a few small CTAs per SM that all take long: placed before the SMs
-// are free they pile up on some (an exact fp32 product of 512 two-warp CTAs took 1.4 to 1.6 times as long).
+// Launches that may begin while the kernel before them in the stream still runs, behind a kernel that calls let_successor_begin();
+// behind any other, and in front of an ordinary launch, the order of the stream is the ordinary one.
+// Behind a predecessor: the kernel calls after_predecessor() before it touches any memory. What then overlaps is the launch, the
+// CTAs' start and their set-up (barriers, tensor memory), which a chain of kernels of 4 to 15 us pays one after the other otherwise.
+// A kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that it needs.
+// The products are launched that way, and the attention forward where it is small; the memory-bound kernels only let a product
+// behind them begin. Launched early themselves they gain less than they cost, since CTAs that are placed before the SMs are
+// free pile up on some: us, every launch ordinary / as it is / every grid of up to 8 CTAs per SM early: block without gradients,
+// 768 wide, 16 tokens 45.0 / 41.1 / 40.4, 333 tokens 52.0 / 48.3 / 52.5, 2048 wide, 1111 tokens 146 / 142 / 152; feed-forward sublayer
+// forward and backward, 2048 wide, 128 tokens 128 / 123 / 132.
 // Side by side, where two kernels need nothing of each other: the first, launched in the ordinary way, calls
-// let_successor_begin(), so that all that ran before it is complete by then; the second, launched by otb_launch_early, touches
-// memory at once and lets one thread call wait_for_predecessor() at its end, so that what follows in the stream waits for both.
-// Behind anything but such a kernel, and in front of it, the order of the stream is the ordinary one.
+// let_successor_begin(), so that all that ran before it is complete by then; the second touches memory at once and lets one
+// thread call wait_for_predecessor() at its end, so that what follows in the stream waits for both.
 __device__ __forceinline__ void let_successor_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_predecessor() {
@@ -112,18 +114,16 @@ inline int otb_launch_args(bool early, const void* kern, dim3 grid, dim3 block, 
   return rc;
 }
 template <typename... P, typename... A>
+inline int otb_launch_if_early(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  return otb_launch_args<P...>(early, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
 inline int otb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  return otb_launch_args<P...>(false, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
+  return otb_launch_if_early(false, kern, grid, block, smem, s, args...);
 }
 template <typename... P, typename... A>
 inline int otb_launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  return otb_launch_args<P...>(true, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
-}
-constexpr unsigned CHAIN_CTAS_PER_SM = 8;
-template <typename... P, typename... A>
-inline int otb_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  const bool small = (unsigned long)grid.x * grid.y * grid.z <= (unsigned long)CHAIN_CTAS_PER_SM * otb_sm_count();
-  return otb_launch_args<P...>(small, reinterpret_cast<const void*>(kern), grid, block, smem, s, static_cast<P>(args)...);
+  return otb_launch_if_early(true, kern, grid, block, smem, s, args...);
 }
 
 #define OTB_CUDA_CHECK_RET(expr)              \

@@ -30,7 +30,7 @@ namespace {
 template <typename T, int MAXC>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                                          float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
-  after_predecessor();
+  let_successor_begin();
   const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
 template <typename T>
 __global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                         float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
-  after_predecessor();
+  let_successor_begin();
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -130,7 +130,7 @@ template <typename T, int MAXC>
 __global__ void __launch_bounds__(NORM_SLAB * 32) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                                                     const float* __restrict__ rstd_in, T* __restrict__ dx,
                                                                     float* __restrict__ dgamma_partial, long rows, int D, float inv_d) {
-  after_predecessor();
+  let_successor_begin();
   extern __shared__ float prod[];  // [NORM_SLAB][MAXC * 256] when dgamma is wanted
   const long slab = blockIdx.x;
   const int lane = threadIdx.x & 31, wrow = threadIdx.x >> 5;
@@ -215,7 +215,6 @@ __global__ void __launch_bounds__(NORM_SLAB * 32) rmsnorm_bwd_kernel(const T* __
 // log-depth instead of a serial chain. Logical row j lives at v[j * row_stride * D]. A missing partner leaves the
 // value untouched (never "+ 0.0", which would turn -0.0 into +0.0).
 __global__ void __launch_bounds__(256) pair_tree_cols_stage_kernel(float* __restrict__ v, long n, long row_stride, int D) {
-  after_predecessor();
   __shared__ float sm[64][33];
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;  // 32 columns x 8 row-threads
   const int col = blockIdx.x * 32 + c;
@@ -236,7 +235,7 @@ inline int pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
   while (n > 1) {
     const long groups = (n + 63) / 64;
     dim3 grid((D + 31) / 32, (unsigned)groups);
-    if (const int rc = otb_chain(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D)) return rc;
+    if (const int rc = otb_launch(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D)) return rc;
     n = groups;
     stride *= 64;
   }
@@ -257,7 +256,6 @@ __device__ __forceinline__ float half_butterfly(float v) {
 template <typename T>
 __global__ void __launch_bounds__(256) head_rmsnorm_fwd_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, T* __restrict__ y, long ldy,
                                                               float* __restrict__ rstd_out, long rows, int heads, int D, float inv_d, float eps) {
-  after_predecessor();
   const long row = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
   const int c = (threadIdx.x & 15) * 8;
   const bool on = row < rows && c < D;
@@ -289,7 +287,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) head_rmsnorm_bwd_kernel(const T* __restrict__ dy, long lddy, const T* __restrict__ x, long ldx, const T* __restrict__ w,
                                                               const float* __restrict__ rstd_in, T* __restrict__ dx, long lddx,
                                                               float* __restrict__ dgamma_partial, long rows, int heads, int D, float inv_d) {
-  after_predecessor();
+  let_successor_begin();
   __shared__ float prod[16][128];
   const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
   const long row = (long)blockIdx.x * 16 + r;
@@ -394,7 +392,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restric
                                        float* __restrict__ rstd_out, const float* __restrict__ cosb,
                                        const float* __restrict__ sinb, long rows, int heads, int D, int seq_len,
                                        int do_norm, float inv_d, float eps) {
-  after_predecessor();
+  let_successor_begin();
   long row;
   int head0;
   if (!rope_place<NH>(rows, heads, row, head0)) return;
@@ -446,7 +444,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restric
                                        const float* __restrict__ rstd_in, T* __restrict__ din, long ld_din,
                                        const float* __restrict__ cosb, const float* __restrict__ sinb, long rows,
                                        int heads, int D, int seq_len, int do_norm, float inv_d) {
-  after_predecessor();
+  let_successor_begin();
   long row;
   int head0;
   if (!rope_place<NH>(rows, heads, row, head0)) return;
@@ -543,7 +541,7 @@ __device__ __forceinline__ void swiglu8_bwd(const Raw8<T>& rg, const Raw8<T>& ru
 // One thread per group of eight, wherever its row is.
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* __restrict__ gu, T* __restrict__ h, long rows, int F) {
-  after_predecessor();
+  let_successor_begin();
   const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (idx >= rows * F) return;
   const long row = idx / F;
@@ -555,7 +553,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* __restric
 }
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_bwd_flat_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, long rows, int F) {
-  after_predecessor();
+  let_successor_begin();
   const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (idx >= rows * F) return;
   const long row = idx / F, at = row * 2 * F + (idx - row * F);
@@ -575,7 +573,7 @@ constexpr int SWIGLU_MAX_THREADS = 384;
 inline bool swiglu_per_row(long rows, int F) { return F >= 1024 && rows >= 2048 && rows <= 0x7fffffffL; }
 template <typename T>
 __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ h, int F) {
-  after_predecessor();
+  let_successor_begin();
   const T* gr = gu + (long)blockIdx.x * 2 * F;
   T* hr = h + (long)blockIdx.x * F;
   for (int c0 = threadIdx.x * 8; c0 < F; c0 += blockDim.x * 16) {
@@ -598,7 +596,7 @@ __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T*
 // d_gate_up [rows, 2F] from dh [rows, F]
 template <typename T>
 __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, int F) {
-  after_predecessor();
+  let_successor_begin();
   const T* gr = gu + (long)blockIdx.x * 2 * F;
   const T* dr = dh + (long)blockIdx.x * F;
   T* or_ = dgu + (long)blockIdx.x * 2 * F;
@@ -694,7 +692,7 @@ template <typename T, int CE_UNROLL, bool TEST>
 __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ logits, const long* __restrict__ labels,
                                                               float* __restrict__ ce_out, float* __restrict__ lse_out,
                                                               long rows, int V, float two_z, float scale, int write_grad) {
-  after_predecessor();
+  let_successor_begin();
   using namespace tc05;
   __shared__ float sh[32];
   const long row = blockIdx.x;
@@ -759,7 +757,6 @@ inline int ce_form(long rows, int V, bool bf16) {
 // mode 0: sum x, 1: sum x*x (fma chain). out[0] = result * post_scale.
 __global__ void __launch_bounds__(1024) det_sum_kernel(const float* __restrict__ x, long n, int mode, float post_scale,
                                                         float* __restrict__ out) {
-  after_predecessor();
   __shared__ float sh[32];
   float acc = 0.0f;
   for (long i = threadIdx.x; i < n; i += 1024) {
@@ -774,7 +771,6 @@ __global__ void __launch_bounds__(1024) det_sum_kernel(const float* __restrict__
 template <typename T>
 __global__ void embedding_fwd_kernel(const long* __restrict__ ids, const T* __restrict__ table, T* __restrict__ out,
                                      long rows, int D) {
-  after_predecessor();
   const long row = blockIdx.x;
   const long id = ids[row];
   const uint4* src = reinterpret_cast<const uint4*>(table + id * D);
@@ -836,7 +832,7 @@ inline bool four_aligned(const void* p, long ld, int bf16) { return ld % 4 == 0 
 extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long rows, int D, float inv_d,
                                float eps, int dtype, void* stream) {
   if (D % 8) return -2;
-#define RF(KERN) return otb_chain(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
+#define RF(KERN) return otb_launch(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
 #define RFC(MAXC) RF((rmsnorm_fwd_kernel<T, MAXC>))
   if (!rmsnorm_in_registers(rows, D, dtype)) {
     DISPATCH_T(dtype, RF(rmsnorm_fwd_wide_kernel<T>);)
@@ -858,7 +854,7 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
 #define RB(MAXC)                                                                                                          \
   DISPATCH_T(dtype, {                                                                                                     \
     if (const int rc = otb_allow_smem<rmsnorm_bwd_kernel<T, MAXC>>(NORM_SLAB * 256 * MAXC * 4)) return rc;                   \
-    launched = otb_chain(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
+    launched = otb_launch(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
                                                                                      dgamma_partial, rows, D, inv_d);     \
   })
   if (D <= 256) { RB(1) } else if (D <= 1024) { RB(4) } else if (D <= 2048) { RB(8) } else { RB(16) }
@@ -870,14 +866,14 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
 extern "C" int otb_head_rmsnorm_fwd(const void* x, long ldx, const void* w, void* y, long ldy, float* rstd, long rows, int heads, int D,
                                     float inv_d, float eps, int dtype, void* stream) {
   if (D % 8 || D > 128 || ldx % 8 || ldy % 8) return -2;
-  DISPATCH_T(dtype, return otb_chain(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
+  DISPATCH_T(dtype, return otb_launch(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
                                                                                           D, inv_d, eps);)
 }
 extern "C" int otb_head_rmsnorm_bwd(const void* dy, long lddy, const void* x, long ldx, const void* w, const float* rstd, void* dx, long lddx,
                                     float* dgamma_partial, long rows, int heads, int D, float inv_d, int dtype, void* stream) {
   if (D % 8 || D > 128 || lddy % 8 || ldx % 8 || lddx % 8) return -2;
   int launched = 0;
-  DISPATCH_T(dtype, launched = otb_chain(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
+  DISPATCH_T(dtype, launched = otb_launch(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
                                                                                           (T*)dx, lddx, dgamma_partial, rows, heads, D, inv_d);)
   if (launched || !dgamma_partial) return launched;
   return pair_tree_cols_launch(dgamma_partial, (rows + NORM_SLAB - 1) / NORM_SLAB, D, S(stream));
@@ -893,7 +889,7 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
                                    float inv_d, float eps, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(in, ld_in, dtype) && four_aligned(out, ld_out, dtype);
-#define QF(V, NH) DISPATCH_T(dtype, return otb_chain(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QF(V, NH) DISPATCH_T(dtype, return otb_launch(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d, eps);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QF(true, 1) } else { QF(false, 1) }
@@ -907,7 +903,7 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
                                    int D, int seq_len, int do_norm, float inv_d, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(dout, ld_dout, dtype) && four_aligned(in, ld_in, dtype) && four_aligned(din, ld_din, dtype);
-#define QB(V, NH) DISPATCH_T(dtype, return otb_chain(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QB(V, NH) DISPATCH_T(dtype, return otb_launch(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QB(true, 1) } else { QB(false, 1) }
@@ -919,35 +915,35 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
 extern "C" int otb_swiglu_fwd(const void* gu, void* h, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, return otb_chain(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
+    DISPATCH_T(dtype, return otb_launch(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
   } else {
-    DISPATCH_T(dtype, return otb_chain(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
+    DISPATCH_T(dtype, return otb_launch(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
   }
 }
 extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, return otb_chain(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
+    DISPATCH_T(dtype, return otb_launch(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
   } else {
-    DISPATCH_T(dtype, return otb_chain(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
+    DISPATCH_T(dtype, return otb_launch(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
   }
 }
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
 #define CE(U, TEST) \
-  DISPATCH_T(dtype, return otb_chain(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+  DISPATCH_T(dtype, return otb_launch(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
   const int form = ce_form(rows, V, dtype);
   if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
 }
 extern "C" int otb_det_sum(const float* x, long n, int mode, float post_scale, float* out, void* stream) {
-  return otb_chain(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
+  return otb_launch(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
 }
 extern "C" int otb_embedding_fwd(const long* ids, const void* table, void* out, long rows, int D, int dtype,
                                  void* stream) {
   if (D % 8) return -2;
-  DISPATCH_T(dtype, return otb_chain(embedding_fwd_kernel<T>, (unsigned)rows, 128, 0, S(stream), ids, (const T*)table, (T*)out, rows,
+  DISPATCH_T(dtype, return otb_launch(embedding_fwd_kernel<T>, (unsigned)rows, 128, 0, S(stream), ids, (const T*)table, (T*)out, rows,
                                                                                     D);)
 }
 extern "C" int otb_embedding_bwd(const void* dy, const long* sorted_ids, const long* sorted_tok, long n, float* dW, int D,

@@ -769,8 +769,8 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   int grid = tiles < max_ctas ? tiles : max_ctas;
   if (grid < 1) grid = 1;
   const int group_m = 8;
-  return otb_chain(kern, grid, NUM_THREADS, L::TOTAL, stream, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m,
-                   scale_a, scale_b, status, TpNone{});
+  return otb_launch_early(kern, grid, NUM_THREADS, L::TOTAL, stream, ta, tb, tc, C, reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, group_m,
+                          scale_a, scale_b, status, TpNone{});
 }
 
 template <int BN, int STAGES, bool B_MN, int EPI, int TP>

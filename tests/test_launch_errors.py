@@ -1,5 +1,6 @@
 """What an entry point returns when a launch is refused, against a fake runtime: an early launch that is refused is tried in the
-ordinary way; an error is returned by the call whose launch it was, once, and nothing that depends on that launch follows it."""
+ordinary way; an error is returned by the call whose launch it was, once, and nothing that depends on that launch follows it. And
+which launches are early: products, the attention forward on half the chip, dQ beside dK/dV."""
 import pytest
 from fake_cudart import run_with_fake
 
@@ -48,8 +49,9 @@ single = {
 # a single launch: refused early only, then both ways; the next call is not charged with it
 ONE = HEAD + r"""
 for name, call in single.items():
+    early = name in ("gemm", "attn_fwd", "attn_fwd_64")
     fake.fake_reset()
-    assert call() == 0 and fake.fake_launched() == fake.fake_launched_early() == 1, name
+    assert call() == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (1, early), name
     fake.fake_reset()
     fake.fake_refuse_launch(EARLY, 0, 1, 801)
     assert call() == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (1, 0), name
@@ -58,7 +60,14 @@ for name, call in single.items():
     fake.fake_refuse_launch(ORDINARY, 0, 1, 701)
     assert call() == 701 and fake.fake_launched() == 0, name
     assert fake.fake_pending() == 0, name
+    fake.fake_reset()
     assert call() == 0, name
+for T, early in ((18 * 256, True), (18 * 256 + 1, False), (64 * 256, False)):  # 4 heads: 72, 76 and 256 pairs of query tiles, 148 SMs
+    fake.fake_reset()
+    assert attn_fwd(128, T) == attn_fwd(64, T) == 0 and fake.fake_launched_early() == 2 * early, T
+for M in (1, 4096, 148 * 128):
+    fake.fake_reset()
+    assert gemm(M) == 0 and fake.fake_launched_early() == 1, M
 fake.fake_reset()
 fake.fake_refuse_launch(EARLY, 0, 1, 701)  # a CTA pair's launch has a cluster attribute and no second try
 assert gemm(1 << 16) == 701 and fake.fake_pending() == 0
@@ -71,9 +80,9 @@ SEVERAL = HEAD + r"""
 for D in (64, 128):
     for T in (128, 100):  # both forms of dK/dV
         fake.fake_reset()
-        assert attn_bwd(D, T) == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (3, 2)
+        assert attn_bwd(D, T) == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (3, 1)
         fake.fake_reset()
-        fake.fake_refuse_launch(EARLY, 0, 2, 801)
+        fake.fake_refuse_launch(EARLY, 0, 1, 801)
         assert attn_bwd(D, T) == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (3, 0)
         for nth in range(3):
             fake.fake_reset()
@@ -81,8 +90,8 @@ for D in (64, 128):
             fake.fake_refuse_launch(ORDINARY, nth, 1, 701)
             assert attn_bwd(D, T) == 701 and fake.fake_launched() == nth and fake.fake_pending() == 0, (D, T, nth)
         fake.fake_reset()
-        fake.fake_refuse_launch(EARLY, 1, 1, 801)
-        fake.fake_refuse_launch(ORDINARY, 0, 1, 701)  # dK/dV by itself
+        fake.fake_refuse_launch(EARLY, 0, 1, 801)
+        fake.fake_refuse_launch(ORDINARY, 1, 1, 701)  # dK/dV by itself
         assert attn_bwd(D, T) == 701 and fake.fake_launched() == 1 and fake.fake_pending() == 0, (D, T)
 for call, rows in ((rmsnorm_bwd, 64), (rmsnorm_bwd, 8 * 1200), (head_rmsnorm_bwd, 64), (head_rmsnorm_bwd, 16 * 1200)):
     fake.fake_reset()

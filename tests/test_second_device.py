@@ -25,7 +25,6 @@ for dev in (0, 1, 0, 1):
         assert calls(D) == (0, 0, 0), (dev, D, calls(D))
     counts.append(fake.fake_asked())
 assert fake.fake_launched() == 4 * 2 * (1 + 3 + 1)
-assert fake.fake_launched_early() == 4 * 2 * 1  # the norm's: a small grid in a chain
 assert counts[1] == 2 * counts[0] and counts[3] == counts[1], counts  # once per kernel and device
 print("ok")
 """
