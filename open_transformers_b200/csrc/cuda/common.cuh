@@ -80,9 +80,14 @@ inline int otb_allow_smem(int bytes) {
 // free pile up on some: us, every launch ordinary / as it is / every grid of up to 8 CTAs per SM early: block without gradients,
 // 768 wide, 16 tokens 45.0 / 41.1 / 40.4, 333 tokens 52.0 / 48.3 / 52.5, 2048 wide, 1111 tokens 146 / 142 / 152; feed-forward sublayer
 // forward and backward, 2048 wide, 128 tokens 128 / 123 / 132.
+// A kernel that waits exists while what it reads is still being written. Its inputs, and what it both reads and writes, are
+// therefore not __restrict__ and not read by __ldg: either would tell the compiler that nothing changes them while the kernel
+// runs, and let it take a load past the wait, whose "memory" clobber covers only what others may write. Buffers that are only
+// written may be __restrict__, as what goes into them follows from loads behind the wait.
 // Side by side, where two kernels need nothing of each other: the first, launched in the ordinary way, calls
 // let_successor_begin(), so that all that ran before it is complete by then; the second touches memory at once and lets one
-// thread call wait_for_predecessor() at its end, so that what follows in the stream waits for both.
+// thread call wait_for_predecessor() at its end, so that what follows in the stream waits for both. It reads nothing that its
+// predecessor writes and may say so.
 __device__ __forceinline__ void let_successor_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_predecessor() {

@@ -175,8 +175,8 @@ template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool I8, int TP, ty
 __global__ void __launch_bounds__(TP >= 2 ? NUM_THREADS + 128 : NUM_THREADS, 1)
 gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, void* __restrict__ Cv,
-                 const __nv_bfloat16* __restrict__ R, int M, int N, int K, long ldc, long ldr, int group_m,
-                 const float* __restrict__ scale_a, const float* __restrict__ scale_b, uint32_t* __restrict__ status,
+                 const __nv_bfloat16* R, int M, int N, int K, long ldc, long ldr, int group_m,
+                 const float* scale_a, const float* scale_b, uint32_t* __restrict__ status,
                  const __grid_constant__ TPA tp) {
   static_assert(!I8 || (!A_MN && !B_MN), "the int8 path takes K-major operands only");
   static_assert(TP == 0 || !I8, "the tensor-parallel variants are bf16");
@@ -552,7 +552,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           // dequantise: the int32 sum is exact; float(acc) rounds once, then one multiply by sa * sb[col]
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const float sb = col + j < N ? __ldg(scale_b + col + j) : 0.0f;
+            const float sb = col + j < N ? scale_b[col + j] : 0.0f;
             v[j] = __float_as_uint(__fmul_rn(__int2float_rn((int)v[j]), __fmul_rn(sa0, sb)));
           }
         }

@@ -33,3 +33,40 @@ def test_entry_points_called_across_files_are_declared_once():
         header = next(iter(declared[name]))
         for user in defined[name] | called[name]:
             assert header == user or '#include "%s"' % header in (CUDA / user).read_text(), (name, user, header)
+
+
+def _kernels(text: str):
+    """(name, parameters, body) of every __global__ function."""
+    for m in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\s*\(", text):
+        def close(i, pair):
+            depth = 1
+            while depth:
+                depth += {pair[0]: 1, pair[1]: -1}.get(text[i], 0)
+                i += 1
+            return i
+        end = close(m.end(), "()")
+        start = text.index("{", end) + 1
+        yield m[1], text[m.end():end], text[start:close(start, "{}")]
+
+
+WRITTEN_ONLY = {"O", "Cv", "lse_out", "status"}
+
+
+def test_kernels_that_wait_promise_nothing_of_what_they_read():
+    """A kernel that is launched while its predecessor still writes must not call its inputs unchanging: the compiler might take
+    a load past the wait. It has to wait in the first place, and the early kernel of a pair at its end."""
+    waiting, early, launched = set(), set(), set()
+    for path in sorted(CUDA.glob("*.cu")):
+        text = _source(path)
+        for name, params, body in _kernels(text):
+            if "after_predecessor()" in body:
+                waiting.add(name)
+                assert "__ldg" not in re.sub(r"if constexpr \(TP == 1\).*?\n    }\n  }\n", "", body, flags=re.S), name
+                for const, p in re.findall(r"(const\s+)?[\w:]+\s*\*\s*__restrict__\s+(\w+)", params):
+                    assert not const and p in WRITTEN_ONLY, (name, p)
+            elif "wait_for_predecessor()" in body:
+                early.add(name)
+        aliases = dict(re.findall(r"auto (\w+) = [^;]*?\b(\w+_kernel)\b", text))
+        launched |= {aliases.get(n, n) for n in re.findall(r"\botb_launch_(?:early\(|if_early\(\s*\w+,)\s*(\w+)", text)}
+    assert waiting == {"attn_fwd2_kernel", "gemm_tc05_kernel"} and early == {"attn_bwd_q2_kernel"}
+    assert launched == waiting | early, launched
