@@ -735,11 +735,22 @@ bool pair_wins(int M, int N, int K, bool mn_major, bool i8, int max_ctas, double
   return N > 128 && K > (i8 ? PAIR_ABOVE_K_I8 : PAIR_ABOVE_K) && tiles >= max_ctas / 2 && max_ctas >= 2 &&
          (!mn_major || 2.0 * M * N * K <= PAIR_MN_FLOPS) && PAIR_GAIN * tile_efficiency(M, N, 2 * BM, 256, max_ctas / 2) > single;
 }
-// Where even 64-wide tiles fit the chip in one wave, more SMs share the loads and each has less to load, multiply and store
-// (wider and 64-wide tiles, us: 333 x 768 x 768 with residual 8.8 and 6.0, 1111 x 768 x 2048 13.0 and 9.7, the data gradient
-// 1111 x 768 x 4096 17.8 and 14.8, the weight gradient 768 x 2048 x 1111 9.1 and 7.8; nowhere longer). In a second wave
-// they would read A twice as often as 128-wide ones.
+// Where even 64-wide tiles fit the chip in one wave, more SMs share the loads and each has less to load, multiply and store: 0.92 to
+// 0.97 of the wider tile's time as a plain product, 0.73 to 0.90 with a residual, 0.88 to 0.93 as an accumulated weight gradient
+// (us, wider and 64-wide: 333 x 768 x 768 5.1 and 4.8, with residual 7.4 and 5.7, 1111 x 768 x 2048 8.9 and 8.6, 640 x 768 x 2048
+// with residual 10.3 and 9.0, weight gradient 9.6 and 8.6; worst, tall and 128 columns wide, 9472 x 128 x 768, 5.3 and 5.4). In a
+// second wave they would read A twice as often as 128-wide ones.
+// But a small A is read by every tile at once, from few places of the L2: below 128 KB of it more than 32 columns of tiles take up to
+// 1.5 times as long as half as many wider ones (16 x 4096 x 768 5.0 and 5.7, 28 x 4096 x 2048 1.23 times, 8 x 4096 x 4096 1.21), from
+// there on they win (32 x 4096 x 2048 and 16 x 4096 x 4096 0.95; 80 x 5632 x 768, 123 KB, 1.10, 100 x 5632 x 768 0.97), as do up
+// to 32 columns of any A (1 to 96 rows x 2048 x 256 to 2048 0.92 to 0.99).
 constexpr int SLIM = 64;
+constexpr int SLIM_ANY_A = 32;             // columns of tiles
+constexpr long SLIM_A_ELEMS = 128 << 9;    // 128 KB of bf16
+bool slim_wins(int M, int N, int K, int max_ctas) {
+  const long tiles_n = (N + SLIM - 1) / SLIM;
+  return (M + BM - 1) / BM * tiles_n <= max_ctas && (tiles_n <= SLIM_ANY_A || (long)M * K >= SLIM_A_ELEMS);
+}
 // Tile of a product: columns of a single CTA's tile, or PAIR_TILE.
 constexpr int PAIR_TILE = 512;
 int choose_tile(int M, int N, int K, bool mn_major, bool i8, int max_ctas) {
@@ -754,7 +765,7 @@ int choose_tile(int M, int N, int K, bool mn_major, bool i8, int max_ctas) {
     const double e256 = N >= 256 ? tile_efficiency(M, N, BM, 256, max_ctas) : 0.0;
     BN = e256 >= e128 ? 256 : 128;
     single = BN == 256 ? e256 : e128;
-    if ((long)((M + BM - 1) / BM) * ((N + SLIM - 1) / SLIM) <= max_ctas) return SLIM;
+    if (slim_wins(M, N, K, max_ctas)) return SLIM;
   }
   return pair_wins(M, N, K, mn_major, i8, max_ctas, single) ? PAIR_TILE : BN;
 }

@@ -1,4 +1,5 @@
-"""The rule that chooses a product's tile, asked on the host for 148 SMs: where CTA pairs (512) take over from single CTAs."""
+"""The rule that chooses a product's tile, asked on the host for 148 SMs: where CTA pairs (512) take over from single CTAs, and
+where 64-wide tiles, which have to fit the chip in one wave, take over from wider ones."""
 import pytest
 
 from open_transformers_b200 import build_native
@@ -27,3 +28,21 @@ def test_no_pairs_on_one_cta():
     if not (build_native.EXT / "libotb_cuda.so").exists():
         pytest.skip("the CUDA library is not built here")
     assert cuda_lib().otb_gemm_tile(16384, 5632, 2048, 0, 0, 1) in (128, 256)
+
+
+@pytest.mark.parametrize("mn", [0, 1])
+@pytest.mark.parametrize("M,N,K,sms,slim", [
+    (1, 8, 8, 148, True), (333, 768, 768, 148, True), (1111, 768, 2048, 148, True),           # 1, 36 and 108 tiles
+    (37 * 128, 256, 72, 148, True), (37 * 128 + 1, 256, 72, 148, False),                       # 148 tiles, and one row more
+    (128, 148 * 64, 2048, 148, True), (128, 148 * 64 + 8, 2048, 148, False),                   # 148, and eight columns more
+    (1, 2048, 8, 148, True), (16, 2048, 768, 148, True), (1, 2056, 2048, 148, False),          # 32 columns of tiles, and 33
+    (31, 4096, 2048, 148, False), (32, 4096, 2048, 148, True), (16, 4096, 4096, 148, True),    # 33 and more: from 128 KB of A on
+    (16, 4096, 768, 148, False), (85, 5632, 768, 148, False), (86, 5632, 768, 148, True),
+    (148 * 128, 64, 64, 148, True), (148 * 128, 72, 64, 148, False),                           # narrow results of many rows
+    (128, 64, 64, 1, True), (128, 72, 64, 1, False), (333, 768, 768, 35, False), (333, 768, 768, 36, True),  # a capped grid
+])
+def test_where_slim_tiles_end(M, N, K, sms, slim, mn):
+    if not (build_native.EXT / "libotb_cuda.so").exists():
+        pytest.skip("the CUDA library is not built here")
+    assert (cuda_lib().otb_gemm_tile(M, N, K, mn, 0, sms) == 64) == slim
+    assert cuda_lib().otb_gemm_tile(M, N, K, 0, 1, sms) != 64  # int8 products keep their tiles
