@@ -185,15 +185,17 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 
 template <int TM, int TN, int RM, int RN, int RES = 0>
 int launch_gemm_f32(const float* A, const float* B, float* C, const float* R, int M, int N, int K, long lda, long ldb, long ldc, long ldr,
-                    int a_mn, int b_mn, int epi, int vec, cudaStream_t s) {
+                    int a_mn, int b_mn, int epi, int vec, cudaStream_t s, bool predicate = true) {
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-  // Predicated loads pay with two MN-major operands, the weight gradients (256 x 704 x 2048 71.5 -> 46.5 us, 1408 x 256 x 2048 85.4 ->
-  // 68.3, 4096 x 4096 x 512 411 -> 376), and with two K-major ones in 64-wide tiles (2048 x 1408 x 256 66.7 -> 61.2); not in
-  // 128-wide ones (4096 x 4096 x 512 465 -> 480) and not with one of each kind (2048 x 256 x 1408 75 -> 78).
-  const bool whole = (vec & 3) == 3 && (a_mn ? M : K) % 4 == 0 && (b_mn ? N : K) % 4 == 0;
+  // Predicated loads, us, branches and predicated. They pay with two MN-major operands, the weight gradients, in 32-wide tiles (704 x 256 x
+  // 2048 72.1 and 46.6, accumulating 70.3 and 57.3; 128 x 128 x 64 4.4 and 3.3), in 64-wide ones (but see the caller), and in 128-wide
+  // ones that store (4096 x 4096 x 512 411 and 376, 8192 x 4096 x 256 411 and 375), not in those that accumulate (450 and 472, 477 and
+  // 514); and with two K-major ones that store from 64-wide tiles (2048 x 1408 x 256 66.1 and 61.2, 768 x 2048 x 1000 129.9 and
+  // 125.0), not accumulating (38.7 and 39.9, 125.5 and 128.5) nor in 128-wide ones (464 and 480). Elsewhere they differ in both directions.
+  const bool whole = predicate && (vec & 3) == 3 && (a_mn ? M : K) % 4 == 0 && (b_mn ? N : K) % 4 == 0;
 #define GF(AM, BM, E)                                                                                    \
   do {                                                                                                   \
-    constexpr bool PAYS = AM == BM && (AM || TM == 64);                                                  \
+    constexpr bool PAYS = E == 2 ? AM && BM && TM < 128 : AM == BM && (AM || TM == 64);                  \
     auto kern = whole && PAYS ? gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, PAYS>                    \
                               : gemm_f32_kernel<TM, TN, RM, RN, RES, AM, BM, E, false>;                  \
     kern<<<grid, F32Tile<TM, TN, RM, RN>::NT, 0, s>>>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, vec);     \
@@ -833,7 +835,11 @@ extern "C" int otb_gemm_f32(const float* A, const float* B, float* C, const floa
     // tiles: 127 and 154). An MN-major B takes fewer registers and fits three as it is, but for the accumulating epilogue.
     auto cost = [&](long r) { return r * ((tiles(64) + r * sms - 1) / (r * sms)); };
     if ((!b_mn || epi == 2) && cost(3) < cost(2)) return launch_gemm_f32<64, 64, 4, 4, 3>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
-    return launch_gemm_f32<64, 64, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
+    // With predicated loads a store of two MN-major operands has registers for two tiles per SM only, which pays where that many make
+    // clearly fewer turns (branches and three, predicated and two, us: 456 tiles 37.9 and 35.1, 588 114 and 92; but 384 tiles 95 and
+    // 128, 704 50.0 and 51.3, 896 60.5 and 62.2, 1152 67.5 and 68.1).
+    const bool predicate = !a_mn || !b_mn || epi == 2 || 4 * cost(2) <= 3 * cost(3);
+    return launch_gemm_f32<64, 64, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s, predicate);
   }
   return launch_gemm_f32<32, 32, 4, 4>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, vec, s);
 }

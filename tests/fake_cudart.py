@@ -18,11 +18,13 @@ static int device, last;
 static struct { const void* f; int dev, bytes; } asked[256];
 static int n_asked;
 static int fake_launches, fake_early;
+static const void* fake_f;
 int fake_refuse_next;
 static int code[2], skip[2], times[2];  /* launches that are refused: [0] ordinary, [1] early */
 void fake_set_device(int d) { device = d; }
 int fake_asked(void) { return n_asked; }
 int fake_launched(void) { return fake_launches; }
+const void* fake_last(void) { return fake_f; }
 int fake_launched_early(void) { return fake_early; }
 void fake_refuse(void) { fake_refuse_next = 1; }
 void fake_refuse_launch(int early, int after, int n, int rc) { code[early] = rc; skip[early] = after; times[early] = n; }
@@ -45,6 +47,7 @@ static int launch(int early, const void* f, dim3_ g, size_t smem) {
     if (asked[i].f == f && asked[i].dev == device && asked[i].bytes > most) most = asked[i].bytes;
   if (smem > (size_t)most || !g.x || !g.y || !g.z) return last = 1;
   ++fake_launches;
+  fake_f = f;
   return 0;
 }
 int cudaLaunchKernel(const void* f, dim3_ g, dim3_ b, void** args, size_t smem, void* stream) { return launch(0, f, g, smem); }
