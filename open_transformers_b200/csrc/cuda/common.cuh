@@ -70,16 +70,19 @@ inline int otb_allow_smem(int bytes) {
   return 0;
 }
 
-// Launches that may begin while the kernel before them in the stream still runs, behind a kernel that calls let_successor_begin();
-// behind any other, and in front of an ordinary launch, the order of the stream is the ordinary one.
-// Behind a predecessor: the kernel calls after_predecessor() before it touches any memory. What then overlaps is the launch, the
-// CTAs' start and their set-up (barriers, tensor memory), which a chain of kernels of 4 to 15 us pays one after the other otherwise.
-// A kernel lets its own successor begin as soon as all its CTAs are there, so the successor never takes a place that it needs.
-// The products are launched that way, and the attention forward where it is small; the memory-bound kernels only let a product
-// behind them begin. Launched early themselves they gain less than they cost, since CTAs that are placed before the SMs are
-// free pile up on some: us, every launch ordinary / as it is / every grid of up to 8 CTAs per SM early: block without gradients,
-// 768 wide, 16 tokens 45.0 / 41.1 / 40.4, 333 tokens 52.0 / 48.3 / 52.5, 2048 wide, 1111 tokens 146 / 142 / 152; feed-forward sublayer
-// forward and backward, 2048 wide, 128 tokens 128 / 123 / 132.
+// Launches that may begin before the kernel in front of them in the stream has ended: at its end without the pause of an
+// ordinary launch, or, where that kernel calls let_successor_begin(), as soon as all its CTAs are there. In front of an ordinary
+// launch the order of the stream is the ordinary one.
+// Behind a predecessor: the kernel waits for it before it touches any memory. What overlaps is the launch, the CTAs' start and
+// their set-up (barriers, tensor memory), which a chain of kernels of 4 to 15 us pays one after the other otherwise. The memory-bound
+// kernels and the products are launched that way, and the attention forward where it is small. Which of them lets its successor
+// begin is what decides: memory-bound kernels and the attention do where a product follows, whose CTAs take an SM each; a product does
+// not, since small CTAs that are placed while it runs pile up on the SMs that happen to have room (what it costs is a product behind a
+// product: 333 x 768 x 768 with residual back to back 6.9 ordinary, 6.4 so, 5.9 with the former letting go). us, every launch ordinary / so /
+// every small grid early and every kernel letting go at its start: block without gradients, 768 wide, 16 tokens 45.0 / 39.4 / 40.4, 333
+// tokens 52.0 / 47.5 / 52.6, 2048 wide, 128 tokens 78.2 / 72.8 / 79.3, 1111 tokens 146 / 142 / 152; feed-forward sublayer forward and
+// backward, 2048 wide, 128 tokens 128 / 125 / 132. With the memory-bound kernels launched in the ordinary way a block of 333 tokens takes
+// 48.1, and a micro-batch of the two-layer fp32 decoder 2065 instead of 2007.
 // A kernel that waits exists while what it reads is still being written. Its inputs, and what it both reads and writes, are
 // therefore not __restrict__ and not read by __ldg: either would tell the compiler that nothing changes them while the kernel
 // runs, and let it take a load past the wait, whose "memory" clobber covers only what others may write. Buffers that are only

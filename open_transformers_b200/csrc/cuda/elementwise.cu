@@ -28,9 +28,9 @@ namespace {
 // scaling, so all of its loads are in flight at once and x is read once. MAXC = max number of 8-wide column chunks per
 // lane (D <= 256 * MAXC).
 template <typename T, int MAXC>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
+__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* x, const T* w, T* __restrict__ y,
                                                          float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
-  let_successor_begin();
+  after_predecessor();
   const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -74,11 +74,12 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
     }
   }
 }
-// The same row of any width: x is read twice, the second time from the nearer caches.
-template <typename T>
-__global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
-                                        float* __restrict__ rstd_out, long rows, int D, float inv_d, float eps) {
-  let_successor_begin();
+// The same row of any width: x is read twice, the second time from the nearer caches, U groups of eight columns per lane and turn,
+// all loaded before any is stored (behind a store the next turn's loads would wait).
+template <typename T, int U>
+__global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const T* x, const T* w, T* __restrict__ y, float* __restrict__ rstd_out, long rows,
+                                                              int D, float inv_d, float eps) {
+  after_predecessor();
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -94,19 +95,34 @@ __global__ void rmsnorm_fwd_wide_kernel(const T* __restrict__ x, const T* __rest
   const float rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
   if (lane == 0) rstd_out[row] = rstd;
   T* yr = y + row * D;
-  for (int c = lane * 8; c < D; c += 256) {
-    float f[8], o[8];
-    Vec8<T>::load(xr + c, f);
-    if (w) {
-      float g[8];
-      Vec8<T>::load(w + c, g);
+  for (int c0 = lane * 8; c0 < D; c0 += 256 * U) {
+    Raw8<T> rx[U], rw[U];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(__fmul_rn(f[e], rstd), g[e]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(f[e], rstd);
+    for (int u = 0; u < U; ++u) {
+      const int c = c0 + u * 256;
+      if (c < D) {
+        rx[u].load(xr + c);
+        if (w) rw[u].load(w + c);
+      }
     }
-    Vec8<T>::store(yr + c, o);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = c0 + u * 256;
+      if (c < D) {
+        float f[8], o[8];
+        rx[u].unpack(f);
+        if (w) {
+          float g[8];
+          rw[u].unpack(g);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(__fmul_rn(f[e], rstd), g[e]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(f[e], rstd);
+        }
+        Vec8<T>::store(yr + c, o);
+      }
+    }
   }
 }
 
@@ -127,10 +143,10 @@ inline bool rmsnorm_in_registers(long rows, int D, bool bf16) {
 // MAXC = max number of 8-wide column chunks per lane (D <= 256 * MAXC).
 constexpr int NORM_SLAB = 8;
 template <typename T, int MAXC>
-__global__ void __launch_bounds__(NORM_SLAB * 32) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                                                                    const float* __restrict__ rstd_in, T* __restrict__ dx,
+__global__ void __launch_bounds__(NORM_SLAB * 32) rmsnorm_bwd_kernel(const T* dy, const T* x, const T* w,
+                                                                    const float* rstd_in, T* __restrict__ dx,
                                                                     float* __restrict__ dgamma_partial, long rows, int D, float inv_d) {
-  let_successor_begin();
+  wait_for_predecessor();
   extern __shared__ float prod[];  // [NORM_SLAB][MAXC * 256] when dgamma is wanted
   const long slab = blockIdx.x;
   const int lane = threadIdx.x & 31, wrow = threadIdx.x >> 5;
@@ -214,7 +230,8 @@ __global__ void __launch_bounds__(NORM_SLAB * 32) rmsnorm_bwd_kernel(const T* __
 // same kernel is then applied to the 64-strided group roots (levels 64..2048), and so on: identical association,
 // log-depth instead of a serial chain. Logical row j lives at v[j * row_stride * D]. A missing partner leaves the
 // value untouched (never "+ 0.0", which would turn -0.0 into +0.0).
-__global__ void __launch_bounds__(256) pair_tree_cols_stage_kernel(float* __restrict__ v, long n, long row_stride, int D) {
+__global__ void __launch_bounds__(256) pair_tree_cols_stage_kernel(float* v, long n, long row_stride, int D) {
+  wait_for_predecessor();
   __shared__ float sm[64][33];
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;  // 32 columns x 8 row-threads
   const int col = blockIdx.x * 32 + c;
@@ -235,7 +252,7 @@ inline int pair_tree_cols_launch(float* v, long n, int D, cudaStream_t s) {
   while (n > 1) {
     const long groups = (n + 63) / 64;
     dim3 grid((D + 31) / 32, (unsigned)groups);
-    if (const int rc = otb_launch(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D)) return rc;
+    if (const int rc = otb_launch_early(pair_tree_cols_stage_kernel, grid, 256, 0, s, v, n, stride, D)) return rc;
     n = groups;
     stride *= 64;
   }
@@ -254,8 +271,9 @@ __device__ __forceinline__ float half_butterfly(float v) {
   return v;
 }
 template <typename T>
-__global__ void __launch_bounds__(256) head_rmsnorm_fwd_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, T* __restrict__ y, long ldy,
+__global__ void __launch_bounds__(256) head_rmsnorm_fwd_kernel(const T* x, long ldx, const T* w, T* __restrict__ y, long ldy,
                                                               float* __restrict__ rstd_out, long rows, int heads, int D, float inv_d, float eps) {
+  wait_for_predecessor();
   const long row = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
   const int c = (threadIdx.x & 15) * 8;
   const bool on = row < rows && c < D;
@@ -284,10 +302,10 @@ __global__ void __launch_bounds__(256) head_rmsnorm_fwd_kernel(const T* __restri
 }
 // dx and the dgamma partials of NORM_SLAB-row slabs (rows = (token, head) pairs); two slabs per CTA.
 template <typename T>
-__global__ void __launch_bounds__(256) head_rmsnorm_bwd_kernel(const T* __restrict__ dy, long lddy, const T* __restrict__ x, long ldx, const T* __restrict__ w,
-                                                              const float* __restrict__ rstd_in, T* __restrict__ dx, long lddx,
+__global__ void __launch_bounds__(256) head_rmsnorm_bwd_kernel(const T* dy, long lddy, const T* x, long ldx, const T* w,
+                                                              const float* rstd_in, T* __restrict__ dx, long lddx,
                                                               float* __restrict__ dgamma_partial, long rows, int heads, int D, float inv_d) {
-  let_successor_begin();
+  wait_for_predecessor();
   __shared__ float prod[16][128];
   const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
   const long row = (long)blockIdx.x * 16 + r;
@@ -388,11 +406,11 @@ __device__ __forceinline__ bool rope_place(long rows, int heads, long& row, int&
 __device__ __forceinline__ int rope_pos(long row, int seq_len) { return row >> 31 ? (int)(row % seq_len) : (int)((unsigned)row % (unsigned)seq_len); }
 
 template <typename T, bool VEC, int NH>
-__global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restrict__ in, long ld_in, T* __restrict__ out, long ld_out,
-                                       float* __restrict__ rstd_out, const float* __restrict__ cosb,
-                                       const float* __restrict__ sinb, long rows, int heads, int D, int seq_len,
+__global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* in, long ld_in, T* __restrict__ out, long ld_out,
+                                       float* __restrict__ rstd_out, const float* cosb,
+                                       const float* sinb, long rows, int heads, int D, int seq_len,
                                        int do_norm, float inv_d, float eps) {
-  let_successor_begin();
+  after_predecessor();
   long row;
   int head0;
   if (!rope_place<NH>(rows, heads, row, head0)) return;
@@ -440,11 +458,11 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* __restric
 }
 
 template <typename T, bool VEC, int NH>
-__global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* __restrict__ dout, long ld_dout, const T* __restrict__ in, long ld_in,
-                                       const float* __restrict__ rstd_in, T* __restrict__ din, long ld_din,
-                                       const float* __restrict__ cosb, const float* __restrict__ sinb, long rows,
+__global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(const T* dout, long ld_dout, const T* in, long ld_in,
+                                       const float* rstd_in, T* __restrict__ din, long ld_din,
+                                       const float* cosb, const float* sinb, long rows,
                                        int heads, int D, int seq_len, int do_norm, float inv_d) {
-  let_successor_begin();
+  after_predecessor();
   long row;
   int head0;
   if (!rope_place<NH>(rows, heads, row, head0)) return;
@@ -540,8 +558,8 @@ __device__ __forceinline__ void swiglu8_bwd(const Raw8<T>& rg, const Raw8<T>& ru
 }
 // One thread per group of eight, wherever its row is.
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* __restrict__ gu, T* __restrict__ h, long rows, int F) {
-  let_successor_begin();
+__global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* gu, T* __restrict__ h, long rows, int F) {
+  after_predecessor();
   const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (idx >= rows * F) return;
   const long row = idx / F;
@@ -552,8 +570,8 @@ __global__ void __launch_bounds__(256) swiglu_fwd_flat_kernel(const T* __restric
   swiglu8(g, u, h + idx);
 }
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_bwd_flat_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, long rows, int F) {
-  let_successor_begin();
+__global__ void __launch_bounds__(256) swiglu_bwd_flat_kernel(const T* gu, const T* dh, T* __restrict__ dgu, long rows, int F) {
+  after_predecessor();
   const long idx = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (idx >= rows * F) return;
   const long row = idx / F, at = row * 2 * F + (idx - row * F);
@@ -572,8 +590,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_flat_kernel(const T* __restric
 constexpr int SWIGLU_MAX_THREADS = 384;
 inline bool swiglu_per_row(long rows, int F) { return F >= 1024 && rows >= 2048 && rows <= 0x7fffffffL; }
 template <typename T>
-__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ h, int F) {
-  let_successor_begin();
+__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T* gu, T* __restrict__ h, int F) {
+  after_predecessor();
   const T* gr = gu + (long)blockIdx.x * 2 * F;
   T* hr = h + (long)blockIdx.x * F;
   for (int c0 = threadIdx.x * 8; c0 < F; c0 += blockDim.x * 16) {
@@ -595,8 +613,8 @@ __global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_fwd_kernel(const T*
 }
 // d_gate_up [rows, 2F] from dh [rows, F]
 template <typename T>
-__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dh, T* __restrict__ dgu, int F) {
-  let_successor_begin();
+__global__ void __launch_bounds__(SWIGLU_MAX_THREADS) swiglu_bwd_kernel(const T* gu, const T* dh, T* __restrict__ dgu, int F) {
+  after_predecessor();
   const T* gr = gu + (long)blockIdx.x * 2 * F;
   const T* dr = dh + (long)blockIdx.x * F;
   T* or_ = dgu + (long)blockIdx.x * 2 * F;
@@ -689,10 +707,10 @@ __device__ __forceinline__ void ce_grad(T* __restrict__ xr, int V, tc05::f2 l2, 
   }
 }
 template <typename T, int CE_UNROLL, bool TEST>
-__global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* __restrict__ logits, const long* __restrict__ labels,
+__global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* logits, const long* labels,
                                                               float* __restrict__ ce_out, float* __restrict__ lse_out,
                                                               long rows, int V, float two_z, float scale, int write_grad) {
-  let_successor_begin();
+  after_predecessor();
   using namespace tc05;
   __shared__ float sh[32];
   const long row = blockIdx.x;
@@ -755,8 +773,9 @@ inline int ce_form(long rows, int V, bool bf16) {
 
 // sum (or sum of squares) of n floats: element i -> thread i % 1024, ascending fold, block_tree_sum.
 // mode 0: sum x, 1: sum x*x (fma chain). out[0] = result * post_scale.
-__global__ void __launch_bounds__(1024) det_sum_kernel(const float* __restrict__ x, long n, int mode, float post_scale,
+__global__ void __launch_bounds__(1024) det_sum_kernel(const float* x, long n, int mode, float post_scale,
                                                         float* __restrict__ out) {
+  wait_for_predecessor();
   __shared__ float sh[32];
   float acc = 0.0f;
   for (long i = threadIdx.x; i < n; i += 1024) {
@@ -832,10 +851,12 @@ inline bool four_aligned(const void* p, long ld, int bf16) { return ld % 4 == 0 
 extern "C" int otb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long rows, int D, float inv_d,
                                float eps, int dtype, void* stream) {
   if (D % 8) return -2;
-#define RF(KERN) return otb_launch(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
+#define RF(KERN) return otb_launch_early(KERN, blocks_for(rows, 8), 256, 0, S(stream), (const T*)x, (const T*)w, (T*)y, rstd, rows, D, inv_d, eps)
 #define RFC(MAXC) RF((rmsnorm_fwd_kernel<T, MAXC>))
   if (!rmsnorm_in_registers(rows, D, dtype)) {
-    DISPATCH_T(dtype, RF(rmsnorm_fwd_wide_kernel<T>);)
+    // four groups per turn take more registers, which large tensors need for rows in flight (us, two and four: 64 x 2048 3.3 and 3.2, 4096 x
+    // 2048 7.0 and 5.5, 8192 x 2048 9.6 and 9.2, 8192 x 5120 40.2 and 31.4; 16384 x 2048 23.1 and 24.6, 16384 x 1024 8.9 and 9.4)
+    if (rows <= 64L * otb_sm_count()) { DISPATCH_T(dtype, RF((rmsnorm_fwd_wide_kernel<T, 4>));) } else { DISPATCH_T(dtype, RF((rmsnorm_fwd_wide_kernel<T, 2>));) }
   } else if (dtype) {
     using T = __nv_bfloat16;
     if (D <= 256) RFC(1); else if (D <= 768) RFC(3); else RFC(16);
@@ -854,7 +875,7 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
 #define RB(MAXC)                                                                                                          \
   DISPATCH_T(dtype, {                                                                                                     \
     if (const int rc = otb_allow_smem<rmsnorm_bwd_kernel<T, MAXC>>(NORM_SLAB * 256 * MAXC * 4)) return rc;                   \
-    launched = otb_launch(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
+    launched = otb_launch_early(rmsnorm_bwd_kernel<T, MAXC>, (unsigned)slabs, NORM_SLAB * 32, dgamma_partial ? NORM_SLAB * 256 * MAXC * 4 : 0, S(stream), (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, \
                                                                                      dgamma_partial, rows, D, inv_d);     \
   })
   if (D <= 256) { RB(1) } else if (D <= 1024) { RB(4) } else if (D <= 2048) { RB(8) } else { RB(16) }
@@ -866,14 +887,14 @@ extern "C" int otb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
 extern "C" int otb_head_rmsnorm_fwd(const void* x, long ldx, const void* w, void* y, long ldy, float* rstd, long rows, int heads, int D,
                                     float inv_d, float eps, int dtype, void* stream) {
   if (D % 8 || D > 128 || ldx % 8 || ldy % 8) return -2;
-  DISPATCH_T(dtype, return otb_launch(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
+  DISPATCH_T(dtype, return otb_launch_early(head_rmsnorm_fwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)x, ldx, (const T*)w, (T*)y, ldy, rstd, rows, heads,
                                                                                           D, inv_d, eps);)
 }
 extern "C" int otb_head_rmsnorm_bwd(const void* dy, long lddy, const void* x, long ldx, const void* w, const float* rstd, void* dx, long lddx,
                                     float* dgamma_partial, long rows, int heads, int D, float inv_d, int dtype, void* stream) {
   if (D % 8 || D > 128 || lddy % 8 || ldx % 8 || lddx % 8) return -2;
   int launched = 0;
-  DISPATCH_T(dtype, launched = otb_launch(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
+  DISPATCH_T(dtype, launched = otb_launch_early(head_rmsnorm_bwd_kernel<T>, blocks_for(rows, 16), 256, 0, S(stream), (const T*)dy, lddy, (const T*)x, ldx, (const T*)w, rstd,
                                                                                           (T*)dx, lddx, dgamma_partial, rows, heads, D, inv_d);)
   if (launched || !dgamma_partial) return launched;
   return pair_tree_cols_launch(dgamma_partial, (rows + NORM_SLAB - 1) / NORM_SLAB, D, S(stream));
@@ -889,7 +910,7 @@ extern "C" int otb_qknorm_rope_fwd(const void* in, long ld_in, void* out, long l
                                    float inv_d, float eps, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(in, ld_in, dtype) && four_aligned(out, ld_out, dtype);
-#define QF(V, NH) DISPATCH_T(dtype, return otb_launch(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QF(V, NH) DISPATCH_T(dtype, return otb_launch_early(qknorm_rope_fwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)in, ld_in, (T*)out, ld_out, rstd, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d, eps);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QF(true, 1) } else { QF(false, 1) }
@@ -903,7 +924,7 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
                                    int D, int seq_len, int do_norm, float inv_d, int dtype, void* stream) {
   if (D % 4 || D > 128) return -2;
   const bool vec = four_aligned(dout, ld_dout, dtype) && four_aligned(in, ld_in, dtype) && four_aligned(din, ld_din, dtype);
-#define QB(V, NH) DISPATCH_T(dtype, return otb_launch(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
+#define QB(V, NH) DISPATCH_T(dtype, return otb_launch_early(qknorm_rope_bwd_kernel<T, V, NH>, blocks_for(rows * ((heads + NH - 1) / NH), 8), 256, 0, S(stream),  \
                         (const T*)dout, ld_dout, (const T*)in, ld_in, rstd, (T*)din, ld_din, cosb, sinb, rows, heads, D, seq_len, do_norm, inv_d);)
   if (rope_one_head(rows, heads)) {
     if (vec) { QB(true, 1) } else { QB(false, 1) }
@@ -915,30 +936,30 @@ extern "C" int otb_qknorm_rope_bwd(const void* dout, long ld_dout, const void* i
 extern "C" int otb_swiglu_fwd(const void* gu, void* h, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, return otb_launch(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
+    DISPATCH_T(dtype, return otb_launch_early(swiglu_fwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (T*)h, F);)
   } else {
-    DISPATCH_T(dtype, return otb_launch(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
+    DISPATCH_T(dtype, return otb_launch_early(swiglu_fwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (T*)h, rows, F);)
   }
 }
 extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long rows, int F, int dtype, void* stream) {
   if (F % 8) return -2;
   if (swiglu_per_row(rows, F)) {
-    DISPATCH_T(dtype, return otb_launch(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
+    DISPATCH_T(dtype, return otb_launch_early(swiglu_bwd_kernel<T>, (unsigned)rows, swiglu_threads(F), 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, F);)
   } else {
-    DISPATCH_T(dtype, return otb_launch(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
+    DISPATCH_T(dtype, return otb_launch_early(swiglu_bwd_flat_kernel<T>, blocks_for(rows * F / 8, 256), 256, 0, S(stream), (const T*)gu, (const T*)dh, (T*)dgu, rows, F);)
   }
 }
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
 #define CE(U, TEST) \
-  DISPATCH_T(dtype, return otb_launch(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+  DISPATCH_T(dtype, return otb_launch_early(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
   const int form = ce_form(rows, V, dtype);
   if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
 }
 extern "C" int otb_det_sum(const float* x, long n, int mode, float post_scale, float* out, void* stream) {
-  return otb_launch(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
+  return otb_launch_early(det_sum_kernel, 1, 1024, 0, S(stream), x, n, mode, post_scale, out);
 }
 extern "C" int otb_embedding_fwd(const long* ids, const void* table, void* out, long rows, int D, int dtype,
                                  void* stream) {

@@ -269,7 +269,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (TP == 0 && !PAIR) after_predecessor();
+  if constexpr (TP == 0 && !PAIR) wait_for_predecessor();
 
   // tile -> (m, n): groups of `group_m` row-tiles sweep all column tiles, so that the A rows of
   // a group and the B columns being swept stay L2-resident across the CTAs working on them.

@@ -1,6 +1,6 @@
 """What an entry point returns when a launch is refused, against a fake runtime: an early launch that is refused is tried in the
 ordinary way; an error is returned by the call whose launch it was, once, and nothing that depends on that launch follows it. And
-which launches are early: products, the attention forward on half the chip, dQ beside dK/dV."""
+which launches are early: products, memory-bound kernels, the attention forward on half the chip, dQ beside dK/dV."""
 import pytest
 from fake_cudart import run_with_fake
 
@@ -49,7 +49,7 @@ single = {
 # a single launch: refused early only, then both ways; the next call is not charged with it
 ONE = HEAD + r"""
 for name, call in single.items():
-    early = name in ("gemm", "attn_fwd", "attn_fwd_64")
+    early = name != "embedding_fwd"
     fake.fake_reset()
     assert call() == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (1, early), name
     fake.fake_reset()
@@ -97,6 +97,7 @@ for call, rows in ((rmsnorm_bwd, 64), (rmsnorm_bwd, 8 * 1200), (head_rmsnorm_bwd
     fake.fake_reset()
     assert call(rows) == 0
     launches = fake.fake_launched()
+    assert fake.fake_launched_early() == launches
     assert launches == (2 if rows == 64 else 3)
     for nth in range(launches):
         fake.fake_reset()
