@@ -13,9 +13,10 @@ def _same(dev, host, what):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-# register widths, and one past the last; bf16 keeps rows up to 768, and 2056 to 4096 of 12288 and more, in registers
+# register widths, and one past the last; bf16 keeps rows up to 768, and 2056 to 4096 of 12288 and more, in registers; where rows
+# are read twice, four groups per turn up to 9472 rows (148 SMs) and two above
 @pytest.mark.parametrize("rows,D", [(1, 8), (9, 248), (7, 1032), (3, 4096), (5, 4104), (9, 256), (9, 264), (9, 768), (9, 776), (9, 2048), (12288, 2048),
-                                    (12288, 2056), (12287, 2056), (12289, 4096)])
+                                    (12288, 2056), (12287, 2056), (12289, 4096), (9472, 1032), (9473, 1032), (9473, 4104)])
 def test_rmsnorm_forward_widths(dtype, rows, D):
     g = torch.Generator().manual_seed(D)
     x, w = torch.randn(rows, D, generator=g).to(dtype), torch.randn(D, generator=g).to(dtype)

@@ -1,8 +1,11 @@
 """Fast forms of kernels at the edges of what chooses them, bit for bit against the CPU twin."""
+import ctypes
+
 import pytest
 import torch
 
 from open_transformers_b200.ops import functional as K
+from open_transformers_b200.ops.native import cuda_lib
 
 pytestmark = pytest.mark.gpu
 
@@ -41,13 +44,34 @@ def test_quantiser_near_ties(dtype, qmax, top):
         assert torch.equal(q.cpu()[keep], want_q[keep])
 
 
+# A NaN becomes -qmax wherever it lies, in a whole group of eight or in the ragged end, with a step in or out of the range of the
+# fast division, and leaves its neighbours alone.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("top", [3.0, 2.0**-90, 2.0**120])
+def test_quantiser_of_nan(dtype, top):
+    x = (torch.linspace(-1, 1, 8 * 300 + 5) * top).to(dtype)
+    at = torch.tensor([0, 3, 7, 8, 8 * 150 + 4, 8 * 300 - 1, 8 * 300, 8 * 300 + 4])
+    x[at] = float("nan")
+    q, s = K.quant_act(x.cuda(), 127)
+    want_q, want_s = K.quant_act(x, 127)
+    assert torch.equal(s.cpu(), want_s) and (q.cpu()[at] == -127).all()
+    rest = ~x.isnan()
+    assert torch.equal(q.cpu()[rest], want_q[rest])
+
+
 # 64-wide tiles where all of them fit the chip at once: one tile, ragged columns and rows, a K of one step and of many, the
-# first size past a wave of them
-@pytest.mark.parametrize("M,N,K_", [(1, 8, 8), (130, 200, 64), (129, 72, 520), (37 * 128, 256, 72), (37 * 128 + 1, 256, 72)])
+# last size of one wave of them (rows of four tiles each, by the device's SM count) and the first past it; more than 32 columns of
+# them on 128 KB of A and on less
+@pytest.mark.parametrize("M,N,K_,slim", [(1, 8, 8, True), (130, 200, 64, True), (129, 72, 520, True), ("wave", 256, 72, True), ("wave + 1", 256, 72, False),
+                                            (32, 2056, 2048, True), (24, 2056, 2048, False)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
-def test_slim_gemm_tiles(M, N, K_, a_mn, b_mn):
+def test_slim_gemm_tiles(M, N, K_, slim, a_mn, b_mn):
+    if isinstance(M, str):
+        M = torch.cuda.get_device_properties(0).multi_processor_count // 4 * 128 + (M == "wave + 1")
     g = torch.Generator().manual_seed(M + K_)
     Mr = (M + 7) // 8 * 8 if a_mn else M  # (a row pitch is a multiple of 16 bytes)
+    tile = cuda_lib().otb_gemm_tile(*(ctypes.c_int(v) for v in (Mr, N, K_, a_mn or b_mn, 0, 0)))
+    assert (tile == 64) == slim
     a = torch.randn((K_, Mr) if a_mn else (M, K_), generator=g).bfloat16()
     b = torch.randn((K_, N) if b_mn else (N, K_), generator=g).bfloat16()
     for epi in (K.EPI_STORE, K.EPI_STORE_F32, K.EPI_ACC_F32, K.EPI_RESIDUAL):
