@@ -1,8 +1,8 @@
 // One decoder block without gradients as one host call: the nine launches of norm -> QKV product -> QK-norm / RoPE ->
 // attention -> output product (+ residual) -> norm -> gate/up product -> SwiGLU -> down product (+ residual), each the kernel
 // that the block's modules launch one by one, so the results are the same bits. What bounds the scoring of a short prompt is
-// the host: module calls and autograd functions, about 250 us of Python a block for 90 us of kernels (333 tokens through the
-// six-layer 100M model: 1691 -> 594 us).
+// the host: module calls and autograd functions, about 250 us of Python a block for 50 us of kernels (333 tokens through the
+// six-layer 100M model: 1584 -> 542 us, the launches' own changes included).
 #include "common.cuh"
 #include "entries.cuh"
 
