@@ -5,14 +5,13 @@
 //
 //   attn_fwd2     CTA = (batch, query head, TWO 128-row query tiles); one thread per row; S = Q K^T (TMEM) -> online
 //                 softmax -> P written back over S as bf16 (the A operand of P V) -> O accumulates in TMEM.
-//   attn_bwd_kv2  CTA = (batch, KV head, 128 keys); scores formed transposed (S^T, dP^T: lanes are keys), P^T / dS^T
-//                 written back in place, dV += P^T dO and dK += dS^T Q with the A operand in TMEM; 64-query steps over
-//                 the heads of the group and the query blocks that see these keys, both ascending.
+//   attn_bwd_kv3  CTA = (batch, KV head, 128 keys); scores formed transposed (S^T, dP^T: lanes are keys), P^T / dS^T
+//                 written back in place, dV += P^T dO and dK += dS^T Q with the A operand in TMEM; 128-query steps over
+//                 the heads of the group and the query blocks that see these keys, both ascending; any T.
 //   attn_bwd_q2   CTA = (batch, query head, two query tiles); two threads per row; dS written back over S;
 //                 dQ += dS K with dS in TMEM; 64-key steps ascending.
 //   attn_fwd      (one tile per CTA, four threads per row, P through shared memory, O in registers) serves the int8 P V
-//                 variant; attn_bwd_kv (one score buffer, P / dS through shared memory) serves sequence lengths that
-//                 are not a multiple of 64.
+//                 variant.
 //
 // No atomics, no split accumulation: every output element has one owner CTA and a fixed
 // summation order, so results are identical for any grid, stream or GPU count. The window rule
@@ -78,8 +77,7 @@ struct BarsX : Bars {
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
-// The bf16 forward, dQ and transposed dK/dV kernels are persistent, one CTA per SM (the dK/dV kernel for lengths that are no
-// multiple of 64 and the int8 P V forward are not): every role walks the same list of work items, barrier phases and ring
+// The bf16 forward, dQ and dK/dV kernels are persistent, one CTA per SM (the int8 P V forward is not): every role walks the same list of work items, barrier phases and ring
 // positions running on, so the loads and first products of an item are under way while the previous one's results are read
 // out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about 8 us, were
 // exposed: a quarter of an item's time with a 512-key window. 4 x 4096 tokens, 16 heads x 128, forward and backward: 1790 ->
@@ -746,195 +744,6 @@ __device__ __forceinline__ void bwd_probs(const uint32_t (&vs)[N], const uint32_
   }
 }
 
-// -------------------------------------------------------- backward: dK and dV
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV,
-                   const __grid_constant__ CUtensorMap tmDO, const float* __restrict__ lse,
-                   const float* __restrict__ delta, __nv_bfloat16* __restrict__ dK, long lddk,
-                   __nv_bfloat16* __restrict__ dV, long lddv, int T, int H, int Hkv, int window, float scale,
-                   float c_log2, uint32_t* __restrict__ status) {
-  constexpr int TILE = BQ * D * 2;
-  constexpr int ST = 2;
-  let_successor_begin();
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align1024(smem_raw);
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + TILE;
-  uint8_t* sPdS = sV + TILE;
-  uint8_t* sQ = sPdS + BQ * BKV * 2;  // [ST]
-  uint8_t* sDO = sQ + ST * TILE;      // [ST]
-  Bars* bars = reinterpret_cast<Bars*>(sDO + ST * TILE);
-  uint64_t* kv_full = &bars->b[0];
-  uint64_t* qdo_full = &bars->b[1];   // [ST]
-  uint64_t* qdo_empty = &bars->b[3];  // [ST]
-  uint64_t* sdp_full = &bars->b[5];
-  uint64_t* sdp_empty = &bars->b[6];
-  uint64_t* p_ready = &bars->b[7];
-  uint64_t* dv_done = &bars->b[8];
-  uint64_t* ds_ready = &bars->b[9];
-  uint64_t* dk_done = &bars->b[10];
-  volatile uint32_t* abort_flag = &bars->abort_flag;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = (T + BQ - 1) / BQ;
-  const int kb = (int)((blockIdx.x + g_attn_rotation) % gridDim.x), g = blockIdx.y, b = blockIdx.z;
-  const int G = H / Hkv;
-  const int k0 = kb * BKV;
-  int qlast = nq - 1;
-  if (window > 0) qlast = min(qlast, (k0 + BKV - 1 + window - 1) / BQ);
-  const int nqi = qlast - kb + 1;  // query blocks per head
-  const int n = G * nqi;
-
-  if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int s = 0; s < ST; ++s) { mbar_init(&qdo_full[s], 1); mbar_init(&qdo_empty[s], 1); }
-    mbar_init(sdp_full, 1); mbar_init(sdp_empty, SOFTMAX_WARPS); mbar_init(p_ready, SOFTMAX_WARPS); mbar_init(dv_done, 1);
-    mbar_init(ds_ready, SOFTMAX_WARPS); mbar_init(dk_done, 1);
-    bars->abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) { tmem_alloc(&bars->tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = bars->tmem_slot;
-  const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
-
-  if (warp == 0) {
-    if (elect_one()) {
-      mbar_expect_tx(kv_full, 2 * TILE);
-      load_tile<D>(sK, &tmQK, kv_full, (H + g) * D, k0, b);
-      load_tile<D>(sV, &tmV, kv_full, (H + Hkv + g) * D, k0, b);
-      for (int i = 0; i < n; ++i) {
-        const int st = i % ST;
-        const int h = g * G + i / nqi;
-        const int q0 = (kb + i % nqi) * BQ;
-        if (!mbar_wait(&qdo_empty[st], ((i / ST) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(&qdo_full[st], 2 * TILE);
-        load_tile<D>(sQ + st * TILE, &tmQK, &qdo_full[st], h * D, q0, b);
-        load_tile<D>(sDO + st * TILE, &tmDO, &qdo_full[st], h * D, q0, b);
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idS = make_idesc(128, BKV, 0, 0);   // S = Q K^T, dP = dO V^T
-      constexpr uint32_t idG = make_idesc(128, D, 1, 1);     // dV = P^T dO, dK = dS^T Q
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sPdS);
-      bool ok = mbar_wait(kv_full, 0, abort_flag);
-      auto issue_sdp = [&](int i) {
-        const int st = i % ST;
-        if (!mbar_wait(&qdo_full[st], (i / ST) & 1, abort_flag)) return false;
-        if (!mbar_wait(sdp_empty, (i & 1) ^ 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t aQ = smem_u32(sQ + st * TILE), aDO = smem_u32(sDO + st * TILE);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tS, desc_k(aQ, kk), desc_k(aK, kk), idS, kk != 0);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tDP, desc_k(aDO, kk), desc_k(aV, kk), idS, kk != 0);
-        mma_commit(sdp_full);
-        return true;
-      };
-      if (ok) ok = issue_sdp(0);
-      for (int i = 0; i < n && ok; ++i) {
-        const int st = i % ST;
-        const uint32_t aQ = smem_u32(sQ + st * TILE), aDO = smem_u32(sDO + st * TILE);
-        // S and dP of the next block run while the softmax warps work on this one (they released the buffers
-        // as soon as the values were in registers)
-        if (i + 1 < n) { if (!issue_sdp(i + 1)) { ok = false; break; } }
-        if (!mbar_wait(p_ready, i & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk) mma_f16_ss(tDV, desc_mn(aP, kk), desc_mn(aDO, kk), idG, (i | kk) != 0);
-        mma_commit(dv_done);
-        if (!mbar_wait(ds_ready, i & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk) mma_f16_ss(tDK, desc_mn(aP, kk), desc_mn(aQ, kk), idG, (i | kk) != 0);
-        mma_commit(dk_done);
-        mma_commit(&qdo_empty[st]);
-      }
-    }
-  } else {
-    constexpr int DH = D / NSPLIT;
-    constexpr int CW = DH >= 32 ? 32 : 16;
-    const int qd = warp & 3;
-    const int part = (warp - 2) >> 2;
-    const int r = qd * 32 + lane;
-    const uint32_t lane_off = uint32_t(qd * 32) << 16;
-    bool ok = true;
-    for (int i = 0; i < n && ok; ++i) {
-      const int h = g * G + i / nqi;
-      const int qb = kb + i % nqi;
-      const int qi = qb * BQ + r;
-      const bool row_ok = qi < T;
-      const bool need_mask = (qb == kb) || (window > 0 && k0 < qb * BQ + BQ - window) || (qb * BQ + BQ > T);
-      const float lse_r = row_ok ? lse[((long)b * H + h) * T + qi] : 0.0f;
-      const float dl_r = row_ok ? delta[((long)b * H + h) * T + qi] : 0.0f;
-      if (!mbar_wait(sdp_full, i & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t dsr[KPT / 2], pk[KPT / 2];
-      {
-        uint32_t vs[KPT], vd[KPT];
-        tmem_ld_32x32b_x32(tS + lane_off + part * KPT, vs);
-        tmem_ld_32x32b_x32(tDP + lane_off + part * KPT, vd);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sdp_empty);  // S and dP are in registers: the next block's products may overwrite them
-        if (need_mask) bwd_probs<true, true>(vs, vd, c_log2, lse_r, dl_r, scale, row_ok, k0 + part * KPT, qi, window, pk, dsr);
-        else bwd_probs<false, true>(vs, vd, c_log2, lse_r, dl_r, scale, row_ok, k0 + part * KPT, qi, window, pk, dsr);
-      }
-      // the shared P / dS buffer is free once the previous block's dK product has read it
-      if (i > 0) { if (!mbar_wait(dk_done, (i - 1) & 1, abort_flag)) { ok = false; break; } }
-      uint8_t* base = sPdS + (part >> 1) * 16384;
-#pragma unroll
-      for (int w = 0; w < 4; ++w)
-        *reinterpret_cast<uint4*>(base + swz(r, (part & 1) * 4 + w)) = make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
-      fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_ready);
-      if (!mbar_wait(dv_done, i & 1, abort_flag)) { ok = false; break; }
-#pragma unroll
-      for (int w = 0; w < 4; ++w)
-        *reinterpret_cast<uint4*>(base + swz(r, (part & 1) * 4 + w)) = make_uint4(dsr[4 * w], dsr[4 * w + 1], dsr[4 * w + 2], dsr[4 * w + 3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
-    }
-    if (ok && mbar_wait(dk_done, (n - 1) & 1, abort_flag)) {
-      tc_fence_after();
-      const int kj = k0 + r;  // TMEM lane == key row
-      const bool in_range = kj < T;
-      __nv_bfloat16* dkrow = dK + ((long)b * T + kj) * lddk + (long)g * D + part * DH;
-      __nv_bfloat16* dvrow = dV + ((long)b * T + kj) * lddv + (long)g * D + part * DH;
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-#pragma unroll
-        for (int c = 0; c < DH / CW; ++c) {
-          uint32_t v[CW];
-          tmem_ld_cols<CW>((which ? tDK : tDV) + lane_off + part * DH + c * CW, v);
-          tmem_ld_wait();
-          if (in_range) {
-            uint4* dst = reinterpret_cast<uint4*>((which ? dkrow : dvrow) + c * CW);
-#pragma unroll
-            for (int w = 0; w < CW / 8; ++w)
-              dst[w] = make_uint4(pack_bf16(__uint_as_float(v[8 * w]), __uint_as_float(v[8 * w + 1])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 2]), __uint_as_float(v[8 * w + 3])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 4]), __uint_as_float(v[8 * w + 5])),
-                                  pack_bf16(__uint_as_float(v[8 * w + 6]), __uint_as_float(v[8 * w + 7])));
-          }
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (threadIdx.x == 0 && bars->abort_flag && status) atomicExch(status, 3u);
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
-}
-
 // ------------------------------------------------ backward: dQ, two query tiles per CTA
 // Same organisation as the forward: one CTA owns two adjacent 128-row query tiles, one thread per query row, and the
 // tensor core serves one tile while the other tile's threads do the element math (two threads per row, each with half
@@ -1176,96 +985,127 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
 }
 
 // ------------------------------------------- backward: dK and dV, transposed scores
-// One CTA owns 128 keys of one KV head and walks, head by head of the group and in ascending query order, the 64-row
-// query steps that see those keys. The products are formed TRANSPOSED, S^T = K Q^T and dP^T = V dO^T (128 keys x 64
+// One CTA owns 128 keys of one KV head and walks, head by head of the group and in ascending query order, the 128-row
+// query steps that see those keys. The products are formed TRANSPOSED, S^T = K Q^T and dP^T = V dO^T (128 keys x 128
 // queries), so a tensor-memory lane is a key: the threads of a key row write P^T and dS^T back over their own columns
 // as bf16 pairs and both accumulations, dV += P^T dO and dK += dS^T Q, take their A operand straight from tensor memory.
-// Two score buffers alternate, so the tensor core forms the next step's scores while the 16 element warps (four threads
-// per key row, 16 queries each, no value crosses threads) work on the current one. Per-query statistics (-lse, -delta)
-// arrive through a small bulk copy beside each Q / dO tile. dV and dK accumulate over (head, query) in 16-query
-// tensor-core steps in the same order as the one-buffer kernel above, so the bits are the same.
-// Tensor memory: dV 128 | dK 128 | buffer 0: S^T 64, dP^T 64 | buffer 1: S^T 64, dP^T 64. Needs T % 64 == 0.
-constexpr int KV2_ST = 4;
+// dV and dK accumulate over (head, query) in 16-query tensor-core steps, as the CPU twin does.
+// Steps are 128 queries wide because a product of two shared-memory operands reads all of A whatever its width (128 x 64 takes 60
+// clocks a k-step, 128 x 128 64). That leaves tensor memory for one S^T and one dP^T, and the overlap comes from the order: while
+// the sixteen element warps (four threads per key row, no value crosses threads) turn dP^T into dS^T, the tensor core runs dV and
+// the next S^T; while they make the next P^T, it runs dK and the next dP^T. Each 64-query half of P^T and dS^T is handed over by
+// itself; the probabilities stay in registers (fp32) from the one phase to the other.
+// A 128 x 128 step takes 3500 clocks: P^T 1800 (1250 of the multiply-add pipe), dS^T 750, 600 and 170 waiting for S^T and dP^T.
+// 4 x 4096 tokens, 16 x 128 heads: 538 -> 533 us against 64-query steps with two score buffers (products alone 2900 clocks there);
+// lengths that are no multiple of 64 had a kernel of their own: backward of 333 tokens, 12 x 64, 39.5 -> 25.1 us, 2 x 1000 55.3 -> 36.1.
+// Also measured: two groups of eight warps, one per 64-query buffer (537 us); P^T through shared memory, so that S^T is free early
+// (611: three products of four then take all of the shared-memory bandwidth).
+// Per-query statistics (-lse, -delta) are copied to shared memory by the loading warp, plain loads, so any T will do: rows past
+// the end have dO = 0 and -delta = 0 and add nothing.
+// Tensor memory: dV 128 | dK 128 | S^T 128 | dP^T 128.
+constexpr int KV_QST = 3, KV_DOST = 2;  // Q lives until its dK product, dO until its dV product
 
-struct BarsKV2 {
-  uint64_t kv_full, kv_empty, qdo_full[KV2_ST], qdo_empty[KV2_ST], sdp_full[2], pds_ready[2], acc_done;
+struct BarsKV3 {
+  uint64_t k_full, k_empty, v_full, v_empty, q_full[KV_QST], q_empty[KV_QST], do_full[KV_DOST], do_empty[KV_DOST], stat_full[2], s_full, dp_full,
+      p_ready[2], ds_ready[2], acc_full, acc_empty;
   uint32_t tmem_slot;
   uint32_t abort_flag;
 };
 
-template <bool MASK>
-__device__ __forceinline__ void bwd_probs_t(const uint32_t (&vs)[16], const uint32_t (&vd)[16], const float* __restrict__ nl,
-                                            const float* __restrict__ nd, float c_log2, float scale, int kj, int qbase, int window,
-                                            uint32_t (&pk)[8], uint32_t (&dsr)[8]) {
-  const f2 c2 = pack2(c_log2, c_log2), sc2 = pack2(scale, scale);
+// P^T of 16 queries of the thread's key (0 where hidden), kept as fp32 pairs and packed to bf16. One copy of the arithmetic for
+// pieces with and without hidden pairs: with a copy of each for all four pieces the kernel outgrew the instruction cache (85 K
+// misses an SM at 4 x 4096 tokens, 716 us instead of 533).
+__device__ __forceinline__ void probs_t(const uint32_t (&vs)[16], const float* nl, float c_log2, bool mixed, int kj, int qbase, int window, f2 (&p)[8],
+                                        uint32_t (&pk)[8]) {
+  const f2 c2 = pack2(c_log2, c_log2);
 #pragma unroll
   for (int e = 0; e < 16; e += 4) {
-    const float4 l4 = *reinterpret_cast<const float4*>(nl + e), d4 = *reinterpret_cast<const float4*>(nd + e);
+    const float4 l4 = *reinterpret_cast<const float4*>(nl + e);
+    p[e >> 1] = exp2_attn2(fma2(pack2(__uint_as_float(vs[e]), __uint_as_float(vs[e + 1])), c2, pack2(l4.x, l4.y)));
+    p[(e >> 1) + 1] = exp2_attn2(fma2(pack2(__uint_as_float(vs[e + 2]), __uint_as_float(vs[e + 3])), c2, pack2(l4.z, l4.w)));
+  }
+  if (mixed) {
+    const uint32_t reach = window > 0 ? (uint32_t)window : 0x7FFFFFFFu;  // the queries kj .. kj + reach - 1 see the key
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+      float p0, p1;
+      unpack2(p[e >> 1], p0, p1);
+      if ((uint32_t)(qbase + e - kj) >= reach) p0 = 0.0f;
+      if ((uint32_t)(qbase + e + 1 - kj) >= reach) p1 = 0.0f;
+      p[e >> 1] = pack2(p0, p1);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    float p0, p1;
+    unpack2(p[e], p0, p1);
+    pk[e] = pack_bf16(p0, p1);
+  }
+}
+// dS^T = (P (dP - delta)) scale of the same 16 queries
+__device__ __forceinline__ void dscores_t(const uint32_t (&vd)[16], const float* nd, const f2 (&p)[8], float scale, uint32_t (&pk)[8]) {
+  const f2 sc2 = pack2(scale, scale);
+#pragma unroll
+  for (int e = 0; e < 16; e += 4) {
+    const float4 d4 = *reinterpret_cast<const float4*>(nd + e);
 #pragma unroll
     for (int w = 0; w < 4; w += 2) {
-      const f2 nl2 = w ? pack2(l4.z, l4.w) : pack2(l4.x, l4.y), nd2 = w ? pack2(d4.z, d4.w) : pack2(d4.x, d4.y);
-      f2 p2 = exp2_attn2(fma2(pack2(__uint_as_float(vs[e + w]), __uint_as_float(vs[e + w + 1])), c2, nl2));
-      float p0, p1;
-      unpack2(p2, p0, p1);
-      if constexpr (MASK) {
-        if (key_hidden(kj, qbase + e + w, window)) p0 = 0.0f;
-        if (key_hidden(kj, qbase + e + w + 1, window)) p1 = 0.0f;
-        p2 = pack2(p0, p1);
-      }
-      const f2 d2 = mul2(mul2(p2, add2(pack2(__uint_as_float(vd[e + w]), __uint_as_float(vd[e + w + 1])), nd2)), sc2);
+      const f2 d2 = mul2(mul2(p[(e + w) >> 1], add2(pack2(__uint_as_float(vd[e + w]), __uint_as_float(vd[e + w + 1])), w ? pack2(d4.z, d4.w) : pack2(d4.x, d4.y))), sc2);
       float d0, d1;
       unpack2(d2, d0, d1);
-      pk[(e + w) >> 1] = pack_bf16(p0, p1);
-      dsr[(e + w) >> 1] = pack_bf16(d0, d1);
+      pk[(e + w) >> 1] = pack_bf16(d0, d1);
     }
   }
 }
 
 template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV,
-                    const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmDO64,
+attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                     const float* __restrict__ nlse, const float* __restrict__ ndelta, __nv_bfloat16* __restrict__ dK, long lddk,
                     __nv_bfloat16* __restrict__ dV, long lddv, int B, int T, int H, int Hkv, int window, float scale, float c_log2,
                     uint32_t* __restrict__ status) {
-  constexpr int TILE = BKV * D * 2;  // [128 keys][D]
-  constexpr int QT = HK * D * 2;     // [64 queries][D]
-  constexpr int ST = KV2_ST;
+  constexpr int TILE = BKV * D * 2;
+  constexpr int QST = KV_QST, DOST = KV_DOST;
   let_successor_begin();
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align1024(smem_raw);
-  uint8_t* sK = smem;
+  extern __shared__ __align__(1024) uint8_t smem_kv[];
+  if (smem_u32(smem_kv) & 1023u) {  // no room to align by hand; the first byte that a kernel without static shared memory gets is aligned so
+    if (threadIdx.x == 0 && status) atomicExch(status, 3u);
+    return;
+  }
+  uint8_t* sK = smem_kv;
   uint8_t* sV = sK + TILE;
-  uint8_t* sQ = sV + TILE;           // [ST]
-  uint8_t* sDO = sQ + ST * QT;       // [ST]
-  float* sStat = reinterpret_cast<float*>(sDO + ST * QT);  // [ST][2][64]: -lse, -delta of the step's queries
-  BarsKV2* bars = reinterpret_cast<BarsKV2*>(sStat + ST * 2 * HK);
+  uint8_t* sQ = sV + TILE;            // [QST]
+  uint8_t* sDO = sQ + QST * TILE;     // [DOST]
+  float* sStat = reinterpret_cast<float*>(sDO + DOST * TILE);  // [2][2][128]: -lse, -delta of the step's queries
+  BarsKV3* bars = reinterpret_cast<BarsKV3*>(sStat + 4 * BQ);
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = H / Hkv, nkb = (T + BKV - 1) / BKV, heads = B * Hkv;
   const int items = nkb * heads;
-  // Item -> key block (the first ones are seen by the most queries), KV head, sequence, and the query steps per head
-  struct Item { int k0, g, b, ulo, nqi, n; };
+  // Item -> key block (the first ones are seen by the most queries), KV head, sequence; the 64-query halves that see it, counted
+  // from its own position, and the 128-query steps per head (of the last one, only the first half where the count is odd)
+  struct Item { int k0, g, b, halves, nqi, n; };
   auto item_of = [&](int w) {
     Item it;
     it.k0 = rotated(w / heads, nkb) * BKV;
     it.g = w % heads % Hkv;
     it.b = w % heads / Hkv;
-    it.ulo = it.k0 / HK;
-    int uhi = T / HK - 1;
-    if (window > 0) uhi = min(uhi, (it.k0 + BKV - 1 + window - 1) / HK);
-    it.nqi = uhi - it.ulo + 1;
+    int last = (T - 1) / 64;
+    if (window > 0) last = min(last, (it.k0 + BKV - 1 + window - 1) / 64);
+    it.halves = last - it.k0 / 64 + 1;
+    it.nqi = (it.halves + 1) / 2;
     it.n = G * it.nqi;
     return it;
   };
 
   if (threadIdx.x == 0) {
-    mbar_init(&bars->kv_full, 1);
-    mbar_init(&bars->kv_empty, 1);
-    for (int s = 0; s < ST; ++s) { mbar_init(&bars->qdo_full[s], 1); mbar_init(&bars->qdo_empty[s], 1); }
-    for (int z = 0; z < 2; ++z) { mbar_init(&bars->sdp_full[z], 1); mbar_init(&bars->pds_ready[z], SOFTMAX_WARPS); }
-    mbar_init(&bars->acc_done, 1);
+    mbar_init(&bars->k_full, 1); mbar_init(&bars->k_empty, 1); mbar_init(&bars->v_full, 1); mbar_init(&bars->v_empty, 1);
+    for (int s = 0; s < QST; ++s) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
+    for (int s = 0; s < DOST; ++s) { mbar_init(&bars->do_full[s], 1); mbar_init(&bars->do_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&bars->stat_full[s], 1); mbar_init(&bars->p_ready[s], SOFTMAX_WARPS); mbar_init(&bars->ds_ready[s], SOFTMAX_WARPS); }
+    mbar_init(&bars->s_full, 1); mbar_init(&bars->dp_full, 1);
+    mbar_init(&bars->acc_full, 1); mbar_init(&bars->acc_empty, SOFTMAX_WARPS);
     bars->abort_flag = 0;
     mbar_fence_init();
   }
@@ -1274,142 +1114,224 @@ attn_bwd_kv2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_slot;
-  const uint32_t tDV = tmem, tDK = tmem + 128, tBuf = tmem + 256;
+  const uint32_t tDV = tmem, tDK = tmem + 128, tS = tmem + 256, tDP = tmem + 384;
 
   if (warp == 0) {
-    if (elect_one()) {
-      uint32_t step = 0;  // query steps loaded so far
-      bool ok = true;
-      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
-        const Item it = item_of(w);
-        if (!mbar_wait(&bars->kv_empty, (turn & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(&bars->kv_full, 2 * TILE);
-        load_tile<D>(sK, &tmQK, &bars->kv_full, (H + it.g) * D, it.k0, it.b);
-        load_tile<D>(sV, &tmV, &bars->kv_full, (H + Hkv + it.g) * D, it.k0, it.b);
-        for (int i = 0; i < it.n; ++i, ++step) {
-          const int st = step % ST;
-          const int h = it.g * G + i / it.nqi;
-          const int q0 = (it.ulo + i % it.nqi) * HK;
-          if (!(ok = mbar_wait(&bars->qdo_empty[st], ((step / ST) & 1) ^ 1, abort_flag))) break;
-          mbar_expect_tx(&bars->qdo_full[st], 2 * QT + 2 * HK * 4);
-          load_tile_r<D, HK>(sQ + st * QT, &tmQ64, &bars->qdo_full[st], h * D, q0, it.b);
-          load_tile_r<D, HK>(sDO + st * QT, &tmDO64, &bars->qdo_full[st], h * D, q0, it.b);
-          bulk_load(sStat + st * 2 * HK, nlse + ((long)it.b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
-          bulk_load(sStat + st * 2 * HK + HK, ndelta + ((long)it.b * H + h) * T + q0, HK * 4, &bars->qdo_full[st]);
+    uint32_t c = 0;  // query steps loaded so far
+    bool ok = true;
+    for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
+      const Item it = item_of(w);
+      int h = it.g * G, q0 = it.k0;
+      for (int i = 0; ok && i < it.n; ++i, ++c) {
+        const int qs = c % QST, os = c % DOST;
+        float st[2][4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int q = q0 + x * 32 + lane;
+          const long at = ((long)it.b * H + h) * T + q;
+          st[0][x] = q < T ? nlse[at] : 0.0f;
+          st[1][x] = q < T ? ndelta[at] : 0.0f;
+        }
+        if (lane == 0) {
+          if (i == 0 && (ok = mbar_wait(&bars->k_empty, (turn & 1) ^ 1, abort_flag))) {
+            mbar_expect_tx(&bars->k_full, TILE);
+            load_tile<D>(sK, &tmQK, &bars->k_full, (H + it.g) * D, it.k0, it.b);
+          }
+          if (ok && (ok = mbar_wait(&bars->q_empty[qs], ((c / QST) & 1) ^ 1, abort_flag))) {
+            mbar_expect_tx(&bars->q_full[qs], TILE);
+            load_tile<D>(sQ + qs * TILE, &tmQK, &bars->q_full[qs], h * D, q0, it.b);
+          }
+          if (ok && i == 0 && (ok = mbar_wait(&bars->v_empty, (turn & 1) ^ 1, abort_flag))) {
+            mbar_expect_tx(&bars->v_full, TILE);
+            load_tile<D>(sV, &tmV, &bars->v_full, (H + Hkv + it.g) * D, it.k0, it.b);
+          }
+          if (ok && (ok = mbar_wait(&bars->do_empty[os], ((c / DOST) & 1) ^ 1, abort_flag))) {
+            mbar_expect_tx(&bars->do_full[os], TILE);
+            load_tile<D>(sDO + os * TILE, &tmDO, &bars->do_full[os], h * D, q0, it.b);
+          }
+          // the statistics of two steps ago have been read once that step's dK product is done
+          if (ok && c >= 2) ok = mbar_wait(&bars->q_empty[(c - 2) % QST], ((c - 2) / QST) & 1, abort_flag);
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0);
+        if (!ok) break;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          sStat[(c & 1) * 2 * BQ + x * 32 + lane] = st[0][x];
+          sStat[(c & 1) * 2 * BQ + BQ + x * 32 + lane] = st[1][x];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->stat_full[c & 1]);
+        if ((q0 += BQ) == it.k0 + it.nqi * BQ) {
+          q0 = it.k0;
+          ++h;
         }
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idS = make_idesc(128, HK, 0, 0);  // S^T = K Q^T, dP^T = V dO^T: 128 keys x 64 queries
+      constexpr uint32_t idS = make_idesc(128, BQ, 0, 0);  // S^T = K Q^T, dP^T = V dO^T
       constexpr uint32_t idG = make_idesc(128, D, 0, 1);   // dV = P^T dO, dK = dS^T Q: A in tensor memory, B MN-major
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
-      bool ok = true;
-      uint32_t step = 0;  // query steps before this item: their number decides stage, buffer and phases
-      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
-        const int n = item_of(w).n;
-        if (!(ok = mbar_wait(&bars->kv_full, turn & 1, abort_flag))) break;
-        auto issue_sdp = [&](int i) {
-          const uint32_t c = step + i;
-          const int st = c % ST, z = c & 1;
-          if (!mbar_wait(&bars->qdo_full[st], (c / ST) & 1, abort_flag)) return false;
-          tc_fence_after();
-          const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128, desc_k(aK, kk), desc_k_r<HK>(aQ, kk), idS, kk != 0);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tBuf + z * 128 + 64, desc_k(aV, kk), desc_k_r<HK>(aDO, kk), idS, kk != 0);
-          mma_commit(&bars->sdp_full[z]);
-          if (i + 1 == n) mma_commit(&bars->kv_empty);  // the item's last scores are on their way
-          return true;
-        };
-        ok = issue_sdp(0);
-        if (ok && n > 1) ok = issue_sdp(1);
-        for (int i = 0; i < n && ok; ++i) {
-          const uint32_t c = step + i;
-          const int st = c % ST, z = c & 1;
-          if (!(ok = mbar_wait(&bars->pds_ready[z], (c >> 1) & 1, abort_flag))) break;
-          tc_fence_after();
-          const uint32_t aQ = smem_u32(sQ + st * QT), aDO = smem_u32(sDO + st * QT);
-#pragma unroll
-          for (int kk = 0; kk < HK / 16; ++kk)
-            mma_f16_ts(tDV, tBuf + z * 128 + kk * 16, desc_mn_r<HK>(aDO, kk), idG, (i | kk) != 0);
-#pragma unroll
-          for (int kk = 0; kk < HK / 16; ++kk)
-            mma_f16_ts(tDK, tBuf + z * 128 + 64 + kk * 16, desc_mn_r<HK>(aQ, kk), idG, (i | kk) != 0);
-          mma_commit(&bars->qdo_empty[st]);
-          if (i + 1 == n) mma_commit(&bars->acc_done);
-          if (i + 2 < n) ok = issue_sdp(i + 2);  // into the buffer just consumed
+      // two walks over the same steps: the score products are one step ahead
+      struct Walk { int turn = 0, i = 0, n = 0, q = 0, nqi = 0, halves = 0; uint32_t c = 0; } a, d;  // n = 0: past the last item
+      auto begin = [&](Walk& x) {
+        const int w = work_item(x.turn);
+        x.i = x.n = x.q = x.nqi = x.halves = 0;
+        if (w < items) {
+          const Item it = item_of(w);
+          x.n = it.n;
+          x.nqi = it.nqi;
+          x.halves = it.halves;
         }
-        step += n;
+      };
+      auto next = [&](Walk& x) {
+        ++x.c;
+        if (++x.q == x.nqi) x.q = 0;
+        if (++x.i == x.n) {
+          ++x.turn;
+          begin(x);
+        }
+      };
+      // operands are waited for ahead of the hand-over that the product also needs
+      auto S_ready = [&]() {
+        return !(a.i == 0 && !mbar_wait(&bars->k_full, a.turn & 1, abort_flag)) && mbar_wait(&bars->q_full[a.c % QST], (a.c / QST) & 1, abort_flag);
+      };
+      auto dP_ready = [&]() {
+        return !(a.i == 0 && !mbar_wait(&bars->v_full, a.turn & 1, abort_flag)) && mbar_wait(&bars->do_full[a.c % DOST], (a.c / DOST) & 1, abort_flag);
+      };
+      auto issue_S = [&]() {
+        const uint32_t aQ = smem_u32(sQ + (a.c % QST) * TILE);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tS, desc_k(aK, kk), desc_k(aQ, kk), idS, kk != 0);
+        mma_commit(&bars->s_full);
+        if (a.i == a.n - 1) mma_commit(&bars->k_empty);
+      };
+      auto issue_dP = [&]() {
+        const uint32_t aDO = smem_u32(sDO + (a.c % DOST) * TILE);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tDP, desc_k(aV, kk), desc_k(aDO, kk), idS, kk != 0);
+        mma_commit(&bars->dp_full);
+        if (a.i == a.n - 1) mma_commit(&bars->v_empty);
+      };
+      // one accumulation over the step's queries, half by half as the element warps hand them over
+      auto accumulate = [&](uint32_t tAcc, uint32_t tA, uint32_t aB, uint64_t* ready) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (!mbar_wait(&ready[half], d.c & 1, abort_flag)) return false;
+          tc_fence_after();
+          if (half == 0 || 2 * d.q + 1 < d.halves) {
+#pragma unroll
+            for (int kk = half * 4; kk < half * 4 + 4; ++kk)
+              mma_f16_ts(tAcc, tA + kk * 16, desc_mn(aB, kk), idG, (d.i | kk) != 0);
+          }
+        }
+        return true;
+      };
+      begin(a);
+      d = a;
+      bool ok = true;
+      for (bool first = true; ok && (first || d.n); first = false) {
+        if (a.n && !(ok = S_ready())) break;
+        if (!first) {
+          if (d.i == 0 && !(ok = mbar_wait(&bars->acc_empty, (d.turn & 1) ^ 1, abort_flag))) break;  // the last item's results are read
+          if (!(ok = accumulate(tDV, tS, smem_u32(sDO + (d.c % DOST) * TILE), bars->p_ready))) break;
+        }
+        if (a.n) issue_S();  // over the P^T just consumed
+        if (!first) mma_commit(&bars->do_empty[d.c % DOST]);
+        if (a.n && !(ok = dP_ready())) break;
+        if (!first && !(ok = accumulate(tDK, tDP, smem_u32(sQ + (d.c % QST) * TILE), bars->ds_ready))) break;
+        if (a.n) {
+          issue_dP();
+          next(a);
+        }
+        if (!first) {
+          mma_commit(&bars->q_empty[d.c % QST]);
+          if (d.i == d.n - 1) mma_commit(&bars->acc_full);
+          next(d);
+        }
       }
     }
   } else {
-    constexpr int DH = D / NSPLIT;
     const int quad = warp & 3;
-    const int cq = (warp - 2) >> 2;          // which 16 of the step's 64 queries
+    const int part = (warp - 2) >> 2;        // which 16 queries of a 64-query half, and which quarter of the result's columns
     const int r = quad * 32 + lane;          // key row == TMEM lane
-    const uint32_t lane_off = uint32_t(quad * 32) << 16;
-    uint32_t step = 0;
+    const uint32_t lane_off = (uint32_t(quad * 32) << 16) + part * 16;
+    uint32_t c = 0;
     bool ok = true;
     for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
       const Item it = item_of(w);
-      const int k0 = it.k0, g = it.g, b = it.b, kj = k0 + r;
-      for (int i = 0; i < it.n && ok; ++i, ++step) {
-        const int st = step % ST, z = step & 1;
-        const int q0 = (it.ulo + i % it.nqi) * HK;
-        const int qbase = q0 + cq * 16;
-        // some (key, query) pair of the step is hidden
-        const bool need_mask = (k0 + BKV - 1 > q0) || (window > 0 && k0 <= q0 + HK - 1 - window);
-        if (!mbar_wait(&bars->qdo_full[st], (step / ST) & 1, abort_flag)) { ok = false; break; }  // the statistics are in shared memory
-        if (!mbar_wait(&bars->sdp_full[z], (step >> 1) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t tSt = tBuf + z * 128 + cq * 16 + lane_off, tDPt = tSt + 64;
-        const float* nl = sStat + st * 2 * HK + cq * 16;
-        const float* nd = nl + HK;
-        uint32_t vs[16], vd[16], pk[8], dsr[8];
-        // (512-key window, 4 x 4096 tokens, 16 heads x 128: 222 -> 209 us against position tests in every pair of such a step)
-        const Seen sn = need_mask ? seen(k0 + quad * 32, k0 + quad * 32 + 31, qbase, qbase + 15, window) : VISIBLE;
-        if (sn == HIDDEN) {
+      const int kj = it.k0 + r, klo = it.k0 + quad * 32;
+      int step = 0;
+      for (int i = 0; i < it.n && ok; ++i, ++c, step = step + 1 == it.nqi ? 0 : step + 1) {
+        const int q0 = it.k0 + step * BQ + part * 16;
+        const float* nl = sStat + (c & 1) * 2 * BQ + part * 16;
+        const float* nd = nl + BQ;
+        // two pieces of 16 queries, the second one's values in flight under the first one's arithmetic
+        Seen sn[2];
+        f2 p[2][8];
+        uint32_t v[2][16], pk[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) pk[e] = dsr[e] = 0u;
-        } else {
-          tmem_ld_32x32b_x16(tSt, vs);
-          tmem_ld_32x32b_x16(tDPt, vd);
+        for (int x = 0; x < 2; ++x) sn[x] = seen(klo, klo + 31, q0 + x * 64, q0 + x * 64 + 15, window);
+        if (!mbar_wait(&bars->stat_full[c & 1], (c >> 1) & 1, abort_flag) || !mbar_wait(&bars->s_full, c & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        tmem_ld_32x32b_x16(tS + lane_off, v[0]);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
           tmem_ld_wait();
-          if (sn == MIXED) bwd_probs_t<true>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
-          else bwd_probs_t<false>(vs, vd, nl, nd, c_log2, scale, kj, qbase, window, pk, dsr);
-        }
-        tmem_st_32x32b_x8(tSt, pk);
-        tmem_st_32x32b_x8(tDPt, dsr);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->pds_ready[z]);
-      }
-      ok = ok && mbar_wait(&bars->acc_done, turn & 1, abort_flag);
-      if (ok) {
-        tc_fence_after();
-        const bool in_range = kj < T;
-        __nv_bfloat16* dkrow = dK + ((long)b * T + kj) * lddk + (long)g * D + cq * DH;
-        __nv_bfloat16* dvrow = dV + ((long)b * T + kj) * lddv + (long)g * D + cq * DH;
+          if (x == 0) tmem_ld_32x32b_x16(tS + lane_off + 64, v[1]);
+          if (sn[x] != HIDDEN) probs_t(v[x], nl + x * 64, c_log2, sn[x] == MIXED, kj, q0 + x * 64, window, p[x], pk);
+          else {
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-#pragma unroll
-          for (int c = 0; c < DH / 16; ++c) {
-            uint32_t v[16];
-            tmem_ld_32x32b_x16((which ? tDK : tDV) + lane_off + cq * DH + c * 16, v);
-            tmem_ld_wait();
-            if (in_range) {
-              uint4* dst = reinterpret_cast<uint4*>((which ? dkrow : dvrow) + c * 16);
-#pragma unroll
-              for (int w = 0; w < 2; ++w)
-                dst[w] = make_uint4(pack_bf16(__uint_as_float(v[8 * w]), __uint_as_float(v[8 * w + 1])),
-                                    pack_bf16(__uint_as_float(v[8 * w + 2]), __uint_as_float(v[8 * w + 3])),
-                                    pack_bf16(__uint_as_float(v[8 * w + 4]), __uint_as_float(v[8 * w + 5])),
-                                    pack_bf16(__uint_as_float(v[8 * w + 6]), __uint_as_float(v[8 * w + 7])));
-            }
+            for (int e = 0; e < 8; ++e) pk[e] = 0u;
           }
+          tmem_st_32x32b_x8(tS + lane_off + x * 64, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->p_ready[x]);
+        }
+        if (!mbar_wait(&bars->dp_full, c & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        tmem_ld_32x32b_x16(tDP + lane_off, v[0]);
+        tmem_ld_32x32b_x16(tDP + lane_off + 64, v[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          if (sn[x] != HIDDEN) dscores_t(v[x], nd + x * 64, p[x], scale, pk);
+          else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) pk[e] = 0u;
+          }
+          tmem_st_32x32b_x8(tDP + lane_off + x * 64, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->ds_ready[x]);
+        }
+      }
+      ok = ok && mbar_wait(&bars->acc_full, turn & 1, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      constexpr int DH = D / NSPLIT;
+      const long row = (long)it.b * T + kj;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t v[DH];
+        tmem_ld_cols<DH>((which ? tDK : tDV) + (uint32_t(quad * 32) << 16) + part * DH, v);
+        tmem_ld_wait();
+        if (which == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty);
+        }
+        if (kj < T) {
+          uint4* dst = reinterpret_cast<uint4*>((which ? dK + row * lddk : dV + row * lddv) + (long)it.g * D + part * DH);
+#pragma unroll
+          for (int x = 0; x < DH / 8; ++x)
+            dst[x] = make_uint4(pack_bf16(__uint_as_float(v[8 * x]), __uint_as_float(v[8 * x + 1])),
+                                pack_bf16(__uint_as_float(v[8 * x + 2]), __uint_as_float(v[8 * x + 3])),
+                                pack_bf16(__uint_as_float(v[8 * x + 4]), __uint_as_float(v[8 * x + 5])),
+                                pack_bf16(__uint_as_float(v[8 * x + 6]), __uint_as_float(v[8 * x + 7])));
         }
       }
     }
@@ -1552,10 +1474,9 @@ CUresult encode_3d(CUtensorMap* out, const void* ptr, uint64_t cols, uint64_t T,
 }
 
 template <int D> constexpr int attn_smem_bytes() { return (1 + 2 * 2) * (BQ * D * 2) + BQ * BKV * 2 + 1024 + 512 + 4096; }
-template <int D> constexpr int attn_bwd_smem_bytes() { return (2 + 2 * 2) * (BQ * D * 2) + BQ * BKV * 2 + 1024 + 256; }
 
 template <int D> constexpr int attn_bwd_q2_smem_bytes() { return 4 * (BQ * D * 2) + 2 * 3 * (HK * D * 2) + 1024 + 256; }
-template <int D> constexpr int attn_bwd_kv2_smem_bytes() { return 2 * (BKV * D * 2) + 2 * KV2_ST * (HK * D * 2) + KV2_ST * 2 * HK * 4 + 1024 + 256; }
+template <int D> constexpr int attn_bwd_kv3_smem_bytes() { return (2 + KV_QST + KV_DOST) * (BKV * D * 2) + 4 * BQ * 4 + (int)sizeof(BarsKV3); }
 template <int D> constexpr int attn_fwd2_smem_bytes() { return (2 + 2 * 2) * (BQ * D * 2) + 1024 + 256; }
 
 }  // namespace
@@ -1655,40 +1576,23 @@ extern "C" int otb_attn_bwd(const void* qk, long ldqk, const void* qkv, long ldq
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   const int nq = (T + BQ - 1) / BQ;
   const int nkb = (T + BKV - 1) / BKV;
-  const unsigned gq = persistent_grid((long)((nq + 1) / 2) * H * B), gkv2 = persistent_grid((long)nkb * Hkv * B);
-  const dim3 gkv(nkb, Hkv, B);
+  const unsigned gq = persistent_grid((long)((nq + 1) / 2) * H * B), gkv = persistent_grid((long)nkb * Hkv * B);
   // dQ runs beside dK/dV: its CTAs start on the SMs that the latter leaves free, or as its CTAs end (backward, us, one after the
   // other and so: 2 x 1000 tokens, 12 heads x 64, window 512 83 and 56; 1 x 2048, 16 x 128 198 and 141; 4 x 4096 1018 and 976).
-  const bool kv2 = T % HK == 0;  // the transposed dK/dV kernel walks whole 64-query steps
   const long plane = (long)B * H * T;
-  CUtensorMap tq64, tdo64;
-  if (kv2) {
-    r = encode_3d(&tq64, qk, (uint64_t)ldqk, (uint64_t)T, (uint64_t)B, (uint64_t)ldqk, HK);
-    if (r != CUDA_SUCCESS) return 1000 + (int)r;
-    r = encode_3d(&tdo64, dO, (uint64_t)lddo, (uint64_t)T, (uint64_t)B, (uint64_t)lddo, HK);
-    if (r != CUDA_SUCCESS) return 1000 + (int)r;
-  }
   if (D == 128) {
-    const int rc = otb_allow_smem<attn_bwd_kv_kernel<128>>(attn_bwd_smem_bytes<128>()) |
-                   otb_allow_smem<attn_bwd_kv2_kernel<128>>(attn_bwd_kv2_smem_bytes<128>()) |
-                   otb_allow_smem<attn_bwd_q2_kernel<128>>(attn_bwd_q2_smem_bytes<128>());
+    const int rc = otb_allow_smem<attn_bwd_kv3_kernel<128>>(attn_bwd_kv3_smem_bytes<128>()) | otb_allow_smem<attn_bwd_q2_kernel<128>>(attn_bwd_q2_smem_bytes<128>());
     if (rc) return rc;
-    const int kv = kv2 ? otb_launch(attn_bwd_kv2_kernel<128>, gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<128>(), s, tq, tv, tq64, tdo64, delta + plane,
-                                    delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status)
-                       : otb_launch(attn_bwd_kv_kernel<128>, gkv, ATT_THREADS, attn_bwd_smem_bytes<128>(), s, tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
-                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
+    const int kv = otb_launch(attn_bwd_kv3_kernel<128>, gkv, ATT_THREADS, attn_bwd_kv3_smem_bytes<128>(), s, tq, tv, tdo, delta + plane, delta + 2 * plane, dKp,
+                              lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
     if (kv) return kv;
     return otb_launch_early(attn_bwd_q2_kernel<128>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<128>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T,
                             H, Hkv, window, scale, c_log2, status);
   } else {
-    const int rc = otb_allow_smem<attn_bwd_kv_kernel<64>>(attn_bwd_smem_bytes<64>()) |
-                   otb_allow_smem<attn_bwd_kv2_kernel<64>>(attn_bwd_kv2_smem_bytes<64>()) |
-                   otb_allow_smem<attn_bwd_q2_kernel<64>>(attn_bwd_q2_smem_bytes<64>());
+    const int rc = otb_allow_smem<attn_bwd_kv3_kernel<64>>(attn_bwd_kv3_smem_bytes<64>()) | otb_allow_smem<attn_bwd_q2_kernel<64>>(attn_bwd_q2_smem_bytes<64>());
     if (rc) return rc;
-    const int kv = kv2 ? otb_launch(attn_bwd_kv2_kernel<64>, gkv2, ATT_THREADS, attn_bwd_kv2_smem_bytes<64>(), s, tq, tv, tq64, tdo64, delta + plane,
-                                    delta + 2 * plane, dKp, lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status)
-                       : otb_launch(attn_bwd_kv_kernel<64>, gkv, ATT_THREADS, attn_bwd_smem_bytes<64>(), s, tq, tv, tdo, lse, delta, dKp, lddqk, dVp,
-                                    lddqkv, T, H, Hkv, window, scale, c_log2, status);
+    const int kv = otb_launch(attn_bwd_kv3_kernel<64>, gkv, ATT_THREADS, attn_bwd_kv3_smem_bytes<64>(), s, tq, tv, tdo, delta + plane, delta + 2 * plane, dKp,
+                              lddqk, dVp, lddqkv, B, T, H, Hkv, window, scale, c_log2, status);
     if (kv) return kv;
     return otb_launch_early(attn_bwd_q2_kernel<64>, gq, ATT_THREADS, attn_bwd_q2_smem_bytes<64>(), s, tq, tdo, tk64, tv64, lse, delta, dQp, lddqk, B, T,
                             H, Hkv, window, scale, c_log2, status);
