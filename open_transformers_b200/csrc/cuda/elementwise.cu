@@ -656,9 +656,8 @@ inline int swiglu_threads(int F) {
 // long rows and cost short ones registers, and with them CTAs per SM (ce_form chooses):
 //   TEST: the first pass finds the smallest logit too, and where it is near enough the exponent's clamp is left out;
 //   UNROLL groups per thread are in flight.
-// us for 16384 rows with their gradient; neither / TEST / TEST and four groups: bf16 V 1024 89 / 95 / 130, 8192 211 / 216 / 248,
-// 16384 296 / 296 / 346, 32768 525 / 516 / 568, 65536 986 / 967 / 1073, 98304 1714 / 1672 / 1552; 4000 rows of 128256 622 / 624 /
-// 542. fp32, 4000 rows: 1024 22 / 26 / 36, 8192 60 / 67 / 83, 16384 99 / 104 / 135, 32768 256 / 198 / 225, 65536 611 / 584 / 448;
+// us for 16384 rows with their gradient; neither / TEST / TEST and four groups: bf16 V 32768 525 / 516 / 568, 65536 986 / 967 / 1073, 98304 1714 / 1672 / 1552; 4000 rows of 128256 622 / 624 /
+// 542. fp32, 4000 rows: 16384 99 / 104 / 135, 32768 256 / 198 / 225, 65536 611 / 584 / 448;
 // with a few rows per SM neither helps (64 rows of 128256: 30 / 34 / 37, 149: 52 / - / 60, 600: 222 / 231 / 209).
 constexpr int CE_THREADS = 512, CE_SWEEP = CE_THREADS * 8;
 template <typename T, int CE_UNROLL>
@@ -765,9 +764,89 @@ __global__ void __launch_bounds__(CE_THREADS) ce_zloss_kernel(T* logits, const l
   else ce_grad<T, CE_UNROLL, true>(xr, V, l2, nm2, k2, label, at_label);
 }
 
-// Form of the loss kernel: 0 neither, 1 TEST, 4 TEST and four groups in flight. The lines lie where the figures above cross.
+// Rows of up to GROUPS groups per thread: the row is read once and its e_i stay in registers from the sum to the gradient, which
+// halves both the reading passes and the exponentials. Same chains and trees, so the same bits; rows of fewer than 512 groups
+// take a CTA of fewer threads (the sums that are missing from the tree are zeros in the other form). Bound by memory and, below
+// 2048 columns, by the row's two reductions. us, three passes and so: bf16 64 x 1024 3.4 and 2.5, 16384 x 1024 89 and 21, 8192 x 2048
+// 52 and 22, 8192 x 4096 67 and 46, 8192 x 8192 108 and 64 (4.2 TB/s), 8192 x 12288 139 and 104, 16384 x 16384 296 and 239; fp32 2048 x 1024
+// 12.5 and 5.1, 8192 x 4096 81 and 58, 4000 x 8192 60 and 52, but 4000 x 16384 99 and 108: four groups of fp32 leave too few rows on an SM.
+template <typename T, int GROUPS>
+__global__ void __launch_bounds__(CE_THREADS) ce_zloss_short_kernel(T* logits, const long* labels, float* __restrict__ ce_out, float* __restrict__ lse_out,
+                                                                    int V, float two_z, float scale, int write_grad) {
+  after_predecessor();
+  using namespace tc05;
+  __shared__ float sh[32];
+  const long row = blockIdx.x;
+  T* xr = logits + row * V;
+  const int c0 = threadIdx.x * 8;
+  Raw8<T> raw[GROUPS];
+  ce_fetch(raw, xr, c0, V);
+  const long label = labels[row];
+  if (label < 0) {
+    if (threadIdx.x == 0) { ce_out[row] = 0.0f; lse_out[row] = 0.0f; }
+    if (write_grad) {
+      float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int c = c0; c < V; c += CE_SWEEP) Vec8<T>::store(xr + c, z);
+    }
+    return;
+  }
+  const float x_label = to_f<T>(xr[label]);
+  float mx = -INFINITY;
+#pragma unroll
+  for (int u = 0; u < GROUPS; ++u)
+    if (c0 + u * CE_SWEEP < V) raw[u].largest(mx);
+  mx = block_max(mx, sh);
+  const float LOG2E = 1.44269504088896341f;
+  const f2 l2 = pack2(LOG2E, LOG2E);
+  const float nm = -__fmul_rn(mx, LOG2E);
+  const f2 nm2 = pack2(nm, nm);
+  f2 e2[GROUPS][4], acc2 = pack2(0.0f, 0.0f);
+#pragma unroll
+  for (int u = 0; u < GROUPS; ++u) {
+    if (c0 + u * CE_SWEEP < V) {
+      float f[8];
+      raw[u].unpack(f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        e2[u][e] = exp2_acc2(fma2(pack2(f[2 * e], f[2 * e + 1]), l2, nm2));
+        acc2 = add2(acc2, e2[u][e]);
+      }
+    }
+  }
+  float a0, a1;
+  unpack2(acc2, a0, a1);
+  const float s = block_tree_sum(__fadd_rn(a0, a1), sh);
+  const float lse = __fadd_rn(det_logf(s), mx);
+  if (threadIdx.x == 0) {
+    ce_out[row] = __fadd_rn(lse, -x_label);
+    lse_out[row] = lse;
+  }
+  if (!write_grad) return;
+  const float k = __fmul_rn(__fdiv_rn(__fmaf_rn(two_z, lse, 1.0f), s), scale);
+  const f2 k2 = pack2(k, k);
+  const float at_label = __fmaf_rn(det_exp2_acc(__fmaf_rn(x_label, LOG2E, nm)), k, -scale);
+#pragma unroll
+  for (int u = 0; u < GROUPS; ++u) {
+    const int c = c0 + u * CE_SWEEP;
+    if (c < V) {
+      float o[8];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) unpack2(mul2(e2[u][e], k2), o[2 * e], o[2 * e + 1]);
+      Vec8<T>::store(xr + c, o);
+      if (label >= c && label < c + 8) xr[label] = from_f<T>(at_label);
+    }
+  }
+}
+// threads of a short row's CTA: a power of two of at least one warp
+inline unsigned ce_short_threads(int V) {
+  unsigned t = CE_THREADS;
+  while (t > 32 && (int)(t / 2) * 8 >= V) t /= 2;
+  return t;
+}
+
+// Form of the loss kernel for longer rows: 0 neither, 1 TEST, 4 TEST and four groups in flight. The lines lie where the figures above cross.
 inline int ce_form(long rows, int V, bool bf16) {
-  if (bf16) return V <= 2 * CE_SWEEP ? 0 : V <= 20 * CE_SWEEP ? 1 : 4;
+  if (bf16) return V <= 20 * CE_SWEEP ? 1 : 4;
   return V <= 6 * CE_SWEEP || rows <= 4 * otb_sm_count() ? 0 : V <= 8 * CE_SWEEP ? 1 : 4;
 }
 
@@ -817,7 +896,6 @@ __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const long* __res
     out[c] = accumulate ? __fadd_rn(out[c], acc) : acc;
   }
 }
-
 // elementwise helpers ---------------------------------------------------------
 template <typename TI, typename TO>
 __global__ void cast_kernel(const TI* __restrict__ in, TO* __restrict__ out, long n) {
@@ -954,6 +1032,10 @@ extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* 
   if (V % 8) return -2;
 #define CE(U, TEST) \
   DISPATCH_T(dtype, return otb_launch_early(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
+#define CE_SHORT(GROUPS) \
+  DISPATCH_T(dtype, return otb_launch_early(ce_zloss_short_kernel<T, GROUPS>, (unsigned)rows, ce_short_threads(V), 0, S(stream), (T*)logits, labels, ce, lse, V, two_z, scale, write_grad);)
+  if (V <= CE_SWEEP) { CE_SHORT(1) } else if (V <= 2 * CE_SWEEP) { CE_SHORT(2) } else if (V <= 4 * CE_SWEEP && dtype) { CE_SHORT(4) }
+#undef CE_SHORT
   const int form = ce_form(rows, V, dtype);
   if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
