@@ -26,3 +26,25 @@ def test_loss_rows(V, dtype):
     for grad in (True, False):
         for got, ref in zip(run("cuda", grad), run("cpu", grad)):
             assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("D", [8, 12, 248, 256, 264, 2048, 2056, 4096])  # (12: no whole groups of eight)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_gradient(D, dtype):
+    g = torch.Generator().manual_seed(D)
+    ids = torch.cat([torch.randint(0, 40, (60,), generator=g), torch.full((9,), 7), torch.tensor([49])])  # runs of one to a dozen
+    dy, start = torch.randn(len(ids), D, generator=g).to(dtype), torch.randn(50, D, generator=g)
+    for accumulate in (True, False):
+        out = []
+        for dev in ("cuda", "cpu"):
+            dW = start.to(dev).clone()
+            K.embedding_bwd(dy.to(dev), ids.to(dev), dW, accumulate)
+            out.append(dW.cpu())
+        assert torch.equal(*out)
+    # a gradient that starts between two 16-byte boundaries takes the column-by-column form
+    odd = torch.empty(dy.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(dy).copy_(dy)
+    dW = start.cuda()
+    K.embedding_bwd(odd, ids.cuda(), dW, True)
+    ref = start.clone()
+    K.embedding_bwd(dy, ids, ref, True)
+    assert torch.equal(dW.cpu(), ref)
