@@ -56,7 +56,8 @@ constexpr int SOFTMAX_THREADS = 128 * NSPLIT;
 constexpr int ATT_THREADS = 64 + SOFTMAX_THREADS;
 constexpr int SOFTMAX_WARPS = SOFTMAX_THREADS / 32;
 
-__device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory"); }
+// The four warps that share the rows of a TMEM lane quadrant. (With one barrier for all sixteen warps 4 x 4096 tokens take 784 us, so 768.)
+__device__ __forceinline__ void quadrant_bar(int quad) { asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "n"(32 * NSPLIT) : "memory"); }
 
 // N (16 or 32) consecutive TMEM columns of this thread's lane
 template <int N>
@@ -156,9 +157,12 @@ __device__ __forceinline__ f2 probs_pack(const uint32_t (&sv)[KPT], float c_log2
     }
     lsum2 = add2(lsum2, p2);
     if constexpr (I8) {
-      const uint32_t q0b = (uint32_t)(int)rintf(__fmul_rn(p0, 127.0f)), q1b = (uint32_t)(int)rintf(__fmul_rn(p1, 127.0f));
-      if ((e & 3) == 0) pk[e >> 2] = 0;
-      pk[e >> 2] |= (q0b | (q1b << 8)) << (8 * (e & 3));
+      // rint(127 p) sits in the low byte of 127 p + 1.5 * 2^23. (The product is rounded first, by itself: as packed instructions
+      // the two come out as one multiply-add, whose ties are others.)
+      float t0, t1;
+      unpack2(add2(pack2(__fmul_rn(p0, 127.0f), __fmul_rn(p1, 127.0f)), pack2(12582912.0f, 12582912.0f)), t0, t1);
+      const uint32_t two = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x0040);
+      pk[e >> 2] = (e & 3) == 0 ? two : __byte_perm(pk[e >> 2], two, 0x5410);
     } else {
       pk[e >> 1] = pack_bf16(p0, p1);
     }
@@ -292,8 +296,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
     float m_run = -INFINITY, l_run = 0.0f, alpha_prev = 0.0f;
     float c_prev = 0.0f;  // int8 P V: dequantisation factor (value step / 127) of the block whose P V is pending
     const int nblk = (T + BKV - 1) / BKV;
-    // accumulator word -> fp32 contribution
-    auto pv_val = [&](uint32_t w) { return I8PV ? __fmul_rn(__int2float_rn((int)w), c_prev) : __uint_as_float(w); };
+    // two accumulator words -> fp32 contributions; the integers (below 2^22) become floats by one addition to the bits of 1.5 * 2^23
+    // and one subtraction, both exact. (This and the same for the probabilities, instead of the conversion pipe, a quarter as wide:
+    // 4 x 4096 tokens, 16 heads, 812 -> 784 us; 1 x 2048 94 -> 91.)
+    auto pv_vals = [&](uint32_t w0, uint32_t w1) {
+      if constexpr (!I8PV) return pack2(__uint_as_float(w0), __uint_as_float(w1));
+      const f2 x = add2(pack2(__uint_as_float(w0 + 0x4B400000u), __uint_as_float(w1 + 0x4B400000u)), pack2(-12582912.0f, -12582912.0f));
+      return mul2(x, pack2(c_prev, c_prev));
+    };
     f2 o[DH / 2];
 #pragma unroll
     for (int d = 0; d < DH / 2; ++d) o[d] = pack2(0.0f, 0.0f);
@@ -317,7 +327,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
       float mx = -INFINITY;
       if (ok) mx = need_mask ? scores_max<true>(sv, kbase, qi, window) : scores_max<false>(sv, kbase, qi, window);
       bars->xch[i & 1][part][r] = mx;
-      softmax_bar();
+      quadrant_bar(qd);
 #pragma unroll
       for (int pp = 0; pp < NSPLIT; ++pp) mx = fmaxf(mx, bars->xch[i & 1][pp][r]);
       const float m_new = fmaxf(m_run, __fmul_rn(mx, c_log2));
@@ -342,7 +352,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
             tmem_ld_wait();
 #pragma unroll
             for (int e = 0; e < CW; e += 2)
-              o[(c * CW + e) >> 1] = fma2(o[(c * CW + e) >> 1], a2, pack2(pv_val(v[e]), pv_val(v[e + 1])));
+              o[(c * CW + e) >> 1] = fma2(o[(c * CW + e) >> 1], a2, pv_vals(v[e], v[e + 1]));
           }
         }
       }
@@ -376,7 +386,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
     ok = ok && mbar_wait(pv_full, (n - 1) & 1, abort_flag);
     tc_fence_after();
     bars->xch[n & 1][part][r] = l_run;
-    softmax_bar();
+    quadrant_bar(qd);
     float l_tot = bars->xch[n & 1][0][r];
 #pragma unroll
     for (int pp = 1; pp < NSPLIT; ++pp) l_tot = __fadd_rn(l_tot, bars->xch[n & 1][pp][r]);
@@ -392,7 +402,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
 #pragma unroll
         for (int e = 0; e < CW; e += 2) {
           float a0, a1;
-          unpack2(fma2(o[(c * CW + e) >> 1], pack2(alpha_prev, alpha_prev), pack2(pv_val(v[e]), pv_val(v[e + 1]))), a0, a1);
+          unpack2(fma2(o[(c * CW + e) >> 1], pack2(alpha_prev, alpha_prev), pv_vals(v[e], v[e + 1])), a0, a1);
           pk[e >> 1] = pack_bf16(__fdiv_rn(a0, l_tot), __fdiv_rn(a1, l_tot));
         }
         if (in_range) {

@@ -25,3 +25,14 @@ def test_step_edges(T, H, Hkv, D, window):
     for got, ref in zip(run("cuda"), run("cpu")):
         assert torch.equal(got, ref)
     assert K.kernel_status("cuda") == 0
+
+
+def test_int8_probabilities_are_rounded_twice():
+    """127 p is rounded before it is rounded to an integer: a fused multiply-add differs in a few of these 4 M probabilities."""
+    B, T, H, D = 1, 1000, 4, 128
+    g = torch.Generator().manual_seed(1)
+    qk, qkv = torch.randn(B * T, 2 * H * D, generator=g).to(torch.bfloat16), torch.randn(B * T, 3 * H * D, generator=g).to(torch.bfloat16)
+    for window in (0, 512):
+        got = K.attn_fwd(qk.cuda(), qkv.cuda(), B, T, H, H, D, window, int8_pv=True)
+        for x, ref in zip(got, K.attn_fwd(qk, qkv, B, T, H, H, D, window, int8_pv=True)):
+            assert torch.equal(x.cpu(), ref)
