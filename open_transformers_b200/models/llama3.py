@@ -103,6 +103,25 @@ class Llama3(nn.Module):
     def forward(self, input_ids: torch.Tensor) -> ModelOutput:
         return ModelOutput(self.embedding.project(self.forward_hidden(input_ids)), None)
 
+    def train(self, mode: bool = True):
+        """``nn.Module.train`` in one walk without its attribute machinery: a scoring program calls ``eval()`` before each prompt, and
+        through 73 modules of the six-layer 100M model that took longer (95 us) than two of its blocks take to launch."""
+        if not isinstance(mode, bool):
+            raise ValueError("training mode is expected to be boolean")
+        todo, plain_train, plain_set = [self], nn.Module.train, nn.Module.__setattr__
+        while todo:
+            m = todo.pop()
+            cls = type(m)
+            if m is not self and (cls.train is not plain_train or "train" in m.__dict__):
+                m.train(mode)  # one that does more than this
+                continue
+            if cls.__setattr__ is plain_set:
+                m.__dict__["training"] = mode
+            else:
+                m.training = mode
+            todo.extend(c for c in m._modules.values() if c is not None)
+        return self
+
     def num_parameters(self) -> int:
         return sum(p.numel() for p in self.parameters())
 

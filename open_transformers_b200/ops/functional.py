@@ -7,6 +7,7 @@ native library is an error. Activations are bf16 (tensor-core family) or fp32 (e
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
 import torch
@@ -277,6 +278,14 @@ def swiglu_bwd(gu: torch.Tensor, dh: torch.Tensor) -> torch.Tensor:
 _block_fwd = packed_entry("otb_block_fwd", "20q4d3q")
 
 
+@functools.lru_cache(maxsize=256)
+def _block_scratch(rows: int, d: int, H: int, Hkv: int, D: int, inner: int, bf: int) -> int:
+    """Bytes of work space of a block call: a function of the sizes alone (5 us of argument objects a call otherwise)."""
+    need = cuda_lib().otb_block_fwd_scratch
+    need.restype = ctypes.c_long
+    return need(L(rows), I(d), I(H), I(Hkv), I(D), I(inner), I(bf))
+
+
 def block_fwd(x, norm1, wqkv, wo, norm2, wgu, wdown, cos, sin, H: int, Hkv: int, D: int, window: int, qk_norm: bool, eps1: float, eps2: float,
               eps_qk: float) -> torch.Tensor:
     """Decoder block on CUDA activations ``x`` [B, T, d] in one native call (csrc/cuda/block.cu): the launches of ``rmsnorm_fwd``,
@@ -286,9 +295,7 @@ def block_fwd(x, norm1, wqkv, wo, norm2, wgu, wdown, cos, sin, H: int, Hkv: int,
     inner = wdown.shape[1]
     y = torch.empty_like(x)
     bf = is_bf16(x)
-    need = cuda_lib().otb_block_fwd_scratch
-    need.restype = ctypes.c_long
-    scratch = torch.empty(need(L(B * T), I(d), I(H), I(Hkv), I(D), I(inner), I(bf)), dtype=torch.uint8, device=x.device)
+    scratch = torch.empty(_block_scratch(B * T, d, H, Hkv, D, inner, bf), dtype=torch.uint8, device=x.device)
     check(_block_fwd(x.data_ptr(), y.data_ptr(), scratch.data_ptr(), norm1.data_ptr(), wqkv.data_ptr(), wo.data_ptr(), norm2.data_ptr(),
                      wgu.data_ptr(), wdown.data_ptr(), cos.data_ptr(), sin.data_ptr(), B, T, d, H, Hkv, D, inner, window, qk_norm, eps1, eps2,
                      eps_qk, 1.0 / math.sqrt(D), bf, _status_ptr(x), raw_stream()), "block_fwd")
