@@ -170,6 +170,38 @@ __device__ __forceinline__ f2 probs_pack(const uint32_t (&sv)[KPT], float c_log2
   return lsum2;
 }
 
+// N outputs of a row divided by its sum l, packed to bf16 pairs; y = 1 / l correctly rounded. IEEE divisions without the divider: two
+// steps q <- q + (a - q l) y from q = a y give the correctly rounded quotient where nothing over- or underflows (Markstein, IBM J. Res.
+// Dev. 34, 1990); a warp with a value outside those bounds (a zero, whose sign the steps may lose, an infinity or a NaN among them)
+// divides. Called by whole warps. (The divider's checks keep its instructions from overlapping: with it the 128 of a row took 10 thousand
+// clocks, a third of an item with a 512-key window. us, divider and so: forward 1 x 16 tokens 8.6 and 6.9, 1 x 333 13.6 and 11.9, 1 x 2048 57
+// and 54, 4 x 4096 388 and 362, with a 512-key window 176 and 163; int8 P V 1 x 2048 89 and 82, 4 x 4096 768 and 701, window 334 and 309.)
+template <int N>
+__device__ __forceinline__ void divide_pack(const float (&a)[N], float l, float y, uint32_t (&pk)[N / 2]) {
+  float lo = fabsf(a[0]), hi = lo;
+#pragma unroll
+  for (int e = 1; e < N; ++e) {
+    lo = fminf(lo, fabsf(a[e]));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(hi) : "f"(fabsf(a[e])));
+  }
+  if (__all_sync(0xffffffffu, l >= 0x1p-20f && l <= 0x1p40f && lo >= 0x1p-60f && hi <= 0x1p80f)) {
+    const f2 y2 = pack2(y, y), nl2 = pack2(-l, -l);
+#pragma unroll
+    for (int e = 0; e < N; e += 2) {
+      const f2 a2 = pack2(a[e], a[e + 1]);
+      f2 q = mul2(a2, y2);
+      q = fma2(fma2(q, nl2, a2), y2, q);
+      q = fma2(fma2(q, nl2, a2), y2, q);
+      float q0, q1;
+      unpack2(q, q0, q1);
+      pk[e >> 1] = pack_bf16(q0, q1);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < N; e += 2) pk[e >> 1] = pack_bf16(__fdiv_rn(a[e], l), __fdiv_rn(a[e + 1], l));
+  }
+}
+
 // ---------------------------------------------------------------------------- forward
 template <int D, bool I8PV>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
@@ -392,6 +424,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
     for (int pp = 1; pp < NSPLIT; ++pp) l_tot = __fadd_rn(l_tot, bars->xch[n & 1][pp][r]);
     if (ok) {
       const bool in_range = qi < T;
+      const float y = __frcp_rn(l_tot);
       __nv_bfloat16* orow = O + ((long)b * T + qi) * ldo + (long)h * D + part * DH;
 #pragma unroll
       for (int c = 0; c < DH / CW; ++c) {
@@ -399,12 +432,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
         tmem_ld_cols<CW>(tPV + lane_off + part * DH + c * CW, v);
         tmem_ld_wait();
         uint32_t pk[CW / 2];
+        float a[CW];
 #pragma unroll
-        for (int e = 0; e < CW; e += 2) {
-          float a0, a1;
-          unpack2(fma2(o[(c * CW + e) >> 1], pack2(alpha_prev, alpha_prev), pv_vals(v[e], v[e + 1])), a0, a1);
-          pk[e >> 1] = pack_bf16(__fdiv_rn(a0, l_tot), __fdiv_rn(a1, l_tot));
-        }
+        for (int e = 0; e < CW; e += 2) unpack2(fma2(o[(c * CW + e) >> 1], pack2(alpha_prev, alpha_prev), pv_vals(v[e], v[e + 1])), a[e], a[e + 1]);
+        divide_pack<CW>(a, l_tot, y, pk);
         if (in_range) {
 #pragma unroll
           for (int w = 0; w < CW / 8; ++w)
@@ -699,6 +730,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
       if (ok) {
         const float l_tot = __fadd_rn(__fadd_rn(__fadd_rn(l_run[0], l_run[1]), l_run[2]), l_run[3]);
         const bool in_range = qi < T;
+        const float y = __frcp_rn(l_tot);
         __nv_bfloat16* orow = O + ((long)b * T + qi) * ldo + (long)h * D;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -706,9 +738,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
           tmem_ld_32x32b_x32(tO + c * 32, v);
           tmem_ld_wait();
           uint32_t pk[16];
+          float a[32];
 #pragma unroll
-          for (int e = 0; e < 32; e += 2)
-            pk[e >> 1] = pack_bf16(__fdiv_rn(__uint_as_float(v[e]), l_tot), __fdiv_rn(__uint_as_float(v[e + 1]), l_tot));
+          for (int e = 0; e < 32; ++e) a[e] = __uint_as_float(v[e]);
+          divide_pack<32>(a, l_tot, y, pk);
           if (in_range) {
 #pragma unroll
             for (int w = 0; w < 4; ++w)
