@@ -556,59 +556,62 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
     if (elect_one()) {
       constexpr uint32_t idS = make_idesc(128, BKV, 0, 0);
       constexpr uint32_t idPV = make_idesc(128, D, 0, 1);
+      // Scores are formed one step ahead, across the boundaries of items: the next item's first ones go right behind this one's last P V,
+      // while the softmax warps still divide and store. us, from the next item's beginning and so: 1 x 2048 tokens 54.4 and 52.0, 4 x 4096
+      // 363 and 357, with a 512-key window 163 and 152; 8 x 2048, 4 x 64 heads, 53.8 and 52.0. (The same in dQ: 1033 to 1046 for the whole
+      // backward, windowed 366 to 360; not taken.)
+      uint32_t ring = 0, blocks[2] = {0, 0};  // key blocks so far; those of each tile
+      // this step's item and key block, and those of the step whose scores are formed now: one further, in the next item after the last
+      Item it, ahead = item_of(work_item(0));
+      int turn = -1, i = 0, ahead_i = 0;
       bool ok = true;
-      uint32_t ring = 0, parity[2] = {0, 0};  // key blocks before this item; P tiles consumed per tile
-      for (int turn = 0, w; ok && (w = work_item(turn)) < items; ++turn) {
-        const Item it = item_of(w);
-        const int n = it.n;
-        if (!(ok = mbar_wait(&bars->q_full, turn & 1, abort_flag))) break;
-        bool first[2] = {true, true};
-        auto k_ready = [&](int i) { return mbar_wait(&bars->k_full[(ring + i) % ST], ((ring + i) / ST) & 1, abort_flag); };
-        // S of tile X (block i); K stage not released
-        auto issue_S1 = [&](int X, int i) {
-          const uint32_t aK = smem_u32(sK + ((ring + i) % ST) * TILE), aQ = smem_u32(sQ + X * TILE);
+      for (bool first = true; ok; first = false) {
+        bool scores = ahead_i < ahead.n, k_here = false;
+        for (int X = 0; X < 2 && ok; ++X) {
+          if (!first && it.act(X, it.jlo + i)) {
+            const int j = it.jlo + i, st = (ring - 1) % ST;
+            if (!(ok = mbar_wait(&bars->v_full[st], ((ring - 1) / ST) & 1, abort_flag) && mbar_wait(&bars->p_ready[X], blocks[X] & 1, abort_flag))) break;
+            ++blocks[X];
+            tc_fence_after();
+            const uint32_t aV = smem_u32(sV + st * TILE);
+            const bool fresh = j == (X == 0 ? it.jlo : it.jloB);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 128, desc_k(aQ, kk), desc_k(aK, kk), idS, kk != 0);
-          mma_commit(&bars->s_full[X]);
-        };
-        if (!(ok = k_ready(0))) break;
-        tc_fence_after();
-        for (int X = 0; X < 2; ++X)
-          if (it.act(X, it.jlo)) issue_S1(X, 0);
-        mma_commit(&bars->k_empty[ring % ST]);
-        for (int i = 0; i < n && ok; ++i) {
-          const int st = (ring + i) % ST, j = it.jlo + i;
-          const bool more = i + 1 < n;
-          bool k_next = false;  // K of block i + 1 is in shared memory
-          for (int X = 0; X < 2 && ok; ++X) {
-            if (it.act(X, j)) {
-              if (!(ok = mbar_wait(&bars->p_ready[X], parity[X] & 1, abort_flag))) break;
-              ++parity[X];
-              if (!(ok = mbar_wait(&bars->v_full[st], ((ring + i) / ST) & 1, abort_flag))) break;
-              tc_fence_after();
-              const uint32_t aV = smem_u32(sV + st * TILE);
-#pragma unroll
-              for (int kk = 0; kk < BKV / 16; ++kk)
-                mma_f16_ts(tmem + 256 + X * 128, tmem + X * 128 + kk * 8, desc_mn(aV, kk), idPV, !first[X] || kk != 0);
-              first[X] = false;
-              if (j == (X == 0 ? it.jhiA : it.jhiB)) mma_commit(&bars->o_done[X]);
-            }
-            // this tile's next S goes right behind its P V (it overwrites the P just consumed)
-            if (more && it.act(X, j + 1)) {
-              if (!k_next) {
-                if (!(ok = k_ready(i + 1))) break;
-                tc_fence_after();
-                k_next = true;
-              }
-              issue_S1(X, i + 1);
-            }
+            for (int kk = 0; kk < BKV / 16; ++kk)
+              mma_f16_ts(tmem + 256 + X * 128, tmem + X * 128 + kk * 8, desc_mn(aV, kk), idPV, !fresh || kk != 0);
+            if (j == (X == 0 ? it.jhiA : it.jhiB)) mma_commit(&bars->o_done[X]);
           }
-          if (!ok) break;
-          mma_commit(&bars->v_empty[st]);
-          if (more) mma_commit(&bars->k_empty[(ring + i + 1) % ST]);
-          if (i + 2 == n || n == 1) mma_commit(&bars->q_empty);  // the item's last scores are on their way
+          // this tile's next S goes right behind its P V (it overwrites the P just consumed)
+          if (scores && ahead.act(X, ahead.jlo + ahead_i)) {
+            if (!k_here) {
+              if (ahead_i == 0 && !(ok = mbar_wait(&bars->q_full, (turn + 1) & 1, abort_flag))) break;
+              if (!(ok = mbar_wait(&bars->k_full[ring % ST], (ring / ST) & 1, abort_flag))) break;
+              tc_fence_after();
+              k_here = true;
+            }
+            const uint32_t aK = smem_u32(sK + (ring % ST) * TILE), aQ = smem_u32(sQ + X * TILE);
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk) mma_f16_ss(tmem + X * 128, desc_k(aQ, kk), desc_k(aK, kk), idS, kk != 0);
+            mma_commit(&bars->s_full[X]);
+          }
         }
-        ring += n;
+        if (!ok) break;
+        if (!first) mma_commit(&bars->v_empty[(ring - 1) % ST]);
+        if (!scores) break;
+        mma_commit(&bars->k_empty[ring % ST]);
+        if (ahead_i == ahead.n - 1) mma_commit(&bars->q_empty);  // the item's last scores are on their way
+        if (ahead_i == 0) {
+          it = ahead;
+          ++turn;
+        }
+        i = ahead_i;
+        ++ring;
+        if (++ahead_i == ahead.n) {
+          const int w = work_item(turn + 1);
+          if (w < items) {
+            ahead = item_of(w);
+            ahead_i = 0;
+          }
+        }
       }
     }
   } else {
