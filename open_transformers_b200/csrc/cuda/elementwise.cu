@@ -428,6 +428,23 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* in, long 
 #pragma unroll
     for (int pr = 0; pr < 2; ++pr) { c[pr] = cosb[at + pr]; s[pr] = sinb[at + pr]; }
   }
+  // The heads' sums first, then lane i finds the root of head i: one square root and division for all of them. (Every lane finding every
+  // head's: 16384 tokens x 20 heads x 128 38.9 us, so 35.6; 1000 x 16 x 64 4.8 and 4.2.)
+  float rstd = 0.0f;
+  if (do_norm) {
+    float mine = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NH; ++i) {
+      float f[4] = {0.f, 0.f, 0.f, 0.f}, acc = 0.0f;
+      if (active && i < n) raw[i].unpack(f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc = __fmaf_rn(f[e], f[e], acc);
+      const float ss = warp_butterfly(acc);
+      if (lane == i) mine = ss;
+    }
+    rstd = det_rsqrtf(__fadd_rn(__fmul_rn(mine, inv_d), eps));
+    if (lane < n) rstd_out[row * heads + head0 + lane] = rstd;
+  }
   T* o = out + row * ld_out + (long)head0 * D + lane * 4;
 #pragma unroll
   for (int i = 0; i < NH; ++i) {
@@ -435,14 +452,9 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(const T* in, long 
     float f[4] = {0.f, 0.f, 0.f, 0.f};
     if (active) raw[i].unpack(f);
     if (do_norm) {
-      float acc = 0.0f;
+      const float r = __shfl_sync(0xffffffffu, rstd, i);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc = __fmaf_rn(f[e], f[e], acc);
-      const float ss = warp_butterfly(acc);
-      const float rstd = det_rsqrtf(__fadd_rn(__fmul_rn(ss, inv_d), eps));
-      if (lane == 0) rstd_out[row * heads + head0 + i] = rstd;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = __fmul_rn(f[e], rstd);
+      for (int e = 0; e < 4; ++e) f[e] = __fmul_rn(f[e], r);
     }
     if (active) {
       float r[4];
