@@ -89,6 +89,10 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 __device__ __forceinline__ int work_item(int turn) {
   return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
+// The element warps of these kernels do not leave an item where a bounded wait gives up: a lane that gave up alone would be missing from
+// the tensor-memory accesses, votes and shuffles that follow, and the others would wait for it without a limit. It waits no more,
+// the warp goes on with whatever values are there, and at the item's end votes whether to store them and go on to the next. (A vote
+// at each wait, us: forward and backward at 4 x 4096 tokens with a 512-key window 619 and 635.)
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
@@ -379,15 +383,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
       const uint32_t tSb = tS + (i & 1) * 128 + part * KPT + lane_off;
       // the thread's 32 raw scores stay in registers for both passes; once they are there the S buffer is free
       uint32_t sv[KPT];
-      if (ok) {
-        tmem_ld_32x32b_x32(tSb, sv);
-        tmem_ld_wait();
-      }
+      tmem_ld_32x32b_x32(tSb, sv);
+      tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(&s_empty[i & 1]);
-      float mx = -INFINITY;
-      if (ok) mx = need_mask ? scores_max<true>(sv, kbase, qi, window) : scores_max<false>(sv, kbase, qi, window);
+      if (lane == 0) mbar_arrive(&s_empty[i & 1]);
+      float mx = need_mask ? scores_max<true>(sv, kbase, qi, window) : scores_max<false>(sv, kbase, qi, window);
       bars->xch[i & 1][part][r] = mx;
       quadrant_bar(qd);
 #pragma unroll
@@ -396,42 +397,36 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
       const float m_safe = (m_new == -INFINITY) ? 0.0f : m_new;
       const float alpha = det_exp2_attn(__fadd_rn(m_run, -m_safe));
       // probabilities and the quarter-row sum first (independent of O), while the tensor core finishes the previous P V
-      f2 lsum2 = pack2(0.0f, 0.0f);
       uint32_t pk[KPT / 2];
-      if (ok)
-        lsum2 = need_mask ? probs_pack<true, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk)
-                          : probs_pack<false, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk);
+      const f2 lsum2 = need_mask ? probs_pack<true, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk)
+                                 : probs_pack<false, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk);
       // deferred accumulation of the previous block's P V (its completion also frees the P buffer)
       if (i > 0) {
         ok = ok && mbar_wait(pv_full, (i - 1) & 1, abort_flag);
         tc_fence_after();
-        if (ok) {
-          const f2 a2 = pack2(alpha_prev, alpha_prev);
+        const f2 a2 = pack2(alpha_prev, alpha_prev);
 #pragma unroll
-          for (int c = 0; c < DH / CW; ++c) {
-            uint32_t v[CW];
-            tmem_ld_cols<CW>(tPV + lane_off + part * DH + c * CW, v);
-            tmem_ld_wait();
+        for (int c = 0; c < DH / CW; ++c) {
+          uint32_t v[CW];
+          tmem_ld_cols<CW>(tPV + lane_off + part * DH + c * CW, v);
+          tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < CW; e += 2)
-              o[(c * CW + e) >> 1] = fma2(o[(c * CW + e) >> 1], a2, pv_vals(v[e], v[e + 1]));
-          }
+          for (int e = 0; e < CW; e += 2)
+            o[(c * CW + e) >> 1] = fma2(o[(c * CW + e) >> 1], a2, pv_vals(v[e], v[e + 1]));
         }
       }
-      if (ok) {
-        if (I8PV) {
-          // keys part*32 .. +31 are bytes part*32 .. +31 of the 128-byte row: chunks part*2, part*2 + 1
+      if (I8PV) {
+        // keys part*32 .. +31 are bytes part*32 .. +31 of the 128-byte row: chunks part*2, part*2 + 1
 #pragma unroll
-          for (int w = 0; w < 2; ++w)
-            *reinterpret_cast<uint4*>(sP + swz(r, part * 2 + w)) = make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
-        } else {
-          // keys part*32 .. +31 -> 64-key sub-tile (part >> 1), 16-byte chunks (part & 1) * 4 .. +3 of the row
-          uint8_t* base = sP + (part >> 1) * 16384;
+        for (int w = 0; w < 2; ++w)
+          *reinterpret_cast<uint4*>(sP + swz(r, part * 2 + w)) = make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
+      } else {
+        // keys part*32 .. +31 -> 64-key sub-tile (part >> 1), 16-byte chunks (part & 1) * 4 .. +3 of the row
+        uint8_t* base = sP + (part >> 1) * 16384;
 #pragma unroll
-          for (int w = 0; w < 4; ++w)
-            *reinterpret_cast<uint4*>(base + swz(r, (part & 1) * 4 + w)) =
-                make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
-        }
+        for (int w = 0; w < 4; ++w)
+          *reinterpret_cast<uint4*>(base + swz(r, (part & 1) * 4 + w)) =
+              make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
       }
       float ls0, ls1;
       unpack2(lsum2, ls0, ls1);
@@ -443,9 +438,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(p_ready);
+      if (lane == 0) mbar_arrive(p_ready);
     }
     ok = ok && mbar_wait(pv_full, (n - 1) & 1, abort_flag);
+    ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
     bars->xch[n & 1][part][r] = l_run;
     quadrant_bar(qd);
@@ -658,9 +654,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
       const int q0 = (it.tile0 + X) * BQ, qi = q0 + r, h = it.h, b = it.b;
       const int jloX = X == 0 ? it.jlo : it.jloB, jhiX = X == 0 ? it.jhiA : it.jhiB;
       float m_run = -INFINITY, l_run[NSPLIT] = {0.0f, 0.0f, 0.0f, 0.0f};
-      for (int j = jloX; j <= jhiX && ok; ++j) {
+      for (int j = jloX; j <= jhiX; ++j) {
         const bool need_mask = (j == jhiX) || (window > 0 && j * BKV < q0 + BQ - window);
-        if (!mbar_wait(&bars->s_full[X], scores & 1, abort_flag)) { ok = false; break; }
+        ok = ok && mbar_wait(&bars->s_full[X], scores & 1, abort_flag);
         ++scores;
         tc_fence_after();
         // pass 1: row maximum. Fully visible blocks take the unrolled path with the next 32 columns already in flight
@@ -758,6 +754,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
         if (lane == 0) mbar_arrive(&bars->p_ready[X]);
       }
       ok = ok && mbar_wait(&bars->o_done[X], outputs & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
       ++outputs;
       tc_fence_after();
       if (ok) {
@@ -1006,11 +1003,11 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
       const float lse_r = row_ok ? lse[((long)b * H + h) * T + qi] : 0.0f;
       const float dl_r = row_ok ? delta[((long)b * H + h) * T + qi] : 0.0f;
       const int uloX = X == 0 ? it.ulo : it.uloB, uhiX = X == 0 ? it.uhiA : it.uhiB;
-      for (int u = uloX; u <= uhiX && ok; ++u) {
+      for (int u = uloX; u <= uhiX; ++u) {
         const int k0 = u * HK;
         // some (row, key) pair of this step is hidden, or the tile has rows past the end of the sequence
         const bool need_mask = (k0 + HK - 1 > q0) || (window > 0 && k0 <= q0 + BQ - 1 - window) || (q0 + BQ > T);
-        if (!mbar_wait(&bars->sdp_full[X], scores & 1, abort_flag)) { ok = false; break; }
+        ok = ok && mbar_wait(&bars->sdp_full[X], scores & 1, abort_flag);
         ++scores;
         tc_fence_after();
         // dS (bf16 pairs, 8 columns per 16 keys) goes over the thread's own score columns, which it has read by then
@@ -1030,6 +1027,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         if (lane == 0) mbar_arrive(&bars->ds_ready[X]);
       }
       ok = ok && mbar_wait(&bars->dq_done[X], outputs & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
       ++outputs;
       tc_fence_after();
       if (ok) {
@@ -1337,7 +1335,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
       const Item it = item_of(w);
       const int kj = it.k0 + r, klo = it.k0 + quad * 32;
       int step = 0;
-      for (int i = 0; i < it.n && ok; ++i, ++c, step = step + 1 == it.nqi ? 0 : step + 1) {
+      for (int i = 0; i < it.n; ++i, ++c, step = step + 1 == it.nqi ? 0 : step + 1) {
         const int q0 = it.k0 + step * BQ + part * 16;
         const float* nl = sStat + (c & 1) * 2 * BQ + part * 16;
         const float* nd = nl + BQ;
@@ -1347,7 +1345,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
         uint32_t v[2][16], pk[8];
 #pragma unroll
         for (int x = 0; x < 2; ++x) sn[x] = seen(klo, klo + 31, q0 + x * 64, q0 + x * 64 + 15, window);
-        if (!mbar_wait(&bars->stat_full[c & 1], (c >> 1) & 1, abort_flag) || !mbar_wait(&bars->s_full, c & 1, abort_flag)) { ok = false; break; }
+        ok = ok && mbar_wait(&bars->stat_full[c & 1], (c >> 1) & 1, abort_flag) && mbar_wait(&bars->s_full, c & 1, abort_flag);
         tc_fence_after();
         tmem_ld_32x32b_x16(tS + lane_off, v[0]);
 #pragma unroll
@@ -1365,7 +1363,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->p_ready[x]);
         }
-        if (!mbar_wait(&bars->dp_full, c & 1, abort_flag)) { ok = false; break; }
+        ok = ok && mbar_wait(&bars->dp_full, c & 1, abort_flag);
         tc_fence_after();
         tmem_ld_32x32b_x16(tDP + lane_off, v[0]);
         tmem_ld_32x32b_x16(tDP + lane_off + 64, v[1]);
@@ -1385,6 +1383,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
         }
       }
       ok = ok && mbar_wait(&bars->acc_full, turn & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       constexpr int DH = D / NSPLIT;

@@ -458,7 +458,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tile_coord(t, tm, tn);
           const uint32_t buf = lt & 1;
           const uint32_t bph = (lt >> 1) & 1;
-          if (!mbar_wait(&tempty_bar[buf], bph ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&tempty_bar[buf], bph ^ 1, abort_flag)) { ok = false; break; }
           uint32_t got = 1;
           if (lane == 0) got = wait_peer_flag(tp.flags_in + ((long)tm * tiles_n + tn) * 4 + q, tp.seq, abort_flag) ? 1u : 0u;
           got = __shfl_sync(0xffffffffu, got, 0);
@@ -506,7 +506,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       const uint32_t buf = lt & 1;
       const uint32_t bph = (lt >> 1) & 1;
-      if (!mbar_wait(&tfull_bar[buf], bph, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&tfull_bar[buf], bph, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int row0 = tm * TM + half * BM + q * 32;  // first row of this warp
       const long row = row0 + lane;

@@ -65,6 +65,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   *abort_flag = 1;
   return false;
 }
+// The same by a whole warp, with one answer for all of its lanes: tensor-memory accesses, votes and shuffles take every lane, and lanes
+// that went on alone would wait there without a limit. (Lanes look at the barrier and at the abort word one by one; the phase
+// cannot pass by while this warp has not arrived, so a vote that one lane spoils is held again.)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  for (uint32_t i = 0; i < TC05_SPIN_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 1023u) == 1023u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
 
 // ------------------------------------------------------- CTA pairs (2-CTA clusters) -----
 // The same shared-memory location in the pair's first CTA: in the shared::cluster window bit 24 of an address tells the two

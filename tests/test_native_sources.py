@@ -71,3 +71,39 @@ def test_kernels_that_wait_promise_nothing_of_what_they_read():
         launched |= {aliases.get(n, n) for n in re.findall(r"\botb_launch_(?:early\(|if_early\(\s*\w+,)\s*(\w+)", text)}
     assert early == {"attn_bwd_q2_kernel"}
     assert launched | {"rmsnorm_fwd_wide_kernel"} == waiting | early, launched ^ (waiting | early)
+
+
+def test_warps_give_up_together():
+    """What whole warps do after a bounded wait (tensor-memory accesses, votes, shuffles) needs all of their lanes: lanes that left alone
+    would keep the others waiting without a limit. Outside code that one lane runs, a wait has one answer for the warp, or only adds to
+    ``ok``, which decides nothing before the warp has voted on it."""
+    waits = {}
+    for path in sorted(CUDA.glob("*.cu")):
+        text = _source(path)
+        for name, _, body in _kernels(text):
+            blocks = [(False, False)]  # of each open block: whether a single lane runs it, whether it is a loop that goes on while ``ok``
+            voted = True
+            for m in re.finditer(r"[{}]|\bmbar_wait(?:_cluster|_warp)?\(|\bok\b", body):
+                before, after = body[:m.start()], body[m.start():m.start() + 200]
+                if m[0] == "{":
+                    one_lane = re.search(r"if \((?:half == 0 && )?(?:elect_one\(\)|lane == 0)\) $", before)
+                    head = before[before.rfind("\n"):]
+                    blocks.append((bool(one_lane) or blocks[-1][0], bool(re.search(r"\b(?:for|while) \(.*\bok\b", head))))
+                elif m[0] == "}":
+                    one_lane, loop = blocks.pop()
+                    assert voted or not loop, (path.name, name)
+                elif not blocks[-1][0]:
+                    if m[0] == "mbar_wait_warp(":
+                        waits.setdefault(name, set()).add("one answer")
+                    elif m[0] != "ok":
+                        assert re.search(r"\n\s*ok = ok &&[^;]*$", before), (path.name, name, after)
+                        waits.setdefault(name, set()).add("a vote at the end")
+                        voted = False
+                    elif after.startswith("ok = __all_sync(0xffffffffu, ok);"):
+                        voted = True
+                    else:
+                        adds = re.match(r"ok = ok && mbar_wait\(", after) or re.search(r"ok = $", before) and after.startswith("ok && mbar_wait(") \
+                            or before.endswith("__all_sync(0xffffffffu, ")
+                        assert voted or adds, (path.name, name, after)
+            assert voted, (path.name, name)
+    assert waits == {"gemm_tc05_kernel": {"one answer"}, **{"attn_%s_kernel" % k: {"a vote at the end"} for k in ("fwd", "fwd2", "bwd_q2", "bwd_kv3")}}
