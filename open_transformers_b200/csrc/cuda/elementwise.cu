@@ -1103,7 +1103,7 @@ extern "C" int otb_embedding_fwd(const long* ids, const void* table, void* out, 
 extern "C" int otb_embedding_bwd(const void* dy, const long* sorted_ids, const long* sorted_tok, long n, float* dW, int D,
                                  int accumulate, int dtype, void* stream) {
   if (n <= 0) return 0;
-  const bool wide = D % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dW)) & 15) == 0;
+  const bool wide = D > 0 && D % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dW)) & 15) == 0;
   const unsigned threads = wide ? (unsigned)(D < 2048 ? (D / 8 + 31) / 32 * 32 : 256) : 256u;
   DISPATCH_T(dtype, return otb_launch(wide ? embedding_bwd8_kernel<T> : embedding_bwd_kernel<T>, (unsigned)n, threads, 0, S(stream), (const T*)dy,
                                       sorted_ids, sorted_tok, n, dW, D, accumulate);)

@@ -1,6 +1,6 @@
 """A stand-in for the few CUDA runtime calls that the native library's host code makes, to run that code without a GPU: it keeps
-count of the launches, refuses those that need more shared memory than the current device was asked for, and refuses others on
-request. Preloaded into a child process, which sees no device."""
+count of the launches, refuses those that need more shared memory than the current device was asked for and those of no threads or
+too many, and refuses others on request. Preloaded into a child process, which sees no device."""
 import os
 import subprocess
 import sys
@@ -40,19 +40,20 @@ int cudaFuncSetAttribute(const void* f, int attr, int value) {
 }
 static int encode(void) { return 0; }
 int cudaGetDriverEntryPoint(const char* name, void** f, unsigned long long flags, int* found) { *f = (void*)encode; *found = 0; return 0; }
-static int launch(int early, const void* f, dim3_ g, size_t smem) {
+static int launch(int early, const void* f, dim3_ g, dim3_ b, size_t smem) {
   int most = 48 << 10, i;
   if (times[early] && skip[early]-- <= 0) { --times[early]; return last = code[early]; }
   for (i = 0; i < n_asked; ++i)
     if (asked[i].f == f && asked[i].dev == device && asked[i].bytes > most) most = asked[i].bytes;
   if (smem > (size_t)most || !g.x || !g.y || !g.z) return last = 1;
+  if (!b.x || !b.y || !b.z || b.x * b.y * b.z > 1024) return last = 9;
   ++fake_launches;
   fake_f = f;
   return 0;
 }
-int cudaLaunchKernel(const void* f, dim3_ g, dim3_ b, void** args, size_t smem, void* stream) { return launch(0, f, g, smem); }
+int cudaLaunchKernel(const void* f, dim3_ g, dim3_ b, void** args, size_t smem, void* stream) { return launch(0, f, g, b, smem); }
 int cudaLaunchKernelExC(const config_* c, const void* f, void** args) {
-  int rc = launch(1, f, c->grid, c->smem);
+  int rc = launch(1, f, c->grid, c->block, c->smem);
   if (!rc) ++fake_early;
   return rc;
 }

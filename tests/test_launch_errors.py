@@ -108,6 +108,17 @@ print("ok")
 """
 
 
-@pytest.mark.parametrize("child", [ONE, SEVERAL], ids=["one launch", "several launches"])
+# threads by the width of a row: some at every width, no columns at all among them
+WIDTHS = HEAD + r"""
+for D in (0, 8, 12, 248, 256, 264, 2040, 2048, 2056, 1 << 20):
+    for bf16 in (0, 1):
+        fake.fake_reset()
+        assert lib.otb_embedding_bwd(P, P, P, L(8), P, I(D), I(1), I(bf16), N) == 0 and fake.fake_launched() == 1, D
+        assert lib.otb_ce_zloss(P, P, P, P, L(8), I(D // 8 * 8), F(1.0), F(1.0), I(1), I(bf16), N) == 0 and fake.fake_launched() == 2, D
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("child", [ONE, SEVERAL, WIDTHS], ids=["one launch", "several launches", "widths"])
 def test_refused_launches(child, tmp_path):
     run_with_fake(child, tmp_path)
