@@ -89,10 +89,12 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 __device__ __forceinline__ int work_item(int turn) {
   return turn * (int)gridDim.x + (turn & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
 }
-// The element warps of these kernels do not leave an item where a bounded wait gives up: a lane that gave up alone would be missing from
-// the tensor-memory accesses, votes and shuffles that follow, and the others would wait for it without a limit. It waits no more,
-// the warp goes on with whatever values are there, and at the item's end votes whether to store them and go on to the next. (A vote
-// at each wait, us: forward and backward at 4 x 4096 tokens with a 512-key window 619 and 635.)
+// A lane of an element warp never leaves an item alone where a bounded wait gives up: it would be missing from the tensor-memory accesses,
+// votes and shuffles that follow, and the others would wait for it without a limit. dK/dV votes at each wait (mbar_wait_warp). In the
+// forward kernels and dQ a warp goes on with whatever values are there, and votes at the item's end whether to store them and go on: by
+// its lanes' own answers, which then wait no more, or in dQ by the abort word. Each kernel has the form that costs it least. us
+// against waits that lanes left one by one, 4 x 4096 tokens, 16 heads x 128: dK/dV and dQ 944 and 936, windowed (512 keys) 344 and 346; with
+// answers kept in dQ and the abort word in dK/dV 352. Forward 350 and 352; 2 % more with the abort word at a few hundred tokens.
 // byte offset of the 16-byte chunk `ch` (0..7) of row r in a [rows][128 B] 128B-swizzled tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t ch) { return r * 128u + ((ch ^ (r & 7u)) << 4); }
 
@@ -1007,7 +1009,7 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         const int k0 = u * HK;
         // some (row, key) pair of this step is hidden, or the tile has rows past the end of the sequence
         const bool need_mask = (k0 + HK - 1 > q0) || (window > 0 && k0 <= q0 + BQ - 1 - window) || (q0 + BQ > T);
-        ok = ok && mbar_wait(&bars->sdp_full[X], scores & 1, abort_flag);
+        mbar_wait(&bars->sdp_full[X], scores & 1, abort_flag);
         ++scores;
         tc_fence_after();
         // dS (bf16 pairs, 8 columns per 16 keys) goes over the thread's own score columns, which it has read by then
@@ -1026,8 +1028,8 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->ds_ready[X]);
       }
-      ok = ok && mbar_wait(&bars->dq_done[X], outputs & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
+      mbar_wait(&bars->dq_done[X], outputs & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, *abort_flag == 0);
       ++outputs;
       tc_fence_after();
       if (ok) {
@@ -1335,7 +1337,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
       const Item it = item_of(w);
       const int kj = it.k0 + r, klo = it.k0 + quad * 32;
       int step = 0;
-      for (int i = 0; i < it.n; ++i, ++c, step = step + 1 == it.nqi ? 0 : step + 1) {
+      for (int i = 0; i < it.n && ok; ++i, ++c, step = step + 1 == it.nqi ? 0 : step + 1) {
         const int q0 = it.k0 + step * BQ + part * 16;
         const float* nl = sStat + (c & 1) * 2 * BQ + part * 16;
         const float* nd = nl + BQ;
@@ -1345,7 +1347,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
         uint32_t v[2][16], pk[8];
 #pragma unroll
         for (int x = 0; x < 2; ++x) sn[x] = seen(klo, klo + 31, q0 + x * 64, q0 + x * 64 + 15, window);
-        ok = ok && mbar_wait(&bars->stat_full[c & 1], (c >> 1) & 1, abort_flag) && mbar_wait(&bars->s_full, c & 1, abort_flag);
+        if (!mbar_wait_warp(&bars->stat_full[c & 1], (c >> 1) & 1, abort_flag) || !mbar_wait_warp(&bars->s_full, c & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         tmem_ld_32x32b_x16(tS + lane_off, v[0]);
 #pragma unroll
@@ -1363,7 +1365,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->p_ready[x]);
         }
-        ok = ok && mbar_wait(&bars->dp_full, c & 1, abort_flag);
+        if (!mbar_wait_warp(&bars->dp_full, c & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         tmem_ld_32x32b_x16(tDP + lane_off, v[0]);
         tmem_ld_32x32b_x16(tDP + lane_off + 64, v[1]);
@@ -1382,8 +1384,7 @@ attn_bwd_kv3_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
           if (lane == 0) mbar_arrive(&bars->ds_ready[x]);
         }
       }
-      ok = ok && mbar_wait(&bars->acc_full, turn & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = ok && mbar_wait_warp(&bars->acc_full, turn & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       constexpr int DH = D / NSPLIT;

@@ -75,8 +75,8 @@ def test_kernels_that_wait_promise_nothing_of_what_they_read():
 
 def test_warps_give_up_together():
     """What whole warps do after a bounded wait (tensor-memory accesses, votes, shuffles) needs all of their lanes: lanes that left alone
-    would keep the others waiting without a limit. Outside code that one lane runs, a wait has one answer for the warp, or only adds to
-    ``ok``, which decides nothing before the warp has voted on it."""
+    would keep the others waiting without a limit. Outside code that one lane runs, a wait has one answer for the warp, or its answer is
+    left alone or only added to ``ok``, and nothing is decided before the warp has voted on that or on the abort word."""
     waits = {}
     for path in sorted(CUDA.glob("*.cu")):
         text = _source(path)
@@ -96,14 +96,17 @@ def test_warps_give_up_together():
                     if m[0] == "mbar_wait_warp(":
                         waits.setdefault(name, set()).add("one answer")
                     elif m[0] != "ok":
-                        assert re.search(r"\n\s*ok = ok &&[^;]*$", before), (path.name, name, after)
-                        waits.setdefault(name, set()).add("a vote at the end")
+                        adds, alone = re.search(r"\n\s*ok = ok &&[^;]*$", before), re.search(r"[;}{]\s*$", before) and re.match(r"mbar_wait\([^;]*\);", after)
+                        assert adds or alone, (path.name, name, after)
+                        waits.setdefault(name, set()).add("a vote on the answers" if adds else "a vote on the abort word")
                         voted = False
-                    elif after.startswith("ok = __all_sync(0xffffffffu, ok);"):
+                    elif re.match(r"ok = __all_sync\(0xffffffffu, (?:ok|\*abort_flag == 0)\);", after):
+                        assert voted or ("abort_flag" in after[:40]) == ("a vote on the abort word" in waits[name]), (path.name, name)
                         voted = True
                     else:
                         adds = re.match(r"ok = ok && mbar_wait\(", after) or re.search(r"ok = $", before) and after.startswith("ok && mbar_wait(") \
                             or before.endswith("__all_sync(0xffffffffu, ")
                         assert voted or adds, (path.name, name, after)
             assert voted, (path.name, name)
-    assert waits == {"gemm_tc05_kernel": {"one answer"}, **{"attn_%s_kernel" % k: {"a vote at the end"} for k in ("fwd", "fwd2", "bwd_q2", "bwd_kv3")}}
+    assert waits == {"gemm_tc05_kernel": {"one answer"}, "attn_bwd_kv3_kernel": {"one answer"}, "attn_bwd_q2_kernel": {"a vote on the abort word"},
+                     "attn_fwd_kernel": {"a vote on the answers"}, "attn_fwd2_kernel": {"a vote on the answers"}}
