@@ -38,7 +38,7 @@ inline float rbf(float x) { return det_bf2f(det_f2bf(x)); }
 inline bool masked_pair(int qi, int kj, int window) { return kj > qi || (window > 0 && kj <= qi - window); }
 
 // i8pv: P V on the int8 grid (values quantised per (KV head, 128-key block), probabilities q = rint(127 p), exact
-// integer sums, one fp32 dequantisation per block) - the twin of attn_fwd_kernel<128, true>.
+// integer sums, one fp32 dequantisation per block) - the twin of attn_fwd_i8pv_kernel.
 int attn_fwd_tc(const void* qk, long ldqk, const void* qkv, long ldqkv, void* O, long ldo, float* lse, int B, int T, int H, int Hkv, int D,
                 int window, float c_log2, int i8pv = 0) {
   const int G = H / Hkv;

@@ -10,8 +10,8 @@
 //                 the heads of the group and the query blocks that see these keys, both ascending; any T.
 //   attn_bwd_q2   CTA = (batch, query head, two query tiles); two threads per row; dS written back over S;
 //                 dQ += dS K with dS in TMEM; 64-key steps ascending.
-//   attn_fwd      (one tile per CTA, four threads per row, P through shared memory, O in registers) serves the int8 P V
-//                 variant.
+//   attn_fwd_i8pv the forward with P V in int8: one tile per CTA, four threads per row, P through shared memory, O in
+//                 registers.
 //
 // No atomics, no split accumulation: every output element has one owner CTA and a fixed
 // summation order, so results are identical for any grid, stream or GPU count. The window rule
@@ -21,7 +21,7 @@
 // Row sums: each 32-key quarter keeps two ascending chains (even / odd keys) that are added per block;
 // the four quarter sums are combined ((l0 + l1) + l2) + l3 at the end.
 //
-// int8-PV variant of the forward (I8PV): V is quantised beforehand to int8 per (KV head, 128-key block) with one
+// int8-PV variant of the forward: V is quantised beforehand to int8 per (KV head, 128-key block) with one
 // fp32 step per block (quant_v_kernel), the probabilities are quantised on the fly to q = rint(127 p), P V runs on
 // the int8 tensor cores (tcgen05 kind::i8, exact int32 sums over the 128 keys of a block) and is dequantised in
 // fp32: O = O*alpha + float(sum) * (step / 127). Softmax statistics stay fp32 on the unquantised probabilities;
@@ -238,13 +238,12 @@ __device__ __forceinline__ void divide_pack(const float (&a)[N], float l, float 
   }
 }
 
-// ---------------------------------------------------------------------------- forward
-template <int D, bool I8PV>
+// ------------------------------------------------- forward with P V in int8
 __global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV,
-                __nv_bfloat16* __restrict__ O, long ldo, float* __restrict__ lse_out, int T, int H, int Hkv, int window,
-                float scale, float c_log2, const float* __restrict__ vstep, uint32_t* __restrict__ status) {
-  static_assert(!I8PV || D == 128, "the int8 P V path needs 128-byte value rows");
+attn_fwd_i8pv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O, long ldo,
+                     float* __restrict__ lse_out, int T, int H, int Hkv, int window, float c_log2, const float* __restrict__ vstep,
+                     uint32_t* __restrict__ status) {
+  constexpr int D = 128;  // 128-byte value rows
   constexpr int TILE = BQ * D * 2;
   constexpr int ST = 2;
   extern __shared__ uint8_t smem_raw[];
@@ -305,19 +304,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
         mbar_expect_tx(&k_full[st], TILE);
         load_tile<D>(sK + st * TILE, &tmQK, &k_full[st], (H + g) * D, k0, b);
         if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag)) break;
-        if (I8PV) {  // int8 values: [128 keys][D bytes], one swizzle row per key
-          mbar_expect_tx(&v_full[st], BKV * D);
-          tma_load_3d(sV + st * TILE, &tmV, &v_full[st], g * D, k0, b);
-        } else {
-          mbar_expect_tx(&v_full[st], TILE);
-          load_tile<D>(sV + st * TILE, &tmV, &v_full[st], (H + Hkv + g) * D, k0, b);
-        }
+        mbar_expect_tx(&v_full[st], BKV * D);  // int8 values: [128 keys][D bytes], one swizzle row per key
+        tma_load_3d(sV + st * TILE, &tmV, &v_full[st], g * D, k0, b);
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idS = make_idesc(128, BKV, 0, 0);
-      constexpr uint32_t idPV = I8PV ? make_idesc(128, D, 0, 1, 2, 1) : make_idesc(128, D, 0, 1);
+      constexpr uint32_t idPV = make_idesc(128, D, 0, 1, 2, 1);
       const uint32_t aQ = smem_u32(sQ), aP = smem_u32(sP);
       bool ok = mbar_wait(q_full, 0, abort_flag);
       auto issue_S = [&](int i) {
@@ -340,15 +334,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
         if (!mbar_wait(&v_full[st], (i / ST) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t aV = smem_u32(sV + st * TILE);
-        if (I8PV) {
-          // P: [128 rows][128 int8 keys] K-major, 32 keys per instruction; V: [128 keys][128 int8] MN-major, 32 key rows per instruction
+        // P: [128 rows][128 int8 keys] K-major, 32 keys per instruction; V: [128 keys][128 int8] MN-major, 32 key rows per instruction
 #pragma unroll
-          for (int kk = 0; kk < BKV / 32; ++kk)
-            mma_i8_ss(tPV, make_smem_desc(aP + kk * 32, 16, 1024), make_smem_desc(aV + kk * 4096, 16384, 1024), idPV, kk != 0);
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) mma_f16_ss(tPV, desc_k(aP, kk), desc_mn(aV, kk), idPV, kk != 0);
-        }
+        for (int kk = 0; kk < BKV / 32; ++kk)
+          mma_i8_ss(tPV, make_smem_desc(aP + kk * 32, 16, 1024), make_smem_desc(aV + kk * 4096, 16384, 1024), idPV, kk != 0);
         mma_commit(pv_full);
         mma_commit(&v_empty[st]);
       }
@@ -362,13 +351,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
     const int qi = q0 + r;                 // query position
     const uint32_t lane_off = uint32_t(qd * 32) << 16;
     float m_run = -INFINITY, l_run = 0.0f, alpha_prev = 0.0f;
-    float c_prev = 0.0f;  // int8 P V: dequantisation factor (value step / 127) of the block whose P V is pending
+    float c_prev = 0.0f;  // dequantisation factor (value step / 127) of the block whose P V is pending
     const int nblk = (T + BKV - 1) / BKV;
     // two accumulator words -> fp32 contributions; the integers (below 2^22) become floats by one addition to the bits of 1.5 * 2^23
     // and one subtraction, both exact. (This and the same for the probabilities, instead of the conversion pipe, a quarter as wide:
     // 4 x 4096 tokens, 16 heads, 812 -> 784 us; 1 x 2048 94 -> 91.)
     auto pv_vals = [&](uint32_t w0, uint32_t w1) {
-      if constexpr (!I8PV) return pack2(__uint_as_float(w0), __uint_as_float(w1));
       const f2 x = add2(pack2(__uint_as_float(w0 + 0x4B400000u), __uint_as_float(w1 + 0x4B400000u)), pack2(-12582912.0f, -12582912.0f));
       return mul2(x, pack2(c_prev, c_prev));
     };
@@ -400,8 +388,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
       const float alpha = det_exp2_attn(__fadd_rn(m_run, -m_safe));
       // probabilities and the quarter-row sum first (independent of O), while the tensor core finishes the previous P V
       uint32_t pk[KPT / 2];
-      const f2 lsum2 = need_mask ? probs_pack<true, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk)
-                                 : probs_pack<false, I8PV>(sv, c_log2, m_safe, kbase, qi, window, pk);
+      const f2 lsum2 = need_mask ? probs_pack<true, true>(sv, c_log2, m_safe, kbase, qi, window, pk)
+                                 : probs_pack<false, true>(sv, c_log2, m_safe, kbase, qi, window, pk);
       // deferred accumulation of the previous block's P V (its completion also frees the P buffer)
       if (i > 0) {
         ok = ok && mbar_wait(pv_full, (i - 1) & 1, abort_flag);
@@ -417,26 +405,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant_
             o[(c * CW + e) >> 1] = fma2(o[(c * CW + e) >> 1], a2, pv_vals(v[e], v[e + 1]));
         }
       }
-      if (I8PV) {
-        // keys part*32 .. +31 are bytes part*32 .. +31 of the 128-byte row: chunks part*2, part*2 + 1
+      // keys part*32 .. +31 are bytes part*32 .. +31 of the 128-byte row: chunks part*2, part*2 + 1
 #pragma unroll
-        for (int w = 0; w < 2; ++w)
-          *reinterpret_cast<uint4*>(sP + swz(r, part * 2 + w)) = make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
-      } else {
-        // keys part*32 .. +31 -> 64-key sub-tile (part >> 1), 16-byte chunks (part & 1) * 4 .. +3 of the row
-        uint8_t* base = sP + (part >> 1) * 16384;
-#pragma unroll
-        for (int w = 0; w < 4; ++w)
-          *reinterpret_cast<uint4*>(base + swz(r, (part & 1) * 4 + w)) =
-              make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
-      }
+      for (int w = 0; w < 2; ++w)
+        *reinterpret_cast<uint4*>(sP + swz(r, part * 2 + w)) = make_uint4(pk[4 * w], pk[4 * w + 1], pk[4 * w + 2], pk[4 * w + 3]);
       float ls0, ls1;
       unpack2(lsum2, ls0, ls1);
       const float lsum = __fadd_rn(ls0, ls1);
       l_run = __fmaf_rn(l_run, alpha, lsum);
       m_run = m_new;
       alpha_prev = alpha;
-      if (I8PV) c_prev = __fmul_rn(vstep[((long)b * Hkv + g) * nblk + j], 1.0f / 127.0f);
+      c_prev = __fmul_rn(vstep[((long)b * Hkv + g) * nblk + j], 1.0f / 127.0f);
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
@@ -792,13 +771,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant
 
 // Backward element math for a thread's KPT (score, dP) pairs: p = exp2(s * c - lse) (0 where hidden or the row is out of
 // range), ds = (p * (dp - delta)) * scale; both packed to bf16 pairs.
-template <bool MASK, bool WANT_P, int N = KPT>
-__device__ __forceinline__ void bwd_probs(const uint32_t (&vs)[N], const uint32_t (&vd)[N], float c_log2, float lse_r, float dl_r,
-                                          float scale, bool row_ok, int kbase, int qi, int window, uint32_t (&pk)[N / 2],
-                                          uint32_t (&dsr)[N / 2]) {
+template <bool MASK>
+__device__ __forceinline__ void dscores(const uint32_t (&vs)[16], const uint32_t (&vd)[16], float c_log2, float lse_r, float dl_r,
+                                        float scale, bool row_ok, int kbase, int qi, int window, uint32_t (&dsr)[8]) {
   const f2 c2 = pack2(c_log2, c_log2), nl2 = pack2(-lse_r, -lse_r), nd2 = pack2(-dl_r, -dl_r), sc2 = pack2(scale, scale);
 #pragma unroll
-  for (int e = 0; e < N; e += 2) {
+  for (int e = 0; e < 16; e += 2) {
     f2 p2 = exp2_attn2(fma2(pack2(__uint_as_float(vs[e]), __uint_as_float(vs[e + 1])), c2, nl2));
     if constexpr (MASK) {
       float p0, p1;
@@ -811,11 +789,6 @@ __device__ __forceinline__ void bwd_probs(const uint32_t (&vs)[N], const uint32_
     float d0, d1;
     unpack2(d2, d0, d1);
     dsr[e >> 1] = pack_bf16(d0, d1);
-    if constexpr (WANT_P) {
-      float p0, p1;
-      unpack2(p2, p0, p1);
-      pk[e >> 1] = pack_bf16(p0, p1);
-    }
   }
 }
 
@@ -1015,12 +988,12 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         // dS (bf16 pairs, 8 columns per 16 keys) goes over the thread's own score columns, which it has read by then
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          uint32_t sa[16], da[16], pk[8], unused[8];
+          uint32_t sa[16], da[16], pk[8];
           tmem_ld_32x32b_x16(tS + c * 16, sa);
           tmem_ld_32x32b_x16(tDP + c * 16, da);
           tmem_ld_wait();
-          if (need_mask) bwd_probs<true, false, 16>(sa, da, c_log2, lse_r, dl_r, scale, row_ok, k0 + hf * 32 + c * 16, qi, window, unused, pk);
-          else bwd_probs<false, false, 16>(sa, da, c_log2, lse_r, dl_r, scale, true, 0, 0, 0, unused, pk);
+          if (need_mask) dscores<true>(sa, da, c_log2, lse_r, dl_r, scale, row_ok, k0 + hf * 32 + c * 16, qi, window, pk);
+          else dscores<false>(sa, da, c_log2, lse_r, dl_r, scale, true, 0, 0, 0, pk);
           tmem_st_32x32b_x8(tS + c * 8, pk);
         }
         tmem_st_wait();
@@ -1547,7 +1520,7 @@ CUresult encode_3d(CUtensorMap* out, const void* ptr, uint64_t cols, uint64_t T,
   });
 }
 
-template <int D> constexpr int attn_smem_bytes() { return (1 + 2 * 2) * (BQ * D * 2) + BQ * BKV * 2 + 1024 + 512 + 4096; }
+constexpr int attn_fwd_i8pv_smem_bytes() { return (1 + 2 * 2) * (BQ * 128 * 2) + BQ * BKV * 2 + 1024 + 512 + 4096; }
 
 template <int D> constexpr int attn_bwd_q2_smem_bytes() { return 4 * (BQ * D * 2) + 2 * 3 * (HK * D * 2) + 1024 + 256; }
 template <int D> constexpr int attn_bwd_kv3_smem_bytes() { return (2 + KV_QST + KV_DOST) * (BKV * D * 2) + 4 * BQ * 4 + (int)sizeof(BarsKV3); }
@@ -1609,10 +1582,10 @@ extern "C" int otb_attn_fwd_i8pv(const void* qk, long ldqk, const void* qkv, lon
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
   const float c_log2 = (float)((double)scale * 1.4426950408889634);
   dim3 grid((T + BQ - 1) / BQ, H, B);
-  const int rc = otb_allow_smem<attn_fwd_kernel<128, true>>(attn_smem_bytes<128>());
+  const int rc = otb_allow_smem<attn_fwd_i8pv_kernel>(attn_fwd_i8pv_smem_bytes());
   if (rc) return rc;
-  attn_fwd_kernel<128, true><<<grid, ATT_THREADS, attn_smem_bytes<128>(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, T, H, Hkv, window,
-                                                                               scale, c_log2, vstep, status);
+  attn_fwd_i8pv_kernel<<<grid, ATT_THREADS, attn_fwd_i8pv_smem_bytes(), s>>>(tq, tv, (__nv_bfloat16*)O, ldo, lse, T, H, Hkv, window, c_log2, vstep,
+                                                                             status);
   return (int)cudaGetLastError();
 }
 

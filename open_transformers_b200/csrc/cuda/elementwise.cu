@@ -1081,14 +1081,25 @@ extern "C" int otb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long ro
 extern "C" int otb_ce_zloss(void* logits, const long* labels, float* ce, float* lse, long rows, int V, float two_z,
                             float scale, int write_grad, int dtype, void* stream) {
   if (V % 8) return -2;
-#define CE(U, TEST) \
-  DISPATCH_T(dtype, return otb_launch_early(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad);)
-#define CE_SHORT(GROUPS) \
-  DISPATCH_T(dtype, return otb_launch_early(ce_zloss_short_kernel<T, GROUPS>, (unsigned)rows, ce_short_threads(V), 0, S(stream), (T*)logits, labels, ce, lse, V, two_z, scale, write_grad);)
-  if (V <= CE_SWEEP) { CE_SHORT(1) } else if (V <= 2 * CE_SWEEP) { CE_SHORT(2) } else if (V <= 4 * CE_SWEEP && dtype) { CE_SHORT(4) }
+  using bf16 = __nv_bfloat16;
+#define CE(T, U, TEST) \
+  return otb_launch_early(ce_zloss_kernel<T, U, TEST>, (unsigned)rows, CE_THREADS, 0, S(stream), (T*)logits, labels, ce, lse, rows, V, two_z, scale, write_grad)
+#define CE_SHORT(T, GROUPS) \
+  return otb_launch_early(ce_zloss_short_kernel<T, GROUPS>, (unsigned)rows, ce_short_threads(V), 0, S(stream), (T*)logits, labels, ce, lse, V, two_z, scale, write_grad)
+  if (dtype) {
+    if (V <= CE_SWEEP) CE_SHORT(bf16, 1);
+    if (V <= 2 * CE_SWEEP) CE_SHORT(bf16, 2);
+    if (V <= 4 * CE_SWEEP) CE_SHORT(bf16, 4);
+    if (ce_form(rows, V, true) == 1) CE(bf16, 1, true);
+    CE(bf16, 4, true);
+  }
+  if (V <= CE_SWEEP) CE_SHORT(float, 1);
+  if (V <= 2 * CE_SWEEP) CE_SHORT(float, 2);
+  const int form = ce_form(rows, V, false);
+  if (form == 0) CE(float, 1, false);
+  if (form == 1) CE(float, 1, true);
+  CE(float, 4, true);
 #undef CE_SHORT
-  const int form = ce_form(rows, V, dtype);
-  if (form == 0) { CE(1, false) } else if (form == 1) { CE(1, true) } else { CE(4, true) }
 #undef CE
 }
 extern "C" int otb_det_sum(const float* x, long n, int mode, float post_scale, float* out, void* stream) {

@@ -109,4 +109,4 @@ def test_warps_give_up_together():
                         assert voted or adds, (path.name, name, after)
             assert voted, (path.name, name)
     assert waits == {"gemm_tc05_kernel": {"one answer"}, "attn_bwd_kv3_kernel": {"one answer"}, "attn_bwd_q2_kernel": {"a vote on the abort word"},
-                     "attn_fwd_kernel": {"a vote on the answers"}, "attn_fwd2_kernel": {"a vote on the answers"}}
+                     "attn_fwd_i8pv_kernel": {"a vote on the answers"}, "attn_fwd2_kernel": {"a vote on the answers"}}
