@@ -56,7 +56,8 @@ constexpr int SOFTMAX_THREADS = 128 * NSPLIT;
 constexpr int ATT_THREADS = 64 + SOFTMAX_THREADS;
 constexpr int SOFTMAX_WARPS = SOFTMAX_THREADS / 32;
 
-// The four warps that share the rows of a TMEM lane quadrant. (With one barrier for all sixteen warps 4 x 4096 tokens take 784 us, so 768.)
+// The four warps that share the rows of a TMEM lane quadrant. (With one barrier for all sixteen warps 4 x 4096 tokens took 784 us, so 768, when
+// the kernel still used the divider and spilled; 651 now.)
 __device__ __forceinline__ void quadrant_bar(int quad) { asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "n"(32 * NSPLIT) : "memory"); }
 
 // N (16 or 32) consecutive TMEM columns of this thread's lane
@@ -78,12 +79,12 @@ struct BarsX : Bars {
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
-// The bf16 forward, dQ and dK/dV kernels are persistent, one CTA per SM (the int8 P V forward is not): every role walks the same list of work items, barrier phases and ring
-// positions running on, so the loads and first products of an item are under way while the previous one's results are read
-// out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about 8 us, were
-// exposed: a quarter of an item's time with a 512-key window. 4 x 4096 tokens, 16 heads x 128, forward and backward: 1790 ->
-// 1612 us full causal, 744 -> 691 us windowed. Where every item has a CTA of its own the walk costs a little: forward 1 x 2048
-// 56 -> 59 us, 1 x 333 x 12 heads x 64 14.6 -> 15.1.) Item r * gridDim + c of the list goes to CTA c in even turns
+// The bf16 forward, dQ and dK/dV kernels are persistent, one CTA per SM (the int8 P V forward is not): every role walks the same list of work
+// items, barrier phases and ring positions running on, so the loads and first products of an item are under way while the previous
+// one's results are read out of tensor memory and stored. (As one CTA per item, set-up, first loads and the epilogue of each, about
+// 8 us, were exposed: a quarter of an item's time with a 512-key window. When it was made, forward and backward of 4 x 4096 tokens, 16 heads
+// x 128, went from 1790 to 1612 us full causal, 744 to 691 windowed. Where every item has a CTA of its own the walk costs 1 to 5 % of the
+// forward: 1 x 2048 56 and 59 us, 1 x 333 x 12 heads x 64 14.6 and 15.1, then; those take 52 and 11.5 now.) Item r * gridDim + c of the list goes to CTA c in even turns
 // r and to the mirrored CTA in odd ones; the list is sorted by falling work (but for a lone last tile, which comes first), so
 // the sums come out nearly even.
 __device__ __forceinline__ int work_item(int turn) {
@@ -1043,7 +1044,10 @@ attn_bwd_q2_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
 // the sixteen element warps (four threads per key row, no value crosses threads) turn dP^T into dS^T, the tensor core runs dV and
 // the next S^T; while they make the next P^T, it runs dK and the next dP^T. Each 64-query half of P^T and dS^T is handed over by
 // itself; the probabilities stay in registers (fp32) from the one phase to the other.
-// A 128 x 128 step takes 3500 clocks: P^T 1800 (1250 of the multiply-add pipe), dS^T 750, 600 and 170 waiting for S^T and dP^T.
+// A 128 x 128 step takes 3720 clocks of the whole launch: P^T 1800 (1250 of the multiply-add pipe), dS^T 750, 600 and 170 waiting for S^T and
+// dP^T, and 400 between these and in the items' results. A step of which only the first half holds queries takes as long as a whole one:
+// 40 x 64 tokens, 16 heads on 4 of 128, 46.5 us with 64-query steps, 50.9 so. (Leaving the padding's arithmetic out: 49.8 there, but 923 -> 954
+// for 4 x 4096 tokens, 16 heads on 8.)
 // 4 x 4096 tokens, 16 x 128 heads: 538 -> 533 us against 64-query steps with two score buffers (products alone 2900 clocks there);
 // lengths that are no multiple of 64 had a kernel of their own: backward of 333 tokens, 12 x 64, 39.5 -> 25.1 us, 2 x 1000 55.3 -> 36.1.
 // Also measured: two groups of eight warps, one per 64-query buffer (537 us); P^T through shared memory, so that S^T is free early

@@ -2,7 +2,7 @@
 // attention -> output product (+ residual) -> norm -> gate/up product -> SwiGLU -> down product (+ residual), each the kernel
 // that the block's modules launch one by one, so the results are the same bits. What bounds the scoring of a short prompt is
 // the host: module calls and autograd functions, about 250 us of Python a block for 50 us of kernels (333 tokens through the
-// six-layer 100M model: 1584 -> 542 us, the launches' own changes included).
+// six-layer 100M model: 1584 -> 542 us, the launches' own changes included; 440 with the model's walk in train() and a table of scratch sizes).
 #include "common.cuh"
 #include "entries.cuh"
 

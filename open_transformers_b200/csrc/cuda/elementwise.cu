@@ -656,7 +656,7 @@ inline int swiglu_threads(int F) {
 }
 
 // --------------------------------------------------------- fused CE + z-loss
-// One CTA of 512 threads per row of logits [rows, V] (V % 8 == 0). With m = max of the row and L = log2(e):
+// One CTA per row of logits [rows, V] (V % 8 == 0), of 512 threads or, for rows of fewer than 512 groups of 8, of fewer. With m = max of the row and L = log2(e):
 //   e_i = exp2(fma(x_i, L, -(m * L)))        (det_exp2_acc, evaluated two at a time with packed fp32 arithmetic)
 //   s   = sum e_i: the 8-element group g = i / 8 belongs to thread g % 512; a thread keeps two ascending chains, the
 //         even and the odd elements of its groups, adds them, and the 512 thread sums go through block_tree_sum
@@ -664,12 +664,13 @@ inline int swiglu_threads(int F) {
 // and the row is overwritten with d loss / d logits = e_i * k - onehot * scale, k = ((1 + 2 z lse) / s) * scale
 // (scale = 1 / (tokens * accum), host reciprocal; the label's element is fma(e, k, -scale)).
 // Rows with label < 0 are ignored: zero loss, zero gradient.
-// Bound by instructions, not by the three reads (the maximum of bf16 logits is taken two at a time as bf16). Two things help
-// long rows and cost short ones registers, and with them CTAs per SM (ce_form chooses):
+// Rows too long for the registers (the form below) are read three times, once from memory. They are bound by instructions, not by
+// the reads (the maximum of bf16 logits is taken two at a time as bf16). Two things help the longest and cost others registers, and with
+// them CTAs per SM (ce_form chooses):
 //   TEST: the first pass finds the smallest logit too, and where it is near enough the exponent's clamp is left out;
 //   UNROLL groups per thread are in flight.
-// us for 16384 rows with their gradient; neither / TEST / TEST and four groups: bf16 V 32768 525 / 516 / 568, 65536 986 / 967 / 1073, 98304 1714 / 1672 / 1552; 4000 rows of 128256 622 / 624 /
-// 542. fp32, 4000 rows: 16384 99 / 104 / 135, 32768 256 / 198 / 225, 65536 611 / 584 / 448;
+// us for 16384 rows with their gradient; neither / TEST / TEST and four groups: bf16 V 32768 525 / 516 / 568, 65536 986 / 967 / 1073, 98304
+// 1714 / 1672 / 1552; 4000 rows of 128256 622 / 624 / 542. fp32, 4000 rows: 16384 99 / 104 / 135, 32768 256 / 198 / 225, 65536 611 / 584 / 448;
 // with a few rows per SM neither helps (64 rows of 128256: 30 / 34 / 37, 149: 52 / - / 60, 600: 222 / 231 / 209).
 constexpr int CE_THREADS = 512, CE_SWEEP = CE_THREADS * 8;
 template <typename T, int CE_UNROLL>

@@ -78,7 +78,7 @@ print("ok")
 # launch would be refused and repeated
 SEVERAL = HEAD + r"""
 for D in (64, 128):
-    for T in (128, 100):  # both forms of dK/dV
+    for T in (128, 100):  # whole and ragged steps
         fake.fake_reset()
         assert attn_bwd(D, T) == 0 and (fake.fake_launched(), fake.fake_launched_early()) == (3, 1)
         fake.fake_reset()
